@@ -79,18 +79,15 @@ __device__ __forceinline__ uint32_t warp_find_owner(uint32_t incl, uint32_t j) {
   return lo;
 }
 
-// Lane-wise minimum of two pairs of 16-bit halves.
-__device__ __forceinline__ uint32_t vmin_u16x2(uint32_t a, uint32_t b) {
-  uint32_t d;
-  asm("min.u16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
-  return d;
+// Whether any of a block's eight coarse coins is at most th (a uniform
+// threshold's coarse half): when none is, no edge of the block is live and
+// none ties.  Two three-way minima of 16-bit pairs clip every coin at th + 1;
+// any smaller half changes the word.  (th = 0xFFFF: every coin is.)
+__device__ __forceinline__ bool block_clipped(const u32x4 &c, uint32_t lim) {
+  return __vimin3_u16x2(__vimin3_u16x2(c.x, c.y, c.z), c.w, lim) != lim;
 }
-
-// Smallest of the eight coarse coins of a block: when it exceeds a uniform
-// threshold's coarse half, no edge of the block is live and none ties.
-__device__ __forceinline__ uint32_t block_min16(const u32x4 &c) {
-  const uint32_t m = vmin_u16x2(vmin_u16x2(c.x, c.y), vmin_u16x2(c.z, c.w));
-  return min(m & 0xFFFFu, m >> 16);
+__device__ __forceinline__ bool block_any_le(const u32x4 &c, uint32_t th) {
+  return block_clipped(c, (th + 1) * 0x10001u) || th == 0xFFFFu;
 }
 
 // Number of 4-edge groups covering [beg, end).
@@ -102,19 +99,6 @@ __device__ __forceinline__ uint32_t group_count(uint32_t beg, uint32_t end) {
 __device__ __forceinline__ uint32_t block_count(uint32_t beg, uint32_t end) {
   return end > beg ? ((end - 1) >> 3) - (beg >> 3) + 1 : 0;
 }
-
-// Coin blocks of a launch: from the key (its schedule added in registers)
-// or from round keys the kernel keeps in parameter space.
-struct KeyCoins {
-  Key k;
-  __device__ __forceinline__ u32x4 block(uint64_t b, uint64_t s) const { return ic_block(k, b, s); }
-};
-struct RoundKeyCoins {
-  const RoundKeys &rk;
-  __device__ __forceinline__ u32x4 block(uint64_t b, uint64_t s) const {
-    return ic_block_rk(rk, b, s);
-  }
-};
 
 // Live edges (bit h: edge 8b + h) of 8-edge coin block b of the in-list
 // [ob, oe) for set s, given the block's coarse coins c: compared with the
@@ -129,7 +113,7 @@ __device__ __forceinline__ uint32_t ic_block_live(const DevGraph &G, Key key, ui
   uint32_t live = 0, tie = 0;
   if (ovt) {
     const uint32_t th = ovt >> 16;
-    if (block_min16(c) > th) return 0u;
+    if (!block_any_le(c, th)) return 0u;
 #pragma unroll
     for (int h = 0; h < 8; ++h) {
       const uint32_t cc = coarse_of(c, h), e = (b << 3) + h;

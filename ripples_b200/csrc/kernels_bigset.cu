@@ -5,14 +5,20 @@
 // 2^20 vertices 1% of the sets carry ~40% of the edge work).  One warp per set
 // (ic_plain_kernel) or one warp per frontier entry (ic_fused_kernel) walks a
 // hub's in-list alone, so those sets set the kernel's length.  Here one CTA
-// grows one such set: level by level, the level's entries are taken a CTA's
-// width at a time; in-lists of at least that many 8-edge coin blocks (hubs)
-// are swept by all threads one list at a time, and the others through their
-// concatenated blocks (a block scan turns block counts into offsets; each
-// thread finds its entry with a forward-only cursor in shared memory).
-// Levels are separated by __syncthreads only.  Coins are the same
-// (set, edge)-keyed Philox draws as every other sampler; a thread takes
-// whole 8-edge coin blocks (one Philox block each).
+// grows one such set, level by level:
+//   * every warp takes a share of the level's entries and sweeps their shorter
+//     lists alone (a warp scan and a shuffle search over their concatenated
+//     8-edge coin blocks: no block-wide scan);
+//   * lists of at least kTileBlocks blocks are listed and dealt to all warps in
+//     tiles of 32 blocks, round robin across lists;
+//   * on a uniform-threshold list a block is only tested against the threshold;
+//     the few that hold a live edge or a tie go to a shared list, and after the
+//     level's barrier all threads take one each: the chain of coin, source
+//     read, bitmap atomic and queue append runs once per level, not inside a
+//     sweep.
+// Coins are the same (set, edge)-keyed Philox draws as every other sampler.
+// What bounds it: the integer-multiply pipe (18 wide multiplies of 4 cycles a
+// coin block); the sweep is written to add as little as possible to them.
 #include "device.cuh"
 #include "launch.h"
 
@@ -24,43 +30,24 @@ namespace {
 // resident per SM (10, 5, 2 or 1: at most 48, 48, 64 or 64 registers a
 // thread), each growing its own set -- more resident CTAs let one set's
 // barrier waits overlap another's work; the autotuner picks the shape per
-// graph.  In-lists of at least BIG_THREADS coin blocks are swept by the
-// whole CTA, one list at a time.
+// graph.
 
-// Exclusive block scan of one u32 per thread; returns the exclusive value and
-// writes the block total to *total.  Uses `warp_tot` (BIG_WARPS entries).
-template <int BIG_THREADS>
-__device__ uint32_t big_block_scan(uint32_t x, uint32_t *warp_tot, uint32_t *total) {
-  constexpr int BIG_WARPS = BIG_THREADS / 32;
-  const uint32_t lane = lane_id(), wid = threadIdx.x >> 5;
-  const uint32_t incl = warp_incl_scan(x);
-  if (lane == 31) warp_tot[wid] = incl;
-  __syncthreads();
-  if (wid == 0) {
-    const uint32_t t = lane < BIG_WARPS ? warp_tot[lane] : 0u;
-    const uint32_t ti = warp_incl_scan(t);
-    if (lane < BIG_WARPS) warp_tot[lane] = ti - t;
-    if (lane == 31) *total = ti;
-  }
-  __syncthreads();
-  const uint32_t r = warp_tot[wid] + incl - x;
-  __syncthreads();
-  return r;
-}
+constexpr uint32_t kTileBlocks = 128;   // lists of at least this many blocks go in tiles
+constexpr uint32_t kBigLong = 256;        // long lists a level may list
+constexpr uint32_t kBigCandidates = 512;  // blocks a level may defer (the rest run in place)
 
 template <int BIG_THREADS>
 __global__ void __launch_bounds__(BIG_THREADS, kBigCtasPerSm(BIG_THREADS))
 ic_bigset_kernel(const __grid_constant__ BigLaunch L) {
-  constexpr int BIG_WARPS = BIG_THREADS / 32;
-  constexpr uint32_t kLongCTA = BIG_THREADS;
-  __shared__ uint32_t s_off[BIG_THREADS + 1];  // exclusive coin-block offsets of the chunk
-  __shared__ uint32_t s_beg[BIG_THREADS], s_end[BIG_THREADS], s_vt[BIG_THREADS];
-  __shared__ uint32_t s_warp[BIG_WARPS];
-  __shared__ uint32_t s_long[BIG_THREADS];  // entries of the chunk with long in-lists
-  __shared__ uint32_t s_idx, s_qlen, s_overflow, s_total, s_nlong;
-  __shared__ unsigned long long s_edges, s_uedges, s_usrc, s_base;
+  constexpr uint32_t WARPS = BIG_THREADS / 32;
+  __shared__ uint4 s_cand[kBigCandidates];  // block, list begin, list end, threshold
+  __shared__ uint32_t s_lbeg[kBigLong], s_lend[kBigLong], s_lvt[kBigLong];
+  __shared__ uint32_t s_ncand[2], s_nlong[2];  // by the level's parity
+  __shared__ uint32_t s_idx, s_qlen, s_overflow;
+  __shared__ uint32_t s_edges, s_uedges, s_usrc;  // a set's in-edges are fewer than 2^32
+  __shared__ unsigned long long s_base;
 
-  const uint32_t tid = threadIdx.x;
+  const uint32_t tid = threadIdx.x, lane = lane_id(), wid = tid >> 5;
   uint32_t *bm = L.bitmaps + (size_t)blockIdx.x * L.bm_words;
   uint32_t *q = L.queues + (size_t)blockIdx.x * L.qcap;
   unsigned long long n_exp = 0, n_edges = 0, n_sets = 0, n_elems = 0, n_uedges = 0, n_usrc = 0;
@@ -78,12 +65,14 @@ ic_bigset_kernel(const __grid_constant__ BigLaunch L) {
       atomicOr(&bm[root >> 5], 1u << (root & 31));
       s_qlen = 1;
       s_overflow = 0;
+      s_ncand[0] = s_nlong[0] = 0;
       s_edges = 0;
       s_uedges = 0;
       s_usrc = 0;
     }
     __syncthreads();
-    uint32_t lo = 0, hi = 1;
+    const CoinSet cs = coin_set(L.rk, s, DOM_IC);
+    uint32_t my_edges = 0, my_uedges = 0, my_usrc = 0;
     // Source u of a live edge joins the set (and the queue) unless there.
     auto reach = [&](uint32_t u) {
       const uint32_t bit = 1u << (u & 31);
@@ -93,79 +82,115 @@ ic_bigset_kernel(const __grid_constant__ BigLaunch L) {
         else s_overflow = 1;
       }
     };
-    // The live edges of 8-edge coin block b of the in-list [ob, oe) given its
-    // coarse coins c; their sources are read then and reached.
-    auto expand_block = [&](uint32_t b, uint32_t ob, uint32_t oe, uint32_t ovt, const u32x4 &c) {
-      uint32_t live = ic_block_live(L.G, L.key, s, b, ob, oe, ovt, c);
+    // The live edges of 8-edge coin block b of the in-list [ob, oe); their
+    // sources are read then and reached.
+    auto expand_block = [&](uint32_t b, uint32_t ob, uint32_t oe, uint32_t ovt) {
+      uint32_t live = ic_block_live(L.G, L.key, s, b, ob, oe, ovt, coin_block(L.rk, cs, b));
       while (live) {
         const uint32_t ed = (b << 3) + (__ffs(live) - 1);
         live &= live - 1;
-        if (ovt) atomicAdd(&s_usrc, 1ull);
+        if (ovt) ++my_usrc;
         reach(__ldg(&L.G.edges[ed].x));
       }
     };
-    while (lo < hi && !s_overflow) {
-      for (uint32_t cb = lo; cb < hi; cb += BIG_THREADS) {
-        const uint32_t e = cb + tid;
+    uint32_t lo = 0, hi = 1, par = 0;
+    bool full = false;  // the queue overflowed: every thread reads it between two barriers
+    while (lo < hi && !full) {
+      // A block of a uniform list that holds a live edge or a tie (or, past
+      // the list's end, neither: the deferred pass looks).
+      auto defer = [&](uint32_t b, uint32_t ob, uint32_t oe, uint32_t ovt) {
+        const uint32_t pos = atomicAdd(&s_ncand[par], 1u);
+        if (pos < kBigCandidates) s_cand[pos] = make_uint4(b, ob, oe, ovt);
+        else expand_block(b, ob, oe, ovt);
+      };
+      // 1. Every warp takes a share of the level's entries: it sweeps their
+      // shorter lists through their concatenated blocks (block j belongs to
+      // the lane whose scanned range holds it) and lists the long ones.
+      const uint32_t share = min(32u, (hi - lo + WARPS - 1) / WARPS);
+      for (uint32_t cb = lo + wid * share; cb < hi; cb += WARPS * share) {
+        const uint32_t e = cb + lane;
         uint32_t beg = 0, end = 0, vt = 0;
-        if (tid == 0) s_nlong = 0;
-        if (e < hi) {
+        if (lane < share && e < hi) {
           const uint32_t v = q[e];
           beg = __ldg(L.G.off + v);
           end = __ldg(L.G.off + v + 1);
           if (L.G.vthr) vt = __ldg(L.G.vthr + v);
-          atomicAdd(&s_edges, (unsigned long long)(end - beg));
-          if (vt) atomicAdd(&s_uedges, (unsigned long long)(end - beg));
+          my_edges += end - beg;
+          if (vt) my_uedges += end - beg;
         }
-        s_beg[tid] = beg;
-        s_end[tid] = end;
-        s_vt[tid] = vt;
-        const uint32_t nb = block_count(beg, end);
-        const bool lng = nb >= kLongCTA;
-        s_off[tid] = big_block_scan<BIG_THREADS>(lng ? 0u : nb, s_warp, &s_total);  // syncs
-        if (tid == 0) s_off[BIG_THREADS] = s_total;
-        if (lng) s_long[atomicAdd(&s_nlong, 1u)] = tid;
-        __syncthreads();
-        // long in-lists (hubs): all threads sweep one list at a time, a
-        // thread taking whole coin blocks, two in flight so that their
-        // dependent Philox rounds interleave
-        const uint32_t nlong = s_nlong;
-        for (uint32_t li = 0; li < nlong; ++li) {
-          const uint32_t a = s_long[li];
-          const uint32_t ob = s_beg[a], oe = s_end[a], ovt = s_vt[a];
-          const uint32_t b_last = (oe - 1) >> 3;
-          uint32_t b = (ob >> 3) + tid;
-          for (; b + BIG_THREADS <= b_last; b += 2 * BIG_THREADS) {
-            const u32x4 c0 = ic_block_rk(L.rk, b, s);
-            const u32x4 c1 = ic_block_rk(L.rk, b + BIG_THREADS, s);
-            expand_block(b, ob, oe, ovt, c0);
-            expand_block(b + BIG_THREADS, ob, oe, ovt, c1);
-          }
-          if (b <= b_last) expand_block(b, ob, oe, ovt, ic_block_rk(L.rk, b, s));
+        uint32_t nb = block_count(beg, end);
+        if (nb >= kTileBlocks) {
+          const uint32_t pos = atomicAdd(&s_nlong[par], 1u);
+          if (pos < kBigLong) {
+            s_lbeg[pos] = beg;
+            s_lend[pos] = end;
+            s_lvt[pos] = vt;
+            nb = 0;
+          }  // (no room: this warp sweeps it with the others)
         }
-        // the other lists through their concatenated coin blocks: entry a
-        // holds block j when s_off[a] <= j < s_off[a + 1]; a thread's j only
-        // grows, so its entry cursor only moves forward
-        const uint32_t total = s_off[BIG_THREADS];
-        uint32_t a = 0;
-        for (uint32_t j = tid; j < total; j += BIG_THREADS) {
-          if (s_off[a + 1] <= j) {
-            uint32_t hi2 = BIG_THREADS;
-            while (hi2 - a > 1) {
-              const uint32_t mid = (a + hi2) >> 1;
-              if (s_off[mid] <= j) a = mid;
-              else hi2 = mid;
+        const uint32_t incl = warp_incl_scan(nb);
+        const uint32_t total = __shfl_sync(FULL, incl, 31);
+        for (uint32_t base = 0; base < total; base += 32) {
+          const uint32_t j = base + lane;
+          const uint32_t owner = warp_find_owner(incl, min(j, total - 1));
+          const uint32_t ob = __shfl_sync(FULL, beg, owner);
+          const uint32_t oe = __shfl_sync(FULL, end, owner);
+          const uint32_t oexcl = __shfl_sync(FULL, incl - nb, owner);
+          const uint32_t ovt = __shfl_sync(FULL, vt, owner);
+          if (j < total) expand_block((ob >> 3) + (j - oexcl), ob, oe, ovt);
+        }
+      }
+      __syncthreads();
+      // 2. The long lists, dealt to the warps a tile of 32 blocks at a time.
+      const uint32_t nlong = min(s_nlong[par], kBigLong);
+      uint32_t deal = wid;  // (wid - tiles dealt so far) mod WARPS: this warp's next tile
+      for (uint32_t a = 0; a < nlong; ++a) {
+        const uint32_t ob = s_lbeg[a], oe = s_lend[a], ovt = s_lvt[a];
+        const uint32_t b_last = (oe - 1) >> 3;
+        const uint32_t ntiles = ((b_last - (ob >> 3)) >> 5) + 1;
+        uint32_t b = (ob >> 3) + (deal & (WARPS - 1)) * 32 + lane;
+        const uint32_t b_stop = (ob >> 3) + ntiles * 32;  // first block past the tiles
+        deal -= ntiles;
+        const uint32_t th = ovt >> 16;
+        if (ovt != 0 && th != 0xFFFFu) {
+          // (blocks past the list's end draw coins nobody looks at: the
+          // deferred pass drops edges outside [ob, oe))
+          const uint32_t lim = (th + 1) * 0x10001u;
+          for (; b + BIG_THREADS < b_stop; b += 2 * BIG_THREADS) {
+            const bool h0 = block_clipped(coin_block(L.rk, cs, b), lim);
+            const bool h1 = block_clipped(coin_block(L.rk, cs, b + BIG_THREADS), lim);
+            if (h0 || h1) {
+              if (h0) defer(b, ob, oe, ovt);
+              if (h1) defer(b + BIG_THREADS, ob, oe, ovt);
             }
           }
-          const uint32_t ob = s_beg[a];
-          const uint32_t b = (ob >> 3) + (j - s_off[a]);
-          expand_block(b, ob, s_end[a], s_vt[a], ic_block_rk(L.rk, b, s));
+          if (b < b_stop && block_clipped(coin_block(L.rk, cs, b), lim)) defer(b, ob, oe, ovt);
+        } else {
+          for (; b <= b_last; b += BIG_THREADS) expand_block(b, ob, oe, ovt);
         }
-        __syncthreads();
       }
+      __syncthreads();
+      // 3. The deferred blocks, a thread each.
+      const uint32_t ncand = min(s_ncand[par], kBigCandidates);
+      if (tid == 0) s_ncand[par ^ 1] = s_nlong[par ^ 1] = 0;
+      for (uint32_t i = tid; i < ncand; i += BIG_THREADS) {
+        const uint4 c = s_cand[i];
+        expand_block(c.x, c.y, c.z, c.w);
+      }
+      __syncthreads();
       lo = hi;
       hi = min(s_qlen, L.qcap);
+      full = s_overflow != 0;
+      par ^= 1;
       __syncthreads();
+    }
+    my_edges = __reduce_add_sync(FULL, my_edges);
+    my_uedges = __reduce_add_sync(FULL, my_uedges);
+    my_usrc = __reduce_add_sync(FULL, my_usrc);
+    if (lane_id() == 0) {
+      atomicAdd(&s_edges, my_edges);
+      atomicAdd(&s_uedges, my_uedges);
+      atomicAdd(&s_usrc, my_usrc);
     }
     const uint32_t qlen = min(s_qlen, L.qcap);
     bool stored = false;

@@ -20,14 +20,15 @@ coin_rate_kernel(const __grid_constant__ RoundKeys rk, Key key, uint32_t blocks_
                  uint32_t thr, unsigned long long *live) {
   const uint64_t tid = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
   const uint64_t s = tid;                                 // one set per thread
-  const uint64_t b0 = tid * (uint64_t)blocks_per_thread;  // its own coin blocks
+  const uint32_t b0 = threadIdx.x * blocks_per_thread;    // its own coin blocks
+  const CoinSet cs = coin_set(rk, s, DOM_IC);
   uint32_t cnt = 0;
   for (uint32_t i = 0; i < blocks_per_thread; ++i) {
-    const u32x4 c = ic_block_rk(rk, b0 + i, s);
-    if (block_min16(c) <= (thr >> 16)) {  // as the samplers: most blocks stop here
+    const u32x4 c = coin_block(rk, cs, b0 + i);
+    if (block_any_le(c, thr >> 16)) {  // as the samplers: most blocks stop here
 #pragma unroll
       for (int h = 0; h < 8; ++h)
-        cnt += ic_live(key, s, ((b0 + i) << 3) + h, coarse_of(c, h), thr);
+        cnt += ic_live(key, s, ((uint64_t)(b0 + i) << 3) + h, coarse_of(c, h), thr);
     }
   }
   for (int d = 16; d > 0; d >>= 1) cnt += __shfl_xor_sync(FULL, cnt, d);

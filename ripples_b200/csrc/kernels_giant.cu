@@ -173,7 +173,7 @@ __global__ void __launch_bounds__(256) giant_expand_kernel(const __grid_constant
             const int bi = __ffsll((long long)mm) - 1;
             mm &= mm - 1;
             const uint64_t sid = L.set_ids[w * 64 + bi];
-            const u32x4 cb = ic_block_rk(L.rk, b, sid);
+            const u32x4 cb = coin_block(L.rk, coin_set(L.rk, sid, DOM_IC), b);
             const uint64_t bit = 1ull << bi;
             uint32_t tie = 0;
 #pragma unroll

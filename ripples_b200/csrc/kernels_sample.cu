@@ -93,11 +93,12 @@ struct SetOutcome {
 // One IC set: reverse BFS from root(s) over live in-edges, warp-cooperative,
 // members in discovery order in W.q.  Sets past `work_cap` in-edges (when
 // nonzero) are abandoned with big = true.
-template <class Coins>
-__device__ __forceinline__ SetOutcome ic_plain_set(const DevGraph &G, Key key, const Coins &coins,
+template <class RK>
+__device__ __forceinline__ SetOutcome ic_plain_set(const DevGraph &G, Key key, const RK &rk,
                                                    uint64_t s, const WarpCtx &W,
                                                    uint64_t work_cap) {
   const uint32_t lane = lane_id();
+  const CoinSet cs = coin_set(rk, s, DOM_IC);
   const uint32_t root = root_of(key, s, G.n);
   if (lane == 0) {
     W.q[0] = root;
@@ -125,7 +126,7 @@ __device__ __forceinline__ SetOutcome ic_plain_set(const DevGraph &G, Key key, c
     qlen += cnt;
   };
   auto block_live = [&](uint32_t b, uint32_t ob, uint32_t oe, uint32_t ovt) -> uint32_t {
-    return ic_block_live(G, key, s, b, ob, oe, ovt, coins.block(b, s));
+    return ic_block_live(G, key, s, b, ob, oe, ovt, coin_block(rk, cs, b));
   };
   // Marks the sources of a block's live edges in the bitmap and queues the
   // new ones: one live edge per lane per pass, every lane voting (live edges
@@ -310,7 +311,7 @@ ic_plain_kernel(DevGraph G, DevPool P, Key key, const __grid_constant__ RoundKey
     if (idx >= count) break;
     const uint32_t rel = ids ? ids[idx] : idx;
     const uint64_t s = first + rel;
-    const SetOutcome o = ic_plain_set(G, key, RoundKeyCoins{rk}, s, W, work_cap);
+    const SetOutcome o = ic_plain_set(G, key, rk, s, W, work_cap);
     if (finish_set(W, o.qlen, o.overflow, s, rel, P, F, o.big)) {
       n_sets += (lane == 0);
       n_elems += (lane == 0) ? o.qlen : 0;
@@ -431,7 +432,7 @@ multi_sample_kernel(MultiLaunch L) {
     const InstanceDesc &D = L.inst[a];
     const uint32_t rel = idx - L.prefix[a];
     const uint64_t s = D.first + rel;
-    const SetOutcome o = D.model == RIP_MODEL_IC ? ic_plain_set(D.G, D.key, KeyCoins{D.key}, s, W, D.work_cap)
+    const SetOutcome o = D.model == RIP_MODEL_IC ? ic_plain_set(D.G, D.key, KeyRounds{D.key}, s, W, D.work_cap)
                                                  : lt_walk_set(D.G, D.key, s, W);
     if (store_set(W, o.qlen, o.overflow, s, D.P, D.first_bad, D.model == RIP_MODEL_IC)) {
       n_sets += 1;

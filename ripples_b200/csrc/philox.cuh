@@ -51,8 +51,12 @@ enum : uint32_t {
 
 RIP_HD void mulhilo32(uint32_t a, uint32_t b, uint32_t &hi, uint32_t &lo) {
 #if defined(__CUDA_ARCH__)
-  hi = __umulhi(a, b);
-  lo = a * b;
+  // one wide multiply (4 issue cycles of the integer-multiply pipe, measured)
+  // for both halves: written as a high and a low product it takes 6 of them
+  uint64_t p;
+  asm("mul.wide.u32 %0, %1, %2;" : "=l"(p) : "r"(a), "r"(b));
+  hi = (uint32_t)(p >> 32);
+  lo = (uint32_t)p;
 #else
   uint64_t p = (uint64_t)a * (uint64_t)b;
   hi = (uint32_t)(p >> 32);
@@ -110,6 +114,16 @@ RIP_HD Key make_key(uint64_t seed) {
 // adding the schedule in registers every round.
 struct RoundKeys {
   uint32_t k0[10], k1[10];
+  RIP_HD uint32_t r0(int r) const { return k0[r]; }
+  RIP_HD uint32_t r1(int r) const { return k1[r]; }
+};
+
+// The same keys added up in registers, for kernels whose key is not a launch
+// parameter.
+struct KeyRounds {
+  Key k;
+  RIP_HD uint32_t r0(int r) const { return k.k0 + (uint32_t)r * 0x9E3779B9u; }
+  RIP_HD uint32_t r1(int r) const { return k.k1 + (uint32_t)r * 0xBB67AE85u; }
 };
 
 RIP_HD RoundKeys round_keys(Key k) {
@@ -119,26 +133,6 @@ RIP_HD RoundKeys round_keys(Key k) {
     rk.k1[r] = k.k1 + (uint32_t)r * 0xBB67AE85u;
   }
   return rk;
-}
-
-// philox() with the round keys given.
-RIP_HD u32x4 philox_rk(uint32_t c0, uint32_t c1, uint32_t c2, uint32_t c3,
-                       const RoundKeys &rk) {
-#if defined(__CUDA_ARCH__)
-#pragma unroll
-#endif
-  for (int r = 0; r < 10; ++r) {
-    uint32_t hi0, lo0, hi1, lo1;
-    mulhilo32(0xD2511F53u, c0, hi0, lo0);
-    mulhilo32(0xCD9E8D57u, c2, hi1, lo1);
-    const uint32_t n0 = hi1 ^ c1 ^ rk.k0[r];
-    const uint32_t n2 = hi0 ^ c3 ^ rk.k1[r];
-    c0 = n0;
-    c1 = lo1;
-    c2 = n2;
-    c3 = lo0;
-  }
-  return u32x4{c0, c1, c2, c3};
 }
 
 RIP_HD uint32_t set_hi(uint64_t s, uint32_t dom) {
@@ -162,9 +156,51 @@ RIP_HD u32x4 ic_block(Key k, uint64_t b, uint64_t s) {
                 set_hi(s, DOM_IC), k.k0, k.k1);
 }
 
-// ic_block() with the launch's round keys.
-RIP_HD u32x4 ic_block_rk(const RoundKeys &rk, uint64_t b, uint64_t s) {
-  return philox_rk((uint32_t)b, (uint32_t)(b >> 32), (uint32_t)s, set_hi(s, DOM_IC), rk);
+// What the coin blocks of one set (or spread replica) share.  A block's
+// counter is (b, 0, s_lo, dom << 24 | s_hi) with b < 2^29 (edge ids are below
+// 2^32), so round 0's product of s_lo, and round 1's product of the word that
+// comes out of it, depend on the set alone: two of a block's twenty wide
+// multiplies are drawn once per set instead of once per block.
+struct CoinSet {
+  uint32_t x2;  // round 0: word 3 ^ key
+  uint32_t x0;  // round 1: word 1 ^ key
+  uint32_t y2;  // round 1: high product ^ key
+  uint32_t z2;  // round 2: word 3 (the low product) ^ key
+};
+
+template <class RK>
+RIP_HD CoinSet coin_set(const RK &rk, uint64_t s, uint32_t dom) {
+  uint32_t hi1, lo1, hi0, lo0;
+  mulhilo32(0xCD9E8D57u, (uint32_t)s, hi1, lo1);
+  mulhilo32(0xD2511F53u, hi1 ^ rk.r0(0), hi0, lo0);
+  return CoinSet{set_hi(s, dom) ^ rk.r1(0), lo1 ^ rk.r0(1), hi0 ^ rk.r1(1), lo0 ^ rk.r1(2)};
+}
+
+// ic_block() (sim_ic_block()) of block b for the set whose CoinSet is given.
+template <class RK>
+RIP_HD u32x4 coin_block(const RK &rk, const CoinSet &S, uint32_t b) {
+  uint32_t hi0, lo0, hi1, lo1;
+  mulhilo32(0xD2511F53u, b, hi0, lo0);              // round 0
+  mulhilo32(0xCD9E8D57u, hi0 ^ S.x2, hi1, lo1);     // round 1
+  uint32_t c0 = hi1 ^ S.x0, c1 = lo1, c2 = lo0 ^ S.y2, c3;
+  mulhilo32(0xD2511F53u, c0, hi0, lo0);             // round 2
+  mulhilo32(0xCD9E8D57u, c2, hi1, lo1);
+  c0 = hi1 ^ c1 ^ rk.r0(2);
+  c2 = hi0 ^ S.z2;
+  c1 = lo1;
+  c3 = lo0;
+#if defined(__CUDA_ARCH__)
+#pragma unroll
+#endif
+  for (int r = 3; r < 10; ++r) {
+    mulhilo32(0xD2511F53u, c0, hi0, lo0);
+    mulhilo32(0xCD9E8D57u, c2, hi1, lo1);
+    c0 = hi1 ^ c1 ^ rk.r0(r);
+    c2 = hi0 ^ c3 ^ rk.r1(r);
+    c1 = lo1;
+    c3 = lo0;
+  }
+  return u32x4{c0, c1, c2, c3};
 }
 
 // Fine (low) 16 bits of the coin of edge e of set s.

@@ -1,0 +1,56 @@
+"""Edges of the kernels' work division: list and set lengths around tiles,
+blocks and hand-over sizes, thresholds at the ends of their range.  Everything
+is integer work, so every comparison is exact."""
+import numpy as np
+import pytest
+
+import ripples_b200 as rb
+from oracle import oracle as O
+
+pytestmark = pytest.mark.gpu
+
+
+def hub_graph(hubs, lengths, probs, n=6000, seed=5):
+    """`hubs` vertices with in-lists of the given lengths (cycled) and one
+    probability each (cycled), half of their sources hubs; the other vertices
+    have one in-edge from a hub at 0.4."""
+    r = np.random.RandomState(seed)
+    lists, w = [], []
+    for v in range(n):
+        if v < hubs:
+            d = lengths[v % len(lengths)]
+            s = np.where(r.rand(d) < 0.5, r.randint(0, hubs, d), r.randint(0, n, d))
+            lists.append(np.sort(s).astype(np.uint32))
+            w.append(np.full(d, probs[(v // len(lengths)) % len(probs)], dtype=np.float32))
+        else:
+            lists.append(np.array([v % hubs], dtype=np.uint32))
+            w.append(np.array([0.4], dtype=np.float32))
+    index = np.zeros(n + 1, dtype=np.uint64)
+    np.cumsum([len(x) for x in lists], out=index[1:])
+    return rb.HostGraph(n, index, np.concatenate(lists), np.concatenate(w))
+
+
+@pytest.mark.parametrize("threads", [128, 256, 1024])
+@pytest.mark.parametrize("hubs,probs", [
+    (64, [1e-3, 2.0 ** -16, 3e-4]),         # few live edges: deferred blocks
+    (400, [0.02, 0.03]),                    # more long lists in a level than are listed
+    (40, [0.5, 65535.5 / 65536, 1.0, 0.0]),  # more deferred blocks than there is room for
+])
+def test_heavy_set_list_tiles(ctx, threads, hubs, probs):
+    # block counts around a tile (32), the listing length (128) and a CTA's width
+    lengths = [1, 250, 256, 257, 1009, 1016, 1024, 1025, 1033, 2040, 2056, 4099]
+    g = hub_graph(hubs, lengths, probs)
+    dg = rb.DeviceGraph(ctx, g, "IC")
+    assert dg.uniform_thresholds()
+    p = rb.Pool(dg)
+    p.heavy_batch(0)
+    p.heavy_block(threads)
+    p.work_caps(64, 0)
+    p.sample(300, seed=9, sampler=rb.SAMPLER_PLAIN)
+    off, vtx = p.export()
+    thr = O.pack("IC", g.index, g.weights)
+    ooff, ovtx, ost = O.sample("IC", g.n, g.index, g.src, thr, 9, 0, 300)
+    assert np.array_equal(off, ooff) and np.array_equal(vtx, ovtx)
+    st = p.stats()
+    assert st[4] == ost[0] and st[5] == ost[1]
+    dg.close()

@@ -24,9 +24,10 @@
 //                   src/gpu/find_most_influential.cc:65-72): cached chunk
 //                   maxima, cover by decrement or recount.
 //
-// All per-set loops use the same warp-level load balancing: a warp takes 32
-// sets, scans their lengths and walks the concatenated elements 32 at a time,
-// each lane finding its set with a 5-step shuffle search.
+// The per-set loops share one load balancing (block_elements): a warp takes up
+// to 32 sets, scans their lengths and walks the concatenated elements, each
+// lane finding its set with a 5-step shuffle search; long sets are spread over
+// the whole block.
 #include <algorithm>
 
 #include "device.cuh"
@@ -44,10 +45,108 @@ __device__ __forceinline__ uint32_t lanemask_lt() {
 
 constexpr uint32_t NONE = 0xFFFFFFFFu;
 
-// Iterates the elements of 32 sets per warp.  `set_of(i)` returns the set
-// index for lane i of the current 32-set window (or a value >= limit for
-// none); `fn(set, vertex, valid)` is called by ALL lanes (valid says whether
-// the lane holds an element) so it may use warp collectives.
+// Sets of at least this many elements are walked by their whole block, 1024
+// elements at a step; the others by the warp that met them.
+constexpr uint32_t kLongSet = 512;
+constexpr uint32_t kBlock = 256;  // threads of every per-set kernel
+constexpr uint32_t kBlockWarps = kBlock / 32;
+
+struct LongSets {  // shared: the long sets a block met in one step
+  uint64_t set[kBlock], off[kBlock];
+  uint32_t len[kBlock];
+  uint32_t n;
+};
+
+// Calls the grid over the elements of sets set_of(i), i in [lo, hi) (~0: none).
+// A warp takes up to 32 sets a step -- fewer when that leaves warps idle: a
+// pool of giant sets has fewer sets than the grid has warps -- scans their
+// lengths and walks the concatenated elements, each lane finding its set with
+// a shuffle search: mixed(set, vertex, valid) is called by all lanes of the
+// warp, so it may use warp collectives.  Elements of a set of kLongSet or more
+// are spread over the block: single(set, vertex), no collectives.  One warp
+// walking a set of 40 000 elements alone took 0.5 ms; a block takes 15 us.
+template <typename SetOf, typename Mixed, typename Single>
+__device__ __forceinline__ void block_elements(const DevPool &P, uint64_t lo, uint64_t hi,
+                                               LongSets &sh, SetOf set_of, Mixed mixed,
+                                               Single single) {
+  const uint32_t lane = lane_id(), wid = threadIdx.x >> 5;
+  if (hi <= lo) return;
+  const uint64_t warps = (uint64_t)gridDim.x * kBlockWarps;
+  const uint64_t per = (hi - lo + warps - 1) / warps;
+  const uint32_t take = per < 32 ? (uint32_t)per : 32u;  // sets a warp takes a step
+  if (threadIdx.x == 0) sh.n = 0;
+  __syncthreads();
+  for (uint64_t base = lo + (uint64_t)blockIdx.x * kBlockWarps * take; base < hi;
+       base += warps * take) {
+    const uint64_t i = base + wid * take + lane;
+    uint64_t s = 0, off = 0;
+    uint32_t len = 0;
+    if (lane < take && i < hi) {
+      s = set_of(i);
+      if (s != ~0ull) {
+        len = P.set_len[s];
+        off = P.set_off[s];
+      }
+    }
+    if (len >= kLongSet) {
+      const uint32_t k = atomicAdd(&sh.n, 1u);
+      sh.set[k] = s;
+      sh.off[k] = off;
+      sh.len[k] = len;
+    }
+    const bool any = __syncthreads_or(len >= kLongSet);
+    if (len >= kLongSet) len = 0;
+    const uint32_t incl = warp_incl_scan(len);
+    const uint32_t total = __shfl_sync(FULL, incl, 31);
+    for (uint32_t j0 = 0; j0 < total; j0 += 64) {
+      uint64_t os[2];
+      uint32_t v[2];
+      bool valid[2];
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const uint32_t j = j0 + 32 * h + lane;
+        valid[h] = j < total;
+        const uint32_t owner = warp_find_owner(incl, valid[h] ? j : total - 1);
+        const uint64_t ooff = __shfl_sync(FULL, off, owner);
+        const uint32_t oexcl = __shfl_sync(FULL, incl - len, owner);
+        os[h] = __shfl_sync(FULL, s, owner);
+        v[h] = valid[h] ? P.vtx[ooff + (j - oexcl)] : NONE;
+      }
+#pragma unroll
+      for (int h = 0; h < 2; ++h)
+        if (j0 + 32 * h < total) mixed(os[h], v[h], valid[h]);
+    }
+    if (any) {
+      const uint32_t n = sh.n;
+      for (uint32_t k = 0; k < n; ++k) {
+        const uint64_t ks = sh.set[k];
+        const uint32_t *vtx = P.vtx + sh.off[k];
+        const uint32_t klen = sh.len[k];
+        for (uint32_t j = threadIdx.x; j < klen; j += 4 * kBlock) {
+          uint32_t v[4];
+#pragma unroll
+          for (int h = 0; h < 4; ++h)
+            if (j + h * kBlock < klen) v[h] = vtx[j + h * kBlock];
+#pragma unroll
+          for (int h = 0; h < 4; ++h)
+            if (j + h * kBlock < klen) single(ks, v[h]);
+        }
+      }
+      __syncthreads();
+      if (threadIdx.x == 0) sh.n = 0;
+      __syncthreads();
+    }
+  }
+}
+
+// The set ids themselves, for walks over sets [0, S).
+struct EverySet {
+  __device__ __forceinline__ uint64_t operator()(uint64_t i) const { return i; }
+};
+
+// Iterates the elements of 32 sets per warp; `fn(set, vertex, valid)` is
+// called by ALL lanes (valid says whether the lane holds an element) so it may
+// use warp collectives.
 template <typename SetOf, typename Fn>
 __device__ __forceinline__ void for_each_element(const DevPool &P,
                                                  uint64_t window_base,
@@ -96,15 +195,13 @@ __device__ __forceinline__ void add_occurrence(uint32_t *count, uint64_t s, uint
     atomicAdd(count + v, (uint32_t)__popc(peers));
 }
 
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(kBlock)
 count_kernel(DevPool P, uint64_t S, uint32_t *count) {
-  const uint64_t gw = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5;
-  const uint64_t nw = ((uint64_t)gridDim.x * blockDim.x) >> 5;
-  for (uint64_t wb = gw * 32; wb < S; wb += nw * 32) {
-    for_each_element(
-        P, wb, S, [](uint64_t i) { return i; },
-        [&](uint64_t s, uint32_t v, bool valid) { add_occurrence(count, s, v, valid); });
-  }
+  __shared__ LongSets sh;
+  block_elements(
+      P, 0, S, sh, EverySet(),
+      [&](uint64_t s, uint32_t v, bool valid) { add_occurrence(count, s, v, valid); },
+      [&](uint64_t, uint32_t v) { atomicAdd(count + v, 1u); });
 }
 
 // Sets of [0, S) holding at least one marked vertex (OPIM-C's FindCoverage,
@@ -128,47 +225,54 @@ coverage_kernel(DevPool P, uint64_t S, const uint32_t *marked, unsigned long lon
   if (lane_id() == 0 && mine) atomicAdd(covered, mine);
 }
 
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(kBlock)
 inverted_kernel(DevPool P, uint64_t S, uint64_t *cursor, uint32_t *inv, uint64_t base) {
-  const uint64_t gw = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5;
-  const uint64_t nw = ((uint64_t)gridDim.x * blockDim.x) >> 5;
-  for (uint64_t wb = gw * 32; wb < S; wb += nw * 32) {
-    for_each_element(
-        P, wb, S, [](uint64_t i) { return i; },
-        [&](uint64_t s, uint32_t v, bool valid) {
-          if (__shfl_sync(FULL, s, 0) == __shfl_sync(FULL, s, 31)) {  // distinct vertices
-            if (valid)
-              inv[atomicAdd((unsigned long long *)cursor + v, 1ull)] = (uint32_t)(base + s);
-            return;
-          }
-          const uint32_t peers = __match_any_sync(FULL, v);
-          const uint32_t leader = __ffs(peers) - 1;
-          unsigned long long b = 0;
-          if (valid && leader == lane_id())
-            b = atomicAdd((unsigned long long *)cursor + v,
-                          (unsigned long long)__popc(peers));
-          b = __shfl_sync(FULL, b, leader);
-          if (valid) inv[b + __popc(peers & lanemask_lt())] = (uint32_t)(base + s);
-        });
-  }
+  __shared__ LongSets sh;
+  unsigned long long *cur = reinterpret_cast<unsigned long long *>(cursor);
+  block_elements(
+      P, 0, S, sh, EverySet(),
+      [&](uint64_t s, uint32_t v, bool valid) {
+        if (__shfl_sync(FULL, s, 0) == __shfl_sync(FULL, s, 31)) {  // distinct vertices
+          if (valid) inv[atomicAdd(cur + v, 1ull)] = (uint32_t)(base + s);
+          return;
+        }
+        const uint32_t peers = __match_any_sync(FULL, v);
+        const uint32_t leader = __ffs(peers) - 1;
+        unsigned long long b = 0;
+        if (valid && leader == lane_id())
+          b = atomicAdd(cur + v, (unsigned long long)__popc(peers));
+        b = __shfl_sync(FULL, b, leader);
+        if (valid) inv[b + __popc(peers & lanemask_lt())] = (uint32_t)(base + s);
+      },
+      [&](uint64_t s, uint32_t v) { inv[atomicAdd(cur + v, 1ull)] = (uint32_t)(base + s); });
 }
 
-// One warp per set of the seed's inverted list.  A set holds each vertex
-// once, so its members are decremented with plain reductions (no result
-// needed, nothing to aggregate).
-__global__ void __launch_bounds__(256) cover_kernel(CoverLaunch C) {
-  const uint64_t gw = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5;
-  const uint64_t nw = ((uint64_t)gridDim.x * blockDim.x) >> 5;
-  const uint32_t lane = lane_id();
+// A reference-heap pick: covers the vertex's uncovered sets and decrements
+// their members with plain reductions (no result needed).  The vertex itself
+// is a member of every one of them and ends at 0: it is written once instead
+// of being decremented by every set at one address.
+__device__ __forceinline__ void cover_sets(const CoverLaunch &C, LongSets &sh) {
   const uint64_t lo = C.inv_off[C.vertex], hi = C.inv_off[C.vertex + 1];
-  for (uint64_t i = lo + gw; i < hi; i += nw) {
-    const uint32_t s = C.inv[i];
-    if (C.covered[s]) continue;  // covered by an earlier seed (warp-uniform)
-    const uint32_t len = C.P.set_len[s];
-    const uint64_t off = C.P.set_off[s];
-    if (lane == 0) C.covered[s] = 1;  // s holds the vertex once: no other warp has s
-    for (uint32_t j = lane; j < len; j += 32) atomicSub(C.count + C.P.vtx[off + j], 1u);
-  }
+  block_elements(
+      C.P, lo, hi, sh,
+      [&](uint64_t i) -> uint64_t {
+        const uint32_t s = C.inv[i];
+        if (C.covered[s]) return ~0ull;  // covered by an earlier seed
+        C.covered[s] = 1;                // s holds the vertex once: no other lane has s
+        return s;
+      },
+      [&](uint64_t, uint32_t v, bool valid) {
+        if (valid && v != C.vertex) atomicSub(C.count + v, 1u);
+      },
+      [&](uint64_t, uint32_t v) {
+        if (v != C.vertex) atomicSub(C.count + v, 1u);
+      });
+  if (blockIdx.x == 0 && threadIdx.x == 0) C.count[C.vertex] = 0u;
+}
+
+__global__ void __launch_bounds__(kBlock) cover_kernel(CoverLaunch C) {
+  __shared__ LongSets sh;
+  cover_sets(C, sh);
 }
 
 // The pick of a sharded selection over the summed counts: the largest
@@ -281,23 +385,13 @@ __global__ void __launch_bounds__(1024) cmax_max_kernel(const unsigned long long
 // the host's candidates for the next pick into `out` (mapped host memory),
 // resets the ticket and publishes `epoch` in *flag after a system-wide fence,
 // so the host polls one word instead of synchronising the stream.
-__global__ void __launch_bounds__(256) cover_gather_kernel(CoverLaunch C, const uint32_t *ids,
+__global__ void __launch_bounds__(kBlock) cover_gather_kernel(CoverLaunch C, const uint32_t *ids,
                                                            uint32_t nids, uint32_t *out,
                                                            unsigned int *done,
                                                            volatile unsigned int *flag,
                                                            unsigned int epoch) {
-  const uint64_t gw = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5;
-  const uint64_t nw = ((uint64_t)gridDim.x * blockDim.x) >> 5;
-  const uint32_t lane = lane_id();
-  const uint64_t lo = C.inv_off[C.vertex], hi = C.inv_off[C.vertex + 1];
-  for (uint64_t i = lo + gw; i < hi; i += nw) {
-    const uint32_t s = C.inv[i];
-    if (C.covered[s]) continue;
-    const uint32_t len = C.P.set_len[s];
-    const uint64_t off = C.P.set_off[s];
-    if (lane == 0) C.covered[s] = 1;
-    for (uint32_t j = lane; j < len; j += 32) atomicSub(C.count + C.P.vtx[off + j], 1u);
-  }
+  __shared__ LongSets sh;
+  cover_sets(C, sh);
   __shared__ bool s_last;
   __syncthreads();
   if (threadIdx.x == 0) {
@@ -367,19 +461,20 @@ __global__ void __launch_bounds__(256) sel_init_kernel(const SelDesc *__restrict
   }
 }
 
-__global__ void __launch_bounds__(256) sel_count_kernel(const SelDesc *__restrict__ dp) {
+__global__ void __launch_bounds__(kBlock) sel_count_kernel(const SelDesc *__restrict__ dp) {
+  __shared__ LongSets sh;
   const SelDesc d = *dp;
-  const uint64_t gw = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5;
-  const uint64_t nw = ((uint64_t)gridDim.x * blockDim.x) >> 5;
   unsigned long long elems = 0;
-  for (uint64_t wb = gw * 32; wb < d.S; wb += nw * 32) {
-    for_each_element(
-        d.P, wb, d.S, [](uint64_t i) { return i; },
-        [&](uint64_t s, uint32_t v, bool valid) {
-          add_occurrence(d.count, s, v, valid);
-          elems += valid ? 1 : 0;
-        });
-  }
+  block_elements(
+      d.P, 0, d.S, sh, EverySet(),
+      [&](uint64_t s, uint32_t v, bool valid) {
+        add_occurrence(d.count, s, v, valid);
+        elems += valid ? 1 : 0;
+      },
+      [&](uint64_t, uint32_t v) {
+        atomicAdd(d.count + v, 1u);
+        ++elems;
+      });
   elems = warp_sum_u64(elems);
   if (lane_id() == 0 && elems) atomicAdd(d.acc + 2, elems);
 }
@@ -450,8 +545,12 @@ __global__ void __launch_bounds__(256) sel_pick_kernel(const SelDesc *__restrict
 // mode: the sets are only marked, every count is cleared and every chunk
 // marked dirty, and sel_recount_kernel counts the sets left.  Both subtract
 // the covered sets' elements from acc[2] (elements of uncovered sets).
-__global__ void __launch_bounds__(256) sel_cover_kernel(const SelDesc *__restrict__ dp,
-                                                        uint32_t i) {
+constexpr uint32_t kDirtyShared = 4096;  // chunks whose dirty flags a block gathers first
+
+__global__ void __launch_bounds__(kBlock) sel_cover_kernel(const SelDesc *__restrict__ dp,
+                                                           uint32_t i) {
+  __shared__ LongSets sh;
+  __shared__ uint8_t s_dirty[kDirtyShared];
   const SelDesc d = *dp;
   const unsigned long long b = d.best[i];
   if ((b >> 32) == 0) return;
@@ -459,7 +558,6 @@ __global__ void __launch_bounds__(256) sel_cover_kernel(const SelDesc *__restric
   const bool recount = d.acc[4] != 0ull;
   const uint64_t tid = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
   const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
-  const uint64_t gw = tid >> 5, nw = stride >> 5;
   const uint32_t lane = lane_id();
   unsigned long long elems = 0;
   if (recount) {
@@ -467,35 +565,56 @@ __global__ void __launch_bounds__(256) sel_cover_kernel(const SelDesc *__restric
     const uint64_t n4 = (uint64_t)d.nchunks * (SEL_CHUNK / 4);
     for (uint64_t x = tid; x < n4; x += stride) c4[x] = make_uint4(0, 0, 0, 0);
     for (uint64_t x = tid; x < d.nchunks; x += stride) d.dirty[x] = 1;
-  }
-  for (uint32_t g = 0; g < d.nseg; ++g) {
-    if (d.seg_first[g] >= d.S) continue;  // the segment's sets are all >= S
-    const uint64_t lo = d.seg_off[g][v], hi = d.seg_off[g][v + 1];
-    if (recount) {  // one thread per entry: mark only
-      for (uint64_t j = lo + tid; j < hi; j += stride) {
-        const uint32_t s = d.seg_inv[g][j];
+    for (uint32_t g = 0; g < d.nseg; ++g) {
+      if (dp->seg_first[g] >= d.S) continue;  // the segment's sets are all >= S
+      const uint64_t lo = dp->seg_off[g][v], hi = dp->seg_off[g][v + 1];
+      for (uint64_t j = lo + tid; j < hi; j += stride) {  // one thread per entry: mark only
+        const uint32_t s = dp->seg_inv[g][j];
         if (s < d.S && !d.covered[s]) {  // s holds v once: no other thread has s
           d.covered[s] = 1;
           elems += d.P.set_len[s];
         }
       }
-      continue;
     }
-    for (uint64_t j = lo + gw; j < hi; j += nw) {  // one warp per entry
-      const uint32_t s = d.seg_inv[g][j];
-      if (s >= d.S || d.covered[s]) continue;  // warp-uniform
-      const uint32_t len = d.P.set_len[s];
-      const uint64_t so = d.P.set_off[s];
-      if (lane == 0) {
-        d.covered[s] = 1;
-        elems += len;
-      }
-      for (uint32_t e = lane; e < len; e += 32) {
-        const uint32_t u = d.P.vtx[so + e];
-        atomicSub(d.count + u, 1u);
-        d.dirty[u / SEL_CHUNK] = 1;
-      }
+  } else {
+    // the chunks a block touches are flagged in shared memory and written out
+    // once (one byte store per element otherwise)
+    const bool local = d.nchunks <= kDirtyShared;
+    if (local)
+      for (uint32_t x = threadIdx.x; x < d.nchunks; x += kBlock) s_dirty[x] = 0;
+    auto take = [&](uint32_t u) {
+      if (u == v) return;  // in every set of the list: written once, below
+      atomicSub(d.count + u, 1u);
+      if (local) s_dirty[u / SEL_CHUNK] = 1;
+      else d.dirty[u / SEL_CHUNK] = 1;
+    };
+    for (uint32_t g = 0; g < d.nseg; ++g) {
+      if (dp->seg_first[g] >= d.S) continue;
+      const uint64_t lo = dp->seg_off[g][v], hi = dp->seg_off[g][v + 1];
+      const uint32_t *inv = dp->seg_inv[g];
+      __syncthreads();
+      block_elements(
+          d.P, lo, hi, sh,
+          [&](uint64_t j) -> uint64_t {
+            const uint32_t s = inv[j];
+            if (s >= d.S || d.covered[s]) return ~0ull;
+            d.covered[s] = 1;  // s holds v once: no other lane has s
+            elems += d.P.set_len[s];
+            return s;
+          },
+          [&](uint64_t, uint32_t u, bool valid) {
+            if (valid) take(u);
+          },
+          [&](uint64_t, uint32_t u) { take(u); });
     }
+    if (tid == 0) {  // every set of [0, S) that held v is covered now
+      d.count[v] = 0u;
+      d.dirty[v / SEL_CHUNK] = 1;
+    }
+    __syncthreads();
+    if (local)
+      for (uint32_t x = threadIdx.x; x < d.nchunks; x += kBlock)
+        if (s_dirty[x]) d.dirty[x] = 1;
   }
   elems = warp_sum_u64(elems);
   if (lane == 0 && elems) atomicAdd(d.acc + 2, (unsigned long long)0 - elems);  // acc[2] -= elems
@@ -503,16 +622,14 @@ __global__ void __launch_bounds__(256) sel_cover_kernel(const SelDesc *__restric
 
 // Recount mode only: count the members of every set in [0, S) still
 // uncovered.
-__global__ void __launch_bounds__(256) sel_recount_kernel(const SelDesc *__restrict__ dp) {
+__global__ void __launch_bounds__(kBlock) sel_recount_kernel(const SelDesc *__restrict__ dp) {
+  __shared__ LongSets sh;
+  if (dp->acc[4] == 0ull) return;
   const SelDesc d = *dp;
-  if (d.acc[4] == 0ull) return;
-  const uint64_t gw = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5;
-  const uint64_t nw = ((uint64_t)gridDim.x * blockDim.x) >> 5;
-  for (uint64_t wb = gw * 32; wb < d.S; wb += nw * 32) {
-    for_each_element(
-        d.P, wb, d.S, [&](uint64_t x) { return d.covered[x] ? ~0ull : x; },
-        [&](uint64_t s, uint32_t v, bool valid) { add_occurrence(d.count, s, v, valid); });
-  }
+  block_elements(
+      d.P, 0, d.S, sh, [&](uint64_t x) -> uint64_t { return d.covered[x] ? ~0ull : x; },
+      [&](uint64_t s, uint32_t v, bool valid) { add_occurrence(d.count, s, v, valid); },
+      [&](uint64_t, uint32_t v) { atomicAdd(d.count + v, 1u); });
 }
 
 // out[i] = count[ids[i]] (ids and out may live in mapped host memory)
@@ -681,7 +798,7 @@ void launch_make_heap(const uint32_t *count, uint32_t n, uint2 *heap, cudaStream
 void launch_count(const DevPool &P, uint64_t num_sets, uint32_t *count,
                   int blocks, cudaStream_t stream) {
   count_launches(1);
-  count_kernel<<<blocks, 256, 0, stream>>>(P, num_sets, count);
+  count_kernel<<<blocks, kBlock, 0, stream>>>(P, num_sets, count);
 }
 
 size_t scan_block_sums_needed(uint32_t n) {
@@ -705,12 +822,12 @@ void launch_build_inverted(const DevPool &P, uint64_t num_sets,
                            uint64_t *cursor, uint32_t *inv, int blocks,
                            cudaStream_t stream, uint64_t base) {
   count_launches(1);
-  inverted_kernel<<<blocks, 256, 0, stream>>>(P, num_sets, cursor, inv, base);
+  inverted_kernel<<<blocks, kBlock, 0, stream>>>(P, num_sets, cursor, inv, base);
 }
 
 void launch_cover(const CoverLaunch &C, cudaStream_t stream) {
   count_launches(1);
-  cover_kernel<<<C.blocks, 256, 0, stream>>>(C);
+  cover_kernel<<<C.blocks, kBlock, 0, stream>>>(C);
 }
 
 void launch_cover_list(const CoverLaunch &C, uint32_t *out, unsigned long long *cursor,
@@ -737,7 +854,7 @@ void launch_cover_gather(const CoverLaunch &C, const uint32_t *ids, uint32_t nid
                          uint32_t *out, unsigned int *done, unsigned int *flag,
                          unsigned int epoch, cudaStream_t stream) {
   count_launches(1);
-  cover_gather_kernel<<<C.blocks, 256, 0, stream>>>(C, ids, nids, out, done, flag, epoch);
+  cover_gather_kernel<<<C.blocks, kBlock, 0, stream>>>(C, ids, nids, out, done, flag, epoch);
 }
 
 void launch_coverage(const DevPool &P, uint64_t S, const uint32_t *marked,
@@ -752,7 +869,7 @@ void launch_sel_init(const SelDesc *d, int blocks, cudaStream_t stream) {
 }
 void launch_sel_count(const SelDesc *d, int blocks, cudaStream_t stream) {
   count_launches(1);
-  sel_count_kernel<<<blocks, 256, 0, stream>>>(d);
+  sel_count_kernel<<<blocks, kBlock, 0, stream>>>(d);
 }
 void launch_sel_pick(const SelDesc *d, uint32_t i, int blocks, cudaStream_t stream) {
   count_launches(1);
@@ -760,8 +877,8 @@ void launch_sel_pick(const SelDesc *d, uint32_t i, int blocks, cudaStream_t stre
 }
 void launch_sel_cover(const SelDesc *d, uint32_t i, int blocks, cudaStream_t stream) {
   count_launches(2);
-  sel_cover_kernel<<<blocks, 256, 0, stream>>>(d, i);
-  sel_recount_kernel<<<blocks, 256, 0, stream>>>(d);
+  sel_cover_kernel<<<blocks, kBlock, 0, stream>>>(d, i);
+  sel_recount_kernel<<<blocks, kBlock, 0, stream>>>(d);
 }
 uint32_t sel_chunk_vertices() { return SEL_CHUNK; }
 

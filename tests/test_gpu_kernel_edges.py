@@ -54,3 +54,28 @@ def test_heavy_set_list_tiles(ctx, threads, hubs, probs):
     st = p.stats()
     assert st[4] == ost[0] and st[5] == ost[1]
     dg.close()
+
+
+SET_LENGTHS = [0, 1, 31, 32, 33, 63, 64, 65, 511, 512, 513, 1023, 1024, 1025, 5000]
+
+
+@pytest.mark.parametrize("tie", [rb.TIE_REF_HEAP, rb.TIE_LOWEST_ID])
+@pytest.mark.parametrize("copies,n", [(1, 6001), (40, 5003), (700, 5200)])
+def test_selection_over_set_lengths(ctx, tie, copies, n):
+    r = np.random.RandomState(copies)
+    lens = np.array(SET_LENGTHS * copies) if copies < 100 else np.array(SET_LENGTHS[:10] * copies)
+    r.shuffle(lens)
+    off = np.zeros(len(lens) + 1, dtype=np.uint64)
+    np.cumsum(lens, out=off[1:])
+    vtx = np.concatenate([r.choice(n, d, replace=False) for d in lens]).astype(np.uint32)
+    g = rb.HostGraph(n, np.zeros(n + 1, np.uint64), np.zeros(0, np.uint32), np.zeros(0, np.float32))
+    dg = rb.DeviceGraph(ctx, g, "IC")
+    p = rb.Pool(dg)
+    p.import_sets(off, vtx)
+    for s in (len(lens), len(lens) // 2 + 1):
+        e = int(off[s])
+        assert np.array_equal(p.count(s), np.bincount(vtx[:e], minlength=n))
+        of, oseeds, ogains, _ = O.select(n, off[: s + 1], vtx[:e], 12, tie)
+        f, seeds, gains = p.select(12, s, tie)
+        assert f == of and seeds.tolist() == oseeds.tolist() and gains.tolist() == ogains.tolist()
+    dg.close()

@@ -59,8 +59,8 @@ int rip_ctx_destroy(rip_ctx *c) {
   dfree(c, c->m_scratch);
   dfree(c, c->m_table);
   dfree(c, c->m_fail);
-  if (c->heap_registered) cudaHostUnregister(c->heap_registered);
   delete c->h_cand;
+  delete c->h_list;
   delete c->h_count;
   delete c->h_meta;
   if (c->ev0) cudaEventDestroy(c->ev0);

@@ -18,6 +18,7 @@
 #include <sys/types.h>
 
 #include "launch.h"
+#include "sparse_heap.h"
 #include "ripples_b200.h"
 
 using namespace rip;
@@ -35,20 +36,6 @@ struct DevMem {
   size_t bytes = 0;
 };
 
-// The reference's heap holds std::pair<vertex, size_t count> ordered by count
-// alone (CompareHeap, include/ripples/streaming_find_most_influential.h:410-418).
-// The heap algorithms only move elements and compare them with the
-// comparator, so an 8-byte {vertex, u32 count} item with the same comparison
-// yields the same sequence of heaps (counts never exceed the number of sets,
-// < 2^32), at half the memory.
-struct HeapItem {
-  uint32_t first;   // vertex
-  uint32_t second;  // count when pushed
-  bool operator==(const HeapItem &o) const { return first == o.first && second == o.second; }
-};
-struct CompareHeap {
-  bool operator()(const HeapItem &a, const HeapItem &b) const { return a.second < b.second; }
-};
 struct PinnedMem;
 
 struct rip_ctx {
@@ -64,10 +51,10 @@ struct rip_ctx {
   // (unique per context, so a flag left by an earlier pick never matches)
   uint32_t cg_epoch = 0;
   // reference-heap selection storage, shared by the context's pools (one
-  // selection runs at a time) and page-locked once
-  std::vector<HeapItem> heap_store;
-  void *heap_registered = nullptr;
-  PinnedMem *h_count = nullptr;  // counts at the start of a selection
+  // selection runs at a time)
+  SparseHeap heap;
+  PinnedMem *h_list = nullptr;   // the heap items a selection keeps
+  PinnedMem *h_count = nullptr;  // whole-array count fetches
   // multi-instance sampler scratch (per warp: bitmap for the largest graph
   // of the launch + queue), instance table, failure pairs
   DevMem m_scratch, m_table, m_fail;
@@ -354,7 +341,7 @@ struct rip_pool {
   bool last_counts_on_device = false;  // last_counts still in `count` only
   bool have_last_counts = false;
   uint32_t cand_fixed = 0;           // first-fetch threshold, % of the last gain (0 = adaptive)
-  DevMem d_heap;                     // heap built on the device
+  DevMem d_heap, d_list, d_hist;     // heap built on the device, its kept items, count buckets
   DevMem s_cmax, s_dirty, s_best, s_desc;  // device lowest-id picks
   // reference-heap picks: completion ticket of the cover-and-gather kernel
   // (zero between launches)

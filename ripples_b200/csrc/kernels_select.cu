@@ -736,63 +736,192 @@ scan_apply_kernel(const uint32_t *in, uint32_t n, const uint64_t *tile_sums,
   }
 }
 
-// libstdc++-compatible sift of make_heap: the hole at `hole` sinks to a leaf
-// along the larger child (the right one unless the left is strictly larger),
-// then `value` rises from there while its parent compares less.  Elements are
-// {vertex, count}; only counts are compared.
-__device__ void adjust_heap_dev(uint2 *h, int64_t hole, int64_t len, uint2 value) {
-  const int64_t top = hole;
-  int64_t child = hole;
-  while (child < (len - 1) / 2) {
-    child = 2 * (child + 1);
-    if (h[child].y < h[child - 1].y) child--;
-    h[hole] = h[child];
-    hole = child;
+// Heap items {vertex, count}: counts below K are all equally small (K = 0:
+// every count is its own key).
+__device__ __forceinline__ uint32_t heap_key(uint2 it, uint32_t K) { return it.y >= K ? it.y : 0u; }
+
+// One stage of the heap build: levels [d0, d0 + L) of the heap as std::make_heap
+// builds it (the parents of one level have disjoint subtrees, so any order
+// within a level gives the same heap).  A block takes 2^g neighbouring subtrees
+// rooted at level d0 and keeps their L levels in shared memory, each as a heap
+// of its own (item i's children at 2i + 1, 2i + 2); a sift that goes deeper goes
+// on in global memory, where the stages below have been built.  Small items
+// need not be ordered among themselves (sparse_heap.h says why), so with K > 0
+// a sift stops where both children are small.
+// Latency-bound: a launch per level took 24 launches and 0.39 ms at n = 2^24
+// (15 and 0.15 ms at 2^20); two stages keep all but the last sifts on chip.
+__global__ void __launch_bounds__(1024)
+heap_stage_kernel(const uint32_t *__restrict__ count, uint2 *heap, uint32_t len, uint32_t d0,
+                  uint32_t L, uint32_t g, uint32_t K) {
+  extern __shared__ uint2 s_item[];
+  const uint64_t first = (uint64_t)blockIdx.x << g;  // the block's first root, within level d0
+  // item i of subtree sub: its position in the heap
+  auto index = [&](uint32_t sub, uint32_t i) -> uint64_t {
+    const uint32_t j = 31u - __clz(i + 1);
+    return (1ull << (d0 + j)) - 1 + ((first + sub) << j) + (i + 1 - (1u << j));
+  };
+  for (uint32_t j = 0; j < L; ++j)
+    for (uint32_t x = threadIdx.x; x < (1u << (g + j)); x += blockDim.x) {
+      const uint64_t p = (1ull << (d0 + j)) - 1 + (first << j) + x;
+      if (p < len)
+        s_item[((x >> j) << L) + (1u << j) - 1 + (x & ((1u << j) - 1))] =
+            make_uint2((uint32_t)p, __ldg(count + p));
+    }
+  __syncthreads();
+  const uint32_t inside = (1u << L) - 1;  // items of a subtree kept here
+  for (int top = (int)L - 1; top >= 0; --top) {
+    for (uint32_t x = threadIdx.x; x < (1u << (g + top)); x += blockDim.x) {
+      const uint32_t sub = x >> top;
+      uint2 *item = s_item + (sub << L);
+      const uint32_t i0 = (1u << top) - 1 + (x & ((1u << top) - 1));
+      uint64_t p = index(sub, i0);
+      if (2 * p + 1 >= len) continue;  // a leaf, or past the end
+      // libstdc++'s __adjust_heap: the hole sinks along the larger child (the
+      // right one unless the left is strictly larger), then the value rises
+      // while its parent is smaller
+      const uint2 value = item[i0];
+      uint32_t i = i0;
+      while (2 * p + 1 < len) {
+        const bool here = 2 * i + 1 < inside;  // both children are, or neither
+        const uint64_t lp = 2 * p + 1;
+        uint2 c = here ? item[2 * i + 1] : heap[lp];
+        uint32_t right = 0;
+        if (lp + 1 < len) {
+          const uint2 r = here ? item[2 * i + 2] : heap[lp + 1];
+          if (!(heap_key(r, K) < heap_key(c, K))) {
+            c = r;
+            right = 1;
+          }
+        }
+        if (c.y < K) break;  // both small
+        if (i < inside) item[i] = c;
+        else heap[p] = c;
+        i = 2 * i + 1 + right;
+        p = lp + right;
+      }
+      while (i > i0) {
+        const uint32_t pi = (i - 1) >> 1;
+        const uint64_t pp = (p - 1) >> 1;
+        const uint2 par = pi < inside ? item[pi] : heap[pp];
+        if (!(heap_key(par, K) < heap_key(value, K))) break;
+        if (i < inside) item[i] = par;
+        else heap[p] = par;
+        i = pi;
+        p = pp;
+      }
+      if (i < inside) item[i] = value;
+      else heap[p] = value;
+    }
+    __syncthreads();
   }
-  if ((len & 1) == 0 && child == (len - 2) / 2) {
-    child = 2 * (child + 1);
-    h[hole] = h[child - 1];
-    hole = child - 1;
-  }
-  int64_t parent = (hole - 1) / 2;
-  while (hole > top && h[parent].y < value.y) {
-    h[hole] = h[parent];
-    hole = parent;
-    parent = (hole - 1) / 2;
-  }
-  h[hole] = value;
+  for (uint32_t j = 0; j < L; ++j)
+    for (uint32_t x = threadIdx.x; x < (1u << (g + j)); x += blockDim.x) {
+      const uint64_t p = (1ull << (d0 + j)) - 1 + (first << j) + x;
+      if (p < len) heap[p] = s_item[((x >> j) << L) + (1u << j) - 1 + (x & ((1u << j) - 1))];
+    }
 }
 
-// heap[v] = {v, count[v]}
-__global__ void heap_fill_kernel(const uint32_t *count, uint32_t n, uint2 *heap) {
-  for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < n; v += gridDim.x * blockDim.x)
-    heap[v] = make_uint2(v, count[v]);
+// hist[count_bucket(c)] += 1 over the counts.
+__global__ void __launch_bounds__(256)
+count_hist_kernel(const uint32_t *__restrict__ count, uint32_t n, uint32_t *hist) {
+  __shared__ uint32_t s_hist[kCountBuckets];
+  for (uint32_t i = threadIdx.x; i < kCountBuckets; i += blockDim.x) s_hist[i] = 0;
+  __syncthreads();
+  // most counts are small and equal: a warp adds each distinct bucket once
+  const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
+  for (uint64_t base = (uint64_t)blockIdx.x * blockDim.x; base < n; base += stride) {
+    const uint64_t v = base + threadIdx.x;
+    const uint32_t b = v < n ? count_bucket(count[v]) : kCountBuckets;
+    const uint32_t peers = __match_any_sync(FULL, b);
+    if (v < n && __ffs(peers) - 1 == (int)lane_id()) atomicAdd(&s_hist[b], __popc(peers));
+  }
+  __syncthreads();
+  for (uint32_t i = threadIdx.x; i < kCountBuckets; i += blockDim.x)
+    if (s_hist[i]) atomicAdd(hist + i, s_hist[i]);
 }
 
-// make_heap's parents [lo, hi] (one depth) in parallel: disjoint subtrees.
-__global__ void heap_level_kernel(uint2 *heap, int64_t len, int64_t lo, int64_t hi) {
-  for (int64_t p = hi - (int64_t)(blockIdx.x * blockDim.x + threadIdx.x); p >= lo;
-       p -= (int64_t)gridDim.x * blockDim.x)
-    adjust_heap_dev(heap, p, len, heap[p]);
+// count[v] = the count of every heap item.
+__global__ void __launch_bounds__(256)
+heap_counts_kernel(const uint2 *__restrict__ heap, uint32_t n, uint32_t *count) {
+  const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
+  for (uint64_t p = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; p < n; p += stride) {
+    const uint2 it = heap[p];
+    count[it.x] = it.y;
+  }
+}
+
+// The heap's items of K or more, in any order: vertices, counts and positions,
+// R of each.
+__global__ void __launch_bounds__(256)
+heap_list_kernel(const uint2 *__restrict__ heap, uint32_t n, uint32_t K, uint32_t R,
+                 uint32_t *list, unsigned int *tail) {
+  const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
+  for (uint64_t base = (uint64_t)blockIdx.x * blockDim.x; base < n; base += stride) {
+    const uint64_t p = base + threadIdx.x;
+    const uint2 it = p < n ? heap[p] : make_uint2(0u, 0u);
+    const bool want = p < n && it.y >= K;
+    const uint32_t bal = __ballot_sync(FULL, want);
+    if (!bal) continue;
+    uint32_t at = 0;
+    if (lane_id() == (uint32_t)(__ffs(bal) - 1)) at = atomicAdd(tail, (unsigned int)__popc(bal));
+    at = __shfl_sync(FULL, at, __ffs(bal) - 1) + __popc(bal & lanemask_lt());
+    if (want && at < R) {
+      list[at] = it.x;
+      list[(size_t)R + at] = it.y;
+      list[2 * (size_t)R + at] = (uint32_t)p;
+    }
+  }
 }
 
 }  // namespace
 
-void launch_make_heap(const uint32_t *count, uint32_t n, uint2 *heap, cudaStream_t stream) {
-  count_launches(1);
-  heap_fill_kernel<<<592, 256, 0, stream>>>(count, n, heap);
-  const int64_t len = n;
-  if (len < 2) return;
-  const int64_t last_parent = (len - 2) / 2;
-  int dmax = 0;
-  while ((((int64_t)2) << dmax) - 1 <= last_parent) ++dmax;
-  for (int d = dmax; d >= 0; --d) {
-    const int64_t lo = (((int64_t)1) << d) - 1;
-    const int64_t hi = std::min<int64_t>(last_parent, (((int64_t)2) << d) - 2);
-    const int blocks = (int)std::min<int64_t>(1184, (hi - lo + 1 + 255) / 256);
+void launch_make_heap(const uint32_t *count, uint32_t n, uint2 *heap, uint32_t K,
+                      cudaStream_t stream) {
+  uint32_t depth = 0;  // levels of the heap
+  while (depth < 32 && ((1ull << depth) - 1) < n) ++depth;
+  // shared memory holds 2^11 items of a lower stage (16 KB, six blocks an SM)
+  // and 2^14 of the top one (128 KB, one block): its sifts are the longest
+  constexpr uint32_t kTop = 14, kStage = 11;
+  static const cudaError_t attr = cudaFuncSetAttribute(
+      heap_stage_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(sizeof(uint2) << kTop));
+  (void)attr;
+  while (depth > 0) {
+    const bool top = depth <= kTop;
+    uint32_t d0 = 0, L = depth, g = 0;
+    if (!top) {
+      d0 = depth > kTop + kStage ? depth - kStage : kTop;
+      L = depth - d0;
+      g = std::min(kStage - L, d0);
+    }
+    // roots of level d0 that exist, 2^g of them a block
+    const uint64_t roots = std::min<uint64_t>(1ull << d0, n - ((1ull << d0) - 1));
+    const uint32_t blocks = (uint32_t)((roots + (1ull << g) - 1) >> g);
+    const uint32_t threads = top ? (L >= 10 ? 1024 : 256) : 256;
     count_launches(1);
-    heap_level_kernel<<<blocks, 256, 0, stream>>>(heap, len, lo, hi);
+    heap_stage_kernel<<<blocks, threads, sizeof(uint2) << (L + g), stream>>>(count, heap, n, d0, L,
+                                                                             g, K);
+    depth = d0;
   }
+}
+
+void launch_count_hist(const uint32_t *count, uint32_t n, uint32_t *hist, cudaStream_t stream) {
+  count_launches(1);
+  cudaMemsetAsync(hist, 0, sizeof(uint32_t) * kCountBuckets, stream);
+  const uint32_t blocks = std::min<uint32_t>(592, (n + 255) / 256);
+  count_hist_kernel<<<blocks, 256, 0, stream>>>(count, n, hist);
+}
+
+void launch_heap_counts(const uint2 *heap, uint32_t n, uint32_t *count, cudaStream_t stream) {
+  count_launches(1);
+  heap_counts_kernel<<<1184, 256, 0, stream>>>(heap, n, count);
+}
+
+void launch_heap_list(const uint2 *heap, uint32_t n, uint32_t K, uint32_t R, uint32_t *list,
+                      unsigned int *tail, cudaStream_t stream) {
+  count_launches(1);
+  cudaMemsetAsync(tail, 0, sizeof(*tail), stream);
+  const uint32_t blocks = std::min<uint32_t>(1184, (n + 255) / 256);
+  heap_list_kernel<<<blocks, 256, 0, stream>>>(heap, n, K, R, list, tail);
 }
 
 void launch_count(const DevPool &P, uint64_t num_sets, uint32_t *count,

@@ -235,9 +235,32 @@ void launch_chunk_pick(const uint32_t *count, uint32_t n, uint8_t *dirty,
 void launch_cover_gather(const CoverLaunch &C, const uint32_t *ids, uint32_t nids,
                          uint32_t *out, unsigned int *done, unsigned int *flag,
                          unsigned int epoch, cudaStream_t stream);
-// Builds the selection max-heap of {vertex, count} on the device, element for
-// element the heap std::make_heap builds (level-parallel).
-void launch_make_heap(const uint32_t *count, uint32_t n, uint2 *heap, cudaStream_t stream);
+// Builds the selection max-heap of {vertex, count} on the device: the items of
+// K or more element for element where std::make_heap puts them (K = 0: all),
+// the others in any order.
+void launch_make_heap(const uint32_t *count, uint32_t n, uint2 *heap, uint32_t K,
+                      cudaStream_t stream);
+// Counts by size: eight buckets per power of two (one per value below 16).
+constexpr uint32_t kCountBuckets = 240;
+__host__ __device__ inline uint32_t count_bucket(uint32_t c) {
+  if (c < 8) return c;
+#if defined(__CUDA_ARCH__)
+  const uint32_t e = 31u - __clz(c);
+#else
+  const uint32_t e = 31u - __builtin_clz(c);
+#endif
+  return ((e - 2) << 3) | ((c >> (e - 3)) & 7u);
+}
+inline uint32_t count_bucket_low(uint32_t b) {  // the smallest count of bucket b
+  return b < 8 ? b : (8u | (b & 7u)) << ((b >> 3) - 1);
+}
+void launch_count_hist(const uint32_t *count, uint32_t n, uint32_t *hist, cudaStream_t stream);
+// count[v] = the count of v's item in a heap launch_make_heap built.
+void launch_heap_counts(const uint2 *heap, uint32_t n, uint32_t *count, cudaStream_t stream);
+// list = the vertices, counts and positions of the R heap items of K or more,
+// R words each (*tail: a device word).
+void launch_heap_list(const uint2 *heap, uint32_t n, uint32_t K, uint32_t R, uint32_t *list,
+                      unsigned int *tail, cudaStream_t stream);
 
 
 // Device-only lowest-id picks of one served query (lives in device memory).

@@ -8,77 +8,27 @@
 // selection
 // ---------------------------------------------------------------------------
 namespace {
-using RefQueue = std::priority_queue<HeapItem, std::vector<HeapItem>, CompareHeap>;
-
-// std::priority_queue that adopts an already-heapified container instead of
-// running make_heap again (its container and comparator are protected
-// members).  pop/push are libstdc++'s own pop_heap/push_heap, as in the
-// reference.
-struct AdoptedQueue : RefQueue {
-  explicit AdoptedQueue(std::vector<HeapItem> &&heap) { this->c = std::move(heap); }
-  std::vector<HeapItem> release() { return std::move(this->c); }
-  const std::vector<HeapItem> &items() const { return this->c; }
-};
-
-// The vertices of every heap item keyed at least T (keys never grow
-// downwards, so subtrees whose root is keyed below T are skipped).  Walked
-// breadth first: the children of a queued node are prefetched when it is
-// queued, so the random reads into the heap array overlap.  Returns the
-// count, or cap + 1 when more than cap items qualify.
-static uint32_t collect_at_least(const std::vector<HeapItem> &h, uint32_t T, uint32_t cap,
-                                 uint32_t *out, std::vector<uint32_t> &queue) {
-  const size_t len = h.size();
-  uint32_t cnt = 0;
+// The items (ids) of every kept heap position keyed at least T (keys never grow
+// downwards, so subtrees whose root is keyed below T are skipped), breadth
+// first.  Returns the count, or cap + 1 when more than cap items qualify.
+static uint32_t collect_at_least(const SparseHeap &heap, uint32_t T, uint32_t cap, uint32_t *out,
+                                 std::vector<size_t> &queue) {
+  uint32_t cnt = 0, id, key;
   queue.clear();
-  if (len && h[0].second >= T) queue.push_back(0);
-  for (size_t head = 0; head < queue.size(); ++head) {
-    const size_t i = queue[head];
-    if (cnt == cap) return cap + 1;
-    out[cnt++] = h[i].first;
-    const size_t l = 2 * i + 1;
-    for (size_t c = l; c < l + 2 && c < len; ++c)
-      if (h[c].second >= T) {
-        queue.push_back((uint32_t)c);
-        if (2 * c + 1 < len) __builtin_prefetch(&h[2 * c + 1]);
-      }
+  auto look = [&](size_t p) {
+    if (!heap.kept_at(p, id, key) || key < T) return;
+    if (cnt < cap) out[cnt] = id;
+    ++cnt;
+    queue.push_back(p);
+  };
+  look(0);
+  for (size_t head = 0; head < queue.size() && cnt <= cap; ++head) {
+    const size_t p = queue[head];
+    look(2 * p + 1);
+    look(2 * p + 2);
   }
-  return cnt;
+  return std::min(cnt, cap + 1);
 }
-
-// Open-addressing map vertex -> fetched count for one pick's candidates.
-struct CountMap {
-  std::vector<uint32_t> key, val;  // key = vertex + 1, 0 = empty
-  uint32_t mask = 0;
-  void reset(uint32_t items) {
-    uint32_t cap = 64;
-    while (cap < 2 * items) cap <<= 1;
-    if (key.size() < cap) {
-      key.assign(cap, 0u);
-      val.resize(cap);
-    } else {
-      std::fill(key.begin(), key.begin() + cap, 0u);
-    }
-    mask = cap - 1;
-  }
-  static uint32_t hash(uint32_t v) { return (v * 2654435761u) ^ (v >> 15); }
-  void put(uint32_t v, uint32_t c) {
-    uint32_t i = hash(v) & mask;
-    while (key[i] != 0u && key[i] != v + 1) i = (i + 1) & mask;
-    key[i] = v + 1;
-    val[i] = c;
-  }
-  bool get(uint32_t v, uint32_t &c) const {
-    uint32_t i = hash(v) & mask;
-    while (key[i] != 0u) {
-      if (key[i] == v + 1) {
-        c = val[i];
-        return true;
-      }
-      i = (i + 1) & mask;
-    }
-    return false;
-  }
-};
 
 // Bit-identical to std::make_heap(v.begin(), v.end(), CompareHeap{}), built
 // level by level in parallel.  libstdc++'s make_heap runs __adjust_heap on
@@ -121,20 +71,30 @@ extern "C" int rip_selftest_heap_device(rip_ctx *c, uint64_t n, uint32_t max_cou
   for (uint64_t i = 0; i < n; ++i) ref[i] = {(uint32_t)i, cnt[i]};
   std::make_heap(ref.begin(), ref.end(), CompareHeap{});
   DevMem d_cnt, d_heap;
+  bool same = true;
   int rc = dalloc(c, d_cnt, 4 * n);
   if (!rc) rc = dalloc(c, d_heap, 8 * n);
   if (!rc) {
     cudaMemcpyAsync(d_cnt.p, cnt.data(), 4 * n, cudaMemcpyHostToDevice, c->stream);
-    launch_make_heap(ptr<uint32_t>(d_cnt), (uint32_t)n, ptr<uint2>(d_heap), c->stream);
-    cudaMemcpyAsync(got.data(), d_heap.p, 8 * n, cudaMemcpyDeviceToHost, c->stream);
-    cudaError_t e = cudaStreamSynchronize(c->stream);
-    if (e == cudaSuccess) e = cudaGetLastError();
-    if (e != cudaSuccess) rc = set_err(c, RIP_ERR_CUDA, "heap selftest: %s", cudaGetErrorString(e));
+    // the whole heap, then only the items of K or more in their places
+    for (uint32_t K : {0u, 1u, max_count / 2, max_count}) {
+      launch_make_heap(ptr<uint32_t>(d_cnt), (uint32_t)n, ptr<uint2>(d_heap), K, c->stream);
+      cudaMemcpyAsync(got.data(), d_heap.p, 8 * n, cudaMemcpyDeviceToHost, c->stream);
+      cudaError_t e = cudaStreamSynchronize(c->stream);
+      if (e == cudaSuccess) e = cudaGetLastError();
+      if (e != cudaSuccess) {
+        rc = set_err(c, RIP_ERR_CUDA, "heap selftest: %s", cudaGetErrorString(e));
+        break;
+      }
+      for (uint64_t i = 0; i < n && same; ++i)
+        same = (got[i].second >= K) == (ref[i].second >= K) &&
+               (ref[i].second < K || got[i] == ref[i]);
+    }
   }
   dfree(c, d_cnt);
   dfree(c, d_heap);
   if (rc) return rc;
-  return ref == got ? 1 : 0;
+  return same ? 1 : 0;
 }
 
 // Diagnostic: checks parallel_make_heap against std::make_heap on n random
@@ -149,7 +109,39 @@ extern "C" int rip_selftest_heap(uint64_t n, uint32_t max_count, uint64_t seed) 
   b = a;
   std::make_heap(b.begin(), b.end(), CompareHeap{});
   parallel_make_heap(a);
-  return a == b ? 1 : 0;
+  if (!(a == b)) return 0;
+  // pops and pushes on the items of K or more against the full heap's
+  for (uint32_t K : {0u, 1u, max_count / 2}) {
+    std::vector<uint32_t> vtx, key, pos;
+    for (uint64_t i = 0; i < n; ++i)
+      if (b[i].second >= K) {
+        vtx.push_back(b[i].first);
+        key.push_back(b[i].second);
+        pos.push_back((uint32_t)i);
+      }
+    SparseHeap h;
+    h.build(n, (uint32_t)vtx.size(), K, key.data(), pos.data());
+    a = b;
+    for (int op = 0; op < 2000 && !a.empty(); ++op) {
+      const HeapItem top = a.front();
+      if (h.top_kept() != (top.second >= K)) return 0;
+      if (top.second < K) break;
+      const uint32_t id = h.top_id();
+      if (vtx[id] != top.first || h.top_key() != top.second) return 0;
+      std::pop_heap(a.begin(), a.end(), CompareHeap{});
+      a.pop_back();
+      h.pop();
+      x = x * 6364136223846793005ull + 1442695040888963407ull;
+      if ((x >> 40) % 5) {  // back with a smaller key
+        const uint32_t k2 = (uint32_t)((x >> 33) % ((uint64_t)top.second + 1));
+        a.push_back(HeapItem{top.first, k2});
+        std::push_heap(a.begin(), a.end(), CompareHeap{});
+        h.push(id, k2, k2 >= K);
+      }
+      if (a.size() != h.size()) return 0;
+    }
+  }
+  return 1;
 }
 
 // The counts left by the last selection still sit in the count buffer; bring
@@ -202,8 +194,9 @@ extern "C" int rip_select_counts(rip_pool *p, uint32_t *counts) {
 }
 
 // Counts sets [0, S) into `count`, builds the vertex -> sets index over them
-// (inv_off, inv) and clears their covered flags; *P_out = index length.
-static int prepare_cover(rip_pool *p, uint64_t S, uint64_t *P_out) {
+// (inv_off, inv) and clears their covered flags; *P_out = index length.  hist
+// (may be null): the counts by bucket, kCountBuckets words.
+static int prepare_cover(rip_pool *p, uint64_t S, uint64_t *P_out, uint32_t *hist = nullptr) {
   rip_ctx *c = p->ctx;
   const uint32_t n = p->g->n;
   TRY(count_sets(p, S));
@@ -213,6 +206,12 @@ static int prepare_cover(rip_pool *p, uint64_t S, uint64_t *P_out) {
   launch_exclusive_scan(ptr<uint32_t>(p->count), ptr<uint64_t>(p->inv_off), n,
                         ptr<uint64_t>(p->scan_sums), c->stream);
   uint64_t P = 0;
+  if (hist) {
+    TRY(dalloc(c, p->d_hist, sizeof(uint32_t) * kCountBuckets));
+    launch_count_hist(ptr<uint32_t>(p->count), n, ptr<uint32_t>(p->d_hist), c->stream);
+    CK(c, cudaMemcpyAsync(hist, p->d_hist.p, sizeof(uint32_t) * kCountBuckets,
+                          cudaMemcpyDeviceToHost, c->stream));
+  }
   CK(c, cudaMemcpyAsync(&P, ptr<uint64_t>(p->inv_off) + n, sizeof(uint64_t),
                         cudaMemcpyDeviceToHost, c->stream));
   CK(c, cudaMemcpyAsync(p->inv_cur.p, p->inv_off.p, sizeof(uint64_t) * ((size_t)n + 1),
@@ -260,7 +259,8 @@ extern "C" int rip_select(rip_pool *p, uint64_t S, uint32_t k, int tiebreak,
   // 1. histogram, 2. vertex -> sets index
   p->have_last_counts = false;  // superseded by this selection
   uint64_t P = 0;
-  TRY(prepare_cover(p, S, &P));
+  uint32_t hist[kCountBuckets];  // counts by size (reference-heap picks)
+  TRY(prepare_cover(p, S, &P, tiebreak == RIP_TIE_REF_HEAP ? hist : nullptr));
   CoverLaunch C = cover_launch(p);
 
   // whole-array count fetches land in the context's page-locked buffer and
@@ -271,7 +271,6 @@ extern "C" int rip_select(rip_pool *p, uint64_t S, uint32_t k, int tiebreak,
   // mapped: candidate vertex ids in, their counts out (reference-heap picks)
   constexpr uint32_t CAND_CAP = 1u << 16;
   TRY(c->h_cand->ensure(c, 16 + 2 * sizeof(uint32_t) * (size_t)CAND_CAP, true));
-  TRY(c->h_count->ensure(c, sizeof(uint32_t) * (size_t)n));
   PinnedMem &h_cand = *c->h_cand, &h_count = *c->h_count;
 
   uint64_t uncovered = S;
@@ -297,45 +296,55 @@ extern "C" int rip_select(rip_pool *p, uint64_t S, uint32_t k, int tiebreak,
     const auto t_h0 = clk::now();
     // InitHeapStorage + std::priority_queue(cmp, std::move(storage)), as the
     // reference builds its heap (streaming_find_most_influential.h:541-544;
-    // counting.h:196-206): the same heap, built level-parallel on the device
-    // and downloaded into page-locked storage the queue adopts as is.
-    // The storage is the context's (page-locked once, reused by every pool);
-    // the guards hand it back on every way out of this block.
-    struct Lease {
-      rip_ctx *c;
-      std::vector<HeapItem> v;
-      explicit Lease(rip_ctx *c_) : c(c_), v(std::move(c_->heap_store)) {}
-      ~Lease() {
-        if (v.capacity()) c->heap_store = std::move(v);
-      }
-    } lease(c);
-    std::vector<HeapItem> &storage = lease.v;
-    if (storage.capacity() < n || !c->heap_registered) {
-      if (c->heap_registered) cudaHostUnregister(c->heap_registered);
-      c->heap_registered = nullptr;
-      std::vector<HeapItem>().swap(storage);
-      storage.reserve(n);
-      storage.resize(n);
-      if (cudaHostRegister(storage.data(), sizeof(HeapItem) * storage.capacity(), 0) ==
-          cudaSuccess) {
-        c->heap_registered = storage.data();
-      } else {
-        cudaGetLastError();  // pageable copy still works, only slower
-      }
-    }
-    storage.resize(n);
+    // counting.h:196-206), of which the host takes the items that can decide a
+    // pick (sparse_heap.h): those whose count is at least K, about kKeep of
+    // them at first, and more -- the pops so far repeated on the larger heap --
+    // if the gains fall below K.  At n = 2^24 the whole heap was 128 MB over
+    // the bus a selection (4.2 of 14.5 ms), and every pop sank to a leaf 24
+    // levels down.
+    constexpr uint32_t kKeep = 16384;
+    constexpr uint32_t kGone = 0xFFFFFFFFu;  // log: the popped item stayed out (a seed)
+    SparseHeap &heap = c->heap;
+    std::vector<uint32_t> ids;  // vertex by item id
+    std::vector<uint32_t> log;  // per pop: the key it went back with, or kGone
+    // an item's count as last fetched, and the fetch (pick) that brought it
+    std::vector<uint32_t> cnt, cnt_at;
+    uint32_t fetch = 0;
+    uint32_t K = 0, R = 0;
     TRY(dalloc(c, p->d_heap, sizeof(uint2) * (size_t)n));
-    launch_make_heap(ptr<uint32_t>(p->count), n, ptr<uint2>(p->d_heap), c->stream);
-    CK(c, cudaGetLastError());
-    CK(c, cudaMemcpyAsync(storage.data(), p->d_heap.p, sizeof(uint2) * (size_t)n,
-                          cudaMemcpyDeviceToHost, c->stream));
-    CK(c, cudaStreamSynchronize(c->stream));
-    AdoptedQueue queue(std::move(storage));
-    struct Return {
-      rip_ctx *c;
-      AdoptedQueue &q;
-      ~Return() { c->heap_store = q.release(); }
-    } give_back{c, queue};
+    if (!c->h_list) c->h_list = new PinnedMem();
+    // Keeps about `want` items: the buckets of the largest counts that hold
+    // no more than that (the first such bucket at least).
+    auto build = [&](uint64_t want, const uint32_t *d_count) -> int {
+      uint64_t kept = 0;
+      uint32_t b = kCountBuckets;
+      while (b > 0 && (kept == 0 || kept + hist[b - 1] <= want)) kept += hist[--b];
+      K = count_bucket_low(b);
+      R = (uint32_t)kept;
+      launch_make_heap(d_count, n, ptr<uint2>(p->d_heap), K, c->stream);
+      const size_t words = 3 * (size_t)R;
+      TRY(dalloc(c, p->d_list, sizeof(uint32_t) * (words + 1)));
+      TRY(c->h_list->ensure(c, sizeof(uint32_t) * words));
+      launch_heap_list(ptr<uint2>(p->d_heap), n, K, R, ptr<uint32_t>(p->d_list),
+                       ptr<unsigned int>(p->d_list) + words, c->stream);
+      CK(c, cudaGetLastError());
+      CK(c, cudaMemcpyAsync(c->h_list->p, p->d_list.p, sizeof(uint32_t) * words,
+                            cudaMemcpyDeviceToHost, c->stream));
+      CK(c, cudaStreamSynchronize(c->stream));
+      const uint32_t *vtx = static_cast<const uint32_t *>(c->h_list->p);
+      ids.assign(vtx, vtx + R);
+      cnt.resize(R);
+      cnt_at.assign(R, 0u);
+      fetch = 0;
+      heap.build(n, R, K, vtx + R, vtx + 2 * (size_t)R);
+      for (uint32_t key : log) {
+        const uint32_t id = heap.top_id();
+        heap.pop();
+        if (key != kGone) heap.push(id, key, key >= K);
+      }
+      return RIP_OK;
+    };
+    TRY(build(kKeep, ptr<uint32_t>(p->count)));
     p->sel_prof[1] += ms_since(t_h0);
     const auto t_p0 = clk::now();
     // The lazy pops of a pick only read the current counts of heap items keyed
@@ -350,17 +359,14 @@ extern "C" int rip_select(rip_pool *p, uint64_t S, uint32_t k, int tiebreak,
     uint32_t *h_cnt = h_ids + CAND_CAP;
     const uint32_t *d_ids = reinterpret_cast<const uint32_t *>(db + 16);
     uint32_t *d_cnt = reinterpret_cast<uint32_t *>(db + 16) + CAND_CAP;
-    CountMap cmap;
-    std::vector<uint32_t> stack;
-    // First pick: every key is still exact, so only the top is examined.
+    std::vector<uint32_t> cand(CAND_CAP);  // the items whose vertices are in h_ids
+    std::vector<size_t> stack;
+    // First pick: every key is still exact.
     bool fresh_all = false, first = true;
-    if (!queue.empty()) {
-      cmap.reset(1);
-      cmap.put(queue.top().first, queue.top().second);
-    }
     double ratio = 0.9;   // recent gain ratio g_i / g_{i-1}
     double margin = 0.9;  // guess = margin * ratio: lowered when a guess misses
     auto fetch_all = [&]() -> int {
+      TRY(h_count.ensure(c, sizeof(uint32_t) * (size_t)n));
       CK(c, cudaMemcpyAsync(h_count.p, p->count.p, sizeof(uint32_t) * (size_t)n,
                             cudaMemcpyDeviceToHost, c->stream));
       CK(c, cudaStreamSynchronize(c->stream));
@@ -387,13 +393,18 @@ extern "C" int rip_select(rip_pool *p, uint64_t S, uint32_t k, int tiebreak,
       const double guess = p->cand_fixed ? p->cand_fixed / 100.0 : margin * ratio;
       return (uint32_t)std::max<double>(1.0, std::floor((double)g_prev * guess));
     };
+    auto collect = [&](uint32_t T) -> uint32_t {
+      const auto t_c0 = clk::now();
+      const uint32_t nc = collect_at_least(heap, T, CAND_CAP, cand.data(), stack);
+      for (uint32_t i = 0; i < std::min(nc, CAND_CAP); ++i) h_ids[i] = ids[cand[i]];
+      p->sel_prof[10] += ms_since(t_c0);
+      return nc;
+    };
     // round-0 collect at T (raised once while too many items qualify);
     // returns the count, CAND_CAP + 1 when still too many
     auto collect0 = [&](uint64_t g_prev, uint32_t &T) -> uint32_t {
       for (;;) {
-        const auto t_c0 = clk::now();
-        const uint32_t nc = collect_at_least(queue.items(), T, CAND_CAP, h_ids, stack);
-        p->sel_prof[10] += ms_since(t_c0);
+        const uint32_t nc = collect(T);
         if (nc > CAND_CAP && T < g_prev) {
           T = (uint32_t)std::min<uint64_t>(g_prev, (uint64_t)T + (g_prev - T + 1) / 2);
           continue;
@@ -401,86 +412,93 @@ extern "C" int rip_select(rip_pool *p, uint64_t S, uint32_t k, int tiebreak,
         return nc;
       }
     };
+    // The counts the next pops can examine, after a cover.
+    auto fetch_candidates = [&](uint64_t g_prev) -> int {
+      uint32_t T = prefetched ? pre_T : first_T(g_prev);
+      for (int round = 0;; ++round) {
+        const bool have = round == 0 && prefetched;
+        const uint32_t nc = have ? pre_nc : round == 0 ? collect0(g_prev, T) : collect(T);
+        p->sel_prof[11] += 1;
+        if (nc > CAND_CAP) {
+          TRY(fetch_all());
+          break;
+        }
+        if (!have) {
+          launch_gather_counts(ptr<uint32_t>(p->count), d_ids, nc, d_cnt, c->stream);
+          CK(c, cudaGetLastError());
+          CK(c, cudaStreamSynchronize(c->stream));
+        }
+        p->sel_prof[5] += nc;
+        ++fetch;
+        uint32_t mc = 0;
+        for (uint32_t i = 0; i < nc; ++i) {
+          const uint32_t cv = *reinterpret_cast<volatile uint32_t *>(h_cnt + i);
+          cnt[cand[i]] = cv;
+          cnt_at[cand[i]] = fetch;
+          mc = std::max(mc, cv);
+        }
+        if (mc >= T || T <= 1) {
+          if (round == 0) margin = std::min(0.97, margin + 0.01);
+          break;
+        }
+        T = std::max<uint32_t>(mc, 1u);  // mc <= m < T: exact next round
+        margin = std::max(0.5, margin - 0.05);
+      }
+      prefetched = false;
+      return RIP_OK;
+    };
+    // The gains fell below K: keep more items.  Every item's count at the
+    // start is still in the heap array.
+    auto keep_more = [&]() -> int {
+      launch_heap_counts(ptr<uint2>(p->d_heap), n, ptr<uint32_t>(p->inv_cur), c->stream);
+      TRY(build(8ull * R, ptr<uint32_t>(p->inv_cur)));
+      prefetched = false;
+      return first || fresh_all ? RIP_OK : fetch_candidates(out_gains.back());
+    };
     while (out_seeds.size() < k && uncovered != 0) {
       const auto t_g0 = clk::now();
-      if (!first) {
-        const uint64_t g_prev = out_gains.back();
-        uint32_t T = prefetched ? pre_T : first_T(g_prev);
-        for (int round = 0;; ++round) {
-          uint32_t nc;
-          if (round == 0 && prefetched) {
-            nc = pre_nc;
-          } else if (round == 0) {
-            nc = collect0(g_prev, T);
-          } else {
-            const auto t_c0 = clk::now();
-            nc = collect_at_least(queue.items(), T, CAND_CAP, h_ids, stack);
-            p->sel_prof[10] += ms_since(t_c0);
-          }
-          p->sel_prof[11] += 1;
-          if (nc > CAND_CAP) {
-            TRY(fetch_all());
-            break;
-          }
-          if (!(round == 0 && prefetched)) {
-            launch_gather_counts(ptr<uint32_t>(p->count), d_ids, nc, d_cnt, c->stream);
-            CK(c, cudaGetLastError());
-            CK(c, cudaStreamSynchronize(c->stream));
-          }
-          p->sel_prof[5] += nc;
-          cmap.reset(nc);
-          uint32_t mc = 0;
-          for (uint32_t i = 0; i < nc; ++i) {
-            const uint32_t cv = *reinterpret_cast<volatile uint32_t *>(h_cnt + i);
-            cmap.put(h_ids[i], cv);
-            mc = std::max(mc, cv);
-          }
-          if (mc >= T || nc == queue.size()) {
-            if (round == 0) margin = std::min(0.97, margin + 0.01);
-            break;
-          }
-          T = std::max<uint32_t>(mc, 1u);  // mc <= m < T: exact next round
-          margin = std::max(0.5, margin - 0.05);
-        }
-        prefetched = false;
-      }
+      if (!first) TRY(fetch_candidates(out_gains.back()));
       p->sel_prof[7] += ms_since(t_g0);
-      HeapItem element;
+      uint32_t id = 0, gain = 0;
       const auto t_q0 = clk::now();
       for (;;) {  // getNextSeed, streaming_find_most_influential.h:560-571
-        if (queue.empty())
-          return set_err(c, RIP_ERR_STATE, "selection heap exhausted");
-        element = queue.top();
-        uint32_t cur = 0;
-        if (fresh_all) {
-          cur = hcount[element.first];
-        } else if (!cmap.get(element.first, cur)) {
-          TRY(fetch_all());
-          cur = hcount[element.first];
-        }
-        queue.pop();
-        p->sel_prof[3] += 1;
-        if (element.second > cur) {
-          element.second = cur;
-          queue.push(element);
+        if (!heap.top_kept()) {
+          if (K == 0) return set_err(c, RIP_ERR_STATE, "selection heap exhausted");
+          TRY(keep_more());
           continue;
         }
+        id = heap.top_id();
+        const uint32_t key = heap.top_key();
+        uint32_t cur = key;
+        if (!first) {
+          if (!fresh_all && cnt_at[id] != fetch) TRY(fetch_all());
+          cur = fresh_all ? hcount[ids[id]] : cnt[id];
+        }
+        heap.pop();
+        p->sel_prof[3] += 1;
+        if (key > cur) {
+          heap.push(id, cur, cur >= K);
+          log.push_back(cur);
+          continue;
+        }
+        log.push_back(kGone);
+        gain = key;
         break;
       }
       p->sel_prof[9] += ms_since(t_q0);
       if (!out_gains.empty() && out_gains.back())
-        ratio = std::min(1.0, (double)element.second / (double)out_gains.back());
-      uncovered -= element.second;
-      out_seeds.push_back(element.first);
-      out_gains.push_back(element.second);
+        ratio = std::min(1.0, (double)gain / (double)out_gains.back());
+      uncovered -= gain;
+      out_seeds.push_back(ids[id]);
+      out_gains.push_back(gain);
       if (out_seeds.size() == k) break;
       const auto t_f0 = clk::now();
-      pre_T = first_T(element.second);
-      pre_nc = collect0(element.second, pre_T);
+      pre_T = first_T(gain);
+      pre_nc = collect0(gain, pre_T);
       if (pre_nc <= FUSED_MAX) {
-        C.vertex = element.first;
+        C.vertex = ids[id];
         C.blocks = (int)std::min<uint64_t>(max_blocks * 4,
-                                           std::max<uint64_t>(1, (element.second + 7) / 8));
+                                           std::max<uint64_t>(1, ((uint64_t)gain + 7) / 8));
         // epochs count per context: the mapped buffer is the context's
         const unsigned int epoch = ++c->cg_epoch;
         *h_flag = 0u;  // the buffer's first word may hold anything before this
@@ -501,7 +519,7 @@ extern "C" int rip_select(rip_pool *p, uint64_t S, uint32_t k, int tiebreak,
         std::atomic_thread_fence(std::memory_order_acquire);
         prefetched = true;
       } else {
-        TRY(cover(element.first, element.second));
+        TRY(cover(ids[id], gain));
       }
       p->sel_prof[7] += ms_since(t_f0);
       fresh_all = first = false;

@@ -81,3 +81,26 @@ def test_selection_over_set_lengths(ctx, tie, copies, n):
         f, seeds, gains = p.select(12, s, tie)
         assert f == of and seeds.tolist() == oseeds.tolist() and gains.tolist() == ogains.tolist()
     dg.close()
+
+
+@pytest.mark.parametrize("k,hot", [(6, 40), (60, 25000)])
+def test_reference_heap_keeps_more_items(ctx, k, hot):
+    """The first seed covers most sets, so the gains fall below the counts the
+    host kept at first (n above what it keeps): the kept heap grows, down to
+    counts of one and, once every set with members is covered, of zero."""
+    n, r = 40003, np.random.RandomState(hot)
+    sets = [np.concatenate([[0], 1 + r.choice(hot, 30, replace=False)]) for _ in range(900)]
+    sets += [np.array([hot + 1 + i, hot + 2 + i]) for i in range(0, 40, 2)] + [np.array([], int)]
+    off = np.zeros(len(sets) + 1, dtype=np.uint64)
+    np.cumsum([len(x) for x in sets], out=off[1:])
+    vtx = np.concatenate(sets).astype(np.uint32)
+    g = rb.HostGraph(n, np.zeros(n + 1, np.uint64), np.zeros(0, np.uint32), np.zeros(0, np.float32))
+    dg = rb.DeviceGraph(ctx, g, "IC")
+    p = rb.Pool(dg)
+    p.import_sets(off, vtx)
+    of, oseeds, ogains, _ = O.select(n, off, vtx, k, rb.TIE_REF_HEAP)
+    for guess in (0, 100, 3):  # adaptive, too high, too low first fetches
+        p.select_guess(guess)
+        f, seeds, gains = p.select(k, tiebreak=rb.TIE_REF_HEAP)
+        assert f == of and seeds.tolist() == oseeds.tolist() and gains.tolist() == ogains.tolist()
+    dg.close()

@@ -90,7 +90,7 @@ int rip_ctx_stream(rip_ctx *ctx, void **stream);
 /* Number of kernels this library has launched in the process so far. */
 uint64_t rip_kernel_launches(void);
 /* Measured ceiling of the IC coin function on this device: coins per second
- * of a kernel that only draws coins (Philox4x32-10, four per block) the way a
+ * of a kernel that only draws coins (Philox4x32-10, eight per block) the way a
  * uniform-threshold in-list is expanded, at full occupancy, no memory
  * traffic.  The roofline of the samplers on weighted-cascade graphs, which
  * are bound by this arithmetic rather than by HBM.  No reference counterpart. */
@@ -207,7 +207,7 @@ int rip_pool_configure(rip_pool *p, uint32_t colors, uint32_t slots,
 /* Edge-work budgets (in-edges read) after which a one-set-per-warp set, or a
  * fused CTA batch, is handed to the CTA-per-set sampler, whose 32 warps split
  * each level's edge groups (the heavy tail of IC sampling on skewed graphs);
- * 0 disables the hand-over.  Defaults 2^18 and 2^23.  Results do not depend on
+ * 0 disables the hand-over.  Defaults 2^14 and 2^23.  Results do not depend on
  * these values. */
 int rip_pool_work_caps(rip_pool *p, uint64_t plain_cap, uint64_t fused_cap);
 
@@ -219,18 +219,19 @@ int rip_pool_work_caps(rip_pool *p, uint64_t plain_cap, uint64_t fused_cap);
  * heavy sets fill the GPU as they do at full size):
  *   0 plain (one set per warp), heavy sets past 2^18 in-edges -> grid-wide BFS
  *   1 plain, heavy past 2^14 in-edges -> grid-wide BFS
- *   2 plain, heavy past 2^18 -> one CTA per set
+ *   2 plain, heavy past 2^14 -> one CTA per set, block shape by the number of
+ *     heavy sets of a launch (what untuned graphs run where sets stay small)
  *   3/4/5 fused 64/128/256 colours, batches past 2^23 -> heavy path
  *   6/7 as 0/2 with the one-set-per-warp kernel capped at 48 registers
  *       (40 resident warps per SM instead of 32)
  *   8 as 2 with 256-thread CTAs for the heavy sets (5 sets growing per SM
- *       instead of 1: the block-shape axis; candidates 0-2 use 1024-thread
+ *       instead of 1: the block-shape axis; candidates 0-1 use 1024-thread
  *       CTAs, 6-7 256-thread ones), 9 the same with heavy sets from 2^16
  *       in-edges
  * writes the wall times to ms[] (may be null; a candidate dropped after the
  * screen keeps its screen time) and the fastest to *choice, and
  * keeps it for the graph: pools created afterwards start from it and
- * RIP_SAMPLER_AUTO runs it.  Untuned graphs run configuration 0 for AUTO.  LT
+ * RIP_SAMPLER_AUTO runs it.  Untuned graphs run the plain sampler for AUTO.  LT
  * graphs have one sampler (choice 0).  Sets never depend on the choice.  No
  * reference counterpart (the reference fixes its GPU colour width). */
 #define RIP_TUNE_CANDIDATES 10
@@ -265,14 +266,16 @@ int rip_pool_plain_occupancy(rip_pool *p, int blocks_per_sm);
  * regime of supercritical graphs, where many sets hold a large share of the
  * graph and overlap).  Default 32 on IC graphs whose reverse BFS is
  * supercritical -- the expected live in-edges of an edge's source,
- * sum over edges (u->v) of sum_{w->u} p(w->u) / m, above 1.1 -- else 0
+ * sum over edges (u->v) of sum_{w->u} p(w->u) / m, above 1.1 -- and which have
+ * at least 2^21 edges, else 0
  * (weighted cascade: at most 1); 0 = always one CTA per set.  An autotuned graph's pools start from its
  * tuned value.  Results do not depend on it.  No reference counterpart (the reference's GPU BFS,
  * include/ripples/gpu/bfs.h:1338-1680, has one colour-batched path). */
 int rip_pool_heavy_batch(rip_pool *p, uint32_t min_sets);
 
 /* Block shape of the one-CTA-per-set kernel for heavy IC sets: 128, 256, 512
- * or 1024 threads, 10, 5, 2 or 1 of them resident per SM (default 256; an
+ * or 1024 threads, 10, 5, 2 or 1 of them resident per SM (default: by the
+ * number of heavy sets of a launch, smaller blocks for more sets; an
  * autotuned graph's pools start from its tuned value).  Smaller CTAs grow
  * more sets per SM at once, each with fewer threads.  Results do not depend on it.  No reference counterpart. */
 int rip_pool_heavy_block(rip_pool *p, uint32_t threads);

@@ -42,7 +42,7 @@ static int setup_vthr(rip_ctx *c, rip_graph *g) {
   g->branching = total / (double)g->m;
   // grid-wide multi-colour BFS for heavy sets only where sets grow large and
   // overlap (a supercritical reverse BFS); else one CTA per heavy set
-  g->default_giant_min = g->branching > kSupercritical ? 32u : 0u;
+  g->default_giant_min = g->branching > kSupercritical && g->m >= kGiantEdges ? 32u : 0u;
   return RIP_OK;
 }
 

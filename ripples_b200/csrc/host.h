@@ -232,6 +232,20 @@ struct PinnedMem {
 // per set.
 constexpr double kSupercritical = 1.1;
 
+// Edges from which supercritical graphs do so: on a smaller graph one CTA
+// finishes a set before the grid has been through its levels.
+constexpr uint64_t kGiantEdges = 1ull << 21;
+
+// In-edges of a set after which a warp leaves it to the heavy-set path.  A
+// warp takes 256 of them in about a microsecond and a launch ends with its
+// slowest warp, so a late hand-over is a tail: 600 sets of 250 000 in-edges
+// on a 2^14-vertex graph took 4.5 ms at 2^18 and 1.8 ms at 2^14, 200 000 sets
+// of a 300 007-vertex Erdos-Renyi graph 8.6 and 6.3 ms.  What a warp has done
+// is done again, up to the cap per heavy set: at 2^24 vertices, weighted
+// cascade, 2^14 to 2^16 measure the same (41.7-42.4 ms for 400 000 sets; 2^18
+// 45.6).
+constexpr uint64_t kPlainCap = 1ull << 14;
+
 struct rip_graph {
   rip_ctx *ctx;
   uint32_t n;
@@ -258,9 +272,9 @@ struct rip_graph {
     bool set = false;
     int sampler = RIP_SAMPLER_PLAIN;
     uint32_t colors = 64, giant_min = 32;
-    uint64_t cap_plain = 1ull << 18, cap_fused = 1ull << 23;
+    uint64_t cap_plain = kPlainCap, cap_fused = 1ull << 23;
     int plain_occupancy = 0;
-    uint32_t big_threads = 256;
+    uint32_t big_threads = 0;
   } tuned;
   DevGraph view() {
     return DevGraph{n, m, ptr<uint32_t>(off), ptr<uint2>(edges),
@@ -294,6 +308,7 @@ struct PoolMeta {  // device-side bookkeeping block (one D2H reads it all)
   unsigned int fail_count;
   unsigned int next;
   unsigned int fused_dirty;
+  unsigned int big_count;
 };
 
 constexpr uint64_t kNoShard = ~0ull;
@@ -321,10 +336,12 @@ struct rip_pool {
   uint32_t giant_min = 32;  // heavy sets that switch to the grid-wide BFS (0 = never)
   int auto_sampler = RIP_SAMPLER_PLAIN;  // what RIP_SAMPLER_AUTO runs (IC)
   int plain_occupancy = 0;   // IC one-set-per-warp kernel variant (0 or 5)
-  uint64_t cap_plain = 1ull << 18;  // in-edges per set before a warp hands it over
+  uint64_t cap_plain = kPlainCap;   // in-edges per set before a warp hands it over
   uint64_t cap_fused = 1ull << 23;  // in-edges per fused batch before handing over
   uint64_t big_sets = 0;            // sets grown one CTA each (diagnostic)
-  uint32_t big_threads = 256;       // block shape of the CTA-per-set kernel (128-1024)
+  // block shape of the CTA-per-set kernel: 128-1024 threads, 0 = by the number
+  // of heavy sets of a launch (big_shape)
+  uint32_t big_threads = 0;
   uint32_t colors = 64;      // fused colour width (64/128/256)
   uint32_t fused_slots = 0;  // 0 = size from the budget
   uint32_t lcap_pref = 0;    // 0 = default frontier-log capacity

@@ -176,6 +176,7 @@ static uint32_t default_warps(rip_pool *p, uint32_t qcap) {
 static int sample_fused(rip_pool *p, uint64_t seed, uint64_t first, uint32_t count);
 static int sample_big(rip_pool *p, uint64_t seed, uint64_t first,
                       const std::vector<uint32_t> &ids);
+static int sample_big_listed(rip_pool *p, uint64_t seed, uint64_t first, uint32_t count);
 
 // One set per warp (IC BFS / LT walk).  IC sets whose edge work exceeds the
 // per-set cap are handed to the CTA-per-set sampler; sets that outgrow the warp
@@ -201,6 +202,14 @@ static int sample_warp_per_set(rip_pool *p, uint64_t seed, uint64_t first,
     ids = ptr<uint32_t>(p->ids_b);
   }
   const bool capped = g->model == RIP_MODEL_IC && p->cap_plain != 0;
+  // sets handed over stay on the device, up to 2^20 of them (b_ids has room
+  // for those that fail there too)
+  const uint32_t big_cap = capped ? std::min<uint32_t>(count, 1u << 20) : 0;
+  uint32_t n_big = 0;
+  if (capped) {
+    TRY(dalloc(c, p->b_ids, sizeof(uint32_t) * 2 * (size_t)big_cap));
+    CK(c, cudaMemsetAsync(&dm->big_count, 0, sizeof(unsigned int), c->stream));
+  }
   std::vector<uint32_t> big, retry;
   for (int attempt = 0; attempt < 64; ++attempt) {
     CK(c, cudaMemsetAsync(&dm->fail_count, 0, sizeof(unsigned int), c->stream));
@@ -220,6 +229,11 @@ static int sample_warp_per_set(rip_pool *p, uint64_t seed, uint64_t first,
     L.qcap = p->qcap;
     L.work_cap = capped ? p->cap_plain : 0;
     L.F = FailList{ptr<uint32_t>(p->ids_a), &dm->fail_count, &dm->first_bad};
+    if (capped) {
+      L.F.big = ptr<uint32_t>(p->b_ids);
+      L.F.big_count = &dm->big_count;
+      L.F.big_cap = big_cap;
+    }
     L.st = Stats{dm->stats};
     L.threads = 256;
     L.occupancy = p->plain_occupancy;
@@ -238,6 +252,7 @@ static int sample_warp_per_set(rip_pool *p, uint64_t seed, uint64_t first,
     cudaEventElapsedTime(&kms, c->ev0, c->ev1);
     p->kernel_ms += kms;
     p->kernel_launches++;
+    if (capped) n_big = std::min<uint32_t>(m.big_count, big_cap);
     if (m.fail_count == 0) {
       p->num_elems = m.cursor;
       break;
@@ -277,6 +292,7 @@ static int sample_warp_per_set(rip_pool *p, uint64_t seed, uint64_t first,
     todo = (uint32_t)retry.size();
     if (attempt == 63) return set_err(c, RIP_ERR_DEVICE, "sampler did not converge after retries");
   }
+  if (n_big) TRY(sample_big_listed(p, seed, first, n_big));
   if (!big.empty()) {
     std::sort(big.begin(), big.end());
     TRY(sample_big(p, seed, first, big));
@@ -290,13 +306,25 @@ static int sample_warp_per_set(rip_pool *p, uint64_t seed, uint64_t first,
 static int ensure_big_scratch(rip_pool *p, uint32_t slots, uint32_t qcap) {
   rip_ctx *c = p->ctx;
   const uint64_t bm_words = (((uint64_t)p->g->n + 31) / 32 + 7) & ~7ull;
-  if (p->b_scratch.p && p->b_slots == slots && p->b_qcap == qcap) return RIP_OK;
+  if (p->b_scratch.p && p->b_slots >= slots && p->b_qcap == qcap) return RIP_OK;
   const size_t bytes = (size_t)slots * (bm_words * 4 + (size_t)qcap * 4);
   TRY(dalloc(c, p->b_scratch, bytes));
   CK(c, cudaMemsetAsync(p->b_scratch.p, 0, (size_t)slots * bm_words * 4, c->stream));
   p->b_slots = slots;
   p->b_qcap = qcap;
   return RIP_OK;
+}
+
+// Block shape for `count` heavy sets: many sets run best one to a small block
+// (more of them in flight, fewer warps at a barrier), few need larger ones to
+// fill the device.  Sampling 400 000 sets at 2^24 vertices, weighted cascade
+// (20 000 to 60 000 heavy sets a launch): 41.7 ms with 128 threads, 44.5 with
+// 256, 55 with 512; 600 heavy sets of a 2^14-vertex graph: 1.62 ms with 512
+// threads, 1.79 with 256, 2.17 with 128, 1.93 with 1024.
+static uint32_t big_shape(const rip_pool *p, uint32_t count) {
+  if (p->big_threads) return p->big_threads;
+  const uint32_t sms = (uint32_t)p->ctx->num_sms;
+  return count >= 20 * sms ? 128 : count > 5 * sms ? 256 : count > sms ? 512 : 1024;
 }
 
 // Grows the sets first+ids[i] 64*cw at a time, each batch by the whole grid
@@ -417,30 +445,46 @@ static int sample_giant(rip_pool *p, uint64_t seed, uint64_t first,
   return RIP_OK;
 }
 
-// Grows the sets first+ids[i], one 1024-thread CTA each.
+// Grows the sets first+ids[i].
 static int sample_big(rip_pool *p, uint64_t seed, uint64_t first,
-                      const std::vector<uint32_t> &ids_in) {
-  if (ids_in.empty()) return RIP_OK;
-  if (p->giant_min && ids_in.size() >= p->giant_min) return sample_giant(p, seed, first, ids_in);
+                      const std::vector<uint32_t> &ids) {
+  if (ids.empty()) return RIP_OK;
+  if (p->giant_min && ids.size() >= p->giant_min) return sample_giant(p, seed, first, ids);
+  rip_ctx *c = p->ctx;
+  TRY(dalloc(c, p->b_ids, sizeof(uint32_t) * ids.size() * 2));
+  CK(c, cudaMemcpyAsync(p->b_ids.p, ids.data(), sizeof(uint32_t) * ids.size(),
+                        cudaMemcpyHostToDevice, c->stream));
+  return sample_big_listed(p, seed, first, (uint32_t)ids.size());
+}
+
+// The same for `count` ids in b_ids (which has room for twice as many), one
+// CTA each unless the grid-wide BFS takes them.
+static int sample_big_listed(rip_pool *p, uint64_t seed, uint64_t first, uint32_t count) {
   rip_ctx *c = p->ctx;
   rip_graph *g = p->g;
+  if (p->giant_min && count >= p->giant_min) {
+    std::vector<uint32_t> ids(count);
+    CK(c, cudaMemcpyAsync(ids.data(), p->b_ids.p, sizeof(uint32_t) * count,
+                          cudaMemcpyDeviceToHost, c->stream));
+    CK(c, cudaStreamSynchronize(c->stream));
+    std::sort(ids.begin(), ids.end());
+    return sample_giant(p, seed, first, ids);
+  }
   const uint64_t bm_words = (((uint64_t)g->n + 31) / 32 + 7) & ~7ull;
-  uint32_t qcap = p->b_qcap ? p->b_qcap : std::min<uint32_t>(g->n, 1u << 20);
+  const uint32_t qcap = p->b_qcap ? p->b_qcap : std::min<uint32_t>(g->n, 1u << 18);
   auto slots_for = [&](uint32_t q) {
     const size_t per = bm_words * 4 + (size_t)q * 4;
     size_t avail = c->budget > c->used ? c->budget - c->used : 0;
     avail += p->b_scratch.bytes;
-    // one slot per resident CTA
-    const uint64_t max_slots = (uint64_t)c->num_sms * kBigCtasPerSm((int)p->big_threads);
+    // one slot per resident CTA of the smallest shape a launch may take
+    const uint64_t max_slots =
+        (uint64_t)c->num_sms * kBigCtasPerSm(p->big_threads ? (int)p->big_threads : 128);
     return (uint32_t)std::max<uint64_t>(1, std::min<uint64_t>(max_slots, (avail / 4) / per));
   };
   TRY(ensure_big_scratch(p, slots_for(qcap), qcap));
-  std::vector<uint32_t> ids = ids_in;
+  uint32_t *ids = ptr<uint32_t>(p->b_ids), *failed = ids + count;
   PoolMeta *dm = p->dmeta();
-  for (int attempt = 0; attempt < 32 && !ids.empty(); ++attempt) {
-    TRY(dalloc(c, p->b_ids, sizeof(uint32_t) * ids.size() * 2));
-    CK(c, cudaMemcpyAsync(p->b_ids.p, ids.data(), sizeof(uint32_t) * ids.size(),
-                          cudaMemcpyHostToDevice, c->stream));
+  for (int attempt = 0; attempt < 32 && count; ++attempt) {
     CK(c, cudaMemsetAsync(&dm->fail_count, 0, sizeof(unsigned int), c->stream));
     CK(c, cudaMemsetAsync(&dm->next, 0, sizeof(unsigned int), c->stream));
     CK(c, cudaMemsetAsync(&dm->first_bad, 0xFF, sizeof(unsigned long long), c->stream));
@@ -449,17 +493,18 @@ static int sample_big(rip_pool *p, uint64_t seed, uint64_t first,
     L.P = p->view();
     L.key = make_key(seed);
     L.first = first;
-    L.count = (uint32_t)ids.size();
-    L.ids = ptr<uint32_t>(p->b_ids);
+    L.count = count;
+    L.ids = ids;
     L.next = &dm->next;
     L.bitmaps = ptr<uint32_t>(p->b_scratch);
     L.bm_words = bm_words;
     L.queues = ptr<uint32_t>(p->b_scratch) + (size_t)p->b_slots * bm_words;
     L.qcap = p->b_qcap;
-    L.F = FailList{ptr<uint32_t>(p->b_ids) + ids.size(), &dm->fail_count, &dm->first_bad};
+    L.F = FailList{failed, &dm->fail_count, &dm->first_bad};
     L.st = Stats{dm->stats};
-    L.blocks = (int)std::min<uint32_t>(p->b_slots, (uint32_t)ids.size());
-    L.threads = (int)p->big_threads;
+    L.threads = (int)big_shape(p, count);
+    L.blocks = (int)std::min<uint32_t>(
+        std::min<uint32_t>(p->b_slots, (uint32_t)(c->num_sms * kBigCtasPerSm(L.threads))), count);
     CK(c, cudaEventRecord(c->ev0, c->stream));
     launch_ic_bigset(L, c->stream);
     CK(c, cudaGetLastError());
@@ -470,7 +515,7 @@ static int sample_big(rip_pool *p, uint64_t seed, uint64_t first,
     cudaEventElapsedTime(&kms, c->ev0, c->ev1);
     p->kernel_ms += kms;
     p->kernel_launches++;
-    p->big_sets += ids.size() - m.fail_count;
+    p->big_sets += count - m.fail_count;
     if (m.fail_count == 0) {
       p->num_elems = m.cursor;
       return RIP_OK;
@@ -478,9 +523,6 @@ static int sample_big(rip_pool *p, uint64_t seed, uint64_t first,
     const unsigned long long cur = std::min<unsigned long long>(m.cursor, m.first_bad);
     CK(c, cudaMemcpyAsync(&dm->cursor, &cur, sizeof(cur), cudaMemcpyHostToDevice, c->stream));
     p->num_elems = cur;
-    std::vector<uint32_t> failed(m.fail_count);
-    CK(c, cudaMemcpyAsync(failed.data(), ptr<uint32_t>(p->b_ids) + ids.size(),
-                          sizeof(uint32_t) * m.fail_count, cudaMemcpyDeviceToHost, c->stream));
     CK(c, cudaStreamSynchronize(c->stream));
     if (m.first_bad != ~0ull) {
       TRY(ensure_elems(p, std::max<uint64_t>(p->cap * 2, cur + (1u << 20))));
@@ -490,9 +532,10 @@ static int sample_big(rip_pool *p, uint64_t seed, uint64_t first,
     } else {
       return set_err(c, RIP_ERR_DEVICE, "big-set sampler failed with full-size queues");
     }
-    ids.swap(failed);
+    std::swap(ids, failed);
+    count = m.fail_count;
   }
-  return ids.empty() ? RIP_OK : set_err(c, RIP_ERR_DEVICE, "big-set sampler did not converge");
+  return count ? set_err(c, RIP_ERR_DEVICE, "big-set sampler did not converge") : RIP_OK;
 }
 
 // ---------------------------------------------------------------------------
@@ -681,7 +724,7 @@ extern "C" int rip_graph_autotune(rip_graph *g, uint64_t seed, uint32_t pilot, d
   static const Cand cands[RIP_TUNE_CANDIDATES] = {
       {RIP_SAMPLER_PLAIN, 64, 1ull << 18, 1ull << 23, 32, 0, 1024},
       {RIP_SAMPLER_PLAIN, 64, 1ull << 14, 1ull << 23, 32, 0, 1024},
-      {RIP_SAMPLER_PLAIN, 64, 1ull << 18, 1ull << 23, 0, 0, 1024},
+      {RIP_SAMPLER_PLAIN, 64, kPlainCap, 1ull << 23, 0, 0, 0},
       {RIP_SAMPLER_FUSED, 64, 1ull << 18, 1ull << 23, 32, 0, 1024},
       {RIP_SAMPLER_FUSED, 128, 1ull << 18, 1ull << 23, 32, 0, 1024},
       {RIP_SAMPLER_FUSED, 256, 1ull << 18, 1ull << 23, 32, 0, 1024},

@@ -41,6 +41,7 @@ struct WarpCtx {
   uint32_t *bm;  // visited bitmap, ceil(n/32) words
   uint32_t *q;   // queue, qcap entries
   uint32_t qcap;
+  uint32_t *seen = nullptr;  // LT: the walk's revisit filter (shared memory)
 };
 
 // Writes the finished set to the pool (unless it overflowed) and clears the
@@ -212,80 +213,111 @@ __device__ __forceinline__ SetOutcome ic_plain_set(const DevGraph &G, Key key, c
   return SetOutcome{qlen, overflow, big, set_exp, set_edges, set_uedges, set_usrc};
 }
 
+// Revisit filter of a walk: kSeenBits bits per warp in shared memory.
+constexpr uint32_t kSeenBits = 2048;
+constexpr uint32_t kSeenWords = kSeenBits / 32;
+constexpr uint32_t kProbe = 128;  // records a search step reads, four a lane
+
 // One LT set: the single-predecessor walk from root(s) (see lt_walk_kernel).
-// A revisit is found by scanning the walk so far (the warp's queue, 32
-// entries per load, L1-resident): walks are short (tens of steps), so this
-// costs less than a visited-bitmap atomic and needs no bitmap at all.  After a
-// pick, the next vertex's offsets and (degree <= 32) its in-edges are
-// requested before the scan.
+// A step is a chain of two dependent reads: the vertex's offsets, then 128 of
+// its in-edge records, four a lane.  Lists of up to 128 edges are read whole.
+// A longer one is entered where the threshold would lie if the cumulative
+// weights grew evenly: with weights drawn independently they stray from that
+// by about sqrt(degree) / 3 edges, so consecutive records decide up to some
+// thousand edges and points a few edges apart narrow a longer list to one more
+// read; a list that strays further is split evenly in 128.  (A 32-way search
+// took two steps past 32 edges, three past 1024, four past 32 768.)  The
+// revisit test first asks a bit of a small filter, which costs no memory
+// latency, and scans the walk (the warp's queue) only when it is set.
 __device__ __forceinline__ SetOutcome lt_walk_set(const DevGraph &G, Key key, uint64_t s,
                                                   const WarpCtx &W) {
   const uint32_t lane = lane_id();
+  auto seen_hash = [](uint32_t v) { return (v * 0x9E3779B1u) >> 21; };  // 11 bits
   uint32_t cur = root_of(key, s, G.n);
-  if (lane == 0) W.q[0] = cur;
+#pragma unroll
+  for (uint32_t i = 0; i < kSeenWords; i += 32) W.seen[i + lane] = 0u;
+  __syncwarp();
+  if (lane == 0) {
+    W.q[0] = cur;
+    W.seen[seen_hash(cur) >> 5] = 1u << (seen_hash(cur) & 31);
+  }
   __syncwarp();
   uint32_t qlen = 1;
   bool overflow = false;
   unsigned long long set_exp = 0, set_edges = 0;
-  uint32_t lo = __ldg(G.off + cur), hi = __ldg(G.off + cur + 1);
-  // the current vertex's in-edges when it has at most 32 (lane j: edge lo + j)
-  bool have = false;
-  uint2 rec = make_uint2(0u, 0u);
   for (;;) {
-    set_exp += (lane == 0);
-    if (hi == lo) break;
+    const uint32_t lo = __ldg(G.off + cur), hi = __ldg(G.off + cur + 1);
     const uint32_t t = lt_threshold(key, s, cur);
-    if (!have) {
-      // 32-ary search for the first edge whose cumulative threshold exceeds t
-      bool none = false;
-      while (hi - lo > 32) {
-        const uint32_t stride = (hi - lo + 31) / 32;
-        const uint32_t p = min(lo + (lane + 1) * stride - 1, hi - 1);
-        const bool pred = t < __ldg(&G.edges[p].y);
-        const uint32_t bal = __ballot_sync(FULL, pred);
-        set_edges += (lane == 0) ? 32 : 0;
-        if (bal == 0) {  // even the last edge's cumulative weight is <= t
-          none = true;
-          break;
+    set_exp += (lane == 0);
+    // the first edge of [a, b) whose cumulative threshold exceeds t
+    uint32_t a = lo, b = hi, u = 0;
+    bool found = false, guess = true;
+    while (a < b) {
+      const uint32_t d = b - a;
+      uint32_t start = a, stride = 1;
+      if (d > kProbe) {
+        if (guess) {
+          // points kept four standard deviations to either side
+          if (d > 4096u) stride = 1u + (uint32_t)(sqrtf((float)d) * (2.5f / kProbe));
+          const uint32_t at = __umulhi(t, d), half = stride * (kProbe / 2);
+          start = a + min(at > half ? at - half : 0u, d - 1u - stride * (kProbe - 1));
+          guess = false;
+        } else {
+          stride = (d + kProbe - 1) / kProbe;
+          start = a + stride - 1;
         }
-        const uint32_t L = __ffs(bal) - 1;
-        const uint32_t nlo = lo + L * stride;
-        hi = min(hi, lo + (L + 1) * stride);
-        lo = nlo;
       }
-      if (none) break;
-      const uint32_t e = lo + lane;
-      rec = make_uint2(0u, 0u);
-      if (e < hi) rec = __ldg(&G.edges[e]);
+      uint2 rec[kProbe / 32];
+      uint32_t first = kProbe;  // the first point above t
+#pragma unroll
+      for (uint32_t i = 0; i < kProbe / 32; ++i) {
+        const uint32_t e = start + min((i * 32 + lane) * stride, b - 1 - start);
+        rec[i] = make_uint2(0u, 0u);
+        if (i * 32 < d) rec[i] = __ldg(&G.edges[e]);
+      }
+#pragma unroll
+      for (uint32_t i = 0; i < kProbe / 32; ++i) {
+        const uint32_t bal = __ballot_sync(FULL, i * 32 < d && t < rec[i].y);
+        if (bal && first == kProbe) {
+          first = i * 32 + __ffs(bal) - 1;
+          u = __shfl_sync(FULL, rec[i].x, first & 31);
+        }
+      }
+      set_edges += (lane == 0) ? min(d, kProbe) : 0;
+      if (first == kProbe) {  // every point at or below t
+        a = start + min((kProbe - 1) * stride, b - 1 - start) + 1;
+        continue;
+      }
+      const uint32_t p = start + min(first * stride, b - 1 - start);
+      const uint32_t below = first ? start + (first - 1) * stride + 1 : a;  // first not ruled out
+      if (below == p) {
+        found = true;
+        break;
+      }
+      a = below;
+      b = p + 1;
     }
-    const uint32_t bal = __ballot_sync(FULL, lo + lane < hi && t < rec.y);
-    set_edges += (lane == 0) ? (hi - lo) : 0;
-    if (bal == 0) break;  // no in-edge picked: the walk ends here
-    const uint32_t u = __shfl_sync(FULL, rec.x, __ffs(bal) - 1);
-    const uint32_t lo2 = __ldg(G.off + u), hi2 = __ldg(G.off + u + 1);
-    // u's in-edges, requested before the revisit scan
-    have = hi2 - lo2 <= 32;
-    if (have) {
-      const uint32_t e = lo2 + lane;
-      rec = make_uint2(0u, 0u);
-      if (e < hi2) rec = __ldg(&G.edges[e]);
-    }
+    if (!found) break;  // no in-edge picked: the walk ends here
+    const uint32_t h = seen_hash(u);
     bool seen = false;
-    for (uint32_t b = 0; b < qlen && !seen; b += 32) {
-      const uint32_t j = b + lane;
-      seen = __any_sync(FULL, j < qlen && W.q[j] == u);
-    }
+    if ((W.seen[h >> 5] >> (h & 31)) & 1u)
+      for (uint32_t k = 0; k < qlen && !seen; k += 32) {
+        const uint32_t j = k + lane;
+        seen = __any_sync(FULL, j < qlen && W.q[j] == u);
+      }
     if (seen) break;
     if (qlen + 1 > W.qcap) {
       overflow = true;
       break;
     }
-    if (lane == 0) W.q[qlen] = u;
+    __syncwarp();
+    if (lane == 0) {
+      W.q[qlen] = u;
+      W.seen[h >> 5] |= 1u << (h & 31);
+    }
     __syncwarp();
     ++qlen;
     cur = u;
-    lo = lo2;
-    hi = hi2;
   }
   __syncwarp();
   return SetOutcome{qlen, overflow, false, set_exp, set_edges};
@@ -343,22 +375,19 @@ ic_plain_kernel(DevGraph G, DevPool P, Key key, const __grid_constant__ RoundKey
   }
 }
 
-// One walk per warp.  Each step needs the chosen in-edge of the current
-// vertex: a 32-ary search over the cumulative thresholds (one probe per lane
-// per round, log32(in-degree) rounds), finishing with one 8-byte load per lane
-// so the lane that holds the pick also holds its source id.  Walks are chains
-// of dependent loads; the kernel is bound to 32 registers (up to 64 resident
-// warps per SM) and the host launches 32 warps per SM: a launch lasts about
-// as long as its longest walk either way, and the free warp slots serve
-// other queries' kernels.
-__global__ void __launch_bounds__(256, 8)
+// One walk per warp (lt_walk_set).  Walks are chains of dependent loads; a
+// launch lasts about as long as its longest walk, so the host launches 32 warps
+// per SM and the free warp slots serve other queries' kernels.
+__global__ void __launch_bounds__(256, 5)
 lt_walk_kernel(DevGraph G, DevPool P, Key key, uint64_t first, uint32_t count,
                const uint32_t *ids, unsigned int *next, uint32_t *bitmaps,
                uint64_t bm_words, uint32_t *queues, uint32_t qcap, FailList F,
                Stats st) {
   const uint32_t lane = lane_id();
   const uint64_t w = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  WarpCtx W{bitmaps + w * bm_words, queues + w * (uint64_t)qcap, qcap};
+  __shared__ uint32_t s_seen[8][kSeenWords];
+  WarpCtx W{bitmaps + w * bm_words, queues + w * (uint64_t)qcap, qcap,
+            s_seen[threadIdx.x >> 5]};
   unsigned long long n_exp = 0, n_edges = 0, n_sets = 0, n_elems = 0;
 
   for (;;) {
@@ -398,7 +427,9 @@ __global__ void __launch_bounds__(256)
 multi_sample_kernel(MultiLaunch L) {
   const uint32_t lane = lane_id();
   const uint64_t w = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  WarpCtx W{L.bitmaps + w * L.bm_words, L.queues + w * (uint64_t)L.qcap, L.qcap};
+  __shared__ uint32_t s_seen[8][kSeenWords];
+  WarpCtx W{L.bitmaps + w * L.bm_words, L.queues + w * (uint64_t)L.qcap, L.qcap,
+            s_seen[threadIdx.x >> 5]};
   // counters of the instance the warp is on, flushed when it moves on
   uint32_t cur = ~0u;
   unsigned long long n_exp = 0, n_edges = 0, n_sets = 0, n_elems = 0, n_uedges = 0, n_usrc = 0;

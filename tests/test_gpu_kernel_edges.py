@@ -104,3 +104,36 @@ def test_reference_heap_keeps_more_items(ctx, k, hot):
         f, seeds, gains = p.select(k, tiebreak=rb.TIE_REF_HEAP)
         assert f == of and seeds.tolist() == oseeds.tolist() and gains.tolist() == ogains.tolist()
     dg.close()
+
+
+def star_graph(degrees, weights, n=30000, seed=11):
+    """Vertex v < len(degrees) has degrees[v] in-edges, the others one from a
+    small vertex; weights 'equal', 'random', 'skewed' or 'short' (sum 0.5)."""
+    r = np.random.RandomState(seed)
+    lists, w = [], []
+    for v in range(n):
+        d = degrees[v] if v < len(degrees) else 1
+        s = r.randint(0, len(degrees) if v >= len(degrees) or r.rand() < 0.3 else n, d)
+        x = {"equal": np.ones(d), "random": r.rand(d) + 1e-9, "short": np.ones(d),
+             "skewed": np.where(r.rand(d) < 0.02, 1.0, 1e-5)}[weights]
+        lists.append(np.sort(s).astype(np.uint32))
+        w.append((x / x.sum() * (0.5 if weights == "short" else 1.0)).astype(np.float32))
+    index = np.zeros(n + 1, dtype=np.uint64)
+    np.cumsum([len(x) for x in lists], out=index[1:])
+    return rb.HostGraph(n, index, np.concatenate(lists), np.concatenate(w))
+
+
+@pytest.mark.parametrize("weights", ["equal", "random", "skewed", "short"])
+def test_lt_walk_search_over_list_lengths(ctx, weights):
+    # read whole up to 128 edges, one guessed read up to 4096, then two
+    g = star_graph([1, 2, 31, 32, 33, 127, 128, 129, 160, 1023, 1024, 1025, 4095, 4096, 4097,
+                    9000, 20000], weights)
+    dg = rb.DeviceGraph(ctx, g, "LT")
+    assert np.array_equal(dg.thresholds(), O.pack("LT", g.index, g.weights))
+    p = rb.Pool(dg)
+    p.sample(6000, seed=3)
+    off, vtx = p.export()
+    ooff, ovtx, ost = O.sample("LT", g.n, g.index, g.src, O.pack("LT", g.index, g.weights), 3, 0,
+                               6000)
+    assert np.array_equal(off, ooff) and np.array_equal(vtx, ovtx) and p.stats()[4] == ost[0]
+    dg.close()

@@ -30,6 +30,8 @@
 // the whole block.
 #include <algorithm>
 
+#include <cooperative_groups.h>
+
 #include "device.cuh"
 #include "launch.h"
 
@@ -48,14 +50,15 @@ constexpr uint32_t NONE = 0xFFFFFFFFu;
 // Sets of at least this many elements are walked by their whole block, 1024
 // elements at a step; the others by the warp that met them.
 constexpr uint32_t kLongSet = 512;
-constexpr uint32_t kBlock = 256;  // threads of every per-set kernel
-constexpr uint32_t kBlockWarps = kBlock / 32;
+constexpr uint32_t kBlock = 256;  // threads of the per-set kernels
 
-struct LongSets {  // shared: the long sets a block met in one step
-  uint64_t set[kBlock], off[kBlock];
-  uint32_t len[kBlock];
+template <uint32_t THREADS>
+struct LongSetsOf {  // shared: the long sets a block met in one step
+  uint64_t set[THREADS], off[THREADS];
+  uint32_t len[THREADS];
   uint32_t n;
 };
+using LongSets = LongSetsOf<kBlock>;
 
 // Calls the grid over the elements of sets set_of(i), i in [lo, hi) (~0: none).
 // A warp takes up to 32 sets a step -- fewer when that leaves warps idle: a
@@ -65,18 +68,19 @@ struct LongSets {  // shared: the long sets a block met in one step
 // warp, so it may use warp collectives.  Elements of a set of kLongSet or more
 // are spread over the block: single(set, vertex), no collectives.  One warp
 // walking a set of 40 000 elements alone took 0.5 ms; a block takes 15 us.
-template <typename SetOf, typename Mixed, typename Single>
+template <uint32_t THREADS, typename SetOf, typename Mixed, typename Single>
 __device__ __forceinline__ void block_elements(const DevPool &P, uint64_t lo, uint64_t hi,
-                                               LongSets &sh, SetOf set_of, Mixed mixed,
-                                               Single single) {
+                                               LongSetsOf<THREADS> &sh, SetOf set_of,
+                                               Mixed mixed, Single single) {
+  constexpr uint32_t WARPS = THREADS / 32;
   const uint32_t lane = lane_id(), wid = threadIdx.x >> 5;
   if (hi <= lo) return;
-  const uint64_t warps = (uint64_t)gridDim.x * kBlockWarps;
+  const uint64_t warps = (uint64_t)gridDim.x * WARPS;
   const uint64_t per = (hi - lo + warps - 1) / warps;
   const uint32_t take = per < 32 ? (uint32_t)per : 32u;  // sets a warp takes a step
   if (threadIdx.x == 0) sh.n = 0;
   __syncthreads();
-  for (uint64_t base = lo + (uint64_t)blockIdx.x * kBlockWarps * take; base < hi;
+  for (uint64_t base = lo + (uint64_t)blockIdx.x * WARPS * take; base < hi;
        base += warps * take) {
     const uint64_t i = base + wid * take + lane;
     uint64_t s = 0, off = 0;
@@ -122,14 +126,14 @@ __device__ __forceinline__ void block_elements(const DevPool &P, uint64_t lo, ui
         const uint64_t ks = sh.set[k];
         const uint32_t *vtx = P.vtx + sh.off[k];
         const uint32_t klen = sh.len[k];
-        for (uint32_t j = threadIdx.x; j < klen; j += 4 * kBlock) {
+        for (uint32_t j = threadIdx.x; j < klen; j += 4 * THREADS) {
           uint32_t v[4];
 #pragma unroll
           for (int h = 0; h < 4; ++h)
-            if (j + h * kBlock < klen) v[h] = vtx[j + h * kBlock];
+            if (j + h * THREADS < klen) v[h] = vtx[j + h * THREADS];
 #pragma unroll
           for (int h = 0; h < 4; ++h)
-            if (j + h * kBlock < klen) single(ks, v[h]);
+            if (j + h * THREADS < klen) single(ks, v[h]);
         }
       }
       __syncthreads();
@@ -430,6 +434,13 @@ __global__ void __launch_bounds__(kBlock) cover_gather_kernel(CoverLaunch C, con
 // each; a cover marks the chunks it decrements dirty and the next pick
 // re-reads only those, then reduces the chunk maxima in the last block.
 constexpr uint32_t SEL_CHUNK = 1024;
+constexpr uint32_t kLoopCtas = 8, kLoopThreads = 512;
+constexpr uint32_t kLoopChunks = 2048;  // chunk maxima a block keeps
+// Elements of a round up to which one cluster makes all its picks: the two
+// rounds just below it of a weighted-cascade query on 2^20 Erdos-Renyi vertices
+// took 3.5 ms this way and 3.7 grid-wide; far above it the first covers alone
+// keep eight SMs busy longer than the grid takes for all picks.
+constexpr double kLoopElements = 8.0 * (1 << 20);
 
 __device__ __forceinline__ unsigned long long sel_key(uint32_t c, uint32_t v) {
   return ((unsigned long long)c << 32) | (unsigned long long)(~v);
@@ -479,6 +490,34 @@ __global__ void __launch_bounds__(kBlock) sel_count_kernel(const SelDesc *__rest
   if (lane_id() == 0 && elems) atomicAdd(d.acc + 2, elems);
 }
 
+// Whether a pick's cover recounts: its g sets hold about g x the mean
+// uncovered set size; when that outweighs the rest, recounting the rest is
+// less work than decrementing (either way the counts are exact).
+__device__ __forceinline__ bool sel_recounts(unsigned long long g, unsigned long long left,
+                                             unsigned long long sets, uint32_t n) {
+  const unsigned long long est =
+      sets ? (unsigned long long)((double)g * (double)left / (double)sets) : 0ull;
+  return est > (left > est ? left - est : 0ull) + n / 4;
+}
+
+// The largest key of chunk c's counts (a warp).
+__device__ __forceinline__ unsigned long long sel_chunk_max(const SelDesc &d, uint64_t c) {
+  const uint32_t lane = lane_id();
+  const uint4 *src = reinterpret_cast<const uint4 *>(d.count + c * SEL_CHUNK);
+  unsigned long long key = 0;
+#pragma unroll
+  for (uint32_t j = 0; j < SEL_CHUNK / 128; ++j) {
+    const uint32_t q = j * 32 + lane;
+    const uint4 x = __ldcg(src + q);
+    const uint32_t v = (uint32_t)(c * SEL_CHUNK) + 4 * q;
+    key = umax64(key, umax64(umax64(sel_key(x.x, v), sel_key(x.y, v + 1)),
+                             umax64(sel_key(x.z, v + 2), sel_key(x.w, v + 3))));
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) key = umax64(key, __shfl_xor_sync(FULL, key, o));
+  return key;
+}
+
 // Pick i: refresh the dirty chunk maxima (one warp per chunk), then the last
 // block to finish reduces all chunk maxima into best[i].
 __global__ void __launch_bounds__(256) sel_pick_kernel(const SelDesc *__restrict__ dp,
@@ -492,18 +531,7 @@ __global__ void __launch_bounds__(256) sel_pick_kernel(const SelDesc *__restrict
   const uint64_t nw = ((uint64_t)gridDim.x * blockDim.x) >> 5;
   for (uint64_t c = gw; c < d.nchunks; c += nw) {
     if (!d.dirty[c]) continue;  // warp-uniform
-    const uint4 *src = reinterpret_cast<const uint4 *>(d.count + c * SEL_CHUNK);
-    unsigned long long key = 0;
-#pragma unroll
-    for (uint32_t j = 0; j < SEL_CHUNK / 128; ++j) {
-      const uint32_t q = j * 32 + lane;
-      const uint4 x = __ldcg(src + q);
-      const uint32_t v = (uint32_t)(c * SEL_CHUNK) + 4 * q;
-      key = umax64(key, umax64(umax64(sel_key(x.x, v), sel_key(x.y, v + 1)),
-                               umax64(sel_key(x.z, v + 2), sel_key(x.w, v + 3))));
-    }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) key = umax64(key, __shfl_xor_sync(FULL, key, o));
+    const unsigned long long key = sel_chunk_max(d, c);
     if (lane == 0) {
       d.cmax[c] = key;
       d.dirty[c] = 0;
@@ -527,14 +555,8 @@ __global__ void __launch_bounds__(256) sel_pick_kernel(const SelDesc *__restrict
     for (int w = 0; w < (int)(blockDim.x >> 5); ++w) b = umax64(b, s_red[w]);
     d.best[i] = b;
     *d.done_blocks = 0;
-    // how the cover of this pick runs: its g sets hold about g x the mean
-    // uncovered set size; when that outweighs the rest, recounting the rest
-    // is less work than decrementing (either way the counts are exact)
     const unsigned long long g = b >> 32, left = d.acc[2], sets = d.acc[3];
-    const unsigned long long est = sets ? (unsigned long long)((double)g * (double)left /
-                                                               (double)sets)
-                                        : 0ull;
-    d.acc[4] = (est > (left > est ? left - est : 0ull) + d.n / 4) ? 1ull : 0ull;
+    d.acc[4] = sel_recounts(g, left, sets, d.n) ? 1ull : 0ull;  // how the cover of this pick runs
     d.acc[3] = sets > g ? sets - g : 0ull;
   }
 }
@@ -547,6 +569,75 @@ __global__ void __launch_bounds__(256) sel_pick_kernel(const SelDesc *__restrict
 // the covered sets' elements from acc[2] (elements of uncovered sets).
 constexpr uint32_t kDirtyShared = 4096;  // chunks whose dirty flags a block gathers first
 
+// Decrement mode: marks v's uncovered sets in [0, S) covered and takes them out
+// of the counts; adds their elements to `elems` (per thread).  The chunks a
+// block touches are flagged in shared memory and written out once (one byte
+// store per element otherwise).
+template <uint32_t THREADS>
+__device__ __forceinline__ void sel_cover_sets(const SelDesc *__restrict__ dp, const SelDesc &d,
+                                               uint32_t v, LongSetsOf<THREADS> &sh,
+                                               uint8_t *s_dirty, unsigned long long &elems) {
+  const bool local = d.nchunks <= kDirtyShared;
+  if (local)
+    for (uint32_t x = threadIdx.x; x < d.nchunks; x += THREADS) s_dirty[x] = 0;
+  auto take = [&](uint32_t u) {
+    if (u == v) return;  // in every set of the list: written once, below
+    atomicSub(d.count + u, 1u);
+    if (local) s_dirty[u / SEL_CHUNK] = 1;
+    else d.dirty[u / SEL_CHUNK] = 1;
+  };
+  for (uint32_t g = 0; g < d.nseg; ++g) {
+    if (dp->seg_first[g] >= d.S) continue;  // the segment's sets are all >= S
+    const uint64_t lo = dp->seg_off[g][v], hi = dp->seg_off[g][v + 1];
+    const uint32_t *inv = dp->seg_inv[g];
+    __syncthreads();
+    block_elements(
+        d.P, lo, hi, sh,
+        [&](uint64_t j) -> uint64_t {
+          const uint32_t s = inv[j];
+          if (s >= d.S || __ldcg(d.covered + s)) return ~0ull;
+          d.covered[s] = 1;  // s holds v once: no other lane has s
+          elems += d.P.set_len[s];
+          return s;
+        },
+        [&](uint64_t, uint32_t u, bool valid) {
+          if (valid) take(u);
+        },
+        [&](uint64_t, uint32_t u) { take(u); });
+  }
+  if (blockIdx.x == 0 && threadIdx.x == 0) {  // every set of [0, S) that held v is covered now
+    d.count[v] = 0u;
+    d.dirty[v / SEL_CHUNK] = 1;
+  }
+  __syncthreads();
+  if (local)
+    for (uint32_t x = threadIdx.x; x < d.nchunks; x += THREADS)
+      if (s_dirty[x]) d.dirty[x] = 1;
+}
+
+// Recount mode, first half: marks v's uncovered sets, clears the counts and
+// flags every chunk.
+__device__ __forceinline__ void sel_mark_sets(const SelDesc *__restrict__ dp, const SelDesc &d,
+                                              uint32_t v, unsigned long long &elems) {
+  const uint64_t tid = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
+  const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
+  uint4 *c4 = reinterpret_cast<uint4 *>(d.count);
+  const uint64_t n4 = (uint64_t)d.nchunks * (SEL_CHUNK / 4);
+  for (uint64_t x = tid; x < n4; x += stride) c4[x] = make_uint4(0, 0, 0, 0);
+  for (uint64_t x = tid; x < d.nchunks; x += stride) d.dirty[x] = 1;
+  for (uint32_t g = 0; g < d.nseg; ++g) {
+    if (dp->seg_first[g] >= d.S) continue;
+    const uint64_t lo = dp->seg_off[g][v], hi = dp->seg_off[g][v + 1];
+    for (uint64_t j = lo + tid; j < hi; j += stride) {  // one thread per entry: mark only
+      const uint32_t s = dp->seg_inv[g][j];
+      if (s < d.S && !__ldcg(d.covered + s)) {  // s holds v once: no other thread has s
+        d.covered[s] = 1;
+        elems += d.P.set_len[s];
+      }
+    }
+  }
+}
+
 __global__ void __launch_bounds__(kBlock) sel_cover_kernel(const SelDesc *__restrict__ dp,
                                                            uint32_t i) {
   __shared__ LongSets sh;
@@ -555,69 +646,92 @@ __global__ void __launch_bounds__(kBlock) sel_cover_kernel(const SelDesc *__rest
   const unsigned long long b = d.best[i];
   if ((b >> 32) == 0) return;
   const uint32_t v = ~(uint32_t)(b & 0xFFFFFFFFull);
-  const bool recount = d.acc[4] != 0ull;
-  const uint64_t tid = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
-  const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
-  const uint32_t lane = lane_id();
   unsigned long long elems = 0;
-  if (recount) {
-    uint4 *c4 = reinterpret_cast<uint4 *>(d.count);
-    const uint64_t n4 = (uint64_t)d.nchunks * (SEL_CHUNK / 4);
-    for (uint64_t x = tid; x < n4; x += stride) c4[x] = make_uint4(0, 0, 0, 0);
-    for (uint64_t x = tid; x < d.nchunks; x += stride) d.dirty[x] = 1;
-    for (uint32_t g = 0; g < d.nseg; ++g) {
-      if (dp->seg_first[g] >= d.S) continue;  // the segment's sets are all >= S
-      const uint64_t lo = dp->seg_off[g][v], hi = dp->seg_off[g][v + 1];
-      for (uint64_t j = lo + tid; j < hi; j += stride) {  // one thread per entry: mark only
-        const uint32_t s = dp->seg_inv[g][j];
-        if (s < d.S && !d.covered[s]) {  // s holds v once: no other thread has s
-          d.covered[s] = 1;
-          elems += d.P.set_len[s];
-        }
+  if (d.acc[4] != 0ull) sel_mark_sets(dp, d, v, elems);
+  else sel_cover_sets(dp, d, v, sh, s_dirty, elems);
+  elems = warp_sum_u64(elems);
+  if (lane_id() == 0 && elems) atomicAdd(d.acc + 2, (unsigned long long)0 - elems);  // acc[2] -= elems
+}
+
+// Every pick of a round in one launch: one cluster of kLoopCtas blocks, which
+// meet at cluster barriers instead of kernel boundaries.  Small rounds spend
+// their time between launches: a pick, its cover and the (idle) recount took
+// some 25 us a pick, three launches of a captured graph; here a pick is two
+// cluster barriers and about ten dependent reads, 15 us (twelve queries on six
+// graphs of 4 K to 65 K vertices as one batch: 139 -> 130 ms).  A cluster's
+// eight SMs cannot keep up with a round of many elements, which stays with the
+// grid-wide kernels (kLoopElements).  A block keeps the maxima of every
+// kLoopCtas-th chunk in
+// shared memory and re-reads those a cover flagged.
+__global__ void __cluster_dims__(kLoopCtas, 1, 1) __launch_bounds__(kLoopThreads, 2)
+sel_loop_kernel(const SelDesc *__restrict__ dp) {
+  namespace cg = cooperative_groups;
+  constexpr uint32_t WARPS = kLoopThreads / 32;
+  __shared__ LongSetsOf<kLoopThreads> sh;
+  __shared__ uint8_t s_dirty[kDirtyShared];
+  __shared__ unsigned long long s_cmax[kLoopChunks];
+  __shared__ unsigned long long s_red[WARPS], s_key, s_elems;
+  const SelDesc d = *dp;
+  cg::cluster_group cluster = cg::this_cluster();
+  const uint32_t rank = blockIdx.x, lane = lane_id(), wid = threadIdx.x >> 5;
+  const uint32_t own = d.nchunks > rank ? (d.nchunks - rank + kLoopCtas - 1) / kLoopCtas : 0;
+  // elements of the uncovered sets, and those sets: the same in every block
+  unsigned long long left = __ldcg(d.acc + 2), sets = __ldcg(d.acc + 3);
+  auto block_max = [&](unsigned long long key) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) key = umax64(key, __shfl_xor_sync(FULL, key, o));
+    if (lane == 0) s_red[wid] = key;
+    __syncthreads();
+    if (wid == 0) {
+      key = lane < WARPS ? s_red[lane] : 0ull;
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) key = umax64(key, __shfl_xor_sync(FULL, key, o));
+      if (lane == 0) s_key = key;
+    }
+  };
+  for (uint32_t i = 0; i < d.k; ++i) {
+    for (uint32_t j = wid; j < own; j += WARPS) {
+      const uint32_t c = rank + j * kLoopCtas;
+      if (!__ldcg(d.dirty + c)) continue;  // warp-uniform; all are at the start
+      const unsigned long long key = sel_chunk_max(d, c);
+      if (lane == 0) {
+        s_cmax[j] = key;
+        d.dirty[c] = 0;
       }
     }
-  } else {
-    // the chunks a block touches are flagged in shared memory and written out
-    // once (one byte store per element otherwise)
-    const bool local = d.nchunks <= kDirtyShared;
-    if (local)
-      for (uint32_t x = threadIdx.x; x < d.nchunks; x += kBlock) s_dirty[x] = 0;
-    auto take = [&](uint32_t u) {
-      if (u == v) return;  // in every set of the list: written once, below
-      atomicSub(d.count + u, 1u);
-      if (local) s_dirty[u / SEL_CHUNK] = 1;
-      else d.dirty[u / SEL_CHUNK] = 1;
-    };
-    for (uint32_t g = 0; g < d.nseg; ++g) {
-      if (dp->seg_first[g] >= d.S) continue;
-      const uint64_t lo = dp->seg_off[g][v], hi = dp->seg_off[g][v + 1];
-      const uint32_t *inv = dp->seg_inv[g];
-      __syncthreads();
+    __syncthreads();
+    unsigned long long key = 0;
+    for (uint32_t j = threadIdx.x; j < own; j += kLoopThreads) key = umax64(key, s_cmax[j]);
+    block_max(key);
+    cluster.sync();
+    key = lane < kLoopCtas ? *cluster.map_shared_rank(&s_key, lane) : 0ull;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) key = umax64(key, __shfl_xor_sync(FULL, key, o));
+    if (rank == 0 && threadIdx.x == 0) d.best[i] = key;
+    const unsigned long long g = key >> 32;
+    if (g == 0 || i + 1 == d.k) break;  // the same in every block
+    const uint32_t v = ~(uint32_t)(key & 0xFFFFFFFFull);
+    unsigned long long elems = 0;
+    if (threadIdx.x == 0) s_elems = 0;
+    if (sel_recounts(g, left, sets, d.n)) {
+      sel_mark_sets(dp, d, v, elems);
+      cluster.sync();  // every set marked, every count cleared
       block_elements(
-          d.P, lo, hi, sh,
-          [&](uint64_t j) -> uint64_t {
-            const uint32_t s = inv[j];
-            if (s >= d.S || d.covered[s]) return ~0ull;
-            d.covered[s] = 1;  // s holds v once: no other lane has s
-            elems += d.P.set_len[s];
-            return s;
-          },
-          [&](uint64_t, uint32_t u, bool valid) {
-            if (valid) take(u);
-          },
-          [&](uint64_t, uint32_t u) { take(u); });
-    }
-    if (tid == 0) {  // every set of [0, S) that held v is covered now
-      d.count[v] = 0u;
-      d.dirty[v / SEL_CHUNK] = 1;
+          d.P, 0, d.S, sh, [&](uint64_t x) -> uint64_t { return __ldcg(d.covered + x) ? ~0ull : x; },
+          [&](uint64_t s, uint32_t u, bool valid) { add_occurrence(d.count, s, u, valid); },
+          [&](uint64_t, uint32_t u) { atomicAdd(d.count + u, 1u); });
+    } else {
+      sel_cover_sets(dp, d, v, sh, s_dirty, elems);
     }
     __syncthreads();
-    if (local)
-      for (uint32_t x = threadIdx.x; x < d.nchunks; x += kBlock)
-        if (s_dirty[x]) d.dirty[x] = 1;
+    elems = warp_sum_u64(elems);
+    if (lane == 0 && elems) atomicAdd(&s_elems, elems);
+    cluster.sync();  // the cover is done
+    elems = lane < kLoopCtas ? *cluster.map_shared_rank(&s_elems, lane) : 0ull;
+    left -= warp_sum_u64(elems);
+    sets = sets > g ? sets - g : 0ull;
   }
-  elems = warp_sum_u64(elems);
-  if (lane == 0 && elems) atomicAdd(d.acc + 2, (unsigned long long)0 - elems);  // acc[2] -= elems
+  cluster.sync();  // no block leaves while another may read its shared memory
 }
 
 // Recount mode only: count the members of every set in [0, S) still
@@ -1008,6 +1122,13 @@ void launch_sel_cover(const SelDesc *d, uint32_t i, int blocks, cudaStream_t str
   count_launches(2);
   sel_cover_kernel<<<blocks, kBlock, 0, stream>>>(d, i);
   sel_recount_kernel<<<blocks, kBlock, 0, stream>>>(d);
+}
+void launch_sel_loop(const SelDesc *d, cudaStream_t stream) {
+  count_launches(1);
+  sel_loop_kernel<<<kLoopCtas, kLoopThreads, 0, stream>>>(d);
+}
+bool sel_loop_fits(uint32_t nchunks, double elements) {
+  return nchunks <= kLoopCtas * kLoopChunks && elements <= kLoopElements;
 }
 uint32_t sel_chunk_vertices() { return SEL_CHUNK; }
 

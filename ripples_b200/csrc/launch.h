@@ -299,6 +299,10 @@ void launch_sel_pick(const SelDesc *d, uint32_t i, int blocks, cudaStream_t stre
 // when they hold more elements than every set still uncovered -- recounts the
 // uncovered sets (2 launches; the pick decides which, on the device).
 void launch_sel_cover(const SelDesc *d, uint32_t i, int blocks, cudaStream_t stream);
+// All of a round's picks and covers in one launch, after sel_init (and
+// sel_count): for rounds sel_loop_fits, by chunks and elements of sets [0, S).
+void launch_sel_loop(const SelDesc *d, cudaStream_t stream);
+bool sel_loop_fits(uint32_t nchunks, double elements);
 uint32_t sel_chunk_vertices();
 // out[i] = count[ids[i]], i < m (ids and out 16-byte aligned)
 void launch_gather_counts(const uint32_t *count, const uint32_t *ids, uint32_t m,

@@ -42,8 +42,6 @@ struct SelSlot {
   std::vector<std::pair<uint64_t, std::pair<cudaGraphExec_t, uint64_t>>> execs;
 };
 constexpr size_t MAX_GRAPHS_PER_SLOT = 8;
-// rounds over more elements than this run on full-occupancy grids
-constexpr double WIDE_ROUND_ELEMENTS = 64.0 * 1024 * 1024;
 // queued queries looked at per tick for admission
 constexpr size_t MAX_ADMISSION_SCAN = 1024;
 
@@ -257,12 +255,23 @@ int launch_round(rip_server *s, Active &a) {
   hd->acc = reinterpret_cast<unsigned long long *>(ptr<uint8_t>(sl.ctr) + 64);
   hd->total_elems = 0;
   CK(c, cudaMemcpyAsync(sl.desc.p, hd, sizeof(SelDesc), cudaMemcpyHostToDevice, sl.st));
-  // Rounds over many elements take full-occupancy grids for the count and
-  // the covers (one such round fills the device by itself); small rounds
-  // keep small grids so that many slots' rounds share the device.  The
-  // captured rounds are keyed by k and the grid class.
-  const bool wide = mean_set_size(p) * (double)a.S > WIDE_ROUND_ELEMENTS;
-  const uint64_t key = (uint64_t)k | (wide ? 1ull << 32 : 0ull);
+  // Small rounds: one cluster makes every pick.  The others' counts and covers
+  // take full-occupancy grids (74 blocks, meant to leave room for other slots'
+  // rounds, let one cover of a round of 60 M elements run 9 ms).  The captured
+  // rounds are keyed by k.
+  const double elements = mean_set_size(p) * (double)a.S;
+  if (sel_loop_fits(nchunks, elements)) {
+    const SelDesc *d = ptr<SelDesc>(sl.desc);
+    const int blocks = std::max(8, c->num_sms / 2);
+    launch_sel_init(d, blocks, sl.st);
+    launch_sel_count(d, blocks * 2, sl.st);
+    launch_sel_loop(d, sl.st);
+    CK(c, cudaGetLastError());
+    CK(c, cudaMemcpyAsync(sl.h_best.p, sl.best.p, (size_t)k * 8, cudaMemcpyDeviceToHost, sl.st));
+    s->graph_launches++;
+    return RIP_OK;
+  }
+  const uint64_t key = k;
   size_t gi = 0;
   while (gi < sl.execs.size() && sl.execs[gi].first != key) ++gi;
   if (gi == sl.execs.size()) {
@@ -272,8 +281,8 @@ int launch_round(rip_server *s, Active &a) {
     }
     const SelDesc *d = ptr<SelDesc>(sl.desc);
     const int blocks = std::max(8, c->num_sms / 2);
-    const int count_blocks = wide ? c->num_sms * 8 : blocks * 2;
-    const int cover_blocks = wide ? c->num_sms * 4 : blocks;
+    const int count_blocks = c->num_sms * 8;
+    const int cover_blocks = c->num_sms * 4;
     const uint64_t before = launch_counter();
     cudaGraph_t g = nullptr;
     CK(c, cudaStreamBeginCapture(sl.st, cudaStreamCaptureModeThreadLocal));

@@ -137,3 +137,27 @@ def test_lt_walk_search_over_list_lengths(ctx, weights):
                                6000)
     assert np.array_equal(off, ooff) and np.array_equal(vtx, ovtx) and p.stats()[4] == ost[0]
     dg.close()
+
+
+@pytest.mark.parametrize("copies", [1, 25])
+def test_device_picks_in_one_launch_and_grid_wide(ctx, copies):
+    """Lowest-id picks by one cluster (up to 8 M elements) and by the grid-wide
+    kernels (here 8.8 M): giant first covers (recounts) and small ones, ties."""
+    n, r = 20011, np.random.RandomState(7)
+    sets = [np.unique(np.concatenate([[5], r.randint(0, n, 6000)])) for _ in range(60)]
+    sets += [r.choice(n, 1 + i % 40, replace=False) for i in range(2000)]
+    sets = sets * copies
+    off = np.zeros(len(sets) + 1, dtype=np.uint64)
+    np.cumsum([len(x) for x in sets], out=off[1:])
+    vtx = np.concatenate(sets).astype(np.uint32)
+    assert (len(vtx) > 8 << 20) == (copies > 1)
+    g = rb.HostGraph(n, np.zeros(n + 1, np.uint64), np.zeros(0, np.uint32), np.zeros(0, np.float32))
+    dg = rb.DeviceGraph(ctx, g, "IC")
+    p = rb.Pool(dg)
+    p.import_sets(off, vtx)
+    for s, k in ((len(sets), 40), (len(sets) - 777, 3), (61, 9)):
+        e = int(off[s])
+        of, oseeds, ogains, _ = O.select(n, off[: s + 1], vtx[:e], k, rb.TIE_LOWEST_ID)
+        f, seeds, gains = p.select(k, s, rb.TIE_LOWEST_ID)
+        assert f == of and seeds.tolist() == oseeds.tolist() and gains.tolist() == ogains.tolist()
+    dg.close()

@@ -55,58 +55,117 @@ __device__ __forceinline__ uint64_t sat_add(uint64_t a, uint64_t b) {
   return s > (1ull << 41) ? (1ull << 41) : s;
 }
 
-// One warp per vertex: coalesced 32-edge chunks, a saturating integer warp
-// scan per chunk, carried across chunks.
-__global__ void pack_lt_kernel(const uint64_t *index, const uint32_t *src,
-                               const float *w, uint32_t n, uint64_t m,
-                               uint64_t m_pad, uint2 *edges) {
-  const uint32_t lane = threadIdx.x & 31u;
-  const uint64_t gw = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5;
-  const uint64_t nw = ((uint64_t)gridDim.x * blockDim.x) >> 5;
-  // 32 consecutive vertices per warp: a lane scans its own vertex when it has
-  // at most 32 in-edges (most vertices); the warp scans each larger one
-  // together, 32 edges per step with a shuffle scan
-  for (uint64_t v0 = gw * 32; v0 < n; v0 += nw * 32) {
-    const uint64_t v = v0 + lane;
+__device__ __forceinline__ uint2 lt_record(uint32_t src, uint64_t sum) {
+  const uint64_t c = sum >> 8;
+  return make_uint2(src, c > 0xFFFFFFFFull ? 0xFFFFFFFFu : (uint32_t)c);
+}
+
+// In-lists of at least this many edges are scanned by their whole block.
+constexpr uint32_t kPackLong = 1024;
+
+// A warp takes 32 consecutive vertices, whose edges lie side by side: 32 edges
+// a step, a saturating scan by shuffles that starts anew at every list's first
+// edge.  Long lists are listed (*nlong, longs) for pack_lt_long_kernel.  One
+// kernel that left a hub to its warp took 1.43 ms of the upload of an R-MAT graph
+// with 2^18 vertices and 4 M edges (lists of 30 000, a dependent chain of 32-edge
+// steps; hubs sit side by side); the two take 0.67 ms.
+__global__ void __launch_bounds__(256)
+pack_lt_kernel(const uint64_t *index, const uint32_t *src, const float *w, uint32_t n, uint64_t m,
+               uint64_t m_pad, uint2 *edges, unsigned int *nlong, uint32_t *longs_out) {
+  const uint32_t lane = threadIdx.x & 31u, wid = threadIdx.x >> 5;
+  for (uint64_t v0 = (uint64_t)blockIdx.x * 256; v0 < n; v0 += (uint64_t)gridDim.x * 256) {
+    const uint64_t v = v0 + threadIdx.x;
     uint64_t beg = 0, end = 0;
     if (v < n) {
       beg = index[v];
       end = index[v + 1];
     }
-    if (end - beg <= 32) {
-      uint64_t run = 0;
-      for (uint64_t e = beg; e < end; ++e) {
-        run = sat_add(run, lt_fixed(w[e]));
-        const uint64_t c = run >> 8;
-        edges[e] = make_uint2(src[e], c > 0xFFFFFFFFull ? 0xFFFFFFFFu : (uint32_t)c);
+    const bool lng = end - beg >= kPackLong;
+    if (lng) longs_out[atomicAdd(nlong, 1u)] = (uint32_t)v;
+    // the warp's range, in steps of 32 edges between its long lists
+    const uint64_t wv = v0 + wid * 32;
+    const uint64_t first = __shfl_sync(0xFFFFFFFFu, beg, 0);
+    const uint64_t last = wv < n ? __shfl_sync(0xFFFFFFFFu, end, (uint32_t)min((uint64_t)31, n - 1 - wv))
+                                 : first;
+    const uint32_t longs = __ballot_sync(0xFFFFFFFFu, lng);
+    uint64_t carry = 0;
+    for (uint64_t base = first; base < last;) {
+      uint64_t stop = base + 32 < last ? base + 32 : last;
+      bool skip = false;
+      for (uint32_t l = longs; l; l &= l - 1) {  // (few warps have one)
+        const uint64_t hb = __shfl_sync(0xFFFFFFFFu, beg, __ffs(l) - 1);
+        const uint64_t he = __shfl_sync(0xFFFFFFFFu, end, __ffs(l) - 1);
+        if (base >= hb && base < he) {
+          base = he;
+          skip = true;
+          break;
+        }
+        if (hb > base && hb < stop) stop = hb;
       }
-    }
-    uint32_t big = __ballot_sync(0xFFFFFFFFu, end - beg > 32);
-    while (big) {
-      const uint32_t L = __ffs(big) - 1;
-      big &= big - 1;
-      const uint64_t b = __shfl_sync(0xFFFFFFFFu, beg, L), t = __shfl_sync(0xFFFFFFFFu, end, L);
-      uint64_t carry = 0;
-      for (uint64_t base = b; base < t; base += 32) {
-        const uint64_t e = base + lane;
-        uint64_t x = e < t ? lt_fixed(w[e]) : 0ull;
+      if (skip) continue;
+      const uint64_t e = base + lane;
+      // bit i: edge base + i is the first of its list
+      uint32_t head = 0;
+      if (end > beg && beg >= base && beg < stop) head = 1u << (uint32_t)(beg - base);
+      head = __reduce_or_sync(0xFFFFFFFFu, head);
+      uint64_t x = e < stop ? lt_fixed(w[e]) : 0ull;
+      // lanes back to this edge's list's first edge (or the step's)
+      const uint32_t upto = head & (0xFFFFFFFFu >> (31 - lane));
+      const uint32_t from = upto ? 31u - __clz(upto) : 0u;
 #pragma unroll
-        for (int d = 1; d < 32; d <<= 1) {
-          const uint64_t y = __shfl_up_sync(0xFFFFFFFFu, x, d);
-          if (lane >= (uint32_t)d) x = sat_add(x, y);
-        }
-        x = sat_add(x, carry);
-        if (e < t) {
-          const uint64_t c = x >> 8;
-          edges[e] = make_uint2(src[e], c > 0xFFFFFFFFull ? 0xFFFFFFFFu : (uint32_t)c);
-        }
-        carry = __shfl_sync(0xFFFFFFFFu, x, 31);
+      for (int d = 1; d < 32; d <<= 1) {
+        const uint64_t y = __shfl_up_sync(0xFFFFFFFFu, x, d);
+        if (lane >= from + (uint32_t)d) x = sat_add(x, y);
       }
+      if (!upto) x = sat_add(x, carry);  // the list began in an earlier step
+      if (e < stop) edges[e] = lt_record(src[e], x);
+      carry = __shfl_sync(0xFFFFFFFFu, x, (uint32_t)(stop - base - 1));
+      base = stop;
     }
   }
   const uint64_t tid = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
   const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
   for (uint64_t e = m + tid; e < m_pad; e += stride) edges[e] = make_uint2(0u, 0u);
+}
+
+// The long lists, a block each, 1024 edges a step.
+__global__ void __launch_bounds__(256)
+pack_lt_long_kernel(const uint64_t *index, const uint32_t *src, const float *w, uint2 *edges,
+                    const unsigned int *nlong, const uint32_t *longs) {
+  __shared__ uint64_t s_warp[8], s_carry;
+  const uint32_t lane = threadIdx.x & 31u, wid = threadIdx.x >> 5;
+  for (uint32_t k = blockIdx.x; k < *nlong; k += gridDim.x) {
+    const uint64_t kb = index[longs[k]], ke = index[longs[k] + 1];
+    if (threadIdx.x == 0) s_carry = 0;
+    for (uint64_t base = kb; base < ke; base += 1024) {
+      // four edges a thread, side by side
+      const uint64_t e0 = base + 4 * threadIdx.x;
+      uint64_t x[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        x[i] = e0 + i < ke ? lt_fixed(w[e0 + i]) : 0ull;
+        if (i) x[i] = sat_add(x[i], x[i - 1]);
+      }
+      uint64_t t = x[3];
+#pragma unroll
+      for (int d = 1; d < 32; d <<= 1) {
+        const uint64_t y = __shfl_up_sync(0xFFFFFFFFu, t, d);
+        if (lane >= (uint32_t)d) t = sat_add(t, y);
+      }
+      if (lane == 31) s_warp[wid] = t;
+      __syncthreads();
+      uint64_t before = s_carry;
+      for (uint32_t i = 0; i < wid; ++i) before = sat_add(before, s_warp[i]);
+      const uint64_t prev = __shfl_up_sync(0xFFFFFFFFu, t, 1);
+      if (lane) before = sat_add(before, prev);
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+        if (e0 + i < ke) edges[e0 + i] = lt_record(src[e0 + i], sat_add(before, x[i]));
+      __syncthreads();
+      if (threadIdx.x == 255) s_carry = sat_add(before, x[3]);
+      __syncthreads();
+    }
+  }
 }
 
 }  // namespace
@@ -198,13 +257,18 @@ void launch_uniform_threshold(const uint32_t *off, const uint2 *edges, uint32_t 
   branching_kernel<<<2368, 256, 0, stream>>>(edges, m, lam, reinterpret_cast<double *>(sums + 1));
 }
 
+size_t pack_lt_scratch(uint64_t m) { return sizeof(uint32_t) * (m / kPackLong + 2); }
+
 void launch_pack_lt(const uint64_t *index, const float *w, uint32_t n,
-                    uint64_t m, uint32_t *off, uint2 *edges, const uint32_t *src,
+                    uint64_t m, uint32_t *off, uint2 *edges, const uint32_t *src, void *scratch,
                     cudaStream_t stream) {
-  count_launches(2);
+  count_launches(3);
+  unsigned int *nlong = static_cast<unsigned int *>(scratch);
+  uint32_t *longs = nlong + 1;
+  cudaMemsetAsync(nlong, 0, sizeof(*nlong), stream);
   pack_off_kernel<<<1184, 256, 0, stream>>>(index, n, off);
-  pack_lt_kernel<<<2368, 256, 0, stream>>>(index, src, w, n, m, pad4(m) + 4,
-                                           edges);
+  pack_lt_kernel<<<2368, 256, 0, stream>>>(index, src, w, n, m, pad4(m) + 4, edges, nlong, longs);
+  pack_lt_long_kernel<<<1184, 256, 0, stream>>>(index, src, w, edges, nlong, longs);
 }
 
 }  // namespace rip

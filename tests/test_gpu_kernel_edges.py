@@ -161,3 +161,20 @@ def test_device_picks_in_one_launch_and_grid_wide(ctx, copies):
         f, seeds, gains = p.select(k, s, rb.TIE_LOWEST_ID)
         assert f == of and seeds.tolist() == oseeds.tolist() and gains.tolist() == ogains.tolist()
     dg.close()
+
+
+@pytest.mark.parametrize("total", [0.7, 5.0])
+def test_lt_pack_over_list_lengths(ctx, total):
+    """Cumulative weights of lists that end on and off the scan's 32-edge and
+    1024-edge steps, long ones side by side, empty ones between; sums past 1
+    saturate."""
+    lens = [0, 1, 31, 32, 33, 64, 0, 1023, 1024, 1025, 1024, 4096, 4097, 0, 0, 5000, 7, 100] * 9
+    r = np.random.RandomState(3)
+    index = np.zeros(len(lens) + 1, dtype=np.uint64)
+    np.cumsum(lens, out=index[1:])
+    m = int(index[-1])
+    w = np.concatenate([r.rand(d) * (2 * total / max(d, 1)) for d in lens]).astype(np.float32)
+    g = rb.HostGraph(len(lens), index, r.randint(0, len(lens), m).astype(np.uint32), w)
+    dg = rb.DeviceGraph(ctx, g, "LT")
+    assert np.array_equal(dg.thresholds(), O.pack("LT", g.index, g.weights))
+    dg.close()

@@ -3,11 +3,12 @@
 // The reference measures the quality of a seed set with ripples::simulate
 // (include/ripples/diffusion_simulation.h:73-178, driven replica by replica
 // by tools/simulator.cc); the spread is the number of vertices reached,
-// seeds included.  Here one 512-thread CTA runs one replica at a time with
-// the level loop of the one-CTA-per-heavy-set sampler: a level's entries are
-// taken a CTA's width at a time, a block scan turns their out-edge unit counts into
-// offsets and all warps stride over the concatenated units (IC: 8-edge coin
-// blocks, one Philox block each; LT: 4-edge record groups).
+// seeds included.  Here one CTA runs one replica at a time, level by level, as
+// the one-CTA-per-heavy-set sampler grows a set: warps take 32 of the level's
+// entries at a time and sweep their shorter out-lists through the concatenated
+// 8-edge blocks (a warp scan and a shuffle search, no barrier); lists of
+// kTileBlocks blocks or more are listed and dealt to all warps in 32-block
+// tiles.
 //   IC: out-edge e of a reached vertex fires in replica r iff its coin
 //       (coarse half from sim_ic_block(key, e >> 3, r), fine half from
 //       sim_ic_fine on a coarse tie) is below threshold(e) (BFS over live
@@ -20,6 +21,11 @@
 //       has the distribution of diffusion_simulation.h:129-178's.
 // Either way a replica's reached set is a pure function of (seed, r),
 // whatever the visiting order.
+//
+// What bounds it: latency.  IC draws 90 issue cycles of coins a warp and coin
+// block; a live edge costs round trips.  The reached bitmap sits in shared memory
+// where it fits (n up to about 1.8 million), so a live edge costs none to L2 and
+// the bitmaps leave L2 to the graph.
 #include "device.cuh"
 #include "launch.h"
 
@@ -27,10 +33,204 @@ namespace rip {
 
 namespace {
 
-// four 512-thread CTAs per SM (32 registers a thread: 64 resident warps).
+constexpr uint32_t kTileBlocks = 128;  // lists of at least this many blocks go in tiles
+constexpr uint32_t kSimLong = 256;     // long lists a level may list
+
+__device__ __forceinline__ uint32_t sim_lanemask_lt() {
+  uint32_t m;
+  asm("mov.u32 %0, %%lanemask_lt;" : "=r"(m));
+  return m;
+}
+
+template <bool SHARED, int THREADS>
+__global__ void __launch_bounds__(THREADS, THREADS == 1024 ? 1 : 4)
+spread_ic_kernel(const __grid_constant__ SpreadLaunch L) {
+  constexpr uint32_t WARPS = THREADS / 32;
+  // the targets of a block's edges: kept in registers where there are 64 a
+  // thread, else read again from L1
+  constexpr bool KEEP = THREADS == 1024;
+  extern __shared__ uint4 s_dyn[];  // SHARED: the reached bitmap
+  __shared__ uint32_t s_lbeg[kSimLong], s_lend[kSimLong];
+  __shared__ uint32_t s_qlen, s_nlong[2], s_next[2];  // by the level's parity
+  __shared__ unsigned long long s_rep;
+
+  const uint32_t tid = threadIdx.x, lane = lane_id(), wid = tid >> 5;
+  uint32_t *bm = SHARED ? reinterpret_cast<uint32_t *>(s_dyn)
+                        : L.bitmaps + (size_t)blockIdx.x * L.bm_words;
+  uint32_t *q = L.queues + (size_t)blockIdx.x * L.qcap;
+  const uint32_t words4 = (uint32_t)((L.bm_words + 3) / 4);  // SHARED
+  unsigned long long reached = 0;
+  if (SHARED)
+    for (uint32_t i = tid; i < words4; i += THREADS) s_dyn[i] = make_uint4(0, 0, 0, 0);
+
+  for (;;) {
+    if (tid == 0) {
+      s_rep = atomicAdd(L.next, 1ull);
+      s_qlen = 0;
+      s_nlong[0] = 0;
+      s_next[0] = 0;
+    }
+    __syncthreads();
+    const uint64_t r = s_rep;
+    if (r >= L.replicas) break;
+    // the seeds are the first level (a repeated seed is queued once)
+    for (uint32_t i = tid; i < L.k; i += THREADS) {
+      const uint32_t v = L.seeds[i];
+      const uint32_t bit = 1u << (v & 31);
+      if (!(atomicOr(&bm[v >> 5], bit) & bit)) {
+        const uint32_t pos = atomicAdd(&s_qlen, 1u);
+        if (pos < L.qcap) q[pos] = v;
+      }
+    }
+    const CoinSet cs = coin_set(L.rk, r, DOM_SIM_IC);
+    __syncthreads();
+    // Queues this lane's vertex u (if any) unless it is reached already; all
+    // lanes of the warp call it.
+    auto reach = [&](bool want, uint32_t u) {
+      const uint32_t bit = 1u << (u & 31);
+      const bool isnew = want && !(atomicOr(&bm[u >> 5], bit) & bit);
+      const uint32_t bal = __ballot_sync(FULL, isnew);
+      if (!bal) return;
+      uint32_t pos = 0;
+      if (lane == (uint32_t)(__ffs(bal) - 1)) pos = atomicAdd(&s_qlen, (uint32_t)__popc(bal));
+      pos = __shfl_sync(FULL, pos, __ffs(bal) - 1) + __popc(bal & sim_lanemask_lt());
+      if (isnew && pos < L.qcap) q[pos] = u;
+    };
+    // Draws 8-edge block b's edges in [ob, oe) (an empty range: none) and follows
+    // those that fire, one a lane and pass.  Records are read two at a time (a
+    // pair past the list's end is not read: the record array ends on a 4-edge
+    // boundary).
+    auto expand_block = [&](uint32_t b, uint32_t ob, uint32_t oe) {
+      const uint4 *rp = reinterpret_cast<const uint4 *>(L.G.edges + ((size_t)b << 3));
+      const u32x4 c = coin_block(L.rk, cs, b);
+      uint32_t u[8], live = 0, tie = 0;
+#pragma unroll
+      for (int h = 0; h < 4; ++h) {
+        const uint32_t e0 = (b << 3) + 2 * h;
+        if (KEEP) u[2 * h] = u[2 * h + 1] = 0;
+        if (e0 < oe && e0 + 1 >= ob) {
+          const uint4 x = __ldg(rp + h);
+          if (KEEP) {
+            u[2 * h] = x.x;
+            u[2 * h + 1] = x.z;
+          }
+          const uint32_t c0 = coarse_of(c, 2 * h), c1 = coarse_of(c, 2 * h + 1);
+          if (e0 >= ob) {
+            if (c0 < (x.y >> 16)) live |= 1u << (2 * h);
+            else if (c0 == (x.y >> 16)) tie |= 1u << (2 * h);
+          }
+          if (e0 + 1 < oe) {
+            if (c1 < (x.w >> 16)) live |= 2u << (2 * h);
+            else if (c1 == (x.w >> 16)) tie |= 2u << (2 * h);
+          }
+        }
+      }
+      while (tie) {  // one edge in 65 536: the fine half decides
+        const uint32_t h = __ffs(tie) - 1;
+        tie &= tie - 1;
+        const uint32_t e = (b << 3) + h;
+        if (sim_ic_fine_call(L.key, e, r) < (__ldg(&L.G.edges[e].y) & 0xFFFFu)) live |= 1u << h;
+      }
+      while (__any_sync(FULL, live != 0)) {
+        uint32_t x = 0;
+        bool want = live != 0;
+        if (want) {
+          const uint32_t h = __ffs(live) - 1;
+          live &= live - 1;
+          if (KEEP) {
+#pragma unroll
+            for (int t = 0; t < 8; ++t)
+              if (h == (uint32_t)t) x = u[t];
+          } else {
+            x = __ldg(&L.G.edges[(b << 3) + h].x);
+            const uint32_t word = SHARED ? bm[x >> 5] : __ldcg(&bm[x >> 5]);  // bits are only set
+            want = !((word >> (x & 31)) & 1u);
+          }
+        }
+        reach(want, x);
+      }
+    };
+    uint32_t lo = 0, hi = min(s_qlen, L.qcap), levels = 0, par = 0;
+    __syncthreads();
+    while (lo < hi) {
+      ++levels;  // one BFS level (the seeds are the first)
+      // 1. warps take the level's entries, up to 32 at a time
+      const uint32_t share = min(32u, (hi - lo + WARPS - 1) / WARPS);
+      for (;;) {
+        uint32_t at = 0;
+        if (lane == 0) at = atomicAdd(&s_next[par], share);
+        at = __shfl_sync(FULL, at, 0);
+        if (at >= hi - lo) break;
+        const uint32_t e = lo + at + lane;
+        uint32_t beg = 0, end = 0;
+        if (lane < share && e < hi) {
+          const uint32_t v = q[e];
+          beg = __ldg(L.G.off + v);
+          end = __ldg(L.G.off + v + 1);
+        }
+        uint32_t nb = block_count(beg, end);
+        if (nb >= kTileBlocks) {
+          const uint32_t pos = atomicAdd(&s_nlong[par], 1u);
+          if (pos < kSimLong) {
+            s_lbeg[pos] = beg;
+            s_lend[pos] = end;
+            nb = 0;
+          }  // (no room: this warp sweeps it with the others)
+        }
+        const uint32_t incl = warp_incl_scan(nb);
+        const uint32_t total = __shfl_sync(FULL, incl, 31);
+        for (uint32_t base = 0; base < total; base += 32) {
+          const uint32_t j = base + lane;
+          const uint32_t owner = warp_find_owner(incl, min(j, total - 1));
+          const uint32_t ob = __shfl_sync(FULL, beg, owner);
+          const uint32_t oe = __shfl_sync(FULL, end, owner);
+          const uint32_t oexcl = __shfl_sync(FULL, incl - nb, owner);
+          const bool valid = j < total;
+          expand_block(valid ? (ob >> 3) + (j - oexcl) : 0u, valid ? ob : 0u, valid ? oe : 0u);
+        }
+      }
+      __syncthreads();
+      // 2. the long lists, dealt to the warps a tile of 32 blocks at a time
+      const uint32_t nlong = min(s_nlong[par], kSimLong);
+      if (tid == 0) s_nlong[par ^ 1] = s_next[par ^ 1] = 0;
+      uint32_t deal = wid;  // (wid - tiles dealt so far) mod WARPS: this warp's next tile
+      for (uint32_t a = 0; a < nlong; ++a) {
+        const uint32_t ob = s_lbeg[a], oe = s_lend[a];
+        const uint32_t b_last = (oe - 1) >> 3;
+        const uint32_t ntiles = ((b_last - (ob >> 3)) >> 5) + 1;
+        for (uint32_t t = deal & (WARPS - 1); t < ntiles; t += WARPS) {
+          const uint32_t b = (ob >> 3) + t * 32 + lane;
+          const bool valid = b <= b_last;
+          expand_block(valid ? b : 0u, valid ? ob : 0u, valid ? oe : 0u);
+        }
+        deal -= ntiles;
+      }
+      __syncthreads();
+      lo = hi;
+      hi = min(s_qlen, L.qcap);
+      par ^= 1;
+      __syncthreads();
+    }
+    // every vertex is queued at most once, so qlen <= n = qcap
+    const uint32_t qlen = hi;
+    if (tid == 0) {
+      if (L.sizes) L.sizes[r] = qlen;
+      if (L.levels) L.levels[r] = levels;
+      reached += qlen;
+    }
+    if (SHARED && qlen >= words4) {
+      for (uint32_t i = tid; i < words4; i += THREADS) s_dyn[i] = make_uint4(0, 0, 0, 0);
+    } else {
+      for (uint32_t i = tid; i < qlen; i += THREADS) bm[q[i] >> 5] = 0u;
+    }
+    __syncthreads();
+  }
+  if (tid == 0 && reached) atomicAdd(L.total, reached);
+}
+
+// LT: four 512-thread CTAs per SM (32 registers a thread: 64 resident warps).
 // The kernel waits on L2 latency, so replicas in flight are what move it:
-// one 1024-thread CTA per SM (32 warps) ran 19.3 K replicas/s on the 2^20
-// bench, two of 768 threads 23.1 K, three of 640 25.6 K, four of 512 26.5 K.
+// fewer and larger CTAs (one of 1024 threads, two of 768) were slower.
 constexpr int SIM_THREADS = 512;
 constexpr int SIM_WARPS = SIM_THREADS / 32;
 
@@ -71,12 +271,11 @@ __device__ __forceinline__ uint32_t lt_kept_source(const DevGraph &B, Key key, u
   return __ldg(B.edges + a).x;
 }
 
-template <bool LT>
-__global__ void __launch_bounds__(SIM_THREADS, kSpreadCtasPerSm)
-spread_kernel(SpreadLaunch L) {
+__global__ void __launch_bounds__(SIM_THREADS, 4)
+spread_lt_kernel(SpreadLaunch L) {
   __shared__ uint32_t s_off[SIM_THREADS + 1];
   __shared__ uint32_t s_beg[SIM_THREADS], s_end[SIM_THREADS];
-  __shared__ uint32_t s_v[LT ? SIM_THREADS : 1];  // LT: the entry's vertex
+  __shared__ uint32_t s_v[SIM_THREADS];  // the entry's vertex
   __shared__ uint32_t s_warp[SIM_WARPS];
   __shared__ uint32_t s_qlen, s_total;
   __shared__ unsigned long long s_rep;
@@ -114,11 +313,11 @@ spread_kernel(SpreadLaunch L) {
           const uint32_t v = q[e];
           beg = __ldg(L.G.off + v);
           end = __ldg(L.G.off + v + 1);
-          if (LT) s_v[tid] = v;
+          s_v[tid] = v;
         }
         s_beg[tid] = beg;
         s_end[tid] = end;
-        const uint32_t ng = LT ? group_count(beg, end) : block_count(beg, end);
+        const uint32_t ng = group_count(beg, end);
         s_off[tid] = sim_block_scan(ng, s_warp, &s_total);
         if (tid == 0) s_off[SIM_THREADS] = s_total;
         __syncthreads();
@@ -131,64 +330,22 @@ spread_kernel(SpreadLaunch L) {
             else b = mid;
           }
           const uint32_t ob = s_beg[a], oe = s_end[a];
-          if (LT) {
-            const uint32_t g = (ob >> 2) + (j - s_off[a]);
-            uint2 rec[4];
-            load_group(L.G.edges, g, rec);
-            const uint32_t from = s_v[a];
+          const uint32_t g = (ob >> 2) + (j - s_off[a]);
+          uint2 rec[4];
+          load_group(L.G.edges, g, rec);
+          const uint32_t from = s_v[a];
 #pragma unroll
-            for (int t = 0; t < 4; ++t) {
-              const uint32_t ed = (g << 2) + t;
-              if (ed < ob || ed >= oe) continue;
-              const uint32_t u = rec[t].x;
-              const uint32_t bit = 1u << (u & 31);
-              // a plain read first: reached bits are only ever set
-              if ((__ldcg(&bm[u >> 5]) & bit) || lt_kept_source(L.B, L.key, r, u) != from)
-                continue;
-              if (!(atomicOr(&bm[u >> 5], bit) & bit)) {
-                const uint32_t pos = atomicAdd(&s_qlen, 1u);
-                if (pos < L.qcap) q[pos] = u;
-              }
-            }
-          } else {
-            // an 8-edge coin block: records two at a time (a pair past the
-            // list's end is not read: the record array ends on a 4-edge
-            // boundary), coarse coins first, the fine half on a tie
-            const uint32_t b = (ob >> 3) + (j - s_off[a]);
-            const u32x4 c = sim_ic_block(L.key, b, r);
-            const uint4 *rp = reinterpret_cast<const uint4 *>(L.G.edges + ((size_t)b << 3));
-            uint32_t live = 0, tie = 0;
-#pragma unroll
-            for (int qq = 0; qq < 4; ++qq) {
-              const uint32_t e0 = (b << 3) + 2 * qq;
-              if (e0 < oe && e0 + 1 >= ob) {
-                const uint4 rr = __ldg(rp + qq);
-                const uint32_t c0 = coarse_of(c, 2 * qq), c1 = coarse_of(c, 2 * qq + 1);
-                if (e0 >= ob) {
-                  if (c0 < (rr.y >> 16)) live |= 1u << (2 * qq);
-                  else if (c0 == (rr.y >> 16)) tie |= 1u << (2 * qq);
-                }
-                if (e0 + 1 < oe) {
-                  if (c1 < (rr.w >> 16)) live |= 2u << (2 * qq);
-                  else if (c1 == (rr.w >> 16)) tie |= 2u << (2 * qq);
-                }
-              }
-            }
-            while (tie) {
-              const uint32_t h = __ffs(tie) - 1;
-              tie &= tie - 1;
-              const uint32_t ed = (b << 3) + h;
-              if (sim_ic_fine(L.key, ed, r) < (__ldg(&L.G.edges[ed].y) & 0xFFFFu))
-                live |= 1u << h;
-            }
-            while (live) {
-              const uint32_t u = __ldg(&L.G.edges[(b << 3) + (__ffs(live) - 1)].x);
-              live &= live - 1;
-              const uint32_t bit = 1u << (u & 31);
-              if (!(atomicOr(&bm[u >> 5], bit) & bit)) {
-                const uint32_t pos = atomicAdd(&s_qlen, 1u);
-                if (pos < L.qcap) q[pos] = u;
-              }
+          for (int t = 0; t < 4; ++t) {
+            const uint32_t ed = (g << 2) + t;
+            if (ed < ob || ed >= oe) continue;
+            const uint32_t u = rec[t].x;
+            const uint32_t bit = 1u << (u & 31);
+            // a plain read first: reached bits are only ever set
+            if ((__ldcg(&bm[u >> 5]) & bit) || lt_kept_source(L.B, L.key, r, u) != from)
+              continue;
+            if (!(atomicOr(&bm[u >> 5], bit) & bit)) {
+              const uint32_t pos = atomicAdd(&s_qlen, 1u);
+              if (pos < L.qcap) q[pos] = u;
             }
           }
         }
@@ -211,12 +368,42 @@ spread_kernel(SpreadLaunch L) {
   if (tid == 0 && reached) atomicAdd(L.total, reached);
 }
 
+// Static shared memory of a spread CTA, rounded up.
+constexpr size_t kSpreadStatic = 4096;
+
+template <bool SHARED, int THREADS>
+void launch_ic(const SpreadLaunch &L, size_t shared, cudaStream_t stream) {
+  if (shared)
+    cudaFuncSetAttribute(spread_ic_kernel<SHARED, THREADS>,
+                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shared);
+  spread_ic_kernel<SHARED, THREADS><<<L.blocks, THREADS, shared, stream>>>(L);
+}
+
 }  // namespace
 
-void launch_spread(const SpreadLaunch &L, bool lt, cudaStream_t stream) {
+// IC: four 512-thread CTAs per SM with the bitmap in shared memory where four
+// fit, one 1024-thread CTA where one does, else four with it in global memory.
+// R-MAT, p ~ U(0, 0.1), 50 hubs as seeds, against block-wide scans of every
+// level with the bitmap in global memory: 2^16 vertices, 1500 replicas 2.75 ->
+// 2.59 ms; 2^18 14.9 -> 14.1 (four CTAs; one: 15.2); 2^20 62.8 -> 50.8 (one; in
+// global memory: 59.8); 2^22, 300 replicas 77.7 -> 71.0 (global).
+SpreadShape spread_shape(uint32_t n, bool lt) {
+  const size_t bitmap = (((size_t)n + 127) / 128) * 16;
+  if (lt) return SpreadShape{SIM_THREADS, 4, 0};
+  if (4 * (bitmap + kSpreadStatic + 1024) <= 227 * 1024) return SpreadShape{512, 4, bitmap};
+  if (bitmap + kSpreadStatic <= 227 * 1024 - 1024) return SpreadShape{1024, 1, bitmap};
+  return SpreadShape{512, 4, 0};
+}
+
+void launch_spread(const SpreadLaunch &L0, bool lt, cudaStream_t stream) {
   count_launches(1);
-  if (lt) spread_kernel<true><<<L.blocks, SIM_THREADS, 0, stream>>>(L);
-  else spread_kernel<false><<<L.blocks, SIM_THREADS, 0, stream>>>(L);
+  SpreadLaunch L = L0;
+  L.rk = round_keys(L.key);
+  const SpreadShape s = spread_shape(L.G.n, lt);
+  if (lt) spread_lt_kernel<<<L.blocks, SIM_THREADS, 0, stream>>>(L);
+  else if (s.shared && s.threads == 1024) launch_ic<true, 1024>(L, s.shared, stream);
+  else if (s.shared) launch_ic<true, 512>(L, s.shared, stream);
+  else launch_ic<false, 512>(L, 0, stream);
 }
 
 }  // namespace rip

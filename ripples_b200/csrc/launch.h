@@ -144,6 +144,7 @@ struct SpreadLaunch {
   DevGraph G{};                   // forward CSR: edges[e] = {target, IC threshold}
   DevGraph B{};                   // LT only: backward CSR, edges[j] = {source, cumulative}
   Key key{};
+  RoundKeys rk{};                 // round_keys(key), filled by launch_spread
   const uint32_t *seeds = nullptr;  // k vertex ids < n
   uint32_t k = 0;
   uint64_t replicas = 0;
@@ -151,14 +152,20 @@ struct SpreadLaunch {
   unsigned long long *total = nullptr;  // sum of reached counts (zeroed)
   uint32_t *sizes = nullptr;      // per replica reached count, or null
   uint32_t *levels = nullptr;     // per replica BFS levels (seeds' included), or null
-  uint32_t *bitmaps = nullptr;    // per CTA slot, bm_words words, all-zero
+  uint32_t *bitmaps = nullptr;    // per CTA slot, bm_words words, all-zero (not in shared memory)
   uint64_t bm_words = 0;
   uint32_t *queues = nullptr;     // per CTA slot, qcap = n entries
   uint32_t qcap = 0;
   int blocks = 0;
 };
-// Resident spread CTAs (one replica each at a time) per SM.
-constexpr int kSpreadCtasPerSm = 4;
+// Spread CTAs (one replica each at a time) for a graph of n vertices: threads,
+// CTAs resident per SM, bytes of the reached bitmap in shared memory (0: it is
+// in global memory).
+struct SpreadShape {
+  int threads, per_sm;
+  size_t shared;
+};
+SpreadShape spread_shape(uint32_t n, bool lt);
 void launch_spread(const SpreadLaunch &L, bool lt, cudaStream_t stream);
 void launch_ic_fused(const FusedLaunch &L, cudaStream_t stream);
 // Resident fused CTAs per SM for a colour width (occupancy API).

@@ -239,6 +239,12 @@ RIP_HD uint32_t sim_ic_fine(Key k, uint64_t e, uint64_t r) {
                 set_hi(r, DOM_SIM_IC_FINE), k.k0, k.k1).x & 0xFFFFu;
 }
 
+#if defined(__CUDACC__)
+static __device__ __noinline__ uint32_t sim_ic_fine_call(Key k, uint64_t e, uint64_t r) {
+  return sim_ic_fine(k, e, r);
+}
+#endif
+
 // Threshold of vertex v in LT spread replica r.
 RIP_HD uint32_t sim_lt_threshold(Key k, uint64_t r, uint32_t v) {
   return philox(v, 0u, (uint32_t)r, set_hi(r, DOM_SIM_LT), k.k0, k.k1).x;

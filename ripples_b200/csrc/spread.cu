@@ -24,12 +24,15 @@ int spread_run(rip_graph *g, rip_graph *b, const uint32_t *seeds, uint32_t k,
   if (replicas == 0 || g->n == 0) return RIP_OK;
   CK(c, cudaSetDevice(c->device));
 
-  // per CTA slot: an n-bit visited bitmap and an n-entry queue (a replica
-  // queues every vertex at most once); at most one slot per resident CTA,
-  // fewer when the slots would take more than a quarter of the free budget
+  // per CTA slot: an n-bit visited bitmap (unless the CTAs keep it in shared
+  // memory) and an n-entry queue (a replica queues every vertex at most once);
+  // at most one slot per resident CTA, fewer when the slots would take more
+  // than a quarter of the free budget
+  const SpreadShape shape = spread_shape(g->n, b != nullptr);
   const uint64_t bm_words = ((uint64_t)g->n + 31) / 32;
-  const uint64_t per_slot = 4 * bm_words + 4 * (uint64_t)g->n;
-  uint64_t slots = std::min<uint64_t>(replicas, (uint64_t)c->num_sms * kSpreadCtasPerSm);
+  const uint64_t bm_slot = shape.shared ? 0 : bm_words;
+  const uint64_t per_slot = 4 * bm_slot + 4 * (uint64_t)g->n;
+  uint64_t slots = std::min<uint64_t>(replicas, (uint64_t)c->num_sms * shape.per_sm);
   const uint64_t room = c->budget > c->used ? (c->budget - c->used) / 4 : 0;
   while (slots > 1 && slots * per_slot > room) slots /= 2;
 
@@ -49,7 +52,7 @@ int spread_run(rip_graph *g, rip_graph *b, const uint32_t *seeds, uint32_t k,
   TRY(dalloc(c, B.d_seeds, sizeof(uint32_t) * std::max<uint32_t>(k, 1)));
   if (sizes) TRY(dalloc(c, B.d_sizes, sizeof(uint32_t) * replicas));
   if (levels) TRY(dalloc(c, B.d_levels, sizeof(uint32_t) * replicas));
-  CK(c, cudaMemsetAsync(B.scratch.p, 0, slots * bm_words * 4, c->stream));
+  if (bm_slot) CK(c, cudaMemsetAsync(B.scratch.p, 0, slots * bm_slot * 4, c->stream));
   CK(c, cudaMemsetAsync(B.ctr.p, 0, 2 * sizeof(unsigned long long), c->stream));
   if (k)
     CK(c, cudaMemcpyAsync(B.d_seeds.p, seeds, sizeof(uint32_t) * k, cudaMemcpyHostToDevice,
@@ -68,7 +71,7 @@ int spread_run(rip_graph *g, rip_graph *b, const uint32_t *seeds, uint32_t k,
   L.levels = levels ? ptr<uint32_t>(B.d_levels) : nullptr;
   L.bitmaps = ptr<uint32_t>(B.scratch);
   L.bm_words = bm_words;
-  L.queues = L.bitmaps + slots * bm_words;
+  L.queues = L.bitmaps + slots * bm_slot;
   L.qcap = g->n;
   L.blocks = (int)slots;
   launch_spread(L, b != nullptr, c->stream);

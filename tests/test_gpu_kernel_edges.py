@@ -178,3 +178,24 @@ def test_lt_pack_over_list_lengths(ctx, total):
     dg = rb.DeviceGraph(ctx, g, "LT")
     assert np.array_equal(dg.thresholds(), O.pack("LT", g.index, g.weights))
     dg.close()
+
+
+@pytest.mark.parametrize("n", [20011, 500009, 1900003])
+def test_spread_bitmap_places(ctx, n):
+    """The reached bitmap in shared memory (four CTAs an SM, one) and in global
+    memory; out-lists around a tile and past what a level lists."""
+    r = np.random.RandomState(n % 97)
+    lens = [1, 7, 8, 9, 255, 1016, 1024, 1025, 2049, 5000] * 30
+    src = np.repeat(np.arange(len(lens)), lens)  # out-lists of the first vertices
+    dst = r.randint(0, n, len(src))
+    hub = r.rand(len(src)) < 0.2
+    dst[hub] = r.randint(0, len(lens), hub.sum())
+    g = rb.HostGraph.from_edges(n, src, dst, r.rand(len(src)) * 0.2)
+    dg = rb.DeviceGraph(ctx, g.forward(), "IC")
+    seeds = list(range(12))
+    mean, sizes, levels = rb.spread_ic(dg, seeds, 200, seed=5, with_sizes=True, with_levels=True)
+    f = g.forward()
+    _, o_sizes, o_levels = O.spread_ic(f.n, f.index, f.src, O.pack("IC", f.index, f.weights), seeds,
+                                       200, seed=5, with_levels=True)
+    assert np.array_equal(sizes, o_sizes) and np.array_equal(levels, o_levels)
+    dg.close()

@@ -228,7 +228,7 @@ spread_ic_kernel(const __grid_constant__ SpreadLaunch L) {
   if (tid == 0 && reached) atomicAdd(L.total, reached);
 }
 
-// LT: four 512-thread CTAs per SM (32 registers a thread: 64 resident warps).
+// LT past 65536 vertices: four 512-thread CTAs per SM (32 registers a thread: 64 resident warps).
 // The kernel waits on L2 latency, so replicas in flight are what move it:
 // fewer and larger CTAs (one of 1024 threads, two of 768) were slower.
 constexpr int SIM_THREADS = 512;
@@ -368,6 +368,170 @@ spread_lt_kernel(SpreadLaunch L) {
   if (tid == 0 && reached) atomicAdd(L.total, reached);
 }
 
+// LT with vertex ids of 16 bits.  Sweeping the out-lists of reached vertices
+// tries a vertex once for every reached in-neighbour, each try a search of its
+// in-list by dependent L2 reads.  Once a replica's levels have more out-edges
+// than half the vertices, the in-edge every vertex keeps is drawn instead, once
+// and into shared memory; from there on a level is a scan of 16-bit sources
+// against the reached bitmap, on chip, and no out-list is read.
+// 2^16 vertices, 768 K edges, 20 hubs as seeds, 2000 replicas: 26.1 -> 8.3 ms;
+// 2^12 vertices, 1500 replicas: 1.11 -> 0.28.  The searches' read latency still
+// bounds it, two of them in flight a thread..
+template <int THREADS>
+__global__ void __launch_bounds__(THREADS, THREADS == 1024 ? 1 : 3)
+spread_lt_small_kernel(const __grid_constant__ SpreadLaunch L) {
+  constexpr uint32_t WARPS = THREADS / 32;
+  extern __shared__ uint4 s_dyn[];
+  __shared__ uint32_t s_qlen, s_size;
+  __shared__ unsigned long long s_rep, s_work;
+  const uint32_t tid = threadIdx.x, lane = lane_id(), wid = tid >> 5;
+  const uint32_t n = L.G.n, words = (uint32_t)L.bm_words;
+  uint32_t *bm = reinterpret_cast<uint32_t *>(s_dyn);  // twice: a level's, the next's
+  uint16_t *kept = reinterpret_cast<uint16_t *>(bm + 2 * words);  // own id: none
+  uint32_t *q = L.queues + (size_t)blockIdx.x * L.qcap;
+  unsigned long long reached = 0;
+  for (;;) {
+    if (tid == 0) {
+      s_rep = atomicAdd(L.next, 1ull);
+      s_qlen = s_size = 0;
+      s_work = 0;
+    }
+    for (uint32_t w = tid; w < words; w += THREADS) bm[w] = 0;
+    __syncthreads();
+    const uint64_t r = s_rep;
+    if (r >= L.replicas) break;
+    auto reach = [&](uint32_t u) {  // (every vertex is queued once at most: n = qcap)
+      const uint32_t bit = 1u << (u & 31);
+      if (atomicOr(&bm[u >> 5], bit) & bit) return;
+      const uint32_t pos = atomicAdd(&s_qlen, 1u);
+      if (pos < L.qcap) q[pos] = u;
+    };
+    for (uint32_t i = tid; i < L.k; i += THREADS) reach(L.seeds[i]);
+    __syncthreads();
+    uint32_t lo = 0, hi = min(s_qlen, L.qcap), levels = 0;
+    bool scan = false;
+    while (lo < hi) {
+      ++levels;  // one BFS level (the seeds are the first)
+      unsigned long long work = 0;
+      for (uint32_t e = lo + tid; e < hi; e += THREADS) {
+        const uint32_t v = q[e];
+        work += __ldg(L.G.off + v + 1) - __ldg(L.G.off + v);
+      }
+      work = warp_sum_u64(work);
+      if (lane == 0 && work) atomicAdd(&s_work, work);
+      __syncthreads();
+      if (s_work > n / 2) {
+        scan = true;
+        break;
+      }
+      for (uint32_t cb = lo + wid * 32; cb < hi; cb += WARPS * 32) {
+        const uint32_t e = cb + lane;
+        uint32_t beg = 0, end = 0, v = 0;
+        if (e < hi) {
+          v = q[e];
+          beg = __ldg(L.G.off + v);
+          end = __ldg(L.G.off + v + 1);
+        }
+        const uint32_t ng = group_count(beg, end), incl = warp_incl_scan(ng);
+        const uint32_t total = __shfl_sync(FULL, incl, 31);
+        for (uint32_t base = 0; base < total; base += 32) {
+          const uint32_t j = base + lane;
+          const uint32_t owner = warp_find_owner(incl, min(j, total - 1));
+          const uint32_t ob = __shfl_sync(FULL, beg, owner), oe = __shfl_sync(FULL, end, owner);
+          const uint32_t from = __shfl_sync(FULL, v, owner);
+          const uint32_t g = (ob >> 2) + j - __shfl_sync(FULL, incl - ng, owner);
+          if (j >= total) continue;
+          uint2 rec[4];
+          load_group(L.G.edges, g, rec);
+#pragma unroll
+          for (int t = 0; t < 4; ++t) {
+            const uint32_t ed = (g << 2) + t, u = rec[t].x;
+            if (ed < ob || ed >= oe) continue;
+            const uint32_t word = *(volatile uint32_t *)&bm[u >> 5];  // bits are only set
+            if (!(word >> (u & 31) & 1u) && lt_kept_source(L.B, L.key, r, u) == from) reach(u);
+          }
+        }
+      }
+      __syncthreads();
+      lo = hi;
+      hi = min(s_qlen, L.qcap);
+      __syncthreads();
+    }
+    if (scan) {
+      // the kept sources, two vertices a thread in flight
+      for (uint32_t v0 = tid; v0 < n; v0 += 2 * THREADS) {
+        uint32_t a[2], b[2], t[2];
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+          const uint32_t v = v0 + i * THREADS;
+          a[i] = b[i] = 0;
+          if (v < n) {
+            a[i] = __ldg(L.B.off + v);
+            b[i] = __ldg(L.B.off + v + 1);
+          }
+        }
+        bool some[2];
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+          t[i] = sim_lt_threshold(L.key, r, v0 + i * THREADS);
+          some[i] = a[i] < b[i] && t[i] < __ldg(&L.B.edges[b[i] - 1].y);
+          b[i] = some[i] ? b[i] - 1 : a[i];  // cum[b] > t
+        }
+        while (a[0] < b[0] || a[1] < b[1]) {
+#pragma unroll
+          for (int i = 0; i < 2; ++i) {
+            if (a[i] >= b[i]) continue;
+            const uint32_t mid = a[i] + ((b[i] - a[i]) >> 1);
+            if (__ldg(&L.B.edges[mid].y) > t[i]) b[i] = mid;
+            else a[i] = mid + 1;
+          }
+        }
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+          const uint32_t v = v0 + i * THREADS;
+          if (v < n) kept[v] = (uint16_t)(some[i] ? __ldg(&L.B.edges[a[i]].x) : v);
+        }
+      }
+      __syncthreads();
+      // the level at hand is in the bitmap: a vertex whose source is there and
+      // that is not joins the next one
+      uint32_t cur = 0;
+      for (;;) {
+        const uint32_t *is = bm + cur * words;
+        uint32_t *next = bm + (cur ^ 1) * words;
+        bool grew = false;
+        for (uint32_t w = wid; w < words; w += WARPS) {
+          const uint32_t was = is[w], v = w * 32 + lane;
+          bool joins = false;
+          if (v < n && !(was >> lane & 1u)) {
+            const uint32_t u = kept[v];
+            joins = is[u >> 5] >> (u & 31) & 1u;
+          }
+          const uint32_t add = __ballot_sync(FULL, joins);
+          if (lane == 0) next[w] = was | add;
+          grew = grew || add != 0;
+        }
+        cur ^= 1;
+        if (!__syncthreads_or(grew)) break;
+        ++levels;
+      }
+      uint32_t mine = 0;
+      for (uint32_t w = tid; w < words; w += THREADS) mine += __popc(bm[w]);
+      mine = __reduce_add_sync(FULL, mine);
+      if (lane == 0 && mine) atomicAdd(&s_size, mine);
+      __syncthreads();
+    }
+    if (tid == 0) {
+      const uint32_t size = scan ? s_size : hi;
+      if (L.sizes) L.sizes[r] = size;
+      if (L.levels) L.levels[r] = levels;
+      reached += size;
+    }
+    __syncthreads();
+  }
+  if (tid == 0 && reached) atomicAdd(L.total, reached);
+}
+
 // Static shared memory of a spread CTA, rounded up.
 constexpr size_t kSpreadStatic = 4096;
 
@@ -379,8 +543,17 @@ void launch_ic(const SpreadLaunch &L, size_t shared, cudaStream_t stream) {
   spread_ic_kernel<SHARED, THREADS><<<L.blocks, THREADS, shared, stream>>>(L);
 }
 
+template <int THREADS>
+void launch_lt_small(const SpreadLaunch &L, size_t shared, cudaStream_t stream) {
+  cudaFuncSetAttribute(spread_lt_small_kernel<THREADS>,
+                       cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shared);
+  spread_lt_small_kernel<THREADS><<<L.blocks, THREADS, shared, stream>>>(L);
+}
+
 }  // namespace
 
+// LT: up to 65536 vertices three 512-thread CTAs an SM where their bitmaps and
+// 16-bit sources fit (n up to 32 K), else one of 1024; past that no shared form.
 // IC: four 512-thread CTAs per SM with the bitmap in shared memory where four
 // fit, one 1024-thread CTA where one does, else four with it in global memory.
 // R-MAT, p ~ U(0, 0.1), 50 hubs as seeds, against block-wide scans of every
@@ -389,6 +562,11 @@ void launch_ic(const SpreadLaunch &L, size_t shared, cudaStream_t stream) {
 // global memory: 59.8); 2^22, 300 replicas 77.7 -> 71.0 (global).
 SpreadShape spread_shape(uint32_t n, bool lt) {
   const size_t bitmap = (((size_t)n + 127) / 128) * 16;
+  if (lt && n <= 65536) {  // two bitmaps and the kept sources
+    const size_t bytes = (((size_t)n + 31) / 32 * 8 + 2 * (size_t)n + 15) & ~(size_t)15;
+    if (3 * (bytes + 2048) <= 227 * 1024) return SpreadShape{512, 3, bytes};
+    return SpreadShape{1024, 1, bytes};
+  }
   if (lt) return SpreadShape{SIM_THREADS, 4, 0};
   if (4 * (bitmap + kSpreadStatic + 1024) <= 227 * 1024) return SpreadShape{512, 4, bitmap};
   if (bitmap + kSpreadStatic <= 227 * 1024 - 1024) return SpreadShape{1024, 1, bitmap};
@@ -400,7 +578,9 @@ void launch_spread(const SpreadLaunch &L0, bool lt, cudaStream_t stream) {
   SpreadLaunch L = L0;
   L.rk = round_keys(L.key);
   const SpreadShape s = spread_shape(L.G.n, lt);
-  if (lt) spread_lt_kernel<<<L.blocks, SIM_THREADS, 0, stream>>>(L);
+  if (lt && s.shared && s.threads == 1024) launch_lt_small<1024>(L, s.shared, stream);
+  else if (lt && s.shared) launch_lt_small<512>(L, s.shared, stream);
+  else if (lt) spread_lt_kernel<<<L.blocks, SIM_THREADS, 0, stream>>>(L);
   else if (s.shared && s.threads == 1024) launch_ic<true, 1024>(L, s.shared, stream);
   else if (s.shared) launch_ic<true, 512>(L, s.shared, stream);
   else launch_ic<false, 512>(L, 0, stream);

@@ -199,3 +199,25 @@ def test_spread_bitmap_places(ctx, n):
                                        200, seed=5, with_levels=True)
     assert np.array_equal(sizes, o_sizes) and np.array_equal(levels, o_levels)
     dg.close()
+
+
+@pytest.mark.parametrize("n", [2011, 33000, 65536, 65537])
+def test_spread_lt_swept_and_scanned(ctx, n):
+    """Replicas that stay below the sweep's share of out-edges and replicas that
+    go on over kept sources: 16-bit ids up to 65536 vertices, deep levels."""
+    r = np.random.RandomState(n)
+    chain = 300  # the last ids: one in-edge each
+    src, dst = r.randint(0, n - chain, 4 * n), r.randint(0, n - chain, 4 * n)
+    src[: 2 * n] = r.randint(0, 40, 2 * n)  # hubs
+    src = np.concatenate([src, [7], np.arange(n - chain, n - 1)])
+    dst = np.concatenate([dst, np.arange(n - chain, n)])
+    g = rb.HostGraph.from_edges(n, src, dst).with_weights(rb.WEIGHTS_LT_NORMALIZED, 3, 0.0, 1.0)
+    fg, bg = rb.DeviceGraph(ctx, g.forward(), "IC"), rb.DeviceGraph(ctx, g, "LT")
+    few = [n - 5, 1000, 1000, n - chain]
+    for seeds, replicas in ((few, 40), (few + [7], 40), (list(range(40)), 20), ([], 5)):
+        _, sizes, levels = rb.spread_lt(fg, bg, seeds, replicas, seed=23, with_sizes=True,
+                                        with_levels=True)
+        _, o_sizes, o_levels = O.spread_lt(g, seeds, replicas, seed=23, with_levels=True)
+        assert np.array_equal(sizes, o_sizes) and np.array_equal(levels, o_levels)
+    bg.close()
+    fg.close()

@@ -19,9 +19,14 @@
 //     as every sampler's (coarse halves from an 8-edge Philox block, the fine
 //     half on a tie), so the sets equal those of the one-set-per-warp kernel
 //     and of the CPU restatement bit for bit;
-//   * in-edges are read in aligned 4-edge groups (one 32-byte load, one Philox
-//     block per colour per group) with warp-level load balancing across
-//     entries;
+//   * the (8-edge coin block, colour) pairs of a warp's entries are dealt to its
+//     lanes (pairs.cuh); an entry of more than kShortPairs pairs is listed and
+//     dealt to all warps in tiles after the level's barrier.  What bounds a
+//     batch is its chain of dependent reads: with a lane per 4-edge group,
+//     looping over its colours, a hub's list was one warp's and lanes waited for
+//     the fullest mask (20 011 sets of a 2^14-vertex graph, 128 colours: 10.7
+//     ms; with pairs 6.2, with two live edges a lane and the next records in
+//     flight and no pilot launch 2.8);
 //   * the finished batch is compacted straight into the flat pool: one
 //     atomicAdd reserves all W sets, per-colour shared cursors place members,
 //     and the same pass clears the colour masks (atomicExch) for the next
@@ -31,26 +36,25 @@
 // sets with the one-set-per-warp kernel (identical results).
 #include "device.cuh"
 #include "launch.h"
+#include "pairs.cuh"
 
 namespace rip {
 
 namespace {
 
-__device__ __forceinline__ uint32_t lanemask_lt() {
-  uint32_t m;
-  asm("mov.u32 %0, %%lanemask_lt;" : "=r"(m));
-  return m;
-}
-
-constexpr int FUSED_THREADS = 512;
-constexpr int FUSED_WARPS = FUSED_THREADS / 32;
 constexpr uint32_t kSharedLog = 4096;  // frontier-log entries staged in shared memory
+constexpr uint32_t kFusedLong = 64;    // long entries a level may list
 
-template <int CW>
-__global__ void __launch_bounds__(FUSED_THREADS)
-ic_fused_kernel(FusedLaunch L) {
-  constexpr int W = 64 * CW;
+template <int CW, int FUSED_THREADS>
+__global__ void __launch_bounds__(FUSED_THREADS, 1024 / FUSED_THREADS)
+ic_fused_kernel(const __grid_constant__ FusedLaunch L) {
+  constexpr int W = 64 * CW, FUSED_WARPS = FUSED_THREADS / 32;
+  constexpr uint32_t NW = 2 * CW;  // 32-colour words of a vertex
+  extern __shared__ uint4 s_dyn[];
   __shared__ uint64_t s_set[W];
+  __shared__ uint4 s_cs[W];  // the sets' CoinSets
+  __shared__ uint32_t s_lbeg[kFusedLong], s_lend[kFusedLong], s_lmask[kFusedLong * NW];
+  __shared__ uint32_t s_nlong[2];  // by the level's parity
   __shared__ unsigned long long s_start[W];
   __shared__ uint32_t s_size[W];
   __shared__ uint32_t s_fill[W];
@@ -59,6 +63,7 @@ ic_fused_kernel(FusedLaunch L) {
   __shared__ unsigned long long s_base, s_work;
 
   const uint32_t tid = threadIdx.x, lane = lane_id(), wid = tid >> 5;
+  PairWarp &S = reinterpret_cast<PairWarp *>(s_dyn)[wid];
   const uint32_t slot = blockIdx.x;
   const uint32_t n = L.G.n;
   uint64_t *vis = L.vis + (size_t)slot * n * CW;
@@ -77,6 +82,7 @@ ic_fused_kernel(FusedLaunch L) {
       s_tail = 0;
       s_overflow = 0;
       s_work = 0;
+      s_nlong[0] = s_nlong[1] = 0;
     }
     __syncthreads();
     const uint32_t b = s_batch;
@@ -90,6 +96,8 @@ ic_fused_kernel(FusedLaunch L) {
       if (c < ncol) {
         const uint32_t rel = L.order ? L.order[c0 + c] : c0 + c;
         s_set[c] = L.first + rel;
+        const CoinSet t = coin_set(L.rk, L.first + rel, DOM_IC);
+        s_cs[c] = make_uint4(t.x2, t.x0, t.y2, t.z2);
       }
     }
     __syncthreads();
@@ -112,29 +120,76 @@ ic_fused_kernel(FusedLaunch L) {
     __syncthreads();
     b_exp = b_edges = b_sexp = b_sedges = 0;
     uint32_t lvl_start = 0, lvl_end = min(s_tail, lcap), level = 1;
-    while (lvl_start < lvl_end && !s_overflow) {
+    uint32_t *vis32 = reinterpret_cast<uint32_t *>(vis), *pend32 = reinterpret_cast<uint32_t *>(pend);
+    uint32_t nev = 0;  // live edges in the warp's buffer
+    bool full = s_overflow != 0;
+    __syncthreads();
+    while (lvl_start < lvl_end && !full) {
+      // Live edges, two {edge, colour} a lane: the source joins the colour's
+      // set (and the next level).
+      auto handle = [&](const uint2 *ev, const bool *valid) {
+        uint32_t u[2] = {0, 0};
+        bool push[2] = {false, false};
+#pragma unroll
+        for (int t = 0; t < 2; ++t)
+          if (valid[t]) u[t] = __ldg(&L.G.edges[ev[t].x].x);
+#pragma unroll
+        for (int t = 0; t < 2; ++t) {
+          const uint32_t bit = 1u << (ev[t].y & 31);
+          push[t] = valid[t] &&
+                    !(atomicOr(vis32 + (size_t)u[t] * NW + (ev[t].y >> 5), bit) & bit);
+        }
+#pragma unroll
+        for (int t = 0; t < 2; ++t) {
+          if (!push[t]) continue;
+          atomicOr(pend32 + (size_t)u[t] * NW + (ev[t].y >> 5), 1u << (ev[t].y & 31));
+          atomicAdd(&s_size[ev[t].y], 1u);
+          push[t] = atomicExch(&pflag[u[t]], level + 1) != level + 1;
+        }
+#pragma unroll
+        for (int t = 0; t < 2; ++t) {
+          const uint32_t bal = __ballot_sync(FULL, push[t]);
+          if (!bal) continue;
+          uint32_t pos = 0;
+          if (lane == (uint32_t)(__ffs(bal) - 1)) pos = atomicAdd(&s_tail, __popc(bal));
+          pos = __shfl_sync(FULL, pos, __ffs(bal) - 1) + __popc(bal & pair_lanes_below());
+          if (push[t]) {
+            if (pos < lcap) {
+              if (pos < kSharedLog) s_log[pos] = u[t];
+              else log[pos] = u[t];
+            }
+            else s_overflow = 1;
+          }
+        }
+      };
+      auto sweep = [&](uint32_t npairs) {
+        sweep_pairs(S, npairs, nev, L.G, L.key, L.rk, s_cs, s_set, handle);
+      };
+      // One tile of a long entry whose colours the warp has listed.
+      auto sweep_tile = [&](uint32_t beg, uint32_t end, uint32_t b, uint32_t b_end, uint32_t pc) {
+        const uint32_t step = window_blocks(pc);
+        for (; b < b_end; b += step) sweep(fill_blocks(S, beg, end, b, min(step, b_end - b), pc));
+      };
       // ---- expand level `level`: entries log[lvl_start, lvl_end) ----------
-      for (uint32_t eb = lvl_start + wid * 32; eb < lvl_end; eb += FUSED_WARPS * 32) {
+      const uint32_t share =
+          min(32u, (lvl_end - lvl_start + FUSED_WARPS - 1) / FUSED_WARPS);
+      for (uint32_t eb = lvl_start + wid * share; eb < lvl_end; eb += FUSED_WARPS * share) {
         const uint32_t ei = eb + lane;
         uint64_t mask[CW];
-        uint32_t beg = 0, end = 0, ng = 0;
+        uint32_t beg = 0, end = 0, nb = 0, pc = 0;
 #pragma unroll
         for (int w = 0; w < CW; ++w) mask[w] = 0;
-        if (ei < lvl_end) {
+        if (lane < share && ei < lvl_end) {
           const uint32_t v = ei < kSharedLog ? s_log[ei] : log[ei];
-          uint32_t any = 0;
 #pragma unroll
           for (int w = 0; w < CW; ++w) {
             mask[w] = atomicExch((unsigned long long *)&pend[(size_t)v * CW + w], 0ull);
-            any |= mask[w] != 0;
+            pc += __popcll(mask[w]);
           }
-          if (any) {
+          if (pc) {
             beg = __ldg(L.G.off + v);
             end = __ldg(L.G.off + v + 1);
-            ng = group_count(beg, end);
-            uint32_t pc = 0;
-#pragma unroll
-            for (int w = 0; w < CW; ++w) pc += __popcll(mask[w]);
+            nb = block_count(beg, end);
             b_exp += 1;
             b_edges += end - beg;
             if (L.work_cap) atomicAdd(&s_work, (unsigned long long)(end - beg));
@@ -142,122 +197,73 @@ ic_fused_kernel(FusedLaunch L) {
             b_sedges += (unsigned long long)pc * (end - beg);
           }
         }
-        const uint32_t incl = warp_incl_scan(ng);
-        const uint32_t total = __shfl_sync(FULL, incl, 31);
-        for (uint32_t base = 0; base < total; base += 32) {
-          const uint32_t j = base + lane;
-          const bool valid = j < total;
-          const uint32_t owner = warp_find_owner(incl, valid ? j : total - 1);
-          const uint32_t ob = __shfl_sync(FULL, beg, owner);
-          const uint32_t oe = __shfl_sync(FULL, end, owner);
-          const uint32_t oexcl = __shfl_sync(FULL, incl, owner) -
-                                 __shfl_sync(FULL, ng, owner);
-          uint64_t om[CW];
-#pragma unroll
-          for (int w = 0; w < CW; ++w) om[w] = __shfl_sync(FULL, mask[w], owner);
-          uint64_t live[4][CW];
-          uint32_t u[4];
-#pragma unroll
-          for (int t = 0; t < 4; ++t) {
-            u[t] = 0;
-#pragma unroll
-            for (int w = 0; w < CW; ++w) live[t][w] = 0;
-          }
-          if (valid) {
-            const uint32_t g = (ob >> 2) + (j - oexcl);
-            uint2 rec[4];
-            load_group(L.G.edges, g, rec);
-            bool inr[4];
-#pragma unroll
-            for (int t = 0; t < 4; ++t) {
-              const uint32_t e = (g << 2) + t;
-              inr[t] = e >= ob && e < oe && rec[t].y != 0u;
-              u[t] = rec[t].x;
-            }
-            if (inr[0] | inr[1] | inr[2] | inr[3]) {
-#pragma unroll
-              for (int w = 0; w < CW; ++w) {
-                uint64_t mm = om[w];
-                while (mm) {
-                  const int bi = __ffsll((long long)mm) - 1;
-                  mm &= mm - 1;
-                  const uint64_t sid = s_set[w * 64 + bi];
-                  // this group's four coarse coins: half of the 8-edge block
-                  const u32x4 cb = ic_block(L.key, g >> 1, sid);
-                  const uint32_t hb = (g & 1u) << 2;
-                  const uint64_t bit = 1ull << bi;
-                  uint32_t tie = 0;
-#pragma unroll
-                  for (int t = 0; t < 4; ++t) {
-                    const uint32_t th = rec[t].y >> 16, cc = coarse_of(cb, hb + t);
-                    if (inr[t]) {
-                      if (cc < th) live[t][w] |= bit;
-                      else if (cc == th) tie |= 1u << t;
-                    }
-                  }
-                  while (tie) {  // a coarse tie, one edge in 65 536: the fine half decides
-                    const uint32_t t = __ffs(tie) - 1;
-                    tie &= tie - 1;
-                    const uint32_t thr = t == 0 ? rec[0].y : t == 1 ? rec[1].y : t == 2 ? rec[2].y : rec[3].y;
-                    if (ic_fine_call(L.key, (g << 2) + t, sid) < (thr & 0xFFFFu)) {
-                      if (t == 0) live[0][w] |= bit;
-                      else if (t == 1) live[1][w] |= bit;
-                      else if (t == 2) live[2][w] |= bit;
-                      else live[3][w] |= bit;
-                    }
-                  }
-                }
-              }
-            }
-          }
-          // apply discoveries
-          bool push[4];
-#pragma unroll
-          for (int t = 0; t < 4; ++t) {
-            bool added = false;
+        const bool is_long = pc != 0 && nb > kShortPairs / pc;
+        bool alone = false;  // long, and no room in the list
+        if (is_long) {
+          const uint32_t pos = atomicAdd(&s_nlong[level & 1], 1u);
+          alone = pos >= kFusedLong;
+          if (!alone) {
+            s_lbeg[pos] = beg;
+            s_lend[pos] = end;
 #pragma unroll
             for (int w = 0; w < CW; ++w) {
-              if (live[t][w]) {
-                const uint64_t old = atomicOr(
-                    (unsigned long long *)&vis[(size_t)u[t] * CW + w], live[t][w]);
-                uint64_t add = live[t][w] & ~old;
-                if (add) {
-                  atomicOr((unsigned long long *)&pend[(size_t)u[t] * CW + w], add);
-                  added = true;
-                  while (add) {
-                    const int bi = __ffsll((long long)add) - 1;
-                    add &= add - 1;
-                    atomicAdd(&s_size[w * 64 + bi], 1u);
-                  }
-                }
-              }
-            }
-            push[t] = added && atomicExch(&pflag[u[t]], level + 1) != level + 1;
-          }
-#pragma unroll
-          for (int t = 0; t < 4; ++t) {
-            const uint32_t bal = __ballot_sync(FULL, push[t]);
-            if (!bal) continue;
-            uint32_t pos0 = 0;
-            if (lane == (uint32_t)(__ffs(bal) - 1)) pos0 = atomicAdd(&s_tail, __popc(bal));
-            pos0 = __shfl_sync(FULL, pos0, __ffs(bal) - 1);
-            if (push[t]) {
-              const uint32_t pos = pos0 + __popc(bal & lanemask_lt());
-              if (pos < lcap) {
-                if (pos < kSharedLog) s_log[pos] = u[t];
-                else log[pos] = u[t];
-              }
-              else s_overflow = 1;
+              s_lmask[pos * NW + 2 * w] = (uint32_t)mask[w];
+              s_lmask[pos * NW + 2 * w + 1] = (uint32_t)(mask[w] >> 32);
             }
           }
         }
+        // short entries: those that start in the same kShortPairs of the
+        // running sum share a window
+        const uint32_t pairs = is_long ? 0u : nb * pc;
+        const uint32_t incl = warp_incl_scan(pairs);
+        const uint32_t total = __shfl_sync(FULL, incl, 31);
+        for (uint32_t from = 0; from < total; from += kShortPairs)
+          sweep(fill_window<CW>(S, pairs && (incl - pairs) - from < kShortPairs, beg, end, nb, pc,
+                                mask));
+        for (uint32_t left = __ballot_sync(FULL, alone); left; left &= left - 1) {
+          const uint32_t o = __ffs(left) - 1;
+          const uint32_t ob = __shfl_sync(FULL, beg, o), oe = __shfl_sync(FULL, end, o);
+          const uint32_t opc = __shfl_sync(FULL, pc, o);
+          uint32_t word = 0;
+#pragma unroll
+          for (int w = 0; w < CW; ++w) {
+            const uint64_t m = __shfl_sync(FULL, mask[w], o);
+            if ((lane >> 1) == (uint32_t)w) word = (uint32_t)(m >> (32 * (lane & 1)));
+          }
+          fill_colours(S, word);
+          sweep_tile(ob, oe, ob >> 3, ((oe - 1) >> 3) + 1, opc);
+        }
       }
       __syncthreads();
+      // the long entries, a tile to a warp
+      const uint32_t nlong = min(s_nlong[level & 1], kFusedLong);
+      uint32_t deal = wid;  // (wid - tiles dealt so far) mod FUSED_WARPS: this warp's next tile
+      for (uint32_t a = 0; a < nlong; ++a) {
+        const uint32_t ob = s_lbeg[a], oe = s_lend[a];
+        const uint32_t word = lane < NW ? s_lmask[a * NW + lane] : 0u;
+        const uint32_t pc = __reduce_add_sync(FULL, __popc(word));
+        const uint32_t tb = tile_blocks(pc), b0 = ob >> 3, nb = ((oe - 1) >> 3) - b0 + 1;
+        const uint32_t ntiles = (nb + tb - 1) / tb;
+        uint32_t t = deal & (FUSED_WARPS - 1);
+        deal -= ntiles;
+        if (t >= ntiles) continue;
+        fill_colours(S, word);
+        for (; t < ntiles; t += FUSED_WARPS)
+          sweep_tile(ob, oe, b0 + t * tb, b0 + min(nb, (t + 1) * tb), pc);
+      }
+      drain_events(S, nev, handle);
+      __syncthreads();
+      // a batch that outgrows its edge budget goes to the CTA-per-set sampler;
+      // every thread reads what ends the loop between two barriers
+      const bool over = L.work_cap && s_work > L.work_cap;
+      full = s_overflow != 0 || over;
+      if (tid == 0) {
+        s_nlong[level & 1] = 0;
+        if (over && s_overflow == 0) s_overflow = 3;
+      }
       lvl_start = lvl_end;
       lvl_end = min(s_tail, lcap);
       ++level;
-      // a batch that outgrows its edge budget goes to the CTA-per-set sampler
-      if (tid == 0 && L.work_cap && s_work > L.work_cap && !s_overflow) s_overflow = 3;
       __syncthreads();
     }
     if (s_overflow == 1) {
@@ -346,25 +352,27 @@ ic_fused_kernel(FusedLaunch L) {
 
 }  // namespace
 
-void launch_ic_fused(const FusedLaunch &L, cudaStream_t stream) {
-  count_launches(1);
-  if (L.colors == 64)
-    ic_fused_kernel<1><<<L.blocks, FUSED_THREADS, 0, stream>>>(L);
-  else if (L.colors == 128)
-    ic_fused_kernel<2><<<L.blocks, FUSED_THREADS, 0, stream>>>(L);
-  else
-    ic_fused_kernel<4><<<L.blocks, FUSED_THREADS, 0, stream>>>(L);
+template <int CW, int THREADS>
+static void fused_launch(const FusedLaunch &L, cudaStream_t stream) {
+  constexpr size_t shared = THREADS / 32 * sizeof(PairWarp);
+  cudaFuncSetAttribute(ic_fused_kernel<CW, THREADS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                       (int)shared);
+  ic_fused_kernel<CW, THREADS><<<L.blocks, THREADS, shared, stream>>>(L);
 }
 
-int fused_ctas_per_sm(uint32_t colors) {
-  int nb = 0;
-  if (colors == 64)
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, ic_fused_kernel<1>, FUSED_THREADS, 0);
-  else if (colors == 128)
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, ic_fused_kernel<2>, FUSED_THREADS, 0);
-  else
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, ic_fused_kernel<4>, FUSED_THREADS, 0);
-  return nb > 0 ? nb : 1;
+template <int CW>
+static void fused_launch(const FusedLaunch &L, cudaStream_t stream) {
+  if (L.blocks <= L.num_sms) fused_launch<CW, 1024>(L, stream);
+  else fused_launch<CW, 512>(L, stream);
+}
+
+void launch_ic_fused(const FusedLaunch &L0, cudaStream_t stream) {
+  count_launches(1);
+  FusedLaunch L = L0;
+  L.rk = round_keys(L.key);
+  if (L.colors == 64) fused_launch<1>(L, stream);
+  else if (L.colors == 128) fused_launch<2>(L, stream);
+  else fused_launch<4>(L, stream);
 }
 
 // ---- export gather: sets [first, first+count) -> out, in set-id order -----

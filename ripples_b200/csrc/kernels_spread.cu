@@ -376,7 +376,7 @@ spread_lt_kernel(SpreadLaunch L) {
 // against the reached bitmap, on chip, and no out-list is read.
 // 2^16 vertices, 768 K edges, 20 hubs as seeds, 2000 replicas: 26.1 -> 8.3 ms;
 // 2^12 vertices, 1500 replicas: 1.11 -> 0.28.  The searches' read latency still
-// bounds it, two of them in flight a thread..
+// bounds it, two of them in flight a thread.
 template <int THREADS>
 __global__ void __launch_bounds__(THREADS, THREADS == 1024 ? 1 : 3)
 spread_lt_small_kernel(const __grid_constant__ SpreadLaunch L) {

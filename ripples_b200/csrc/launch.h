@@ -94,6 +94,7 @@ struct FusedLaunch {
   DevGraph G;
   DevPool P;
   Key key;
+  RoundKeys rk{};        // round_keys(key), filled by launch_ic_fused
   uint64_t first;
   uint32_t count;        // number of sets
   const uint32_t *order; // set indices relative to `first`, batch-major (or null)
@@ -110,6 +111,7 @@ struct FusedLaunch {
   FailList F;            // failed batch indices
   Stats st;
   int blocks;            // slots
+  int num_sms = 0;
 };
 
 // IC sets with very large edge work: one 1024-thread CTA per set, the CTA's
@@ -168,8 +170,9 @@ struct SpreadShape {
 SpreadShape spread_shape(uint32_t n, bool lt);
 void launch_spread(const SpreadLaunch &L, bool lt, cudaStream_t stream);
 void launch_ic_fused(const FusedLaunch &L, cudaStream_t stream);
-// Resident fused CTAs per SM for a colour width (occupancy API).
-int fused_ctas_per_sm(uint32_t colors);
+// Resident fused CTAs per SM (of 512 threads; with one slot an SM or less they
+// have 1024).
+constexpr int kFusedCtasPerSm = 2;
 
 // Synthetic graphs on the device (kernels_graphgen.cu).
 inline uint32_t prob_u32_host(double p) {

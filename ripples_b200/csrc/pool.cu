@@ -587,7 +587,7 @@ static int sample_fused(rip_pool *p, uint64_t seed, uint64_t first,
   avail += p->f_vis.bytes + p->f_pend.bytes + p->f_flag.bytes + p->f_log.bytes;
   uint64_t fit = (avail / 2) / std::max<size_t>(per_slot, 1);
   uint64_t want = p->fused_slots ? p->fused_slots
-                                 : (uint64_t)c->num_sms * fused_ctas_per_sm(colors);
+                                 : (uint64_t)c->num_sms * kFusedCtasPerSm;
   uint32_t slots = (uint32_t)std::max<uint64_t>(1, std::min<uint64_t>(want, fit));
   if (p->f_vis.p && p->f_cw == cw && p->f_lcap == lcap && p->f_slots >= 1 &&
       p->f_slots <= slots)
@@ -629,6 +629,7 @@ static int sample_fused(rip_pool *p, uint64_t seed, uint64_t first,
     L.F = FailList{ptr<uint32_t>(p->ids_a), &dm->fail_count, &dm->first_bad};
     L.st = Stats{dm->stats};
     L.blocks = (int)std::min<uint32_t>(p->f_slots, nb);
+    L.num_sms = c->num_sms;
     CK(c, cudaEventRecord(c->ev0, c->stream));
     launch_ic_fused(L, c->stream);
     CK(c, cudaGetLastError());
@@ -864,18 +865,29 @@ extern "C" int rip_sample(rip_pool *p, uint64_t seed, uint64_t count,
   TRY(ensure_sets(p, first + count));
   PoolMeta m;
   TRY(read_meta(p, m));
-  if (m.stats[2] == 0 && count > 4096) {
-    // Fresh pool: sample a pilot of 1024 sets first so the pool is sized from
-    // a measured mean set size (the sets are the same either way).
-    TRY(rip_sample(p, seed, 1024, sampler));
-    return rip_sample(p, seed, count - 1024, sampler);
-  }
+  const bool fused = p->g->model == RIP_MODEL_IC &&
+                     (sampler == RIP_SAMPLER_FUSED ||
+                      (sampler == RIP_SAMPLER_AUTO && p->auto_sampler == RIP_SAMPLER_FUSED));
   double mean = m.stats[2] ? (double)m.stats[3] / (double)m.stats[2] : 8.0;
+  if (m.stats[2] == 0 && count > 4096) {
+    // A fused batch is one CTA's chain of levels, as long in a pilot of a few
+    // batches as in a launch that fills the device (2^14 vertices, 128 colours:
+    // 2.7 ms for 1024 sets, 3.4 for 19 000): up to 64 MB of pool, room for 256
+    // members a set is taken instead (what overflows it is sampled again, as
+    // after a pilot that guessed low).
+    const uint64_t avail = c->budget > c->used ? c->budget - c->used : 0;
+    if (fused && count <= (1u << 16) && avail / 4 >= count * 1024) {
+      mean = 256.0;
+    } else {
+      // Fresh pool: sample a pilot of 1024 sets first so the pool is sized from
+      // a measured mean set size (the sets are the same either way).
+      TRY(rip_sample(p, seed, 1024, sampler));
+      return rip_sample(p, seed, count - 1024, sampler);
+    }
+  }
   TRY(ensure_elems(p, p->num_elems + (uint64_t)(mean * 1.25 * count) + 1024));
   int rc;
-  const bool fused = sampler == RIP_SAMPLER_FUSED ||
-                     (sampler == RIP_SAMPLER_AUTO && p->auto_sampler == RIP_SAMPLER_FUSED);
-  if (p->g->model == RIP_MODEL_IC && fused)
+  if (fused)
     rc = sample_fused(p, seed, first, (uint32_t)count);
   else
     rc = sample_warp_per_set(p, seed, first, (uint32_t)count, nullptr);

@@ -221,3 +221,27 @@ def test_spread_lt_swept_and_scanned(ctx, n):
         assert np.array_equal(sizes, o_sizes) and np.array_equal(levels, o_levels)
     bg.close()
     fg.close()
+
+
+@pytest.mark.parametrize("grid", [False, True])
+@pytest.mark.parametrize("colors,sets", [(64, 60), (128, 300), (256, 500), (256, 4500)])
+def test_colour_pairs(ctx, grid, colors, sets):
+    """Multi-colour levels: masks of one set and of all 256, lists around a
+    window's and a tile's blocks, more long entries in a level than a CTA lists;
+    a fresh pool that its sets overflow."""
+    lengths = [1, 7, 8, 9, 16, 31, 63, 127, 128, 129, 250, 1016, 1024, 1025, 4099]
+    g = hub_graph(400, lengths, [0.02, 0.03, 1e-3, 1.0])
+    dg = rb.DeviceGraph(ctx, g, "IC")
+    p = rb.Pool(dg)
+    p.configure(colors=colors)
+    if grid:  # batches of the whole grid
+        p.heavy_batch(1)
+        p.work_caps(64, 0)
+    p.sample(sets, seed=9, sampler=rb.SAMPLER_PLAIN if grid else rb.SAMPLER_FUSED)
+    off, vtx = p.export()
+    thr = O.pack("IC", g.index, g.weights)
+    ooff, ovtx, ost = O.sample("IC", g.n, g.index, g.src, thr, 9, 0, sets)
+    assert np.array_equal(off, ooff) and np.array_equal(vtx, ovtx)
+    st = p.stats()
+    assert st[4] == ost[0] and st[5] == ost[1]
+    dg.close()

@@ -49,18 +49,19 @@ struct GiantLaunch {
   uint32_t *pflag = nullptr;           // n, zero between batches
   uint32_t *front = nullptr, *front_next = nullptr, *touched = nullptr;  // n each
   uint64_t *masks = nullptr;           // n * cw: the current level's colours per entry
-  uint32_t *ng = nullptr;              // n: coin blocks per entry
-  uint64_t *goff = nullptr;            // n + 1: exclusive scan of ng
-  unsigned int *ctr = nullptr;         // [0] next-frontier tail, [1] touched count
+  uint2 *items = nullptr;              // giant_items(n, m): the level's work
+  unsigned int *ctr = nullptr;         // [0] touched count, [1] next frontier's, [2] items
   uint32_t *sizes = nullptr, *fill = nullptr;  // per colour
   unsigned long long *starts = nullptr;        // per colour: pool offset
   unsigned long long *stats = nullptr;         // the pool's counters
 };
-// what: 0 seed roots, 1 level prep (n_items = frontier size), 2 expand
-// (n_items = frontier size, level), 3 per-colour sizes, 4 scatter (n_items =
-// touched), 5 set offsets/lengths
+// what: 0 seed roots, 1 level prep (n_items = frontier size), 2 expand (level),
+// 3 per-colour sizes, 4 scatter (n_items = touched), 5 set offsets/lengths
 void launch_giant(int what, int cw, const GiantLaunch &L, uint32_t n_items, uint32_t level,
                   int blocks, cudaStream_t s);
+// Work items a level may need: a window of entries, or kPairTile (pairs.cuh) or
+// more coin blocks of one entry.
+inline uint64_t giant_items(uint64_t n, uint64_t m) { return n + (m / 8 + 2 * n) / 16 + 1; }
 
 // One IMM instance of a multi-instance launch.
 struct InstanceDesc {

@@ -341,10 +341,10 @@ static int sample_giant(rip_pool *p, uint64_t seed, uint64_t first,
     TRY(dalloc(c, p->g_state, st_bytes));
     CK(c, cudaMemsetAsync(p->g_state.p, 0, st_bytes, c->stream));
   }
-  // lists: front | next | touched | ng (n u32 each) | masks (n * 4 words) |
-  // goff (n + 1) | scan sums
-  const size_t sums = scan_block_sums_needed((uint32_t)n);
-  const size_t li_bytes = n * 4 * 4 + n * CWMAX * 8 + (n + 1) * 8 + sums * 8;
+  // lists: front | next | touched (n u32 each, 32-byte aligned) | masks (n * 4
+  // words) | work items
+  const size_t n4 = (n * 4 + 31) & ~(size_t)31;
+  const size_t li_bytes = 3 * n4 + n * CWMAX * 8 + giant_items(n, g->m) * sizeof(uint2);
   TRY(dalloc(c, p->g_lists, li_bytes));
   // per colour: set ids (u64) | starts (u64) | sizes | fill (u32) | counters
   TRY(dalloc(c, p->g_col, MAXCOL * 24 + 256));
@@ -358,12 +358,10 @@ static int sample_giant(rip_pool *p, uint64_t seed, uint64_t first,
   L.pend = reinterpret_cast<uint64_t *>(st + n * CWMAX * 8);
   L.pflag = reinterpret_cast<uint32_t *>(st + n * CWMAX * 16);
   L.front = reinterpret_cast<uint32_t *>(li);
-  L.front_next = reinterpret_cast<uint32_t *>(li + n * 4);
-  L.touched = reinterpret_cast<uint32_t *>(li + n * 8);
-  L.ng = reinterpret_cast<uint32_t *>(li + n * 12);
-  L.masks = reinterpret_cast<uint64_t *>(li + n * 16);
-  L.goff = reinterpret_cast<uint64_t *>(li + n * 16 + n * CWMAX * 8);
-  uint64_t *d_sums = reinterpret_cast<uint64_t *>(li + n * 16 + n * CWMAX * 8 + (n + 1) * 8);
+  L.front_next = reinterpret_cast<uint32_t *>(li + n4);
+  L.touched = reinterpret_cast<uint32_t *>(li + 2 * n4);
+  L.masks = reinterpret_cast<uint64_t *>(li + 3 * n4);
+  L.items = reinterpret_cast<uint2 *>(li + 3 * n4 + n * CWMAX * 8);
   L.set_ids = reinterpret_cast<const uint64_t *>(co);
   L.starts = reinterpret_cast<unsigned long long *>(co + MAXCOL * 8);
   L.sizes = reinterpret_cast<uint32_t *>(co + MAXCOL * 16);
@@ -401,19 +399,18 @@ static int sample_giant(rip_pool *p, uint64_t seed, uint64_t first,
     unsigned int hc[2] = {0, 0};
     CK(c, cudaMemcpyAsync(hc, L.ctr, 8, cudaMemcpyDeviceToHost, c->stream));
     CK(c, cudaStreamSynchronize(c->stream));
-    uint32_t nf = hc[0];
+    uint32_t nf = hc[1];
     for (uint32_t level = 1; nf > 0; ++level) {
+      CK(c, cudaMemsetAsync(L.ctr + 1, 0, 8, c->stream));
       launch_giant(1, cw, L, nf, level, blocks, c->stream);
-      launch_exclusive_scan(L.ng, L.goff, nf, d_sums, c->stream);
-      CK(c, cudaMemsetAsync(L.ctr, 0, 4, c->stream));
       launch_giant(2, cw, L, nf, level, blocks, c->stream);
       CK(c, cudaGetLastError());
       CK(c, cudaMemcpyAsync(hc, L.ctr, 8, cudaMemcpyDeviceToHost, c->stream));
       CK(c, cudaStreamSynchronize(c->stream));
       std::swap(L.front, L.front_next);
-      nf = hc[0];
+      nf = hc[1];
     }
-    const uint32_t nt = hc[1];
+    const uint32_t nt = hc[0];
     launch_giant(3, cw, L, nt, 0, blocks, c->stream);
     CK(c, cudaMemcpyAsync(sizes.data(), L.sizes, 4 * ncol, cudaMemcpyDeviceToHost, c->stream));
     CK(c, cudaStreamSynchronize(c->stream));

@@ -302,7 +302,7 @@ giant_expand_kernel(const __grid_constant__ GiantLaunch L, uint32_t level) {
   }
 }
 
-constexpr uint32_t GIANT_CHUNK = 2048;  // touched vertices per block in compaction
+constexpr uint32_t GIANT_CHUNK = 512;  // touched vertices per block in compaction
 
 // Members per colour (block-local histograms, one global add per colour).
 template <int CW>
@@ -327,51 +327,71 @@ __global__ void __launch_bounds__(256) giant_sizes_kernel(GiantLaunch L, uint32_
     if (s_cnt[c]) atomicAdd(L.sizes + c, s_cnt[c]);
 }
 
+// Lane j's result: bit j of every lane's x (a 32 x 32 bit transpose).
+__device__ __forceinline__ uint32_t warp_transpose(uint32_t x) {
+  constexpr uint32_t keep[5] = {0x0000FFFFu, 0x00FF00FFu, 0x0F0F0F0Fu, 0x33333333u, 0x55555555u};
+#pragma unroll
+  for (int k = 0; k < 5; ++k) {
+    const uint32_t s = 16u >> k, m = keep[k], y = __shfl_xor_sync(FULL, x, s);
+    x = lane_id() & s ? (x & ~m) | ((y >> s) & m) : (x & m) | ((y & m) << s);
+  }
+  return x;
+}
+
 // Writes each member into its set's pool range and clears the batch's state.
-// A block takes GIANT_CHUNK touched vertices: counts them per colour,
-// reserves a slice of every colour's range with one atomic each, then places
-// them; positions inside a set are arbitrary (set contents are compared as
-// sets).
+// A block takes GIANT_CHUNK touched vertices: counts them per colour, reserves a
+// slice of every colour's range with one atomic each, then places them;
+// positions inside a set are arbitrary (set contents are compared as sets).  A
+// warp has 32 vertices' masks, transposed: colour by colour, the lanes of its
+// members write side by side.  (A thread that walked its vertex's mask wrote
+// each member to a sector of its own: 0.51 ms for 256 sets of 45 000 members,
+// 0.07 this way, 2.6 TB/s of stores.)
 template <int CW>
 __global__ void __launch_bounds__(256) giant_scatter_kernel(GiantLaunch L, uint32_t nt) {
+  constexpr uint32_t NW = 2 * CW, GROUPS = GIANT_CHUNK / 256;  // groups of 32 a warp
   __shared__ uint32_t s_cnt[64 * CW];
   __shared__ unsigned long long s_at[64 * CW];
-  for (uint32_t c0 = blockIdx.x * GIANT_CHUNK; c0 < nt; c0 += gridDim.x * GIANT_CHUNK) {
-    const uint32_t c1 = min(nt, c0 + GIANT_CHUNK);
+  const uint32_t lane = lane_id(), wid = threadIdx.x >> 5;
+  for (uint64_t c0 = (uint64_t)blockIdx.x * GIANT_CHUNK; c0 < nt;
+       c0 += (uint64_t)gridDim.x * GIANT_CHUNK) {
     for (uint32_t c = threadIdx.x; c < 64 * CW; c += blockDim.x) s_cnt[c] = 0;
     __syncthreads();
-    for (uint32_t i = c0 + threadIdx.x; i < c1; i += blockDim.x) {
-      const uint32_t v = L.touched[i];
+    uint32_t v[GROUPS], has[GROUPS][NW], pos[GROUPS][NW];
 #pragma unroll
-      for (int w = 0; w < CW; ++w) {
-        uint64_t m = L.vis[(size_t)v * CW + w];
-        while (m) {
-          const int bi = __ffsll((long long)m) - 1;
-          m &= m - 1;
-          atomicAdd(&s_cnt[w * 64 + bi], 1u);
-        }
+    for (uint32_t g = 0; g < GROUPS; ++g) {
+      const uint64_t i = c0 + (wid * GROUPS + g) * 32 + lane;
+      uint64_t m[CW], zero[CW];
+#pragma unroll
+      for (int w = 0; w < CW; ++w) m[w] = zero[w] = 0;
+      v[g] = 0;
+      if (i < nt) {
+        v[g] = L.touched[i];
+        load_mask<CW>(L.vis + (size_t)v[g] * CW, m);
+        store_mask<CW>(L.vis + (size_t)v[g] * CW, zero);
+        L.pflag[v[g]] = 0u;
+      }
+#pragma unroll
+      for (uint32_t w = 0; w < NW; ++w) {
+        has[g][w] = warp_transpose((uint32_t)(m[w >> 1] >> (32 * (w & 1))));
+        pos[g][w] = has[g][w] ? atomicAdd(&s_cnt[w * 32 + lane], (uint32_t)__popc(has[g][w])) : 0u;
       }
     }
     __syncthreads();
-    for (uint32_t c = threadIdx.x; c < L.ncol; c += blockDim.x) {
+    for (uint32_t c = threadIdx.x; c < L.ncol; c += blockDim.x)
       s_at[c] = s_cnt[c] ? L.starts[c] + atomicAdd(L.fill + c, s_cnt[c]) : 0ull;
-      s_cnt[c] = 0;
-    }
     __syncthreads();
-    for (uint32_t i = c0 + threadIdx.x; i < c1; i += blockDim.x) {
-      const uint32_t v = L.touched[i];
 #pragma unroll
-      for (int w = 0; w < CW; ++w) {
-        uint64_t m = L.vis[(size_t)v * CW + w];
-        L.vis[(size_t)v * CW + w] = 0ull;
-        while (m) {
-          const int bi = __ffsll((long long)m) - 1;
-          m &= m - 1;
-          const uint32_t c = w * 64 + bi;
-          L.P.vtx[s_at[c] + atomicAdd(&s_cnt[c], 1u)] = v;
+    for (uint32_t g = 0; g < GROUPS; ++g) {
+#pragma unroll
+      for (uint32_t w = 0; w < NW; ++w) {
+        for (uint32_t left = __ballot_sync(FULL, has[g][w] != 0); left; left &= left - 1) {
+          const uint32_t j = __ffs(left) - 1;
+          const uint32_t members = __shfl_sync(FULL, has[g][w], j);
+          const uint32_t at = __shfl_sync(FULL, pos[g][w], j);
+          if (members >> lane & 1u)
+            L.P.vtx[s_at[w * 32 + j] + at + __popc(members & lanemask_lt_g())] = v[g];
         }
       }
-      L.pflag[v] = 0u;
     }
     __syncthreads();
   }

@@ -156,6 +156,67 @@ __device__ __forceinline__ uint32_t ic_block_live(const DevGraph &G, Key key, ui
   return live;
 }
 
+// The source of live edge h (of eight) that tile_live left in src.
+__device__ __forceinline__ uint32_t tile_source(const uint32_t *src, uint32_t h) {
+  uint32_t u = src[0];
+#pragma unroll
+  for (uint32_t i = 1; i < 8; ++i)
+    if (h == i) u = src[i];
+  return u;
+}
+
+// Live edges of the 32 consecutive coin blocks from b0 on of the in-list
+// [ob, oe), whose records hold the thresholds; called by the whole warp.  A
+// lane that reads its own block's records strides 64 bytes: 64 L1 wavefronts a
+// tile, 256 issue cycles of a scheduler's share of L1 against 90 of coins.  So
+// the lanes read the tile's records side by side, two edges a lane and step (16
+// wavefronts), and pass each other the coins through shared memory: word w of
+// the tile's coins belongs to its edges 2w and 2w + 1.  Bit 2i + j of the result
+// is edge 8 b0 + 64 i + 2 lane + j, src[2i + j] its source.  `ahead` of the four
+// steps' records are read before the coins are drawn.
+template <int ahead, class RK, class Fine>
+__device__ __forceinline__ uint32_t tile_live(const DevGraph &G, const RK &rk,
+                                              const CoinSet &cs, uint32_t b0, uint32_t ob,
+                                              uint32_t oe, uint4 *coins, uint32_t *src,
+                                              Fine &&fine) {
+  const uint32_t lane = lane_id(), e0 = (b0 << 3) + 2 * lane;
+  const uint4 *rp = reinterpret_cast<const uint4 *>(G.edges + ((size_t)b0 << 3)) + lane;
+  uint4 rec[4];
+  auto read = [&](int i) {
+    const uint32_t e = e0 + 64 * i;
+    rec[i] = e < oe && e + 1 >= ob ? __ldg(rp + 32 * i) : make_uint4(0, 0, 0, 0);
+  };
+#pragma unroll
+  for (int i = 0; i < ahead; ++i) read(i);
+  const u32x4 c = coin_block(rk, cs, b0 + lane);
+  __syncwarp();
+  coins[lane] = make_uint4(c.x, c.y, c.z, c.w);
+  __syncwarp();
+#pragma unroll
+  for (int i = ahead; i < 4; ++i) read(i);
+  const uint32_t *word = reinterpret_cast<const uint32_t *>(coins) + lane;
+  uint32_t live = 0, tie = 0;
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const uint32_t e = e0 + 64 * i, w = word[32 * i];
+    const uint32_t c0 = w & 0xFFFFu, c1 = w >> 16;
+    const uint32_t t0 = e >= ob ? rec[i].y >> 16 : 0u, t1 = e + 1 < oe ? rec[i].w >> 16 : 0u;
+    src[2 * i] = rec[i].x;
+    src[2 * i + 1] = rec[i].z;
+    if (c0 < t0) live |= 1u << (2 * i);
+    else if (c0 == t0) tie |= 1u << (2 * i);
+    if (c1 < t1) live |= 2u << (2 * i);
+    else if (c1 == t1) tie |= 2u << (2 * i);
+  }
+  while (tie) {  // one edge in 65 536 (and those out of the list): the fine half decides
+    const uint32_t h = __ffs(tie) - 1;
+    tie &= tie - 1;
+    const uint32_t e = e0 + 64 * (h >> 1) + (h & 1);
+    if (e >= ob && e < oe && fine(e) < (__ldg(&G.edges[e].y) & 0xFFFFu)) live |= 1u << h;
+  }
+  return live;
+}
+
 // Loads the 4 edge records of group g (32-byte aligned).
 __device__ __forceinline__ void load_group(const uint2 *edges, uint32_t g,
                                            uint2 rec[4]) {

@@ -345,7 +345,7 @@ __device__ __forceinline__ uint32_t warp_transpose(uint32_t x) {
 // warp has 32 vertices' masks, transposed: colour by colour, the lanes of its
 // members write side by side.  (A thread that walked its vertex's mask wrote
 // each member to a sector of its own: 0.51 ms for 256 sets of 45 000 members,
-// 0.07 this way, 2.6 TB/s of stores.)
+// 0.07 this way.)
 template <int CW>
 __global__ void __launch_bounds__(256) giant_scatter_kernel(GiantLaunch L, uint32_t nt) {
   constexpr uint32_t NW = 2 * CW, GROUPS = GIANT_CHUNK / 256;  // groups of 32 a warp

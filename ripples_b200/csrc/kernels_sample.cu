@@ -42,6 +42,7 @@ struct WarpCtx {
   uint32_t *q;   // queue, qcap entries
   uint32_t qcap;
   uint32_t *seen = nullptr;  // LT: the walk's revisit filter (shared memory)
+  uint4 *coins = nullptr;    // IC: a tile's coins (shared memory)
 };
 
 // Writes the finished set to the pool (unless it overflowed) and clears the
@@ -184,6 +185,24 @@ __device__ __forceinline__ SetOutcome ic_plain_set(const DevGraph &G, Key key, c
       const uint32_t lvt = __shfl_sync(FULL, vt, L);
       const uint32_t b_last = (le - 1) >> 3;
       for (uint32_t base = lb >> 3; base <= b_last && !overflow; base += 32) {
+        if (lvt == 0) {
+          uint32_t src[8];
+          uint32_t live = tile_live<2>(G, rk, cs, base, lb, le, W.coins, src,
+                                       [&](uint32_t e) { return ic_fine_call(key, e, s); });
+          while (__any_sync(FULL, live != 0)) {
+            bool isnew = false;
+            uint32_t nu = 0;
+            if (live) {
+              nu = tile_source(src, __ffs(live) - 1);
+              live &= live - 1;
+              const uint32_t bit = 1u << (nu & 31);
+              isnew = !(atomicOr(&W.bm[nu >> 5], bit) & bit);
+            }
+            append_one(isnew, nu);
+          }
+          __syncwarp();
+          continue;
+        }
         const uint32_t b = base + lane;
         const uint32_t live = b <= b_last ? block_live(b, lb, le, lvt) : 0u;
         take_live(b, live, lvt != 0);
@@ -337,7 +356,9 @@ ic_plain_kernel(DevGraph G, DevPool P, Key key, const __grid_constant__ RoundKey
                 uint64_t work_cap, FailList F, Stats st) {
   const uint32_t lane = lane_id();
   const uint64_t w = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  __shared__ uint4 s_coin[256];
   WarpCtx W{bitmaps + w * bm_words, queues + w * (uint64_t)qcap, qcap};
+  W.coins = s_coin + (threadIdx.x & ~31u);
   unsigned long long n_exp = 0, n_edges = 0, n_sets = 0, n_elems = 0, n_uedges = 0, n_usrc = 0;
 
   for (;;) {
@@ -423,13 +444,18 @@ lt_walk_kernel(DevGraph G, DevPool P, Key key, uint64_t first, uint32_t count,
 // from one counter; index i belongs to the instance a with
 // prefix[a] <= i < prefix[a+1] and is that instance's set first_a + i -
 // prefix[a], grown with that instance's graph, model and seed into its pool.
-__global__ void __launch_bounds__(256)
+// Four blocks an SM (64 registers, some spilled): the walks and sweeps wait for
+// memory, and three blocks of 80 registers took 20.0 ms where four take 19.0
+// (twelve queries' rounds as one batch).
+__global__ void __launch_bounds__(256, 4)
 multi_sample_kernel(MultiLaunch L) {
   const uint32_t lane = lane_id();
   const uint64_t w = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   __shared__ uint32_t s_seen[8][kSeenWords];
+  __shared__ uint4 s_coin[256];
   WarpCtx W{L.bitmaps + w * L.bm_words, L.queues + w * (uint64_t)L.qcap, L.qcap,
             s_seen[threadIdx.x >> 5]};
+  W.coins = s_coin + (threadIdx.x & ~31u);
   // counters of the instance the warp is on, flushed when it moves on
   uint32_t cur = ~0u;
   unsigned long long n_exp = 0, n_edges = 0, n_sets = 0, n_elems = 0, n_uedges = 0, n_usrc = 0;

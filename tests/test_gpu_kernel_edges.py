@@ -245,3 +245,31 @@ def test_colour_pairs(ctx, grid, colors, sets):
     st = p.stats()
     assert st[4] == ost[0] and st[5] == ost[1]
     dg.close()
+
+
+@pytest.mark.parametrize("threads", [0, 128, 512, 1024])
+def test_record_tiles(ctx, threads):
+    """Lists with a threshold per edge, read 32 coin blocks at a time: ends on and
+    off blocks, tiles and the listing length; one warp per set and CTAs."""
+    r = np.random.RandomState(4)
+    g = hub_graph(300, [7, 247, 248, 249, 255, 256, 257, 263, 511, 513, 1000, 1025, 4099], [0.5])
+    w = (r.rand(g.m) * 0.01).astype(np.float32)
+    w[r.rand(g.m) < 0.002] = 1.0
+    w[-5000:] = 0.4
+    g = rb.HostGraph(g.n, g.index, g.src, w)
+    dg = rb.DeviceGraph(ctx, g, "IC")
+    p = rb.Pool(dg)
+    p.heavy_batch(0)
+    if threads:
+        p.heavy_block(threads)
+        p.work_caps(64, 0)
+    else:
+        p.work_caps(0, 0)  # no set is handed over
+    p.sample(400, seed=9, sampler=rb.SAMPLER_PLAIN)
+    off, vtx = p.export()
+    ooff, ovtx, ost = O.sample("IC", g.n, g.index, g.src, O.pack("IC", g.index, g.weights), 9, 0,
+                               400)
+    assert np.array_equal(off, ooff) and np.array_equal(vtx, ovtx)
+    st = p.stats()
+    assert st[4] == ost[0] and st[5] == ost[1]
+    dg.close()

@@ -156,15 +156,6 @@ __device__ __forceinline__ uint32_t ic_block_live(const DevGraph &G, Key key, ui
   return live;
 }
 
-// The source of live edge h (of eight) that tile_live left in src.
-__device__ __forceinline__ uint32_t tile_source(const uint32_t *src, uint32_t h) {
-  uint32_t u = src[0];
-#pragma unroll
-  for (uint32_t i = 1; i < 8; ++i)
-    if (h == i) u = src[i];
-  return u;
-}
-
 // Live edges of the 32 consecutive coin blocks from b0 on of the in-list
 // [ob, oe), whose records hold the thresholds; called by the whole warp.  A
 // lane that reads its own block's records strides 64 bytes: 64 L1 wavefronts a
@@ -172,13 +163,11 @@ __device__ __forceinline__ uint32_t tile_source(const uint32_t *src, uint32_t h)
 // the lanes read the tile's records side by side, two edges a lane and step (16
 // wavefronts), and pass each other the coins through shared memory: word w of
 // the tile's coins belongs to its edges 2w and 2w + 1.  Bit 2i + j of the result
-// is edge 8 b0 + 64 i + 2 lane + j, src[2i + j] its source.  `ahead` of the four
-// steps' records are read before the coins are drawn.
+// is edge 8 b0 + 64 i + 2 lane + j.  `ahead` of the four steps' records are read before the coins are drawn.
 template <int ahead, class RK, class Fine>
 __device__ __forceinline__ uint32_t tile_live(const DevGraph &G, const RK &rk,
                                               const CoinSet &cs, uint32_t b0, uint32_t ob,
-                                              uint32_t oe, uint4 *coins, uint32_t *src,
-                                              Fine &&fine) {
+                                              uint32_t oe, uint4 *coins, Fine &&fine) {
   const uint32_t lane = lane_id(), e0 = (b0 << 3) + 2 * lane;
   const uint4 *rp = reinterpret_cast<const uint4 *>(G.edges + ((size_t)b0 << 3)) + lane;
   uint4 rec[4];
@@ -201,8 +190,6 @@ __device__ __forceinline__ uint32_t tile_live(const DevGraph &G, const RK &rk,
     const uint32_t e = e0 + 64 * i, w = word[32 * i];
     const uint32_t c0 = w & 0xFFFFu, c1 = w >> 16;
     const uint32_t t0 = e >= ob ? rec[i].y >> 16 : 0u, t1 = e + 1 < oe ? rec[i].w >> 16 : 0u;
-    src[2 * i] = rec[i].x;
-    src[2 * i + 1] = rec[i].z;
     if (c0 < t0) live |= 1u << (2 * i);
     else if (c0 == t0) tie |= 1u << (2 * i);
     if (c1 < t1) live |= 2u << (2 * i);

@@ -115,8 +115,8 @@ struct FusedLaunch {
   int num_sms = 0;
 };
 
-// IC sets with very large edge work: one 1024-thread CTA per set, the CTA's
-// warps splitting every level's edge groups (kernels_bigset.cu).
+// IC sets with very large edge work, one CTA of 128 to 1024 threads each
+// (kernels_bigset.cu).
 struct BigLaunch {
   DevGraph G{};
   DevPool P{};

@@ -144,6 +144,21 @@ extern "C" int rip_selftest_heap(uint64_t n, uint32_t max_count, uint64_t seed) 
   return 1;
 }
 
+// Diagnostic: the counts a reference-heap selection with this histogram
+// (kCountBuckets words) keeps, build after build, until it keeps all: smallest
+// count and number of them; returns the builds, `room` when they do not end.
+extern "C" int rip_selftest_keep(const uint32_t *hist, uint32_t *smallest, uint64_t *items,
+                                 uint32_t room) {
+  KeptCounts kept;
+  for (uint32_t i = 0; i < room; ++i) {
+    kept.grow(hist, i ? keep_next(kept) : kKeepFirst);
+    smallest[i] = kept.smallest();
+    items[i] = kept.items;
+    if (smallest[i] == 0) return (int)i + 1;
+  }
+  return (int)room;
+}
+
 // The counts left by the last selection still sit in the count buffer; bring
 // them to the host before anything overwrites that buffer.
 static int settle_last_counts(rip_pool *p) {
@@ -297,12 +312,11 @@ extern "C" int rip_select(rip_pool *p, uint64_t S, uint32_t k, int tiebreak,
     // InitHeapStorage + std::priority_queue(cmp, std::move(storage)), as the
     // reference builds its heap (streaming_find_most_influential.h:541-544;
     // counting.h:196-206), of which the host takes the items that can decide a
-    // pick (sparse_heap.h): those whose count is at least K, about kKeep of
+    // pick (sparse_heap.h): those whose count is at least K, about kKeepFirst of
     // them at first, and more -- the pops so far repeated on the larger heap --
     // if the gains fall below K.  At n = 2^24 the whole heap was 128 MB over
     // the bus a selection (4.2 of 14.5 ms), and every pop sank to a leaf 24
     // levels down.
-    constexpr uint32_t kKeep = 16384;
     constexpr uint32_t kGone = 0xFFFFFFFFu;  // log: the popped item stayed out (a seed)
     SparseHeap &heap = c->heap;
     std::vector<uint32_t> ids;  // vertex by item id
@@ -310,17 +324,15 @@ extern "C" int rip_select(rip_pool *p, uint64_t S, uint32_t k, int tiebreak,
     // an item's count as last fetched, and the fetch (pick) that brought it
     std::vector<uint32_t> cnt, cnt_at;
     uint32_t fetch = 0;
+    KeptCounts kept;
     uint32_t K = 0, R = 0;
     TRY(dalloc(c, p->d_heap, sizeof(uint2) * (size_t)n));
     if (!c->h_list) c->h_list = new PinnedMem();
-    // Keeps about `want` items: the buckets of the largest counts that hold
-    // no more than that (the first such bucket at least).
+    // Keeps more items: the next smaller counts, about `want` of all.
     auto build = [&](uint64_t want, const uint32_t *d_count) -> int {
-      uint64_t kept = 0;
-      uint32_t b = kCountBuckets;
-      while (b > 0 && (kept == 0 || kept + hist[b - 1] <= want)) kept += hist[--b];
-      K = count_bucket_low(b);
-      R = (uint32_t)kept;
+      kept.grow(hist, want);
+      K = kept.smallest();
+      R = (uint32_t)kept.items;
       launch_make_heap(d_count, n, ptr<uint2>(p->d_heap), K, c->stream);
       const size_t words = 3 * (size_t)R;
       TRY(dalloc(c, p->d_list, sizeof(uint32_t) * (words + 1)));
@@ -344,7 +356,7 @@ extern "C" int rip_select(rip_pool *p, uint64_t S, uint32_t k, int tiebreak,
       }
       return RIP_OK;
     };
-    TRY(build(kKeep, ptr<uint32_t>(p->count)));
+    TRY(build(kKeepFirst, ptr<uint32_t>(p->count)));
     p->sel_prof[1] += ms_since(t_h0);
     const auto t_p0 = clk::now();
     // The lazy pops of a pick only read the current counts of heap items keyed
@@ -451,7 +463,7 @@ extern "C" int rip_select(rip_pool *p, uint64_t S, uint32_t k, int tiebreak,
     // start is still in the heap array.
     auto keep_more = [&]() -> int {
       launch_heap_counts(ptr<uint2>(p->d_heap), n, ptr<uint32_t>(p->inv_cur), c->stream);
-      TRY(build(8ull * R, ptr<uint32_t>(p->inv_cur)));
+      TRY(build(keep_next(kept), ptr<uint32_t>(p->inv_cur)));
       prefetched = false;
       return first || fresh_all ? RIP_OK : fetch_candidates(out_gains.back());
     };

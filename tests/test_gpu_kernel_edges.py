@@ -83,14 +83,28 @@ def test_selection_over_set_lengths(ctx, tie, copies, n):
     dg.close()
 
 
-@pytest.mark.parametrize("k,hot", [(6, 40), (60, 25000)])
+@pytest.mark.parametrize("k,hot", [(6, 40), (30, 40), (60, 25000)])
 def test_reference_heap_keeps_more_items(ctx, k, hot):
     """The first seed covers most sets, so the gains fall below the counts the
-    host kept at first (n above what it keeps): the kept heap grows, down to
-    counts of one and, once every set with members is covered, of zero."""
+    host kept at first (n above what it keeps).  k = 6: they stay within them; 30:
+    every set with members is covered and one without is left, counts of zero,
+    which are some 500 times what was kept; 60: all counts in one step."""
     n, r = 40003, np.random.RandomState(hot)
     sets = [np.concatenate([[0], 1 + r.choice(hot, 30, replace=False)]) for _ in range(900)]
     sets += [np.array([hot + 1 + i, hot + 2 + i]) for i in range(0, 40, 2)] + [np.array([], int)]
+    check_reference_heap(ctx, n, sets, k)
+
+
+def test_reference_heap_keeps_a_large_next_bucket(ctx):
+    """Few vertices in two sets each, many in one: the counts of one are 500 times
+    the kept, and the gains fall to them."""
+    first = 100 + 200 * 250
+    sets = [np.concatenate([[i // 2], 100 + 250 * i + np.arange(250)]) for i in range(200)]
+    sets += [np.array([first + i]) for i in range(40)]
+    check_reference_heap(ctx, 60007, sets, 120)
+
+
+def check_reference_heap(ctx, n, sets, k):
     off = np.zeros(len(sets) + 1, dtype=np.uint64)
     np.cumsum([len(x) for x in sets], out=off[1:])
     vtx = np.concatenate(sets).astype(np.uint32)
@@ -101,6 +115,23 @@ def test_reference_heap_keeps_more_items(ctx, k, hot):
     of, oseeds, ogains, _ = O.select(n, off, vtx, k, rb.TIE_REF_HEAP)
     for guess in (0, 100, 3):  # adaptive, too high, too low first fetches
         p.select_guess(guess)
+        f, seeds, gains = p.select(k, tiebreak=rb.TIE_REF_HEAP)
+        assert f == of and seeds.tolist() == oseeds.tolist() and gains.tolist() == ogains.tolist()
+    dg.close()
+
+
+@pytest.mark.parametrize("model,n,sets,k", [("IC", 1 << 20, 1000, 200), ("LT", 1 << 18, 100, 60)])
+def test_reference_heap_on_few_sampled_sets(ctx, model, n, sets, k):
+    """Few sets on many vertices: nearly all counts are zero, most others one."""
+    g = rb.HostGraph.erdos_renyi(n, 8 * n, seed=3).with_weights(
+        rb.WEIGHTS_WC if model == "IC" else rb.WEIGHTS_LT_NORMALIZED, 1, 0.0, 1.0)
+    dg = rb.DeviceGraph(ctx, g, model)
+    p = rb.Pool(dg)
+    for seed in (1, 2, 3):
+        p.clear()
+        p.sample(sets, seed=seed)
+        off, vtx = p.export()
+        of, oseeds, ogains, _ = O.select(n, off, vtx, k, rb.TIE_REF_HEAP)
         f, seeds, gains = p.select(k, tiebreak=rb.TIE_REF_HEAP)
         assert f == of and seeds.tolist() == oseeds.tolist() and gains.tolist() == ogains.tolist()
     dg.close()

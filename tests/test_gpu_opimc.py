@@ -62,3 +62,21 @@ def test_opimc_matches_oracle(ctx, model, eps, tiebreak):
         r1.close()
         r2.close()
         dg.close()
+
+
+def test_opimc_on_a_large_sparse_graph(ctx):
+    """The first pools hold some hundred sets: the picks reach counts of one, which
+    most of the counted vertices have."""
+    g = rb.HostGraph.erdos_renyi(1 << 20, 8 << 20, seed=5).with_weights(rb.WEIGHTS_WC, 1, 0.0, 1.0)
+    dg = rb.DeviceGraph(ctx, g, "IC")
+    r1, r2 = rb.Pool(dg), rb.Pool(dg)
+    try:
+        seeds, rec = rb.opimc(r1, r2, 50, 0.5, 0.05, seed=7)
+        ref = O.opimc("IC", g.n, g.index, g.src, O.pack("IC", g.index, g.weights), 50, 0.5, 0.05,
+                      seed=7)
+        assert seeds.tolist() == ref["seeds"]
+        assert rec.theta == ref["theta"] and rec.rounds == ref["rounds"]
+    finally:
+        r1.close()
+        r2.close()
+        dg.close()

@@ -146,6 +146,29 @@ def test_parallel_heap_is_libstdcxx_make_heap(n, max_count, seed):
     assert _lib.lib.rip_selftest_heap(n, max_count, seed) == 1
 
 
+@pytest.mark.parametrize("counts", [
+    {0: 2000000, 1: 50000, 2: 300},          # the next bucket holds more than eight times the kept
+    {0: 39922, 1: 40, 100: 40, 900: 1},      # down to 0 for sets without members
+    {1: 1 << 22, 1 << 31: 1, 0xFFFFFFFF: 1}, {0: 5}, {7: 1, 8: 20000, 15: 3, 16: 20000, 17: 1},
+    {c: 30 ** (4 - i) for i, c in enumerate([0, 1, 2, 900, 70000])}])
+def test_kept_counts_fall_with_every_build(counts):
+    """A reference-heap selection whose gains fall below what it keeps asks for
+    more: each build has to reach smaller counts, whatever the histogram."""
+    def bucket(c):
+        e = c.bit_length() - 1
+        return c if c < 8 else ((e - 2) << 3) | ((c >> (e - 3)) & 7)
+    hist = np.zeros(240, np.uint32)
+    for c, many in counts.items():
+        hist[bucket(c)] += many
+    smallest, items = np.zeros(250, np.uint32), np.zeros(250, np.uint64)
+    steps = _lib.lib.rip_selftest_keep(hist.ctypes.data, smallest.ctypes.data, items.ctypes.data,
+                                       250)
+    assert 0 < steps < 250 and smallest[steps - 1] == 0 and items[steps - 1] == sum(counts.values())
+    assert (np.diff(smallest[:steps].astype(np.int64)) < 0).all()
+    for s, i in zip(smallest[:steps], items[:steps]):
+        assert i == sum(m for c, m in counts.items() if c >= s)
+
+
 # ---- graph input files (rip_read_tsv / rip_read_binary) ---------------------
 
 def _write(path, text):

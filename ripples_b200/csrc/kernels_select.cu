@@ -989,16 +989,17 @@ heap_list_kernel(const uint2 *__restrict__ heap, uint32_t n, uint32_t K, uint32_
 
 }  // namespace
 
-void launch_make_heap(const uint32_t *count, uint32_t n, uint2 *heap, uint32_t K,
-                      cudaStream_t stream) {
+cudaError_t launch_make_heap(const uint32_t *count, uint32_t n, uint2 *heap, uint32_t K,
+                             cudaStream_t stream) {
   uint32_t depth = 0;  // levels of the heap
   while (depth < 32 && ((1ull << depth) - 1) < n) ++depth;
   // shared memory holds 2^11 items of a lower stage (16 KB, six blocks an SM)
   // and 2^14 of the top one (128 KB, one block): its sifts are the longest
   constexpr uint32_t kTop = 14, kStage = 11;
-  static const cudaError_t attr = cudaFuncSetAttribute(
+  // (per device: the limit belongs to the current one)
+  const cudaError_t e = cudaFuncSetAttribute(
       heap_stage_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(sizeof(uint2) << kTop));
-  (void)attr;
+  if (e != cudaSuccess) return e;
   while (depth > 0) {
     const bool top = depth <= kTop;
     uint32_t d0 = 0, L = depth, g = 0;
@@ -1016,6 +1017,7 @@ void launch_make_heap(const uint32_t *count, uint32_t n, uint2 *heap, uint32_t K
                                                                              g, K);
     depth = d0;
   }
+  return cudaGetLastError();
 }
 
 void launch_count_hist(const uint32_t *count, uint32_t n, uint32_t *hist, cudaStream_t stream) {

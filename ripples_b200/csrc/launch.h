@@ -251,8 +251,8 @@ void launch_cover_gather(const CoverLaunch &C, const uint32_t *ids, uint32_t nid
 // Builds the selection max-heap of {vertex, count} on the device: the items of
 // K or more element for element where std::make_heap puts them (K = 0: all),
 // the others in any order.
-void launch_make_heap(const uint32_t *count, uint32_t n, uint2 *heap, uint32_t K,
-                      cudaStream_t stream);
+cudaError_t launch_make_heap(const uint32_t *count, uint32_t n, uint2 *heap, uint32_t K,
+                             cudaStream_t stream);
 // Counts by size: eight buckets per power of two (one per value below 16).
 constexpr uint32_t kCountBuckets = 240;
 __host__ __device__ inline uint32_t count_bucket(uint32_t c) {

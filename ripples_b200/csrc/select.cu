@@ -78,9 +78,10 @@ extern "C" int rip_selftest_heap_device(rip_ctx *c, uint64_t n, uint32_t max_cou
     cudaMemcpyAsync(d_cnt.p, cnt.data(), 4 * n, cudaMemcpyHostToDevice, c->stream);
     // the whole heap, then only the items of K or more in their places
     for (uint32_t K : {0u, 1u, max_count / 2, max_count}) {
-      launch_make_heap(ptr<uint32_t>(d_cnt), (uint32_t)n, ptr<uint2>(d_heap), K, c->stream);
+      cudaError_t e = launch_make_heap(ptr<uint32_t>(d_cnt), (uint32_t)n, ptr<uint2>(d_heap), K,
+                                       c->stream);
       cudaMemcpyAsync(got.data(), d_heap.p, 8 * n, cudaMemcpyDeviceToHost, c->stream);
-      cudaError_t e = cudaStreamSynchronize(c->stream);
+      if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
       if (e == cudaSuccess) e = cudaGetLastError();
       if (e != cudaSuccess) {
         rc = set_err(c, RIP_ERR_CUDA, "heap selftest: %s", cudaGetErrorString(e));
@@ -333,7 +334,7 @@ extern "C" int rip_select(rip_pool *p, uint64_t S, uint32_t k, int tiebreak,
       kept.grow(hist, want);
       K = kept.smallest();
       R = (uint32_t)kept.items;
-      launch_make_heap(d_count, n, ptr<uint2>(p->d_heap), K, c->stream);
+      CK(c, launch_make_heap(d_count, n, ptr<uint2>(p->d_heap), K, c->stream));
       const size_t words = 3 * (size_t)R;
       TRY(dalloc(c, p->d_list, sizeof(uint32_t) * (words + 1)));
       TRY(c->h_list->ensure(c, sizeof(uint32_t) * words));

@@ -61,3 +61,20 @@ def test_concurrent_contexts_match_alone(model, g):
     # the queries differ from each other (the comparison is not vacuous)
     assert len({tuple(a[0]) for a in alone}) > 1
     assert np.all([a[1] > 0 for a in alone])
+
+
+def test_reference_heap_on_every_device():
+    """Launch limits belong to a device: selections on each one in turn, in one
+    process, answer alike (a heap of 17 levels needs more than 48 KB a block)."""
+    import torch
+    if torch.cuda.device_count() < 2:
+        pytest.skip("one device")
+    g = rb.HostGraph.rmat(16, 8 << 16, seed=3).with_weights(rb.WEIGHTS_WC, 4, 0.0, 1.0)
+    answers = []
+    for device in range(torch.cuda.device_count()):
+        ctx = rb.Context(device)
+        p = rb.Pool(rb.DeviceGraph(ctx, g, "IC"))
+        p.sample(5000, seed=1)
+        answers.append(p.select(20, tiebreak=rb.TIE_REF_HEAP)[1].tolist())
+        ctx.close()
+    assert all(a == answers[0] for a in answers)

@@ -169,6 +169,15 @@ def test_kept_counts_fall_with_every_build(counts):
         assert i == sum(m for c, m in counts.items() if c >= s)
 
 
+def test_launch_limits_are_set_at_each_launch():
+    """A kernel's shared-memory limit belongs to the device that is current when
+    it is set: set once in the process, it is missing on every other device."""
+    csrc = os.path.join(ROOT, "ripples_b200", "csrc")
+    texts = [open(os.path.join(csrc, f)).read() for f in os.listdir(csrc) if f.endswith(".cu")]
+    assert sum(t.count("cudaFuncSetAttribute(") for t in texts) > 0
+    assert not any(re.search(r"\bstatic\b[^;{]*cudaFuncSetAttribute", t) for t in texts)
+
+
 # ---- graph input files (rip_read_tsv / rip_read_binary) ---------------------
 
 def _write(path, text):

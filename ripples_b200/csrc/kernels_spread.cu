@@ -532,22 +532,27 @@ spread_lt_small_kernel(const __grid_constant__ SpreadLaunch L) {
   if (tid == 0 && reached) atomicAdd(L.total, reached);
 }
 
-// Static shared memory of a spread CTA, rounded up.
-constexpr size_t kSpreadStatic = 4096;
+// Shared memory of an SM's CTAs, and what a spread CTA takes besides its dynamic
+// part (static and reserved, rounded up).
+constexpr size_t kSmShared = 227 * 1024;
+constexpr size_t kSpreadStatic = 5120;
+// Dynamic shared memory of the kernels below at most, by CTAs an SM.
+constexpr size_t kIcShared4 = (kSmShared / 4 - kSpreadStatic) & ~(size_t)15;
+constexpr size_t kIcShared1 = kSmShared - kSpreadStatic;
+constexpr size_t lt_shared(size_t n) { return ((n + 31) / 32 * 8 + 2 * n + 15) & ~(size_t)15; }
+constexpr size_t kLtShared3 = kSmShared / 3 - 2048;
+constexpr size_t kLtShared1 = lt_shared(65536);
 
-template <bool SHARED, int THREADS>
-void launch_ic(const SpreadLaunch &L, size_t shared, cudaStream_t stream) {
-  if (shared)
-    cudaFuncSetAttribute(spread_ic_kernel<SHARED, THREADS>,
-                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shared);
-  spread_ic_kernel<SHARED, THREADS><<<L.blocks, THREADS, shared, stream>>>(L);
-}
-
-template <int THREADS>
-void launch_lt_small(const SpreadLaunch &L, size_t shared, cudaStream_t stream) {
-  cudaFuncSetAttribute(spread_lt_small_kernel<THREADS>,
-                       cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shared);
-  spread_lt_small_kernel<THREADS><<<L.blocks, THREADS, shared, stream>>>(L);
+// The limit set is the kernel's largest shape, not this launch's: it belongs to
+// the kernel, and another thread may launch it for a larger graph meanwhile.
+template <class Kernel>
+cudaError_t launch_shared(Kernel kernel, const SpreadLaunch &L, int threads, size_t shared,
+                          size_t limit, cudaStream_t stream) {
+  const cudaError_t e =
+      cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)limit);
+  if (e != cudaSuccess) return e;
+  kernel<<<L.blocks, threads, shared, stream>>>(L);
+  return cudaGetLastError();
 }
 
 }  // namespace
@@ -563,27 +568,31 @@ void launch_lt_small(const SpreadLaunch &L, size_t shared, cudaStream_t stream) 
 SpreadShape spread_shape(uint32_t n, bool lt) {
   const size_t bitmap = (((size_t)n + 127) / 128) * 16;
   if (lt && n <= 65536) {  // two bitmaps and the kept sources
-    const size_t bytes = (((size_t)n + 31) / 32 * 8 + 2 * (size_t)n + 15) & ~(size_t)15;
-    if (3 * (bytes + 2048) <= 227 * 1024) return SpreadShape{512, 3, bytes};
-    return SpreadShape{1024, 1, bytes};
+    const size_t bytes = lt_shared(n);
+    return bytes <= kLtShared3 ? SpreadShape{512, 3, bytes} : SpreadShape{1024, 1, bytes};
   }
   if (lt) return SpreadShape{SIM_THREADS, 4, 0};
-  if (4 * (bitmap + kSpreadStatic + 1024) <= 227 * 1024) return SpreadShape{512, 4, bitmap};
-  if (bitmap + kSpreadStatic <= 227 * 1024 - 1024) return SpreadShape{1024, 1, bitmap};
+  if (bitmap <= kIcShared4) return SpreadShape{512, 4, bitmap};
+  if (bitmap <= kIcShared1) return SpreadShape{1024, 1, bitmap};
   return SpreadShape{512, 4, 0};
 }
 
-void launch_spread(const SpreadLaunch &L0, bool lt, cudaStream_t stream) {
+cudaError_t launch_spread(const SpreadLaunch &L0, bool lt, cudaStream_t stream) {
   count_launches(1);
   SpreadLaunch L = L0;
   L.rk = round_keys(L.key);
   const SpreadShape s = spread_shape(L.G.n, lt);
-  if (lt && s.shared && s.threads == 1024) launch_lt_small<1024>(L, s.shared, stream);
-  else if (lt && s.shared) launch_lt_small<512>(L, s.shared, stream);
-  else if (lt) spread_lt_kernel<<<L.blocks, SIM_THREADS, 0, stream>>>(L);
-  else if (s.shared && s.threads == 1024) launch_ic<true, 1024>(L, s.shared, stream);
-  else if (s.shared) launch_ic<true, 512>(L, s.shared, stream);
-  else launch_ic<false, 512>(L, 0, stream);
+  if (lt && s.shared && s.threads == 1024)
+    return launch_shared(spread_lt_small_kernel<1024>, L, 1024, s.shared, kLtShared1, stream);
+  if (lt && s.shared)
+    return launch_shared(spread_lt_small_kernel<512>, L, 512, s.shared, kLtShared3, stream);
+  if (!lt && s.shared && s.threads == 1024)
+    return launch_shared(spread_ic_kernel<true, 1024>, L, 1024, s.shared, kIcShared1, stream);
+  if (!lt && s.shared)
+    return launch_shared(spread_ic_kernel<true, 512>, L, 512, s.shared, kIcShared4, stream);
+  if (lt) spread_lt_kernel<<<L.blocks, SIM_THREADS, 0, stream>>>(L);
+  else spread_ic_kernel<false, 512><<<L.blocks, 512, 0, stream>>>(L);
+  return cudaGetLastError();
 }
 
 }  // namespace rip

@@ -169,7 +169,7 @@ struct SpreadShape {
   size_t shared;
 };
 SpreadShape spread_shape(uint32_t n, bool lt);
-void launch_spread(const SpreadLaunch &L, bool lt, cudaStream_t stream);
+cudaError_t launch_spread(const SpreadLaunch &L, bool lt, cudaStream_t stream);
 void launch_ic_fused(const FusedLaunch &L, cudaStream_t stream);
 // Resident fused CTAs per SM (of 512 threads; with one slot an SM or less they
 // have 1024).

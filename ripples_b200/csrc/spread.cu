@@ -74,8 +74,7 @@ int spread_run(rip_graph *g, rip_graph *b, const uint32_t *seeds, uint32_t k,
   L.queues = L.bitmaps + slots * bm_slot;
   L.qcap = g->n;
   L.blocks = (int)slots;
-  launch_spread(L, b != nullptr, c->stream);
-  CK(c, cudaGetLastError());
+  CK(c, launch_spread(L, b != nullptr, c->stream));
   unsigned long long total = 0;
   CK(c, cudaMemcpyAsync(&total, L.total, sizeof(total), cudaMemcpyDeviceToHost, c->stream));
   if (sizes)

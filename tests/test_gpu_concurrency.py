@@ -63,6 +63,44 @@ def test_concurrent_contexts_match_alone(model, g):
     assert np.all([a[1] > 0 for a in alone])
 
 
+@pytest.mark.parametrize("model,sizes", [("IC", [300007, 700001, 1200007, 1800001]),
+                                         ("IC", [9001, 100003, 30011, 200003]),
+                                         ("LT", [9001, 20011, 30011, 12007]),
+                                         ("LT", [40009, 65536, 50021, 60013])])
+def test_concurrent_spreads_of_different_sizes(model, sizes):
+    """Four threads launch one kernel with the shared memory their graphs take."""
+    def spread(n, out):
+        ctx = rb.Context(0)
+        g = rb.HostGraph.erdos_renyi(n, 2 * n, seed=n)
+        kind = (rb.WEIGHTS_UNIFORM, 0.1) if model == "IC" else (rb.WEIGHTS_LT_NORMALIZED, 1.0)
+        g = g.with_weights(kind[0], 1, 0.0, kind[1])
+        fg = rb.DeviceGraph(ctx, g.forward(), "IC")
+        bg = rb.DeviceGraph(ctx, g, "LT") if model == "LT" else None
+        for rep in range(30):
+            args = ([1, 2, 3], 20, rep)
+            out.append(rb.spread_lt(fg, bg, *args) if bg else rb.spread_ic(fg, *args))
+        ctx.close()
+
+    alone = [[] for _ in sizes]
+    for n, out in zip(sizes, alone):
+        spread(n, out)
+    got, errors = [[] for _ in sizes], []
+
+    def client(i):
+        try:
+            spread(sizes[i], got[i])
+        except Exception as exc:  # reported after the join
+            errors.append(repr(exc))
+
+    threads = [threading.Thread(target=client, args=(i,)) for i in range(len(sizes))]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not errors, errors
+    assert got == alone
+
+
 def test_reference_heap_on_every_device():
     """Launch limits belong to a device: selections on each one in turn, in one
     process, answer alike (a heap of 17 levels needs more than 48 KB a block)."""

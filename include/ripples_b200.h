@@ -205,10 +205,11 @@ int rip_pool_configure(rip_pool *p, uint32_t colors, uint32_t slots,
                        uint32_t log_capacity);
 
 /* Edge-work budgets (in-edges read) after which a one-set-per-warp set, or a
- * fused CTA batch, is handed to the CTA-per-set sampler, whose 32 warps split
- * each level's edge groups (the heavy tail of IC sampling on skewed graphs);
- * 0 disables the hand-over.  Defaults 2^14 and 2^23.  Results do not depend on
- * these values. */
+ * fused CTA batch, is handed to the CTA-per-set sampler, whose 4 to 32 warps
+ * split each level's coin blocks (the heavy tail of IC sampling on skewed
+ * graphs); 0 disables the hand-over.  Defaults 2^14 (2^18 on graphs of fewer than
+ * 2^21 edges that are not supercritical, see rip_pool_heavy_batch) and 2^23.
+ * Results do not depend on these values. */
 int rip_pool_work_caps(rip_pool *p, uint64_t plain_cap, uint64_t fused_cap);
 
 /* Per-graph sampler autotuner.  Times sets of `seed` on a scratch pool under
@@ -219,15 +220,15 @@ int rip_pool_work_caps(rip_pool *p, uint64_t plain_cap, uint64_t fused_cap);
  * heavy sets fill the GPU as they do at full size):
  *   0 plain (one set per warp), heavy sets past 2^18 in-edges -> grid-wide BFS
  *   1 plain, heavy past 2^14 in-edges -> grid-wide BFS
- *   2 plain, heavy past 2^14 -> one CTA per set, block shape by the number of
- *     heavy sets of a launch (what untuned graphs run where sets stay small)
+ *   2 plain, heavy past the graph's default (2^14 or 2^18, rip_pool_work_caps) ->
+ *     one CTA per set, block shape by the number of heavy sets of a launch
+ *     (what untuned graphs run where sets stay small)
  *   3/4/5 fused 64/128/256 colours, batches past 2^23 -> heavy path
- *   6/7 as 0/2 with the one-set-per-warp kernel capped at 48 registers
+ *   6/7 as 0/8 with the one-set-per-warp kernel capped at 48 registers
  *       (40 resident warps per SM instead of 32)
- *   8 as 2 with 256-thread CTAs for the heavy sets (5 sets growing per SM
- *       instead of 1: the block-shape axis; candidates 0-1 use 1024-thread
- *       CTAs, 6-7 256-thread ones), 9 the same with heavy sets from 2^16
- *       in-edges
+ *   8 plain, heavy past 2^18 -> one 256-thread CTA per set (5 sets growing per
+ *       SM; candidates 0-1 use 1024-thread CTAs, 6-7 256-thread ones), 9 the
+ *       same with heavy sets from 2^16 in-edges
  * writes the wall times to ms[] (may be null; a candidate dropped after the
  * screen keeps its screen time) and the fastest to *choice, and
  * keeps it for the graph: pools created afterwards start from it and

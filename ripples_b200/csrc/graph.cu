@@ -42,7 +42,9 @@ static int setup_vthr(rip_ctx *c, rip_graph *g) {
   g->branching = total / (double)g->m;
   // grid-wide multi-colour BFS for heavy sets only where sets grow large and
   // overlap (a supercritical reverse BFS); else one CTA per heavy set
-  g->default_giant_min = g->branching > kSupercritical && g->m >= kGiantEdges ? 32u : 0u;
+  const bool super = g->branching > kSupercritical;
+  g->default_giant_min = super && g->m >= kGiantEdges ? 32u : 0u;
+  g->default_cap_plain = super || g->m >= kSmallEdges ? kPlainCap : kPlainCapSmall;
   return RIP_OK;
 }
 

@@ -246,6 +246,19 @@ constexpr uint64_t kGiantEdges = 1ull << 21;
 // 45.6).
 constexpr uint64_t kPlainCap = 1ull << 14;
 
+// An early hand-over needs sets that are worth a second launch.  Where the
+// reverse BFS is not supercritical, a graph below this many edges has few sets
+// far past 2^14 in-edges, and the launch that starts those again takes as long
+// as the longest one's chain of levels: weighted cascade, 1500, 20 000 and
+// 150 000 sets, Erdos-Renyi (R-MAT) graphs of degree 8 with 2^19 edges 1.32,
+// 2.43, 3.55 (0.43, 0.83, 1.56) ms at 2^14 and 0.91, 1.53, 2.49 (0.37, 0.73,
+// 1.21) at 2^18; 2^20 edges 1.28, 2.61, 4.07 (0.51, 1.00, 1.86) and 1.09, 1.95,
+// 3.14 (0.59, 1.08, 1.62); 2^21 edges 1.56, 3.35, 5.49 (0.68, 1.19, 2.21) and
+// 1.84, 3.55, 5.37 (1.07, 1.67, 2.32); 2^22 edges 1.88, 4.21, 6.95 (0.82, 1.49,
+// 2.74) and 1.92, 5.96, 8.83 (1.20, 2.21, 3.27).
+constexpr uint64_t kPlainCapSmall = 1ull << 18;
+constexpr uint64_t kSmallEdges = 1ull << 21;
+
 struct rip_graph {
   rip_ctx *ctx;
   uint32_t n;
@@ -266,6 +279,7 @@ struct rip_graph {
   // an untuned graph start with (rip_pool_heavy_batch)
   double branching = 0.0;
   uint32_t default_giant_min = 32;
+  uint64_t default_cap_plain = kPlainCap;  // the hand-over of such pools (rip_pool_work_caps)
   // IC sampler configuration picked by rip_graph_autotune (pools created
   // afterwards start from it; RIP_SAMPLER_AUTO follows `sampler`)
   struct Tuned {

@@ -29,6 +29,7 @@ extern "C" int rip_pool_create(rip_ctx *c, rip_graph *g, rip_pool **out) {
   }
   cudaMemsetAsync(p->meta.p, 0, sizeof(PoolMeta), c->stream);
   p->giant_min = g->default_giant_min;
+  p->cap_plain = g->default_cap_plain;
   if (g->tuned.set) {
     p->auto_sampler = g->tuned.sampler;
     p->colors = g->tuned.colors;
@@ -719,10 +720,10 @@ extern "C" int rip_graph_autotune(rip_graph *g, uint64_t seed, uint32_t pilot, d
     int occupancy;
     uint32_t big_threads;
   };
-  static const Cand cands[RIP_TUNE_CANDIDATES] = {
+  const Cand cands[RIP_TUNE_CANDIDATES] = {
       {RIP_SAMPLER_PLAIN, 64, 1ull << 18, 1ull << 23, 32, 0, 1024},
       {RIP_SAMPLER_PLAIN, 64, 1ull << 14, 1ull << 23, 32, 0, 1024},
-      {RIP_SAMPLER_PLAIN, 64, kPlainCap, 1ull << 23, 0, 0, 0},
+      {RIP_SAMPLER_PLAIN, 64, g->default_cap_plain, 1ull << 23, 0, 0, 0},
       {RIP_SAMPLER_FUSED, 64, 1ull << 18, 1ull << 23, 32, 0, 1024},
       {RIP_SAMPLER_FUSED, 128, 1ull << 18, 1ull << 23, 32, 0, 1024},
       {RIP_SAMPLER_FUSED, 256, 1ull << 18, 1ull << 23, 32, 0, 1024},

@@ -380,7 +380,7 @@ class DeviceGraph:
         return idx, src[: self.m]
 
     TUNE_NAMES = ("plain, heavy>2^18 grid BFS", "plain, heavy>2^14 grid BFS",
-                  "plain, heavy>2^14 CTA per set", "fused 64", "fused 128",
+                  "plain, heavy>default CTA per set", "fused 64", "fused 128",
                   "fused 256", "plain 40 warps/SM, heavy>2^18 grid BFS",
                   "plain 40 warps/SM, heavy>2^18 CTA per set, 256-thread CTAs",
                   "plain, heavy>2^18 CTA per set, 256-thread CTAs",

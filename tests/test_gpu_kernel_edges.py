@@ -56,6 +56,27 @@ def test_heavy_set_list_tiles(ctx, threads, hubs, probs):
     dg.close()
 
 
+@pytest.mark.parametrize("scale,weights,handed", [(15, "wc", False), (19, "wc", True),
+                                                  (14, "uniform", True)])
+def test_sets_are_handed_over_where_it_pays(ctx, scale, weights, handed):
+    """Near-critical graphs below 2^21 edges keep their sets on the warps up to 2^18
+    in-edges (one launch a sample); larger ones and supercritical ones hand them
+    over at 2^14."""
+    kind, hi = (rb.WEIGHTS_WC, 1.0) if weights == "wc" else (rb.WEIGHTS_UNIFORM, 0.2)
+    g = rb.HostGraph.erdos_renyi(1 << scale, 16 << scale, seed=1).with_weights(kind, 2, 0.0, hi)
+    dg = rb.DeviceGraph(ctx, g, "IC")
+    p = rb.Pool(dg)
+    for _ in range(2):  # (the first one grows the pool)
+        p.clear()
+        p.sample(4000, seed=3, sampler=rb.SAMPLER_PLAIN)
+    assert (p.timing()[1] > 1) == handed
+    off, vtx = p.export()
+    thr = O.pack("IC", g.index, g.weights)
+    ooff, ovtx, _ = O.sample("IC", g.n, g.index, g.src, thr, 3, 0, 400)
+    assert np.array_equal(off[:401], ooff) and np.array_equal(vtx[: int(off[400])], ovtx)
+    dg.close()
+
+
 SET_LENGTHS = [0, 1, 31, 32, 33, 63, 64, 65, 511, 512, 513, 1023, 1024, 1025, 5000]
 
 

@@ -248,108 +248,157 @@ constexpr uint32_t kSeenWords = kSeenBits / 32;
 constexpr uint32_t kProbe = 128;  // records a search step reads, four a lane
 
 // One LT set: the single-predecessor walk from root(s) (see lt_walk_kernel).
-// A step is a chain of two dependent reads: the vertex's offsets, then 128 of
-// its in-edge records, four a lane.  Lists of up to 128 edges are read whole.
+// A step is a chain of two dependent reads: the vertex's offsets, then up to 128
+// of its in-edge records, four a lane (most lists have at most 32: one).  Lists
+// of up to 128 edges are read whole.
 // A longer one is entered where the threshold would lie if the cumulative
 // weights grew evenly: with weights drawn independently they stray from that
 // by about sqrt(degree) / 3 edges, so consecutive records decide up to some
 // thousand edges and points a few edges apart narrow a longer list to one more
 // read; a list that strays further is split evenly in 128.  (A 32-way search
-// took two steps past 32 edges, three past 1024, four past 32 768.)  The
-// revisit test first asks a bit of a small filter, which costs no memory
-// latency, and scans the walk (the warp's queue) only when it is set.
+// took two steps past 32 edges, three past 1024, four past 32 768.)
+// Revisits: the first 32 members are in registers, one a lane; a longer walk asks
+// a bit of a small filter, which costs no memory latency, and scans the rest of
+// the walk (the warp's queue) only when it is set.  The next vertex's offsets
+// are on their way meanwhile.  (50 000 walks on Erdos-Renyi graphs of degree 16,
+// 2^14, 2^18, 2^20, 2^21 vertices: 2.3, 11.2, 36, 70 ms; with every member in the
+// filter, read back from the queue 32 at a time: 2.65, 14.7, 53.6, 113.7.)
 __device__ __forceinline__ SetOutcome lt_walk_set(const DevGraph &G, Key key, uint64_t s,
                                                   const WarpCtx &W) {
   const uint32_t lane = lane_id();
   auto seen_hash = [](uint32_t v) { return (v * 0x9E3779B1u) >> 21; };  // 11 bits
   uint32_t cur = root_of(key, s, G.n);
-#pragma unroll
-  for (uint32_t i = 0; i < kSeenWords; i += 32) W.seen[i + lane] = 0u;
-  __syncwarp();
-  if (lane == 0) {
-    W.q[0] = cur;
-    W.seen[seen_hash(cur) >> 5] = 1u << (seen_hash(cur) & 31);
-  }
-  __syncwarp();
+  uint32_t member = lane == 0 ? cur : 0xFFFFFFFFu;  // lane j: the walk's vertex j
+  if (lane == 0) W.q[0] = cur;
   uint32_t qlen = 1;
   bool overflow = false;
-  unsigned long long set_exp = 0, set_edges = 0;
+  uint32_t steps = 0, reads = 0;  // vertices expanded, records read
+  uint32_t lo = __ldg(G.off + cur), hi = __ldg(G.off + cur + 1);
   for (;;) {
-    const uint32_t lo = __ldg(G.off + cur), hi = __ldg(G.off + cur + 1);
     const uint32_t t = lt_threshold(key, s, cur);
-    set_exp += (lane == 0);
-    // the first edge of [a, b) whose cumulative threshold exceeds t
-    uint32_t a = lo, b = hi, u = 0;
-    bool found = false, guess = true;
-    while (a < b) {
-      const uint32_t d = b - a;
-      uint32_t start = a, stride = 1;
-      if (d > kProbe) {
-        if (guess) {
+    ++steps;
+    uint32_t u = 0;
+    // The first of the `many` (at most kProbe) records from e on whose cumulative
+    // threshold exceeds t, and its source u; kProbe: none.
+    auto first_above = [&](uint32_t e, uint32_t many) -> uint32_t {
+      const uint2 *ep = G.edges + e + lane;
+      uint2 rec[kProbe / 32];
+#pragma unroll
+      for (uint32_t i = 0; i < kProbe / 32; ++i) {
+        rec[i] = make_uint2(0u, 0u);
+        if (i * 32 + lane < many) rec[i] = __ldg(ep + i * 32);
+      }
+      reads += many;
+#pragma unroll
+      for (uint32_t i = 0; i < kProbe / 32; ++i) {
+        if (i * 32 >= many) break;
+        const uint32_t bal = __ballot_sync(FULL, t < rec[i].y);
+        if (bal) {
+          const uint32_t at = __ffs(bal) - 1;
+          u = __shfl_sync(FULL, rec[i].x, at);
+          return i * 32 + at;
+        }
+      }
+      return kProbe;
+    };
+    const uint32_t deg = hi - lo;
+    bool found = false;
+    if (deg <= 32) {
+      uint2 rec = make_uint2(0u, 0u);
+      if (lane < deg) rec = __ldg(G.edges + lo + lane);
+      reads += deg;
+      const uint32_t bal = __ballot_sync(FULL, t < rec.y);
+      if (bal) u = __shfl_sync(FULL, rec.x, __ffs(bal) - 1);
+      found = bal != 0;
+    } else if (deg <= kProbe) {
+      found = first_above(lo, deg) != kProbe;
+    } else {
+      // it is in [a, b)
+      uint32_t a = lo, b = hi;
+      for (bool guess = true; a < b; guess = false) {
+        const uint32_t d = b - a;
+        uint32_t start = a, stride = 1;
+        if (d > kProbe && guess) {
           // points kept four standard deviations to either side
           if (d > 4096u) stride = 1u + (uint32_t)(sqrtf((float)d) * (2.5f / kProbe));
           const uint32_t at = __umulhi(t, d), half = stride * (kProbe / 2);
           start = a + min(at > half ? at - half : 0u, d - 1u - stride * (kProbe - 1));
-          guess = false;
-        } else {
+        } else if (d > kProbe) {
           stride = (d + kProbe - 1) / kProbe;
           start = a + stride - 1;
         }
-      }
-      uint2 rec[kProbe / 32];
-      uint32_t first = kProbe;  // the first point above t
-#pragma unroll
-      for (uint32_t i = 0; i < kProbe / 32; ++i) {
-        const uint32_t e = start + min((i * 32 + lane) * stride, b - 1 - start);
-        rec[i] = make_uint2(0u, 0u);
-        if (i * 32 < d) rec[i] = __ldg(&G.edges[e]);
-      }
-#pragma unroll
-      for (uint32_t i = 0; i < kProbe / 32; ++i) {
-        const uint32_t bal = __ballot_sync(FULL, i * 32 < d && t < rec[i].y);
-        if (bal && first == kProbe) {
-          first = i * 32 + __ffs(bal) - 1;
-          u = __shfl_sync(FULL, rec[i].x, first & 31);
+        uint32_t first = kProbe;  // the first point above t
+        if (stride == 1) {
+          const uint32_t many = min(kProbe, b - start);
+          first = first_above(start, many);
+          if (first == kProbe) {
+            a = start + many;
+            continue;
+          }
+          if (first || start == a) {
+            found = true;
+            break;
+          }
+          b = start + 1;
+          continue;
         }
+        uint32_t thr[kProbe / 32];
+#pragma unroll
+        for (uint32_t i = 0; i < kProbe / 32; ++i)
+          thr[i] = __ldg(&G.edges[start + min((i * 32 + lane) * stride, b - 1 - start)].y);
+        reads += kProbe;
+#pragma unroll
+        for (uint32_t i = 0; i < kProbe / 32; ++i) {
+          const uint32_t bal = __ballot_sync(FULL, t < thr[i]);
+          if (bal && first == kProbe) first = i * 32 + __ffs(bal) - 1;
+        }
+        if (first == kProbe) {  // every point at or below t
+          a = start + min((kProbe - 1) * stride, b - 1 - start) + 1;
+          continue;
+        }
+        const uint32_t p = start + min(first * stride, b - 1 - start);
+        if (first) a = start + (first - 1) * stride + 1;  // first not ruled out
+        b = p + 1;
       }
-      set_edges += (lane == 0) ? min(d, kProbe) : 0;
-      if (first == kProbe) {  // every point at or below t
-        a = start + min((kProbe - 1) * stride, b - 1 - start) + 1;
-        continue;
-      }
-      const uint32_t p = start + min(first * stride, b - 1 - start);
-      const uint32_t below = first ? start + (first - 1) * stride + 1 : a;  // first not ruled out
-      if (below == p) {
-        found = true;
-        break;
-      }
-      a = below;
-      b = p + 1;
     }
     if (!found) break;  // no in-edge picked: the walk ends here
+    lo = __ldg(G.off + u);
+    hi = __ldg(G.off + u + 1);
+    bool seen = __any_sync(FULL, member == u);
     const uint32_t h = seen_hash(u);
-    bool seen = false;
-    if ((W.seen[h >> 5] >> (h & 31)) & 1u)
-      for (uint32_t k = 0; k < qlen && !seen; k += 32) {
-        const uint32_t j = k + lane;
-        seen = __any_sync(FULL, j < qlen && W.q[j] == u);
+    if (!seen && qlen > 32 && (W.seen[h >> 5] >> (h & 31)) & 1u)
+      for (uint32_t k = 32; k < qlen && !seen; k += 128) {
+        bool mine = false;
+#pragma unroll
+        for (uint32_t i = 0; i < 4; ++i) {
+          const uint32_t j = k + i * 32 + lane;
+          if (j < qlen) mine |= W.q[j] == u;
+        }
+        seen = __any_sync(FULL, mine);
       }
     if (seen) break;
     if (qlen + 1 > W.qcap) {
       overflow = true;
       break;
     }
-    __syncwarp();
-    if (lane == 0) {
-      W.q[qlen] = u;
-      W.seen[h >> 5] |= 1u << (h & 31);
+    if (qlen < 32) {
+      if (lane == qlen) member = u;
+    } else {
+      __syncwarp();
+      if (qlen == 32) {  // the filter holds the vertices from here on
+#pragma unroll
+        for (uint32_t i = 0; i < kSeenWords; i += 32) W.seen[i + lane] = 0u;
+        __syncwarp();
+      }
+      if (lane == 0) W.seen[h >> 5] |= 1u << (h & 31);
     }
+    if (lane == 0) W.q[qlen] = u;
     __syncwarp();
     ++qlen;
     cur = u;
   }
   __syncwarp();
-  return SetOutcome{qlen, overflow, false, set_exp, set_edges};
+  return SetOutcome{qlen, overflow, false, lane == 0 ? steps : 0u, lane == 0 ? reads : 0u};
 }
 
 }  // namespace
@@ -410,8 +459,11 @@ ic_plain_kernel(DevGraph G, DevPool P, Key key, const __grid_constant__ RoundKey
 
 // One walk per warp (lt_walk_set).  Walks are chains of dependent loads; a
 // launch lasts about as long as its longest walk, so the host launches 32 warps
-// per SM and the free warp slots serve other queries' kernels.
-__global__ void __launch_bounds__(256, 5)
+// per SM and the free warp slots serve other queries' kernels.  Four blocks an SM
+// (63 registers): with five (48, some spilled) small graphs' walks were 8% slower
+// (50 000 on 2^12 R-MAT vertices, degree 30: 0.353 against 0.327 ms; twelve
+// clients' IMMs the same, 15.3 against 15.6 M sets/s).
+__global__ void __launch_bounds__(256, 4)
 lt_walk_kernel(DevGraph G, DevPool P, Key key, uint64_t first, uint32_t count,
                const uint32_t *ids, unsigned int *next, uint32_t *bitmaps,
                uint64_t bm_words, uint32_t *queues, uint32_t qcap, FailList F,

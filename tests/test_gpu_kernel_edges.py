@@ -191,6 +191,27 @@ def test_lt_walk_search_over_list_lengths(ctx, weights):
     dg.close()
 
 
+def test_lt_walk_revisits(ctx):
+    """Walks that come back to their first, 32nd, 33rd, ... vertex: tails into
+    cycles, one in-edge of weight 1 a vertex."""
+    src = []
+    for tail in (0, 1, 30, 31, 32, 33, 100, 700):
+        for cycle in (1, 2, 31, 32, 33, 127, 128, 129, 161, 500):
+            at = len(src)
+            src += list(range(at + 1, at + tail + cycle)) + [at + tail]
+    n = len(src)
+    g = rb.HostGraph(n, np.arange(n + 1, dtype=np.uint64), np.array(src, dtype=np.uint32),
+                     np.ones(n, dtype=np.float32))
+    dg = rb.DeviceGraph(ctx, g, "LT")
+    p = rb.Pool(dg)
+    p.sample(4000, seed=3)
+    off, vtx = p.export()
+    ooff, ovtx, ost = O.sample("LT", n, g.index, g.src, O.pack("LT", g.index, g.weights), 3, 0,
+                               4000)
+    assert np.array_equal(off, ooff) and np.array_equal(vtx, ovtx) and p.stats()[4] == ost[0]
+    dg.close()
+
+
 @pytest.mark.parametrize("copies", [1, 25])
 def test_device_picks_in_one_launch_and_grid_wide(ctx, copies):
     """Lowest-id picks by one cluster (up to 8 M elements) and by the grid-wide

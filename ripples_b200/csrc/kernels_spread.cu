@@ -371,29 +371,42 @@ spread_lt_kernel(SpreadLaunch L) {
 // LT with vertex ids of 16 bits.  Sweeping the out-lists of reached vertices
 // tries a vertex once for every reached in-neighbour, each try a search of its
 // in-list by dependent L2 reads.  Once a replica's levels have more out-edges
-// than half the vertices, the in-edge every vertex keeps is drawn instead, once
-// and into shared memory; from there on a level is a scan of 16-bit sources
-// against the reached bitmap, on chip, and no out-list is read.
-// 2^16 vertices, 768 K edges, 20 hubs as seeds, 2000 replicas: 26.1 -> 8.3 ms;
-// 2^12 vertices, 1500 replicas: 1.11 -> 0.28.  The searches' read latency still
-// bounds it, two of them in flight a thread.
-template <int THREADS>
+// than n / kSweepShare, the in-edge every vertex keeps is drawn instead, once, and
+// no out-list is read any more: a vertex is reached iff the chain of kept sources
+// from it meets a reached vertex.
+// The chains are halved round by round: a vertex whose source is not reached takes
+// its source's source.  (Levels one by one are a pass over all vertices each, and
+// sparse graphs have hundreds of them.)  The halving stops after a round that
+// reaches nobody: of the vertices with a chain to a reached one, not reached yet,
+// the one with the shortest chain has a reached source (sources never skip past
+// the sweep's reached vertices) and joins in the next round.
+// LEVELS: a vertex's level is its chain's length, so the sources are 32-bit words
+// with it (length in the low half), in the queue's place in L2; lengths stay below
+// 2^16 as chains have no vertex twice.
+// 2000 replicas: an R-MAT graph's 20 hubs (2^16 vertices, 768 K edges) 26.1 ms by
+// sweeps to the end, 8.2 by levels, 2.5 by halving; 2^16 Erdos-Renyi vertices of
+// degree 10, 50 (5) seeds 20.6 (11.4), 47.5 (20.3), 3.0 (3.3).  The searches' read
+// latency bounds it, two of them in flight a thread.
+constexpr uint32_t kSweepShare = 64;  // (those 3.0 (3.3) ms: 4.3 (4.8) at 16, 14.6 (11.0) at 2)
+
+template <int THREADS, bool LEVELS>
 __global__ void __launch_bounds__(THREADS, THREADS == 1024 ? 1 : 3)
 spread_lt_small_kernel(const __grid_constant__ SpreadLaunch L) {
   constexpr uint32_t WARPS = THREADS / 32;
   extern __shared__ uint4 s_dyn[];
-  __shared__ uint32_t s_qlen, s_size;
+  __shared__ uint32_t s_qlen, s_size, s_deep;
   __shared__ unsigned long long s_rep, s_work;
   const uint32_t tid = threadIdx.x, lane = lane_id(), wid = tid >> 5;
   const uint32_t n = L.G.n, words = (uint32_t)L.bm_words;
-  uint32_t *bm = reinterpret_cast<uint32_t *>(s_dyn);  // twice: a level's, the next's
-  uint16_t *kept = reinterpret_cast<uint16_t *>(bm + 2 * words);  // own id: none
+  volatile uint32_t *bm = reinterpret_cast<uint32_t *>(s_dyn);
+  volatile uint16_t *kept = reinterpret_cast<uint16_t *>(reinterpret_cast<uint32_t *>(s_dyn) + words);
   uint32_t *q = L.queues + (size_t)blockIdx.x * L.qcap;
+  auto is_reached = [&](uint32_t u) -> bool { return bm[u >> 5] >> (u & 31) & 1u; };
   unsigned long long reached = 0;
   for (;;) {
     if (tid == 0) {
       s_rep = atomicAdd(L.next, 1ull);
-      s_qlen = s_size = 0;
+      s_qlen = s_size = s_deep = 0;
       s_work = 0;
     }
     for (uint32_t w = tid; w < words; w += THREADS) bm[w] = 0;
@@ -402,7 +415,7 @@ spread_lt_small_kernel(const __grid_constant__ SpreadLaunch L) {
     if (r >= L.replicas) break;
     auto reach = [&](uint32_t u) {  // (every vertex is queued once at most: n = qcap)
       const uint32_t bit = 1u << (u & 31);
-      if (atomicOr(&bm[u >> 5], bit) & bit) return;
+      if (atomicOr(const_cast<uint32_t *>(&bm[u >> 5]), bit) & bit) return;
       const uint32_t pos = atomicAdd(&s_qlen, 1u);
       if (pos < L.qcap) q[pos] = u;
     };
@@ -420,7 +433,7 @@ spread_lt_small_kernel(const __grid_constant__ SpreadLaunch L) {
       work = warp_sum_u64(work);
       if (lane == 0 && work) atomicAdd(&s_work, work);
       __syncthreads();
-      if (s_work > n / 2) {
+      if (s_work > n / kSweepShare) {
         scan = true;
         break;
       }
@@ -447,8 +460,7 @@ spread_lt_small_kernel(const __grid_constant__ SpreadLaunch L) {
           for (int t = 0; t < 4; ++t) {
             const uint32_t ed = (g << 2) + t, u = rec[t].x;
             if (ed < ob || ed >= oe) continue;
-            const uint32_t word = *(volatile uint32_t *)&bm[u >> 5];  // bits are only set
-            if (!(word >> (u & 31) & 1u) && lt_kept_source(L.B, L.key, r, u) == from) reach(u);
+            if (!is_reached(u) && lt_kept_source(L.B, L.key, r, u) == from) reach(u);
           }
         }
       }
@@ -458,7 +470,9 @@ spread_lt_small_kernel(const __grid_constant__ SpreadLaunch L) {
       __syncthreads();
     }
     if (scan) {
-      // the kept sources, two vertices a thread in flight
+      uint32_t joined = 0, deep = 0;  // LEVELS: this thread's vertices reached, the longest chain
+      bool grew = false;
+      // the kept sources (none: the vertex itself), two vertices a thread in flight
       for (uint32_t v0 = tid; v0 < n; v0 += 2 * THREADS) {
         uint32_t a[2], b[2], t[2];
 #pragma unroll
@@ -489,42 +503,82 @@ spread_lt_small_kernel(const __grid_constant__ SpreadLaunch L) {
 #pragma unroll
         for (int i = 0; i < 2; ++i) {
           const uint32_t v = v0 + i * THREADS;
-          if (v < n) kept[v] = (uint16_t)(some[i] ? __ldg(&L.B.edges[a[i]].x) : v);
-        }
-      }
-      __syncthreads();
-      // the level at hand is in the bitmap: a vertex whose source is there and
-      // that is not joins the next one
-      uint32_t cur = 0;
-      for (;;) {
-        const uint32_t *is = bm + cur * words;
-        uint32_t *next = bm + (cur ^ 1) * words;
-        bool grew = false;
-        for (uint32_t w = wid; w < words; w += WARPS) {
-          const uint32_t was = is[w], v = w * 32 + lane;
-          bool joins = false;
-          if (v < n && !(was >> lane & 1u)) {
-            const uint32_t u = kept[v];
-            joins = is[u >> 5] >> (u & 31) & 1u;
+          if (v >= n) continue;
+          const uint32_t u = some[i] ? __ldg(&L.B.edges[a[i]].x) : v;
+          if (LEVELS) {
+            __stcg(q + v, u << 16 | (u != v));
+            if (is_reached(u) && !is_reached(v)) {
+              deep = 1;
+              ++joined;
+            }
+          } else {
+            kept[v] = (uint16_t)u;
           }
-          const uint32_t add = __ballot_sync(FULL, joins);
-          if (lane == 0) next[w] = was | add;
-          grew = grew || add != 0;
         }
-        cur ^= 1;
-        if (!__syncthreads_or(grew)) break;
-        ++levels;
       }
-      uint32_t mine = 0;
-      for (uint32_t w = tid; w < words; w += THREADS) mine += __popc(bm[w]);
-      mine = __reduce_add_sync(FULL, mine);
-      if (lane == 0 && mine) atomicAdd(&s_size, mine);
+      if (LEVELS) {
+        do {
+          __syncthreads();
+          grew = false;
+          for (uint32_t v = tid; v < n; v += THREADS) {
+            if (is_reached(v)) continue;
+            const uint32_t x = __ldcg(q + v), u = x >> 16;
+            if (u == v || is_reached(u)) continue;  // no source, or done
+            const uint32_t y = __ldcg(q + u), len = (x + y) & 0xFFFFu;
+            __stcg(q + v, (y & 0xFFFF0000u) | len);
+            if (is_reached(y >> 16)) {
+              grew = true;
+              deep = max(deep, len);
+              ++joined;
+            }
+          }
+        } while (__syncthreads_or(grew));
+        deep = __reduce_max_sync(FULL, deep);
+        if (lane == 0 && deep) atomicMax(&s_deep, deep);
+      } else {
+        do {
+          __syncthreads();
+          grew = false;
+          constexpr uint32_t U = 4;  // words in flight: three dependent reads each
+          for (uint32_t w0 = wid; w0 < words; w0 += U * WARPS) {
+            uint32_t was[U], u[U], to[U];
+            bool open[U], joins[U];
+#pragma unroll
+            for (uint32_t i = 0; i < U; ++i) {
+              const uint32_t w = w0 + i * WARPS;
+              was[i] = FULL;
+              if (w < words) was[i] = bm[w];
+              open[i] = !(was[i] >> lane & 1u) && w * 32 + lane < n;
+            }
+#pragma unroll
+            for (uint32_t i = 0; i < U; ++i)
+              if (open[i]) u[i] = kept[(w0 + i * WARPS) * 32 + lane];
+#pragma unroll
+            for (uint32_t i = 0; i < U; ++i) {
+              joins[i] = open[i] && is_reached(u[i]);
+              if (open[i]) to[i] = kept[u[i]];
+            }
+#pragma unroll
+            for (uint32_t i = 0; i < U; ++i) {
+              const uint32_t w = w0 + i * WARPS;
+              if (open[i] && !joins[i]) kept[w * 32 + lane] = (uint16_t)to[i];
+              const uint32_t add = __ballot_sync(FULL, joins[i]);
+              if (add && lane == 0) bm[w] = was[i] | add;
+              grew = grew || add != 0;
+            }
+          }
+        } while (__syncthreads_or(grew));
+      }
+      for (uint32_t w = tid; w < words; w += THREADS) joined += __popc(bm[w]);
+      joined = __reduce_add_sync(FULL, joined);
+      if (lane == 0 && joined) atomicAdd(&s_size, joined);
       __syncthreads();
+      levels += s_deep;
     }
     if (tid == 0) {
       const uint32_t size = scan ? s_size : hi;
       if (L.sizes) L.sizes[r] = size;
-      if (L.levels) L.levels[r] = levels;
+      if (LEVELS) L.levels[r] = levels;
       reached += size;
     }
     __syncthreads();
@@ -539,7 +593,8 @@ constexpr size_t kSpreadStatic = 5120;
 // Dynamic shared memory of the kernels below at most, by CTAs an SM.
 constexpr size_t kIcShared4 = (kSmShared / 4 - kSpreadStatic) & ~(size_t)15;
 constexpr size_t kIcShared1 = kSmShared - kSpreadStatic;
-constexpr size_t lt_shared(size_t n) { return ((n + 31) / 32 * 8 + 2 * n + 15) & ~(size_t)15; }
+constexpr size_t lt_shared(size_t n) { return ((n + 31) / 32 * 4 + 2 * n + 15) & ~(size_t)15; }
+constexpr size_t kLtLevels = 65536 / 8;
 constexpr size_t kLtShared3 = kSmShared / 3 - 2048;
 constexpr size_t kLtShared1 = lt_shared(65536);
 
@@ -558,16 +613,18 @@ cudaError_t launch_shared(Kernel kernel, const SpreadLaunch &L, int threads, siz
 }  // namespace
 
 // LT: up to 65536 vertices three 512-thread CTAs an SM where their bitmaps and
-// 16-bit sources fit (n up to 32 K), else one of 1024; past that no shared form.
+// 16-bit sources fit (n up to 34 K; with levels: always, the sources are in
+// L2), else one of 1024; past that no shared form.
 // IC: four 512-thread CTAs per SM with the bitmap in shared memory where four
 // fit, one 1024-thread CTA where one does, else four with it in global memory.
 // R-MAT, p ~ U(0, 0.1), 50 hubs as seeds, against block-wide scans of every
 // level with the bitmap in global memory: 2^16 vertices, 1500 replicas 2.75 ->
 // 2.59 ms; 2^18 14.9 -> 14.1 (four CTAs; one: 15.2); 2^20 62.8 -> 50.8 (one; in
 // global memory: 59.8); 2^22, 300 replicas 77.7 -> 71.0 (global).
-SpreadShape spread_shape(uint32_t n, bool lt) {
+SpreadShape spread_shape(uint32_t n, bool lt, bool levels) {
   const size_t bitmap = (((size_t)n + 127) / 128) * 16;
-  if (lt && n <= 65536) {  // two bitmaps and the kept sources
+  if (lt && n <= 65536) {  // the bitmap and the kept sources
+    if (levels) return SpreadShape{512, 3, bitmap};
     const size_t bytes = lt_shared(n);
     return bytes <= kLtShared3 ? SpreadShape{512, 3, bytes} : SpreadShape{1024, 1, bytes};
   }
@@ -581,11 +638,13 @@ cudaError_t launch_spread(const SpreadLaunch &L0, bool lt, cudaStream_t stream) 
   count_launches(1);
   SpreadLaunch L = L0;
   L.rk = round_keys(L.key);
-  const SpreadShape s = spread_shape(L.G.n, lt);
+  const SpreadShape s = spread_shape(L.G.n, lt, L.levels != nullptr);
+  if (lt && s.shared && L.levels)
+    return launch_shared(spread_lt_small_kernel<512, true>, L, 512, s.shared, kLtLevels, stream);
   if (lt && s.shared && s.threads == 1024)
-    return launch_shared(spread_lt_small_kernel<1024>, L, 1024, s.shared, kLtShared1, stream);
+    return launch_shared(spread_lt_small_kernel<1024, false>, L, 1024, s.shared, kLtShared1, stream);
   if (lt && s.shared)
-    return launch_shared(spread_lt_small_kernel<512>, L, 512, s.shared, kLtShared3, stream);
+    return launch_shared(spread_lt_small_kernel<512, false>, L, 512, s.shared, kLtShared3, stream);
   if (!lt && s.shared && s.threads == 1024)
     return launch_shared(spread_ic_kernel<true, 1024>, L, 1024, s.shared, kIcShared1, stream);
   if (!lt && s.shared)

@@ -168,7 +168,7 @@ struct SpreadShape {
   int threads, per_sm;
   size_t shared;
 };
-SpreadShape spread_shape(uint32_t n, bool lt);
+SpreadShape spread_shape(uint32_t n, bool lt, bool levels);
 cudaError_t launch_spread(const SpreadLaunch &L, bool lt, cudaStream_t stream);
 void launch_ic_fused(const FusedLaunch &L, cudaStream_t stream);
 // Resident fused CTAs per SM (of 512 threads; with one slot an SM or less they

@@ -28,7 +28,7 @@ int spread_run(rip_graph *g, rip_graph *b, const uint32_t *seeds, uint32_t k,
   // memory) and an n-entry queue (a replica queues every vertex at most once);
   // at most one slot per resident CTA, fewer when the slots would take more
   // than a quarter of the free budget
-  const SpreadShape shape = spread_shape(g->n, b != nullptr);
+  const SpreadShape shape = spread_shape(g->n, b != nullptr, levels != nullptr);
   const uint64_t bm_words = ((uint64_t)g->n + 31) / 32;
   const uint64_t bm_slot = shape.shared ? 0 : bm_words;
   const uint64_t per_slot = 4 * bm_slot + 4 * (uint64_t)g->n;

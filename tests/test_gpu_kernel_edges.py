@@ -296,6 +296,33 @@ def test_spread_lt_swept_and_scanned(ctx, n):
     fg.close()
 
 
+@pytest.mark.parametrize("n,chain", [(2011, 2000), (33000, 5000), (35000, 34000), (65536, 65535)])
+def test_spread_lt_deep_chains(ctx, n, chain):
+    """Chains of kept sources as long as the graph, cycles, self-loops, vertices that
+    keep no in-edge; sizes with levels and alone (kernels of their own)."""
+    r = np.random.RandomState(n)
+    dst = np.arange(1, n)
+    src = np.where(dst < chain, dst - 1, r.randint(0, n, n - 1))  # past the chain: trees and cycles
+    loops = r.choice(n - 1, 50, replace=False)
+    src[loops[loops > chain]] = dst[loops[loops > chain]]
+    w = np.where(dst < chain, 1.0, 0.9).astype(np.float32)
+    # a second in-edge from far behind for some vertices of the chain
+    more = np.arange(chain // 3, chain, 37)
+    src, dst, w = np.append(src, more // 2), np.append(dst, more), np.append(w, 0.0 * more)
+    w[more - 1], w[n - 1:] = 0.999, 0.001
+    g = rb.HostGraph.from_edges(n, src, dst, w)
+    fg, bg = rb.DeviceGraph(ctx, g.forward(), "IC"), rb.DeviceGraph(ctx, g, "LT")
+    for seeds, replicas in (([0], 12), ([n - 1, 5, chain // 2], 300), (list(range(0, n, 97)), 12)):
+        _, sizes, levels = rb.spread_lt(fg, bg, seeds, replicas, seed=23, with_sizes=True,
+                                        with_levels=True)
+        mean, alone = rb.spread_lt(fg, bg, seeds, replicas, seed=23, with_sizes=True)
+        _, o_sizes, o_levels = O.spread_lt(g, seeds, replicas, seed=23, with_levels=True)
+        assert np.array_equal(sizes, o_sizes) and np.array_equal(levels, o_levels)
+        assert np.array_equal(alone, o_sizes) and mean == o_sizes.mean()
+    bg.close()
+    fg.close()
+
+
 @pytest.mark.parametrize("grid", [False, True])
 @pytest.mark.parametrize("colors,sets", [(64, 60), (128, 300), (256, 500), (256, 4500)])
 def test_colour_pairs(ctx, grid, colors, sets):

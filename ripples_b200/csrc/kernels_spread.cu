@@ -8,7 +8,7 @@
 // entries at a time and sweep their shorter out-lists through the concatenated
 // 8-edge blocks (a warp scan and a shuffle search, no barrier); lists of
 // kTileBlocks blocks or more are listed and dealt to all warps in 32-block
-// tiles.
+// tiles.  Small levels are packed over the whole CTA (kPackEntries).
 //   IC: out-edge e of a reached vertex fires in replica r iff its coin
 //       (coarse half from sim_ic_block(key, e >> 3, r), fine half from
 //       sim_ic_fine on a coarse tie) is below threshold(e) (BFS over live
@@ -24,8 +24,10 @@
 //
 // What bounds it: latency.  IC draws 90 issue cycles of coins a warp and coin
 // block; a live edge costs round trips.  The reached bitmap sits in shared memory
-// where it fits (n up to about 1.8 million), so a live edge costs none to L2 and
-// the bitmaps leave L2 to the graph.
+// where it fits and replicas grow (spread_shape), so a live edge costs none to L2
+// and the bitmaps leave L2 to the graph.
+#include <type_traits>
+
 #include "device.cuh"
 #include "launch.h"
 
@@ -34,7 +36,14 @@ namespace rip {
 namespace {
 
 constexpr uint32_t kTileBlocks = 128;  // lists of at least this many blocks go in tiles
-constexpr uint32_t kSimLong = 256;     // long lists a level may list
+// Levels of at most this many entries are packed, in the 512-thread form with the
+// bitmap in shared memory: a warp's share of a small level leaves lanes without a
+// block, and its passes over live edges wait for each other, which is what replicas
+// of a few thousand vertices spend their time on.  R-MAT, p ~ U(0, 0.02), 5 hubs as
+// seeds, 1500 replicas: 2^16 vertices 0.86 -> 0.75 ms, 2^18 3.67 -> 3.47.  The
+// larger forms lose by it (2^20 vertices, p ~ U(0, 0.1), 50 hubs: 50.9 -> 53.5).
+constexpr uint32_t kPackEntries = 512;
+constexpr uint32_t kSimLong = 256;  // long lists a level may list
 
 __device__ __forceinline__ uint32_t sim_lanemask_lt() {
   uint32_t m;
@@ -49,9 +58,12 @@ spread_ic_kernel(const __grid_constant__ SpreadLaunch L) {
   // the targets of a block's edges: kept in registers where there are 64 a
   // thread, else read again from L1
   constexpr bool KEEP = THREADS == 1024;
+  constexpr bool PACK = SHARED && !KEEP;
   extern __shared__ uint4 s_dyn[];  // SHARED: the reached bitmap
-  __shared__ uint32_t s_lbeg[kSimLong], s_lend[kSimLong];
-  __shared__ uint32_t s_qlen, s_nlong[2], s_next[2];  // by the level's parity
+  constexpr uint32_t ROOM = PACK ? kPackEntries : kSimLong;
+  __shared__ uint32_t s_beg[ROOM], s_end[ROOM];  // a packed level's entries, or long lists
+  __shared__ uint32_t s_off[PACK ? kPackEntries : 1], s_warp[32];
+  __shared__ uint32_t s_qlen, s_nlong, s_next;  // the last two zero between levels
   __shared__ unsigned long long s_rep;
 
   const uint32_t tid = threadIdx.x, lane = lane_id(), wid = tid >> 5;
@@ -67,8 +79,7 @@ spread_ic_kernel(const __grid_constant__ SpreadLaunch L) {
     if (tid == 0) {
       s_rep = atomicAdd(L.next, 1ull);
       s_qlen = 0;
-      s_nlong[0] = 0;
-      s_next[0] = 0;
+      s_nlong = s_next = 0;
     }
     __syncthreads();
     const uint64_t r = s_rep;
@@ -97,10 +108,10 @@ spread_ic_kernel(const __grid_constant__ SpreadLaunch L) {
       if (isnew && pos < L.qcap) q[pos] = u;
     };
     // Draws 8-edge block b's edges in [ob, oe) (an empty range: none) and follows
-    // those that fire, one a lane and pass.  Records are read two at a time (a
-    // pair past the list's end is not read: the record array ends on a 4-edge
-    // boundary).
-    auto expand_block = [&](uint32_t b, uint32_t ob, uint32_t oe) {
+    // those that fire: each lane its own, or (`together`) one a lane and pass, by
+    // the whole warp.  Records are read two at a time (a pair past the list's end
+    // is not read: the record array ends on a 4-edge boundary).
+    auto expand_block = [&](auto together, uint32_t b, uint32_t ob, uint32_t oe) {
       const uint4 *rp = reinterpret_cast<const uint4 *>(L.G.edges + ((size_t)b << 3));
       const u32x4 c = coin_block(L.rk, cs, b);
       uint32_t u[8], live = 0, tie = 0;
@@ -131,7 +142,7 @@ spread_ic_kernel(const __grid_constant__ SpreadLaunch L) {
         const uint32_t e = (b << 3) + h;
         if (sim_ic_fine_call(L.key, e, r) < (__ldg(&L.G.edges[e].y) & 0xFFFFu)) live |= 1u << h;
       }
-      while (__any_sync(FULL, live != 0)) {
+      while (together.value ? __any_sync(FULL, live != 0) : live != 0) {
         uint32_t x = 0;
         bool want = live != 0;
         if (want) {
@@ -143,72 +154,118 @@ spread_ic_kernel(const __grid_constant__ SpreadLaunch L) {
               if (h == (uint32_t)t) x = u[t];
           } else {
             x = __ldg(&L.G.edges[(b << 3) + h].x);
+          }
+          if (!KEEP || !together.value) {
             const uint32_t word = SHARED ? bm[x >> 5] : __ldcg(&bm[x >> 5]);  // bits are only set
             want = !((word >> (x & 31)) & 1u);
           }
         }
-        reach(want, x);
+        if (together.value) {
+          reach(want, x);
+        } else if (want) {
+          const uint32_t bit = 1u << (x & 31);
+          if (!(atomicOr(&bm[x >> 5], bit) & bit)) {
+            const uint32_t pos = atomicAdd(&s_qlen, 1u);
+            if (pos < L.qcap) q[pos] = x;
+          }
+        }
       }
     };
-    uint32_t lo = 0, hi = min(s_qlen, L.qcap), levels = 0, par = 0;
+    constexpr auto alone = std::false_type{};
+    constexpr auto together = std::true_type{};
+    uint32_t lo = 0, hi = min(s_qlen, L.qcap), levels = 0;
     __syncthreads();
     while (lo < hi) {
       ++levels;  // one BFS level (the seeds are the first)
-      // 1. warps take the level's entries, up to 32 at a time
-      const uint32_t share = min(32u, (hi - lo + WARPS - 1) / WARPS);
-      for (;;) {
-        uint32_t at = 0;
-        if (lane == 0) at = atomicAdd(&s_next[par], share);
-        at = __shfl_sync(FULL, at, 0);
-        if (at >= hi - lo) break;
-        const uint32_t e = lo + at + lane;
-        uint32_t beg = 0, end = 0;
-        if (lane < share && e < hi) {
-          const uint32_t v = q[e];
-          beg = __ldg(L.G.off + v);
-          end = __ldg(L.G.off + v + 1);
-        }
-        uint32_t nb = block_count(beg, end);
-        if (nb >= kTileBlocks) {
-          const uint32_t pos = atomicAdd(&s_nlong[par], 1u);
-          if (pos < kSimLong) {
-            s_lbeg[pos] = beg;
-            s_lend[pos] = end;
-            nb = 0;
-          }  // (no room: this warp sweeps it with the others)
+      if (PACK && hi - lo <= kPackEntries) {
+        // a small level: its blocks side by side over the whole CTA
+        const uint32_t e = lo + tid;
+        uint32_t nb = 0;
+        if (tid < kPackEntries) {
+          uint32_t beg = 0, end = 0;
+          if (e < hi) {
+            const uint32_t v = q[e];
+            beg = __ldg(L.G.off + v);
+            end = __ldg(L.G.off + v + 1);
+          }
+          s_beg[tid] = beg;
+          s_end[tid] = end;
+          nb = block_count(beg, end);
         }
         const uint32_t incl = warp_incl_scan(nb);
-        const uint32_t total = __shfl_sync(FULL, incl, 31);
-        for (uint32_t base = 0; base < total; base += 32) {
-          const uint32_t j = base + lane;
-          const uint32_t owner = warp_find_owner(incl, min(j, total - 1));
-          const uint32_t ob = __shfl_sync(FULL, beg, owner);
-          const uint32_t oe = __shfl_sync(FULL, end, owner);
-          const uint32_t oexcl = __shfl_sync(FULL, incl - nb, owner);
-          const bool valid = j < total;
-          expand_block(valid ? (ob >> 3) + (j - oexcl) : 0u, valid ? ob : 0u, valid ? oe : 0u);
+        if (lane == 31) s_warp[wid] = incl;
+        __syncthreads();
+        const uint32_t own = lane < WARPS ? s_warp[lane] : 0u, upto = warp_incl_scan(own);
+        const uint32_t total = __shfl_sync(FULL, upto, 31);
+        const uint32_t before = __shfl_sync(FULL, upto - own, wid);
+        if (tid < kPackEntries) s_off[tid] = before + incl - nb;
+        __syncthreads();
+        for (uint32_t j = tid; j < total; j += THREADS) {
+          uint32_t a = 0, z = hi - lo;  // entry a: s_off[a] <= j < s_off[a + 1]
+          while (z - a > 1) {
+            const uint32_t mid = (a + z) >> 1;
+            if (s_off[mid] <= j) a = mid;
+            else z = mid;
+          }
+          expand_block(alone, (s_beg[a] >> 3) + (j - s_off[a]), s_beg[a], s_end[a]);
         }
-      }
-      __syncthreads();
-      // 2. the long lists, dealt to the warps a tile of 32 blocks at a time
-      const uint32_t nlong = min(s_nlong[par], kSimLong);
-      if (tid == 0) s_nlong[par ^ 1] = s_next[par ^ 1] = 0;
-      uint32_t deal = wid;  // (wid - tiles dealt so far) mod WARPS: this warp's next tile
-      for (uint32_t a = 0; a < nlong; ++a) {
-        const uint32_t ob = s_lbeg[a], oe = s_lend[a];
-        const uint32_t b_last = (oe - 1) >> 3;
-        const uint32_t ntiles = ((b_last - (ob >> 3)) >> 5) + 1;
-        for (uint32_t t = deal & (WARPS - 1); t < ntiles; t += WARPS) {
-          const uint32_t b = (ob >> 3) + t * 32 + lane;
-          const bool valid = b <= b_last;
-          expand_block(valid ? b : 0u, valid ? ob : 0u, valid ? oe : 0u);
+      } else {
+        // 1. warps take the level's entries, up to 32 at a time
+        const uint32_t share = min(32u, (hi - lo + WARPS - 1) / WARPS);
+        for (;;) {
+          uint32_t at = 0;
+          if (lane == 0) at = atomicAdd(&s_next, share);
+          at = __shfl_sync(FULL, at, 0);
+          if (at >= hi - lo) break;
+          const uint32_t e = lo + at + lane;
+          uint32_t beg = 0, end = 0;
+          if (lane < share && e < hi) {
+            const uint32_t v = q[e];
+            beg = __ldg(L.G.off + v);
+            end = __ldg(L.G.off + v + 1);
+          }
+          uint32_t nb = block_count(beg, end);
+          if (nb >= kTileBlocks) {
+            const uint32_t pos = atomicAdd(&s_nlong, 1u);
+            if (pos < kSimLong) {
+              s_beg[pos] = beg;
+              s_end[pos] = end;
+              nb = 0;
+            }  // (no room: this warp sweeps it with the others)
+          }
+          const uint32_t incl = warp_incl_scan(nb);
+          const uint32_t total = __shfl_sync(FULL, incl, 31);
+          for (uint32_t base = 0; base < total; base += 32) {
+            const uint32_t j = base + lane;
+            const uint32_t owner = warp_find_owner(incl, min(j, total - 1));
+            const uint32_t ob = __shfl_sync(FULL, beg, owner);
+            const uint32_t oe = __shfl_sync(FULL, end, owner);
+            const uint32_t oexcl = __shfl_sync(FULL, incl - nb, owner);
+            const bool valid = j < total;
+            expand_block(together, valid ? (ob >> 3) + (j - oexcl) : 0u, valid ? ob : 0u,
+                         valid ? oe : 0u);
+          }
         }
-        deal -= ntiles;
+        __syncthreads();
+        // 2. the long lists, dealt to the warps a tile of 32 blocks at a time
+        const uint32_t nlong = min(s_nlong, kSimLong);
+        uint32_t deal = wid;  // (wid - tiles dealt so far) mod WARPS: this warp's next tile
+        for (uint32_t a = 0; a < nlong; ++a) {
+          const uint32_t ob = s_beg[a], oe = s_end[a];
+          const uint32_t b_last = (oe - 1) >> 3;
+          const uint32_t ntiles = ((b_last - (ob >> 3)) >> 5) + 1;
+          for (uint32_t t = deal & (WARPS - 1); t < ntiles; t += WARPS) {
+            const uint32_t b = (ob >> 3) + t * 32 + lane;
+            const bool valid = b <= b_last;
+            expand_block(together, valid ? b : 0u, valid ? ob : 0u, valid ? oe : 0u);
+          }
+          deal -= ntiles;
+        }
       }
       __syncthreads();
       lo = hi;
       hi = min(s_qlen, L.qcap);
-      par ^= 1;
+      if (tid == 0) s_nlong = s_next = 0;
       __syncthreads();
     }
     // every vertex is queued at most once, so qlen <= n = qcap
@@ -589,7 +646,7 @@ spread_lt_small_kernel(const __grid_constant__ SpreadLaunch L) {
 // Shared memory of an SM's CTAs, and what a spread CTA takes besides its dynamic
 // part (static and reserved, rounded up).
 constexpr size_t kSmShared = 227 * 1024;
-constexpr size_t kSpreadStatic = 5120;
+constexpr size_t kSpreadStatic = 8192;
 // Dynamic shared memory of the kernels below at most, by CTAs an SM.
 constexpr size_t kIcShared4 = (kSmShared / 4 - kSpreadStatic) & ~(size_t)15;
 constexpr size_t kIcShared1 = kSmShared - kSpreadStatic;
@@ -616,12 +673,17 @@ cudaError_t launch_shared(Kernel kernel, const SpreadLaunch &L, int threads, siz
 // 16-bit sources fit (n up to 34 K; with levels: always, the sources are in
 // L2), else one of 1024; past that no shared form.
 // IC: four 512-thread CTAs per SM with the bitmap in shared memory where four
-// fit, one 1024-thread CTA where one does, else four with it in global memory.
+// fit (n up to about 400 K), else one 1024-thread CTA with it where that fits (1.79
+// million) and replicas grow (`super`: the branching factor of a traversal is above
+// kSupercritical), else four with it in global memory.
 // R-MAT, p ~ U(0, 0.1), 50 hubs as seeds, against block-wide scans of every
-// level with the bitmap in global memory: 2^16 vertices, 1500 replicas 2.75 ->
-// 2.59 ms; 2^18 14.9 -> 14.1 (four CTAs; one: 15.2); 2^20 62.8 -> 50.8 (one; in
-// global memory: 59.8); 2^22, 300 replicas 77.7 -> 71.0 (global).
-SpreadShape spread_shape(uint32_t n, bool lt, bool levels) {
+// level with the bitmap in global memory: 2^16 vertices, 1500 replicas 3.63 ->
+// 3.50 ms; 2^18 14.9 -> 14.1 (four CTAs; one: 15.2); 2^20 62.9 -> 50.9 (one; in
+// global memory: 59.8); 2^22, 300 replicas 77.7 -> 71.0 (global).  Replicas that
+// end with a few vertices would wait for each other at one CTA an SM: 2^20
+// Erdos-Renyi vertices, p ~ U(0, 0.06), 100 seeds, 1500 replicas 0.20 ms, 0.14 with
+// four.
+SpreadShape spread_shape(uint32_t n, bool lt, bool levels, bool super) {
   const size_t bitmap = (((size_t)n + 127) / 128) * 16;
   if (lt && n <= 65536) {  // the bitmap and the kept sources
     if (levels) return SpreadShape{512, 3, bitmap};
@@ -630,15 +692,15 @@ SpreadShape spread_shape(uint32_t n, bool lt, bool levels) {
   }
   if (lt) return SpreadShape{SIM_THREADS, 4, 0};
   if (bitmap <= kIcShared4) return SpreadShape{512, 4, bitmap};
-  if (bitmap <= kIcShared1) return SpreadShape{1024, 1, bitmap};
+  if (super && bitmap <= kIcShared1) return SpreadShape{1024, 1, bitmap};
   return SpreadShape{512, 4, 0};
 }
 
-cudaError_t launch_spread(const SpreadLaunch &L0, bool lt, cudaStream_t stream) {
+cudaError_t launch_spread(const SpreadLaunch &L0, bool lt, const SpreadShape &s,
+                          cudaStream_t stream) {
   count_launches(1);
   SpreadLaunch L = L0;
   L.rk = round_keys(L.key);
-  const SpreadShape s = spread_shape(L.G.n, lt, L.levels != nullptr);
   if (lt && s.shared && L.levels)
     return launch_shared(spread_lt_small_kernel<512, true>, L, 512, s.shared, kLtLevels, stream);
   if (lt && s.shared && s.threads == 1024)

@@ -168,8 +168,9 @@ struct SpreadShape {
   int threads, per_sm;
   size_t shared;
 };
-SpreadShape spread_shape(uint32_t n, bool lt, bool levels);
-cudaError_t launch_spread(const SpreadLaunch &L, bool lt, cudaStream_t stream);
+SpreadShape spread_shape(uint32_t n, bool lt, bool levels, bool super);
+cudaError_t launch_spread(const SpreadLaunch &L, bool lt, const SpreadShape &s,
+                          cudaStream_t stream);
 void launch_ic_fused(const FusedLaunch &L, cudaStream_t stream);
 // Resident fused CTAs per SM (of 512 threads; with one slot an SM or less they
 // have 1024).

@@ -28,7 +28,8 @@ int spread_run(rip_graph *g, rip_graph *b, const uint32_t *seeds, uint32_t k,
   // memory) and an n-entry queue (a replica queues every vertex at most once);
   // at most one slot per resident CTA, fewer when the slots would take more
   // than a quarter of the free budget
-  const SpreadShape shape = spread_shape(g->n, b != nullptr, levels != nullptr);
+  const SpreadShape shape = spread_shape(g->n, b != nullptr, levels != nullptr,
+                                         g->branching > kSupercritical);
   const uint64_t bm_words = ((uint64_t)g->n + 31) / 32;
   const uint64_t bm_slot = shape.shared ? 0 : bm_words;
   const uint64_t per_slot = 4 * bm_slot + 4 * (uint64_t)g->n;
@@ -74,7 +75,7 @@ int spread_run(rip_graph *g, rip_graph *b, const uint32_t *seeds, uint32_t k,
   L.queues = L.bitmaps + slots * bm_slot;
   L.qcap = g->n;
   L.blocks = (int)slots;
-  CK(c, launch_spread(L, b != nullptr, c->stream));
+  CK(c, launch_spread(L, b != nullptr, shape, c->stream));
   unsigned long long total = 0;
   CK(c, cudaMemcpyAsync(&total, L.total, sizeof(total), cudaMemcpyDeviceToHost, c->stream));
   if (sizes)

@@ -253,18 +253,21 @@ def test_lt_pack_over_list_lengths(ctx, total):
     dg.close()
 
 
-@pytest.mark.parametrize("n", [20011, 500009, 1900003])
-def test_spread_bitmap_places(ctx, n):
+@pytest.mark.parametrize("n,hi", [(20011, 0.2), (500009, 0.2), (1900003, 0.2), (20011, 0.002),
+                                  (500009, 0.001)])
+def test_spread_bitmap_places(ctx, n, hi):
     """The reached bitmap in shared memory (four CTAs an SM, one) and in global
-    memory; out-lists around a tile and past what a level lists."""
+    memory (large graphs, and wide ones whose replicas stay small); small levels
+    packed over a CTA; out-lists around a tile and past what a level lists."""
     r = np.random.RandomState(n % 97)
     lens = [1, 7, 8, 9, 255, 1016, 1024, 1025, 2049, 5000] * 30
     src = np.repeat(np.arange(len(lens)), lens)  # out-lists of the first vertices
     dst = r.randint(0, n, len(src))
     hub = r.rand(len(src)) < 0.2
     dst[hub] = r.randint(0, len(lens), hub.sum())
-    g = rb.HostGraph.from_edges(n, src, dst, r.rand(len(src)) * 0.2)
+    g = rb.HostGraph.from_edges(n, src, dst, r.rand(len(src)) * hi)
     dg = rb.DeviceGraph(ctx, g.forward(), "IC")
+    assert (dg.branching() > 1.1) == (hi > 0.1)
     seeds = list(range(12))
     mean, sizes, levels = rb.spread_ic(dg, seeds, 200, seed=5, with_sizes=True, with_levels=True)
     f = g.forward()

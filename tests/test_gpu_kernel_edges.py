@@ -267,7 +267,7 @@ def test_spread_bitmap_places(ctx, n, hi):
     dst[hub] = r.randint(0, len(lens), hub.sum())
     g = rb.HostGraph.from_edges(n, src, dst, r.rand(len(src)) * hi)
     dg = rb.DeviceGraph(ctx, g.forward(), "IC")
-    assert (dg.branching() > 1.1) == (hi > 0.1)
+    assert (dg.branching > 1.1) == (hi > 0.1)
     seeds = list(range(12))
     mean, sizes, levels = rb.spread_ic(dg, seeds, 200, seed=5, with_sizes=True, with_levels=True)
     f = g.forward()

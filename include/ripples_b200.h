@@ -320,12 +320,10 @@ int rip_select_profile(rip_pool *p, double out[12]);
  * [0, max_count), with the library's level-parallel heap construction and with
  * std::make_heap; returns 1 when the two are identical element for element. */
 int rip_selftest_heap(uint64_t n, uint32_t max_count, uint64_t seed);
-/* Diagnostic: what reference-heap selections keep of counts with this histogram
- * (240 words: one per count below 16, then eight per power of two), from the
- * first build on until every count is kept: the smallest count and how many
- * items that makes, in smallest[] and items[] (room entries each).  Returns the
- * number of builds, room when they do not come to an end. */
-int rip_selftest_keep(const uint32_t *hist, uint32_t *smallest, uint64_t *items, uint32_t room);
+/* Diagnostic: what a reference-heap selection keeps on the host at first of counts
+ * with this histogram (240 words: one per count below 16, then eight per power of
+ * two): the smallest count and how many items that makes; 0 is the whole heap. */
+int rip_selftest_keep(const uint32_t *hist, uint32_t *smallest, uint64_t *items);
 /* Same check for the device heap build that rip_select uses. */
 int rip_selftest_heap_device(rip_ctx *ctx, uint64_t n, uint32_t max_count, uint64_t seed);
 

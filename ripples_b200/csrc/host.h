@@ -53,7 +53,15 @@ struct rip_ctx {
   // reference-heap selection storage, shared by the context's pools (one
   // selection runs at a time)
   SparseHeap heap;
-  PinnedMem *h_list = nullptr;   // the heap items a selection keeps
+  PinnedMem *h_list = nullptr;   // the heap items a selection keeps, or the full heap
+  // counts by item id, each with the fetch that brought it; `fetch` numbers those
+  // of all the context's selections, so that what one left is never taken for
+  // another's
+  struct Fetched {
+    uint32_t count, at;
+  };
+  std::vector<Fetched> fetched;
+  uint32_t fetch = 0;
   PinnedMem *h_count = nullptr;  // whole-array count fetches
   // multi-instance sampler scratch (per warp: bitmap for the largest graph
   // of the launch + queue), instance table, failure pairs

@@ -268,24 +268,20 @@ __host__ __device__ inline uint32_t count_bucket(uint32_t c) {
 inline uint32_t count_bucket_low(uint32_t b) {  // the smallest count of bucket b
   return b < 8 ? b : (8u | (b & 7u)) << ((b >> 3) - 1);
 }
-// The counts a reference-heap selection keeps on the host: all from bucket `low`
-// on, `items` of them.
-struct KeptCounts {
-  uint32_t low = kCountBuckets;
-  uint64_t items = 0;
-  // Takes in further buckets (hist: the counts by bucket), the largest counts
-  // first: the next one that holds a count whatever its size, so that a caller
-  // who needs smaller counts gets them, then more as long as `want` are not
-  // exceeded.
-  void grow(const uint32_t *hist, uint64_t want) {
-    const uint64_t had = items;
-    while (low > 0 && (items == had || items + hist[low - 1] <= want)) items += hist[--low];
-  }
-  uint32_t smallest() const { return count_bucket_low(low); }  // 0: every count is kept
-};
-// How many items are kept at first, and after the gains fell below those.
-constexpr uint64_t kKeepFirst = 16384;
-inline uint64_t keep_next(const KeptCounts &kept) { return 8 * kept.items; }
+// The smallest count a reference-heap selection keeps on the host at first, and
+// how many items that makes: those of the largest buckets (hist: the counts by
+// bucket) that together hold at most kKeepFirst.  0, every item, where the first
+// bucket with any holds more.
+constexpr uint32_t kKeepFirst = 16384;
+inline uint32_t keep_from(const uint32_t *hist, uint64_t *items) {
+  uint32_t b = kCountBuckets;
+  uint64_t many = 0;
+  while (b > 0 && many + hist[b - 1] <= kKeepFirst) many += hist[--b];
+  if (many == 0)
+    while (b > 0) many += hist[--b];
+  *items = many;
+  return count_bucket_low(b);
+}
 void launch_count_hist(const uint32_t *count, uint32_t n, uint32_t *hist, cudaStream_t stream);
 // count[v] = the count of v's item in a heap launch_make_heap built.
 void launch_heap_counts(const uint2 *heap, uint32_t n, uint32_t *count, cudaStream_t stream);

@@ -8,28 +8,6 @@
 // selection
 // ---------------------------------------------------------------------------
 namespace {
-// The items (ids) of every kept heap position keyed at least T (keys never grow
-// downwards, so subtrees whose root is keyed below T are skipped), breadth
-// first.  Returns the count, or cap + 1 when more than cap items qualify.
-static uint32_t collect_at_least(const SparseHeap &heap, uint32_t T, uint32_t cap, uint32_t *out,
-                                 std::vector<size_t> &queue) {
-  uint32_t cnt = 0, id, key;
-  queue.clear();
-  auto look = [&](size_t p) {
-    if (!heap.kept_at(p, id, key) || key < T) return;
-    if (cnt < cap) out[cnt] = id;
-    ++cnt;
-    queue.push_back(p);
-  };
-  look(0);
-  for (size_t head = 0; head < queue.size() && cnt <= cap; ++head) {
-    const size_t p = queue[head];
-    look(2 * p + 1);
-    look(2 * p + 2);
-  }
-  return std::min(cnt, cap + 1);
-}
-
 // Bit-identical to std::make_heap(v.begin(), v.end(), CompareHeap{}), built
 // level by level in parallel.  libstdc++'s make_heap runs __adjust_heap on
 // every parent from (len-2)/2 down to 0; each call only touches the subtree
@@ -111,17 +89,24 @@ extern "C" int rip_selftest_heap(uint64_t n, uint32_t max_count, uint64_t seed) 
   std::make_heap(b.begin(), b.end(), CompareHeap{});
   parallel_make_heap(a);
   if (!(a == b)) return 0;
-  // pops and pushes on the items of K or more against the full heap's
-  for (uint32_t K : {0u, 1u, max_count / 2}) {
+  // pops and pushes on the items of K or more (0: the full heap) against the full
+  // heap's
+  for (uint32_t K : {0u, 1u, max_count / 2 + 1}) {
     std::vector<uint32_t> vtx, key, pos;
-    for (uint64_t i = 0; i < n; ++i)
-      if (b[i].second >= K) {
-        vtx.push_back(b[i].first);
-        key.push_back(b[i].second);
-        pos.push_back((uint32_t)i);
-      }
+    std::vector<HeapItem> all = b;
     SparseHeap h;
-    h.build(n, (uint32_t)vtx.size(), K, key.data(), pos.data());
+    if (K == 0) {
+      h.adopt(all.data(), n);
+      for (uint64_t i = 0; i < n; ++i) vtx.push_back((uint32_t)i);
+    } else {
+      for (uint64_t i = 0; i < n; ++i)
+        if (b[i].second >= K) {
+          vtx.push_back(b[i].first);
+          key.push_back(b[i].second);
+          pos.push_back((uint32_t)i);
+        }
+      h.build(n, (uint32_t)vtx.size(), key.data(), pos.data());
+    }
     a = b;
     for (int op = 0; op < 2000 && !a.empty(); ++op) {
       const HeapItem top = a.front();
@@ -145,19 +130,11 @@ extern "C" int rip_selftest_heap(uint64_t n, uint32_t max_count, uint64_t seed) 
   return 1;
 }
 
-// Diagnostic: the counts a reference-heap selection with this histogram
-// (kCountBuckets words) keeps, build after build, until it keeps all: smallest
-// count and number of them; returns the builds, `room` when they do not end.
-extern "C" int rip_selftest_keep(const uint32_t *hist, uint32_t *smallest, uint64_t *items,
-                                 uint32_t room) {
-  KeptCounts kept;
-  for (uint32_t i = 0; i < room; ++i) {
-    kept.grow(hist, i ? keep_next(kept) : kKeepFirst);
-    smallest[i] = kept.smallest();
-    items[i] = kept.items;
-    if (smallest[i] == 0) return (int)i + 1;
-  }
-  return (int)room;
+// Diagnostic: what a reference-heap selection keeps of counts with this histogram
+// (kCountBuckets words) at first: the smallest count, and how many items that makes.
+extern "C" int rip_selftest_keep(const uint32_t *hist, uint32_t *smallest, uint64_t *items) {
+  *smallest = keep_from(hist, items);
+  return RIP_OK;
 }
 
 // The counts left by the last selection still sit in the count buffer; bring
@@ -313,43 +290,53 @@ extern "C" int rip_select(rip_pool *p, uint64_t S, uint32_t k, int tiebreak,
     // InitHeapStorage + std::priority_queue(cmp, std::move(storage)), as the
     // reference builds its heap (streaming_find_most_influential.h:541-544;
     // counting.h:196-206), of which the host takes the items that can decide a
-    // pick (sparse_heap.h): those whose count is at least K, about kKeepFirst of
-    // them at first, and more -- the pops so far repeated on the larger heap --
-    // if the gains fall below K.  At n = 2^24 the whole heap was 128 MB over
-    // the bus a selection (4.2 of 14.5 ms), and every pop sank to a leaf 24
-    // levels down.
+    // pick (sparse_heap.h): those whose count is at least K, up to kKeepFirst of
+    // them (at n = 2^24 the whole heap was 128 MB over the bus a selection, 4.2 of
+    // 14.5 ms, and every pop sank to a leaf 24 levels down).  If the gains fall
+    // below K it takes the whole heap and repeats the pops so far on it, some
+    // 16 000.  (Some eight times as many items at a time instead, in four steps,
+    // repeated up to a million pops: an IMM on 2^21 Erdos-Renyi vertices, 100 seeds,
+    // eps 0.2, 11.5 million pops: 4.2 s; the whole heap from the start, with
+    // std::pop_heap: 3.15; so 2.05.)
     constexpr uint32_t kGone = 0xFFFFFFFFu;  // log: the popped item stayed out (a seed)
     SparseHeap &heap = c->heap;
-    std::vector<uint32_t> ids;  // vertex by item id
-    std::vector<uint32_t> log;  // per pop: the key it went back with, or kGone
-    // an item's count as last fetched, and the fetch (pick) that brought it
-    std::vector<uint32_t> cnt, cnt_at;
-    uint32_t fetch = 0;
-    KeptCounts kept;
-    uint32_t K = 0, R = 0;
+    std::vector<uint32_t> ids;  // vertex by item id (of the full heap: the id itself)
+    std::vector<uint32_t> log;  // per pop until then: the key it went back with, or kGone
+    std::vector<rip_ctx::Fetched> &fetched = c->fetched;
+    uint64_t kept = 0;
+    uint32_t K = keep_from(hist, &kept);
     TRY(dalloc(c, p->d_heap, sizeof(uint2) * (size_t)n));
     if (!c->h_list) c->h_list = new PinnedMem();
-    // Keeps more items: the next smaller counts, about `want` of all.
-    auto build = [&](uint64_t want, const uint32_t *d_count) -> int {
-      kept.grow(hist, want);
-      K = kept.smallest();
-      R = (uint32_t)kept.items;
+    auto vertex_of = [&](uint32_t id) { return heap.all() ? id : ids[id]; };
+    // The heap of these counts, of which the items of K or more are kept.
+    auto build = [&](const uint32_t *d_count) -> int {
       CK(c, launch_make_heap(d_count, n, ptr<uint2>(p->d_heap), K, c->stream));
-      const size_t words = 3 * (size_t)R;
-      TRY(dalloc(c, p->d_list, sizeof(uint32_t) * (words + 1)));
+      const uint32_t R = (uint32_t)kept;
+      const size_t words = K ? 3 * (size_t)R : 2 * (size_t)n;
       TRY(c->h_list->ensure(c, sizeof(uint32_t) * words));
-      launch_heap_list(ptr<uint2>(p->d_heap), n, K, R, ptr<uint32_t>(p->d_list),
-                       ptr<unsigned int>(p->d_list) + words, c->stream);
-      CK(c, cudaGetLastError());
-      CK(c, cudaMemcpyAsync(c->h_list->p, p->d_list.p, sizeof(uint32_t) * words,
+      if (K) {
+        TRY(dalloc(c, p->d_list, sizeof(uint32_t) * (words + 1)));
+        launch_heap_list(ptr<uint2>(p->d_heap), n, K, R, ptr<uint32_t>(p->d_list),
+                         ptr<unsigned int>(p->d_list) + words, c->stream);
+        CK(c, cudaGetLastError());
+      }
+      CK(c, cudaMemcpyAsync(c->h_list->p, K ? p->d_list.p : p->d_heap.p, sizeof(uint32_t) * words,
                             cudaMemcpyDeviceToHost, c->stream));
       CK(c, cudaStreamSynchronize(c->stream));
-      const uint32_t *vtx = static_cast<const uint32_t *>(c->h_list->p);
-      ids.assign(vtx, vtx + R);
-      cnt.resize(R);
-      cnt_at.assign(R, 0u);
-      fetch = 0;
-      heap.build(n, R, K, vtx + R, vtx + 2 * (size_t)R);
+      const size_t room = K ? R : n;
+      if (fetched.size() < room) fetched.resize(room, rip_ctx::Fetched{0, 0});
+      if (c->fetch > 0xF0000000u) {  // long before the numbers come round
+        std::fill(fetched.begin(), fetched.end(), rip_ctx::Fetched{0, 0});
+        c->fetch = 0;
+      }
+      ++c->fetch;  // (ids of another heap: no count is known)
+      if (K) {
+        const uint32_t *vtx = static_cast<const uint32_t *>(c->h_list->p);
+        ids.assign(vtx, vtx + R);
+        heap.build(n, R, vtx + R, vtx + 2 * (size_t)R);
+      } else {
+        heap.adopt(static_cast<HeapItem *>(c->h_list->p), n);
+      }
       for (uint32_t key : log) {
         const uint32_t id = heap.top_id();
         heap.pop();
@@ -357,7 +344,7 @@ extern "C" int rip_select(rip_pool *p, uint64_t S, uint32_t k, int tiebreak,
       }
       return RIP_OK;
     };
-    TRY(build(kKeepFirst, ptr<uint32_t>(p->count)));
+    TRY(build(ptr<uint32_t>(p->count)));
     p->sel_prof[1] += ms_since(t_h0);
     const auto t_p0 = clk::now();
     // The lazy pops of a pick only read the current counts of heap items keyed
@@ -373,7 +360,7 @@ extern "C" int rip_select(rip_pool *p, uint64_t S, uint32_t k, int tiebreak,
     const uint32_t *d_ids = reinterpret_cast<const uint32_t *>(db + 16);
     uint32_t *d_cnt = reinterpret_cast<uint32_t *>(db + 16) + CAND_CAP;
     std::vector<uint32_t> cand(CAND_CAP);  // the items whose vertices are in h_ids
-    std::vector<size_t> stack;
+    std::vector<uint32_t> stack;
     // First pick: every key is still exact.
     bool fresh_all = false, first = true;
     double ratio = 0.9;   // recent gain ratio g_i / g_{i-1}
@@ -408,8 +395,8 @@ extern "C" int rip_select(rip_pool *p, uint64_t S, uint32_t k, int tiebreak,
     };
     auto collect = [&](uint32_t T) -> uint32_t {
       const auto t_c0 = clk::now();
-      const uint32_t nc = collect_at_least(heap, T, CAND_CAP, cand.data(), stack);
-      for (uint32_t i = 0; i < std::min(nc, CAND_CAP); ++i) h_ids[i] = ids[cand[i]];
+      const uint32_t nc = heap.collect(T, CAND_CAP, heap.all() ? nullptr : ids.data(), cand.data(),
+                                       h_ids, stack);
       p->sel_prof[10] += ms_since(t_c0);
       return nc;
     };
@@ -442,12 +429,11 @@ extern "C" int rip_select(rip_pool *p, uint64_t S, uint32_t k, int tiebreak,
           CK(c, cudaStreamSynchronize(c->stream));
         }
         p->sel_prof[5] += nc;
-        ++fetch;
+        const uint32_t fetch = ++c->fetch;
         uint32_t mc = 0;
         for (uint32_t i = 0; i < nc; ++i) {
           const uint32_t cv = *reinterpret_cast<volatile uint32_t *>(h_cnt + i);
-          cnt[cand[i]] = cv;
-          cnt_at[cand[i]] = fetch;
+          fetched[cand[i]] = rip_ctx::Fetched{cv, fetch};
           mc = std::max(mc, cv);
         }
         if (mc >= T || T <= 1) {
@@ -460,11 +446,12 @@ extern "C" int rip_select(rip_pool *p, uint64_t S, uint32_t k, int tiebreak,
       prefetched = false;
       return RIP_OK;
     };
-    // The gains fell below K: keep more items.  Every item's count at the
-    // start is still in the heap array.
-    auto keep_more = [&]() -> int {
+    // The gains fell below K.  Every item's count at the start is still in the
+    // heap array.
+    auto keep_all = [&]() -> int {
+      K = 0;
       launch_heap_counts(ptr<uint2>(p->d_heap), n, ptr<uint32_t>(p->inv_cur), c->stream);
-      TRY(build(keep_next(kept), ptr<uint32_t>(p->inv_cur)));
+      TRY(build(ptr<uint32_t>(p->inv_cur)));
       prefetched = false;
       return first || fresh_all ? RIP_OK : fetch_candidates(out_gains.back());
     };
@@ -476,25 +463,25 @@ extern "C" int rip_select(rip_pool *p, uint64_t S, uint32_t k, int tiebreak,
       const auto t_q0 = clk::now();
       for (;;) {  // getNextSeed, streaming_find_most_influential.h:560-571
         if (!heap.top_kept()) {
-          if (K == 0) return set_err(c, RIP_ERR_STATE, "selection heap exhausted");
-          TRY(keep_more());
+          if (heap.all()) return set_err(c, RIP_ERR_STATE, "selection heap exhausted");
+          TRY(keep_all());
           continue;
         }
         id = heap.top_id();
         const uint32_t key = heap.top_key();
         uint32_t cur = key;
         if (!first) {
-          if (!fresh_all && cnt_at[id] != fetch) TRY(fetch_all());
-          cur = fresh_all ? hcount[ids[id]] : cnt[id];
+          if (!fresh_all && fetched[id].at != c->fetch) TRY(fetch_all());
+          cur = fresh_all ? hcount[vertex_of(id)] : fetched[id].count;
         }
         heap.pop();
         p->sel_prof[3] += 1;
         if (key > cur) {
           heap.push(id, cur, cur >= K);
-          log.push_back(cur);
+          if (!heap.all()) log.push_back(cur);
           continue;
         }
-        log.push_back(kGone);
+        if (!heap.all()) log.push_back(kGone);
         gain = key;
         break;
       }
@@ -502,14 +489,14 @@ extern "C" int rip_select(rip_pool *p, uint64_t S, uint32_t k, int tiebreak,
       if (!out_gains.empty() && out_gains.back())
         ratio = std::min(1.0, (double)gain / (double)out_gains.back());
       uncovered -= gain;
-      out_seeds.push_back(ids[id]);
+      out_seeds.push_back(vertex_of(id));
       out_gains.push_back(gain);
       if (out_seeds.size() == k) break;
       const auto t_f0 = clk::now();
       pre_T = first_T(gain);
       pre_nc = collect0(gain, pre_T);
       if (pre_nc <= FUSED_MAX) {
-        C.vertex = ids[id];
+        C.vertex = vertex_of(id);
         C.blocks = (int)std::min<uint64_t>(max_blocks * 4,
                                            std::max<uint64_t>(1, ((uint64_t)gain + 7) / 8));
         // epochs count per context: the mapped buffer is the context's
@@ -532,7 +519,7 @@ extern "C" int rip_select(rip_pool *p, uint64_t S, uint32_t k, int tiebreak,
         std::atomic_thread_fence(std::memory_order_acquire);
         prefetched = true;
       } else {
-        TRY(cover(ids[id], gain));
+        TRY(cover(vertex_of(id), gain));
       }
       p->sel_prof[7] += ms_since(t_f0);
       fresh_all = first = false;

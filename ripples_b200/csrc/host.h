@@ -241,8 +241,12 @@ struct PinnedMem {
 constexpr double kSupercritical = 1.1;
 
 // Edges from which supercritical graphs do so: on a smaller graph one CTA
-// finishes a set before the grid has been through its levels.
-constexpr uint64_t kGiantEdges = 1ull << 21;
+// finishes a set before the grid has been through its levels.  IMM, k = 20,
+// eps = 0.5, grid-wide and one CTA a set: R-MAT (p ~ U(0, 0.1)) with 2.5, 3, 4.2, 6.3
+// and 8.4 million edges 33, 37, 42.7, 56, 59 and 26, 34, 45.0, 66, 64 ms;
+// Erdos-Renyi graphs (three live edges a vertex), whose sets share fewer in-lists, 83,
+// 86, 90, 95, 100 and 52, 54, 57, 68, 75.
+constexpr uint64_t kGiantEdges = 1ull << 22;
 
 // In-edges of a set after which a warp leaves it to the heavy-set path.  A
 // warp takes 256 of them in about a microsecond and a launch ends with its

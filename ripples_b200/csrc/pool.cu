@@ -870,9 +870,11 @@ extern "C" int rip_sample(rip_pool *p, uint64_t seed, uint64_t count,
   if (m.stats[2] == 0 && count > 4096) {
     // A fused batch is one CTA's chain of levels, as long in a pilot of a few
     // batches as in a launch that fills the device (2^14 vertices, 128 colours:
-    // 2.7 ms for 1024 sets, 3.4 for 19 000): up to 64 MB of pool, room for 256
-    // members a set is taken instead (what overflows it is sampled again, as
-    // after a pilot that guessed low).
+    // 2.7 ms for 1024 sets, 3.4 for 19 000): up to 84 MB of pool, room for 256
+    // members a set is taken instead.  What overflows it is sampled again, as
+    // after a pilot that guessed low: still the faster way (first samples of 5000,
+    // 20 000, 60 000 sets of 650 members, 2^15 vertices: 10.5, 12.6, 22.0 ms, 19.2,
+    // 21.1, 27.0 with a pilot; 20 000 of 99 members 3.5 and 6.5).
     const uint64_t avail = c->budget > c->used ? c->budget - c->used : 0;
     if (fused && count <= (1u << 16) && avail / 4 >= count * 1024) {
       mean = 256.0;

@@ -42,11 +42,10 @@ struct FailList {
   uint32_t *ids;          // indices relative to the launch's first set
   unsigned int *count;
   unsigned long long *first_bad_base;  // lowest pool offset of a failed reservation
-  // sets handed over for their edge work go to a list of their own when there
-  // is one with room (it stays on the device), else to ids with FAIL_BIG
-  uint32_t *big = nullptr;
+  // sets handed over for their edge work: a list of their own, downwards from
+  // big_end (a launch with a work cap has one; it stays on the device)
+  uint32_t *big_end = nullptr;
   unsigned int *big_count = nullptr;
-  uint32_t big_cap = 0;  // the list's room: later ones go to ids
 };
 
 // Counters for roofline accounting (see rip_pool_stats in ripples_b200.h).

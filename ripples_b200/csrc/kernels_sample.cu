@@ -80,9 +80,8 @@ __device__ bool finish_set(const WarpCtx &W, uint32_t qlen, bool overflow,
                            const FailList &F, bool big = false, bool clear_bitmap = true) {
   const bool stored = store_set(W, qlen, overflow, s, P, F.first_bad_base, clear_bitmap);
   if (!stored && lane_id() == 0) {
-    const uint32_t pos = big && F.big ? atomicAdd(F.big_count, 1u) : ~0u;
-    if (pos < F.big_cap) F.big[pos] = rel;
-    else F.ids[atomicAdd(F.count, 1u)] = big ? (rel | FAIL_BIG) : rel;
+    if (big) F.big_end[-1 - (int64_t)atomicAdd(F.big_count, 1u)] = rel;
+    else F.ids[atomicAdd(F.count, 1u)] = rel;
   }
   __syncwarp();
   return stored;

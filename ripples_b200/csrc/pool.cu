@@ -177,7 +177,8 @@ static uint32_t default_warps(rip_pool *p, uint32_t qcap) {
 static int sample_fused(rip_pool *p, uint64_t seed, uint64_t first, uint32_t count);
 static int sample_big(rip_pool *p, uint64_t seed, uint64_t first,
                       const std::vector<uint32_t> &ids);
-static int sample_big_listed(rip_pool *p, uint64_t seed, uint64_t first, uint32_t count);
+static int sample_big_listed(rip_pool *p, uint64_t seed, uint64_t first, uint32_t count,
+                             uint32_t *ids, uint32_t *failed);
 
 // One set per warp (IC BFS / LT walk).  IC sets whose edge work exceeds the
 // per-set cap are handed to the CTA-per-set sampler; sets that outgrow the warp
@@ -203,15 +204,11 @@ static int sample_warp_per_set(rip_pool *p, uint64_t seed, uint64_t first,
     ids = ptr<uint32_t>(p->ids_b);
   }
   const bool capped = g->model == RIP_MODEL_IC && p->cap_plain != 0;
-  // sets handed over stay on the device, up to 2^20 of them (b_ids has room
-  // for those that fail there too)
-  const uint32_t big_cap = capped ? std::min<uint32_t>(count, 1u << 20) : 0;
+  // sets handed over stay on the device, in the failure list's other end: a set is
+  // in one of them at most
   uint32_t n_big = 0;
-  if (capped) {
-    TRY(dalloc(c, p->b_ids, sizeof(uint32_t) * 2 * (size_t)big_cap));
-    CK(c, cudaMemsetAsync(&dm->big_count, 0, sizeof(unsigned int), c->stream));
-  }
-  std::vector<uint32_t> big, retry;
+  if (capped) CK(c, cudaMemsetAsync(&dm->big_count, 0, sizeof(unsigned int), c->stream));
+  std::vector<uint32_t> retry;
   for (int attempt = 0; attempt < 64; ++attempt) {
     CK(c, cudaMemsetAsync(&dm->fail_count, 0, sizeof(unsigned int), c->stream));
     CK(c, cudaMemsetAsync(&dm->next, 0, sizeof(unsigned int), c->stream));
@@ -231,9 +228,8 @@ static int sample_warp_per_set(rip_pool *p, uint64_t seed, uint64_t first,
     L.work_cap = capped ? p->cap_plain : 0;
     L.F = FailList{ptr<uint32_t>(p->ids_a), &dm->fail_count, &dm->first_bad};
     if (capped) {
-      L.F.big = ptr<uint32_t>(p->b_ids);
+      L.F.big_end = ptr<uint32_t>(p->ids_a) + count;
       L.F.big_count = &dm->big_count;
-      L.F.big_cap = big_cap;
     }
     L.st = Stats{dm->stats};
     L.threads = 256;
@@ -253,7 +249,7 @@ static int sample_warp_per_set(rip_pool *p, uint64_t seed, uint64_t first,
     cudaEventElapsedTime(&kms, c->ev0, c->ev1);
     p->kernel_ms += kms;
     p->kernel_launches++;
-    if (capped) n_big = std::min<uint32_t>(m.big_count, big_cap);
+    if (capped) n_big = m.big_count;
     if (m.fail_count == 0) {
       p->num_elems = m.cursor;
       break;
@@ -262,17 +258,11 @@ static int sample_warp_per_set(rip_pool *p, uint64_t seed, uint64_t first,
     unsigned long long cur = std::min<unsigned long long>(m.cursor, m.first_bad);
     CK(c, cudaMemcpyAsync(&dm->cursor, &cur, sizeof(cur), cudaMemcpyHostToDevice, c->stream));
     p->num_elems = cur;
-    std::vector<uint32_t> failed(m.fail_count);
-    CK(c, cudaMemcpyAsync(failed.data(), p->ids_a.p, sizeof(uint32_t) * m.fail_count,
+    retry.resize(m.fail_count);
+    CK(c, cudaMemcpyAsync(retry.data(), p->ids_a.p, sizeof(uint32_t) * m.fail_count,
                           cudaMemcpyDeviceToHost, c->stream));
     CK(c, cudaStreamSynchronize(c->stream));
-    retry.clear();
     bool queue_overflow = false;
-    for (uint32_t f : failed) {
-      if (f & FAIL_BIG) big.push_back(f & ~FAIL_BIG);
-      else retry.push_back(f);
-    }
-    if (retry.empty()) break;
     if (m.first_bad != ~0ull) {
       double mean = m.stats[2] ? (double)m.stats[3] / (double)m.stats[2] : 16.0;
       uint64_t need = cur + (uint64_t)(mean * 2.0 * retry.size()) + 4096;
@@ -293,11 +283,9 @@ static int sample_warp_per_set(rip_pool *p, uint64_t seed, uint64_t first,
     todo = (uint32_t)retry.size();
     if (attempt == 63) return set_err(c, RIP_ERR_DEVICE, "sampler did not converge after retries");
   }
-  if (n_big) TRY(sample_big_listed(p, seed, first, n_big));
-  if (!big.empty()) {
-    std::sort(big.begin(), big.end());
-    TRY(sample_big(p, seed, first, big));
-  }
+  if (n_big)  // (the retries are through: ids_b is free)
+    TRY(sample_big_listed(p, seed, first, n_big, ptr<uint32_t>(p->ids_a) + count - n_big,
+                          ptr<uint32_t>(p->ids_b)));
   return RIP_OK;
 }
 
@@ -452,21 +440,23 @@ static int sample_big(rip_pool *p, uint64_t seed, uint64_t first,
   TRY(dalloc(c, p->b_ids, sizeof(uint32_t) * ids.size() * 2));
   CK(c, cudaMemcpyAsync(p->b_ids.p, ids.data(), sizeof(uint32_t) * ids.size(),
                         cudaMemcpyHostToDevice, c->stream));
-  return sample_big_listed(p, seed, first, (uint32_t)ids.size());
+  uint32_t *d_ids = ptr<uint32_t>(p->b_ids);
+  return sample_big_listed(p, seed, first, (uint32_t)ids.size(), d_ids, d_ids + ids.size());
 }
 
-// The same for `count` ids in b_ids (which has room for twice as many), one
-// CTA each unless the grid-wide BFS takes them.
-static int sample_big_listed(rip_pool *p, uint64_t seed, uint64_t first, uint32_t count) {
+// The same for `count` ids on the device, one CTA each unless the grid-wide BFS
+// takes them; `failed` has room for as many, both are written.
+static int sample_big_listed(rip_pool *p, uint64_t seed, uint64_t first, uint32_t count,
+                             uint32_t *ids, uint32_t *failed) {
   rip_ctx *c = p->ctx;
   rip_graph *g = p->g;
   if (p->giant_min && count >= p->giant_min) {
-    std::vector<uint32_t> ids(count);
-    CK(c, cudaMemcpyAsync(ids.data(), p->b_ids.p, sizeof(uint32_t) * count,
-                          cudaMemcpyDeviceToHost, c->stream));
+    std::vector<uint32_t> list(count);
+    CK(c, cudaMemcpyAsync(list.data(), ids, sizeof(uint32_t) * count, cudaMemcpyDeviceToHost,
+                          c->stream));
     CK(c, cudaStreamSynchronize(c->stream));
-    std::sort(ids.begin(), ids.end());
-    return sample_giant(p, seed, first, ids);
+    std::sort(list.begin(), list.end());
+    return sample_giant(p, seed, first, list);
   }
   const uint64_t bm_words = (((uint64_t)g->n + 31) / 32 + 7) & ~7ull;
   const uint32_t qcap = p->b_qcap ? p->b_qcap : std::min<uint32_t>(g->n, 1u << 18);
@@ -480,7 +470,6 @@ static int sample_big_listed(rip_pool *p, uint64_t seed, uint64_t first, uint32_
     return (uint32_t)std::max<uint64_t>(1, std::min<uint64_t>(max_slots, (avail / 4) / per));
   };
   TRY(ensure_big_scratch(p, slots_for(qcap), qcap));
-  uint32_t *ids = ptr<uint32_t>(p->b_ids), *failed = ids + count;
   PoolMeta *dm = p->dmeta();
   for (int attempt = 0; attempt < 32 && count; ++attempt) {
     CK(c, cudaMemsetAsync(&dm->fail_count, 0, sizeof(unsigned int), c->stream));

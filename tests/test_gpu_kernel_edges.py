@@ -376,3 +376,25 @@ def test_record_tiles(ctx, threads):
     st = p.stats()
     assert st[4] == ost[0] and st[5] == ost[1]
     dg.close()
+
+
+def budget_calls():
+    """Calls and device budgets (bytes) that are enough for them: a few KB above the
+    least, which is what the graph, the sets and the smallest scratch take."""
+    def graph(draws, n, weights, hi):
+        return rb.HostGraph.erdos_renyi(n, draws, seed=1).with_weights(weights, 2, 0.0, hi)
+
+    def sample(ctx):
+        p = rb.Pool(rb.DeviceGraph(ctx, graph(1 << 14, 1 << 12, rb.WEIGHTS_UNIFORM, 0.05), "IC"))
+        p.sample(200000, seed=3, sampler=rb.SAMPLER_PLAIN)
+
+    return [pytest.param(sample, 6100000, id="sets that may be handed over")]
+
+
+@pytest.mark.parametrize("call,budget", budget_calls())
+def test_budgets_that_are_enough(call, budget):
+    ctx = rb.Context(0, budget)
+    try:
+        call(ctx)
+    finally:
+        ctx.close()

@@ -68,10 +68,9 @@ extern "C" int rip_graph_upload(rip_ctx *c, const uint64_t *index,
   g->m = m;
   g->model = model;
   const uint64_t m_pad = ((m + 3) & ~3ull) + 4;
-  DevMem d_index, d_src, d_w, d_pack;
+  DevMem d_index, d_src, d_w;
   int rc = RIP_OK;
   do {
-    if (model == RIP_MODEL_LT && (rc = dalloc(c, d_pack, pack_lt_scratch(m)))) break;
     if ((rc = dalloc(c, g->off, sizeof(uint32_t) * ((size_t)n + 1)))) break;
     if ((rc = dalloc(c, g->edges, sizeof(uint2) * m_pad))) break;
     if ((rc = dalloc(c, d_index, sizeof(uint64_t) * ((size_t)n + 1)))) break;
@@ -112,7 +111,7 @@ extern "C" int rip_graph_upload(rip_ctx *c, const uint64_t *index,
     else
       launch_pack_lt(ptr<uint64_t>(d_index), ptr<float>(d_w), n, m,
                      ptr<uint32_t>(g->off), ptr<uint2>(g->edges),
-                     ptr<uint32_t>(d_src), d_pack.p, c->stream);
+                     ptr<uint32_t>(d_src), c->stream);
     e = cudaStreamSynchronize(c->stream);
     if (e == cudaSuccess) e = cudaGetLastError();
     if (e != cudaSuccess)
@@ -121,7 +120,6 @@ extern "C" int rip_graph_upload(rip_ctx *c, const uint64_t *index,
   dfree(c, d_index);
   dfree(c, d_src);
   dfree(c, d_w);
-  dfree(c, d_pack);
   if (rc == RIP_OK) rc = setup_vthr(c, g);
   if (rc != RIP_OK) {
     dfree(c, g->off);
@@ -147,20 +145,17 @@ int pack_device_csr(rip_ctx *c, const uint64_t *d_index, const uint32_t *d_src,
   const uint64_t m_pad = ((m + 3) & ~3ull) + 4;
   int rc = dalloc(c, g->off, sizeof(uint32_t) * ((size_t)n + 1));
   if (!rc) rc = dalloc(c, g->edges, sizeof(uint2) * m_pad);
-  DevMem d_pack;
-  if (!rc && model == RIP_MODEL_LT) rc = dalloc(c, d_pack, pack_lt_scratch(m));
   if (!rc) {
     if (model == RIP_MODEL_IC)
       launch_pack_ic(d_index, d_w, n, m, ptr<uint32_t>(g->off), ptr<uint2>(g->edges), d_src,
                      c->stream);
     else
       launch_pack_lt(d_index, d_w, n, m, ptr<uint32_t>(g->off), ptr<uint2>(g->edges), d_src,
-                     d_pack.p, c->stream);
+                     c->stream);
     cudaError_t e = cudaStreamSynchronize(c->stream);
     if (e == cudaSuccess) e = cudaGetLastError();
     if (e != cudaSuccess) rc = set_err(c, RIP_ERR_CUDA, "pack failed: %s", cudaGetErrorString(e));
   }
-  dfree(c, d_pack);
   if (!rc) rc = setup_vthr(c, g);
   if (rc) {
     dfree(c, g->off);

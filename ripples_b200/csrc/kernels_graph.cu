@@ -257,18 +257,18 @@ void launch_uniform_threshold(const uint32_t *off, const uint2 *edges, uint32_t 
   branching_kernel<<<2368, 256, 0, stream>>>(edges, m, lam, reinterpret_cast<double *>(sums + 1));
 }
 
-size_t pack_lt_scratch(uint64_t m) { return sizeof(uint32_t) * (m / kPackLong + 2); }
-
 void launch_pack_lt(const uint64_t *index, const float *w, uint32_t n,
-                    uint64_t m, uint32_t *off, uint2 *edges, const uint32_t *src, void *scratch,
+                    uint64_t m, uint32_t *off, uint2 *edges, const uint32_t *src,
                     cudaStream_t stream) {
   count_launches(3);
-  unsigned int *nlong = static_cast<unsigned int *>(scratch);
-  uint32_t *longs = nlong + 1;
+  // the offsets' room (n + 1 words) holds the long lists' count and ids until they
+  // are packed
+  unsigned int *nlong = off;
+  uint32_t *longs = off + 1;
   cudaMemsetAsync(nlong, 0, sizeof(*nlong), stream);
-  pack_off_kernel<<<1184, 256, 0, stream>>>(index, n, off);
   pack_lt_kernel<<<2368, 256, 0, stream>>>(index, src, w, n, m, pad4(m) + 4, edges, nlong, longs);
   pack_lt_long_kernel<<<1184, 256, 0, stream>>>(index, src, w, edges, nlong, longs);
+  pack_off_kernel<<<1184, 256, 0, stream>>>(index, n, off);
 }
 
 }  // namespace rip

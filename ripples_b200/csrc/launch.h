@@ -198,10 +198,8 @@ void launch_pack_ic(const uint64_t *index, const float *w, uint32_t n,
                     cudaStream_t stream);
 void launch_validate_csr(const uint64_t *index, const uint32_t *src, uint32_t n, uint64_t m,
                          unsigned long long *bad, cudaStream_t stream);
-// (scratch: pack_lt_scratch(m) bytes)
-size_t pack_lt_scratch(uint64_t m);
 void launch_pack_lt(const uint64_t *index, const float *w, uint32_t n,
-                    uint64_t m, uint32_t *off, uint2 *edges, const uint32_t *src, void *scratch,
+                    uint64_t m, uint32_t *off, uint2 *edges, const uint32_t *src,
                     cudaStream_t stream);
 // Per-vertex uniform IC thresholds (DevGraph::vthr); sums[0] = the edges they
 // cover, sums[1] holds a double whose value / m is the branching factor of a

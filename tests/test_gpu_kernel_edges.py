@@ -388,7 +388,13 @@ def budget_calls():
         p = rb.Pool(rb.DeviceGraph(ctx, graph(1 << 14, 1 << 12, rb.WEIGHTS_UNIFORM, 0.05), "IC"))
         p.sample(200000, seed=3, sampler=rb.SAMPLER_PLAIN)
 
-    return [pytest.param(sample, 6100000, id="sets that may be handed over")]
+    def spread(ctx):
+        g = graph(400000, 100000, rb.WEIGHTS_LT_NORMALIZED, 1.0)
+        fg, bg = rb.DeviceGraph(ctx, g.forward(), "IC"), rb.DeviceGraph(ctx, g, "LT")
+        rb.spread_lt(fg, bg, [1, 2, 3], 50, 1)
+
+    return [pytest.param(sample, 6100000, id="sets that may be handed over"),
+            pytest.param(spread, 12050000, id="LT lists packed")]
 
 
 @pytest.mark.parametrize("call,budget", budget_calls())

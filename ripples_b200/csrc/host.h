@@ -384,7 +384,7 @@ struct rip_pool {
   bool last_counts_on_device = false;  // last_counts still in `count` only
   bool have_last_counts = false;
   uint32_t cand_fixed = 0;           // first-fetch threshold, % of the last gain (0 = adaptive)
-  DevMem d_heap, d_list, d_hist;     // heap built on the device, its kept items, count buckets
+  DevMem d_heap;                     // heap built on the device
   DevMem s_cmax, s_dirty, s_best, s_desc;  // device lowest-id picks
   // reference-heap picks: completion ticket of the cover-and-gather kernel
   // (zero between launches)

@@ -52,7 +52,7 @@ extern "C" int rip_pool_destroy(rip_pool *p) {
   DevMem *all[] = {&p->vtx,     &p->set_off,   &p->set_len,  &p->meta,
                    &p->scratch, &p->ids_a,     &p->ids_b,    &p->f_vis,
                    &p->f_pend,  &p->f_flag,    &p->f_log,    &p->f_order,
-                   &p->b_scratch, &p->b_ids,   &p->d_heap, &p->d_list, &p->d_hist,
+                   &p->b_scratch, &p->b_ids,   &p->d_heap,
                    &p->g_state, &p->g_lists,   &p->g_col,
                    &p->s_cmax,  &p->s_dirty,   &p->s_best,   &p->s_desc,
 

@@ -194,15 +194,15 @@ static int prepare_cover(rip_pool *p, uint64_t S, uint64_t *P_out, uint32_t *his
   const uint32_t n = p->g->n;
   TRY(count_sets(p, S));
   TRY(dalloc(c, p->inv_off, sizeof(uint64_t) * ((size_t)n + 1)));
-  TRY(dalloc(c, p->inv_cur, sizeof(uint64_t) * ((size_t)n + 1)));
+  TRY(dalloc(c, p->inv_cur, std::max(sizeof(uint64_t) * ((size_t)n + 1),
+                                     sizeof(uint32_t) * kCountBuckets)));
   TRY(dalloc(c, p->scan_sums, sizeof(uint64_t) * scan_block_sums_needed(n)));
   launch_exclusive_scan(ptr<uint32_t>(p->count), ptr<uint64_t>(p->inv_off), n,
                         ptr<uint64_t>(p->scan_sums), c->stream);
   uint64_t P = 0;
-  if (hist) {
-    TRY(dalloc(c, p->d_hist, sizeof(uint32_t) * kCountBuckets));
-    launch_count_hist(ptr<uint32_t>(p->count), n, ptr<uint32_t>(p->d_hist), c->stream);
-    CK(c, cudaMemcpyAsync(hist, p->d_hist.p, sizeof(uint32_t) * kCountBuckets,
+  if (hist) {  // (in the cursors' room, before they are set)
+    launch_count_hist(ptr<uint32_t>(p->count), n, ptr<uint32_t>(p->inv_cur), c->stream);
+    CK(c, cudaMemcpyAsync(hist, p->inv_cur.p, sizeof(uint32_t) * kCountBuckets,
                           cudaMemcpyDeviceToHost, c->stream));
   }
   CK(c, cudaMemcpyAsync(&P, ptr<uint64_t>(p->inv_off) + n, sizeof(uint64_t),
@@ -305,6 +305,9 @@ extern "C" int rip_select(rip_pool *p, uint64_t S, uint32_t k, int tiebreak,
     std::vector<rip_ctx::Fetched> &fetched = c->fetched;
     uint64_t kept = 0;
     uint32_t K = keep_from(hist, &kept);
+    // the kept items come in the index cursors' room (the index is built)
+    uint32_t *d_list = ptr<uint32_t>(p->inv_cur);
+    if (3 * kept + 1 > 2 * ((uint64_t)n + 1)) K = 0;
     TRY(dalloc(c, p->d_heap, sizeof(uint2) * (size_t)n));
     if (!c->h_list) c->h_list = new PinnedMem();
     auto vertex_of = [&](uint32_t id) { return heap.all() ? id : ids[id]; };
@@ -315,12 +318,10 @@ extern "C" int rip_select(rip_pool *p, uint64_t S, uint32_t k, int tiebreak,
       const size_t words = K ? 3 * (size_t)R : 2 * (size_t)n;
       TRY(c->h_list->ensure(c, sizeof(uint32_t) * words));
       if (K) {
-        TRY(dalloc(c, p->d_list, sizeof(uint32_t) * (words + 1)));
-        launch_heap_list(ptr<uint2>(p->d_heap), n, K, R, ptr<uint32_t>(p->d_list),
-                         ptr<unsigned int>(p->d_list) + words, c->stream);
+        launch_heap_list(ptr<uint2>(p->d_heap), n, K, R, d_list, d_list + words, c->stream);
         CK(c, cudaGetLastError());
       }
-      CK(c, cudaMemcpyAsync(c->h_list->p, K ? p->d_list.p : p->d_heap.p, sizeof(uint32_t) * words,
+      CK(c, cudaMemcpyAsync(c->h_list->p, K ? (void *)d_list : p->d_heap.p, sizeof(uint32_t) * words,
                             cudaMemcpyDeviceToHost, c->stream));
       CK(c, cudaStreamSynchronize(c->stream));
       const size_t room = K ? R : n;

@@ -393,7 +393,14 @@ def budget_calls():
         fg, bg = rb.DeviceGraph(ctx, g.forward(), "IC"), rb.DeviceGraph(ctx, g, "LT")
         rb.spread_lt(fg, bg, [1, 2, 3], 50, 1)
 
+    def select(ctx):
+        p = rb.Pool(rb.DeviceGraph(ctx, graph(400000, 100000, rb.WEIGHTS_WC, 1.0), "IC"))
+        vtx = np.random.RandomState(1).randint(0, 100000, 400000).astype(np.uint32)
+        p.import_sets(np.arange(0, 400001, 2, dtype=np.uint64), vtx)
+        p.select(20, tiebreak=rb.TIE_REF_HEAP)
+
     return [pytest.param(sample, 6100000, id="sets that may be handed over"),
+            pytest.param(select, 13850000, id="reference heap"),
             pytest.param(spread, 12050000, id="LT lists packed")]
 
 

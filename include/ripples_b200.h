@@ -275,8 +275,8 @@ int rip_pool_plain_occupancy(rip_pool *p, int blocks_per_sm);
 int rip_pool_heavy_batch(rip_pool *p, uint32_t min_sets);
 
 /* Block shape of the one-CTA-per-set kernel for heavy IC sets: 128, 256, 512
- * or 1024 threads, 10, 5, 2 or 1 of them resident per SM (default: by the
- * number of heavy sets of a launch, smaller blocks for more sets; an
+ * or 1024 threads, 10, 5, 2 or 1 of them resident per SM, or 0: by the number
+ * of heavy sets of a launch, smaller blocks for more sets (the default; an
  * autotuned graph's pools start from its tuned value).  Smaller CTAs grow
  * more sets per SM at once, each with fewer threads.  Results do not depend on it.  No reference counterpart. */
 int rip_pool_heavy_block(rip_pool *p, uint32_t threads);

@@ -811,9 +811,9 @@ extern "C" int rip_pool_heavy_batch(rip_pool *p, uint32_t min_sets) {
   return RIP_OK;
 }
 
-// Block shape of the CTA-per-set kernel for heavy IC sets.
+// Block shape of the CTA-per-set kernel for heavy IC sets (0: big_shape's).
 extern "C" int rip_pool_heavy_block(rip_pool *p, uint32_t threads) {
-  if (!p || (threads != 128 && threads != 256 && threads != 512 && threads != 1024))
+  if (!p || (threads != 0 && threads != 128 && threads != 256 && threads != 512 && threads != 1024))
     return RIP_ERR_INVALID;
   p->big_threads = threads;
   return RIP_OK;

@@ -77,6 +77,25 @@ def test_sets_are_handed_over_where_it_pays(ctx, scale, weights, handed):
     dg.close()
 
 
+def test_heavy_block_goes_back_to_its_default(ctx):
+    g = hub_graph(64, [257, 1033, 4099], [1e-3, 0.02])
+    dg = rb.DeviceGraph(ctx, g, "IC")
+    p = rb.Pool(dg)
+    p.heavy_batch(0)
+    p.work_caps(64, 0)
+    sets = []
+    for threads in (0, 128, 1024, 0):
+        p.heavy_block(threads)
+        p.clear()
+        p.sample(300, seed=9, sampler=rb.SAMPLER_PLAIN)
+        sets.append(p.export())
+    assert all(np.array_equal(a, b) for s in sets[1:] for a, b in zip(s, sets[0]))
+    for threads in (1, 64, 2048):
+        with pytest.raises(rb.RipError):
+            p.heavy_block(threads)
+    dg.close()
+
+
 SET_LENGTHS = [0, 1, 31, 32, 33, 63, 64, 65, 511, 512, 513, 1023, 1024, 1025, 5000]
 
 

@@ -268,7 +268,7 @@ int rip_pool_plain_occupancy(rip_pool *p, int blocks_per_sm);
  * graph and overlap).  Default 32 on IC graphs whose reverse BFS is
  * supercritical -- the expected live in-edges of an edge's source,
  * sum over edges (u->v) of sum_{w->u} p(w->u) / m, above 1.1 -- and which have
- * at least 2^22 edges, else 0
+ * at least 7 * 2^19 edges, else 0
  * (weighted cascade: at most 1); 0 = always one CTA per set.  An autotuned graph's pools start from its
  * tuned value.  Results do not depend on it.  No reference counterpart (the reference's GPU BFS,
  * include/ripples/gpu/bfs.h:1338-1680, has one colour-batched path). */

@@ -246,7 +246,7 @@ constexpr double kSupercritical = 1.1;
 // and 8.4 million edges 33, 37, 42.7, 56, 59 and 26, 34, 45.0, 66, 64 ms;
 // Erdos-Renyi graphs (three live edges a vertex), whose sets share fewer in-lists, 83,
 // 86, 90, 95, 100 and 52, 54, 57, 68, 75.
-constexpr uint64_t kGiantEdges = 1ull << 22;
+constexpr uint64_t kGiantEdges = 7ull << 19;
 
 // In-edges of a set after which a warp leaves it to the heavy-set path.  A
 // warp takes 256 of them in about a microsecond and a launch ends with its

@@ -54,6 +54,11 @@ struct Stats {
 };
 
 __device__ __forceinline__ uint32_t lane_id() { return threadIdx.x & 31u; }
+__device__ __forceinline__ uint32_t lanes_below() {  // mask of the lanes before this one
+  uint32_t m;
+  asm("mov.u32 %0, %%lanemask_lt;" : "=r"(m));
+  return m;
+}
 
 __device__ __forceinline__ uint32_t warp_incl_scan(uint32_t x) {
 #pragma unroll

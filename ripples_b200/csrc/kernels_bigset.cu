@@ -57,7 +57,6 @@ ic_bigset_kernel(const __grid_constant__ BigLaunch L) {
   __shared__ unsigned long long s_base;
 
   const uint32_t tid = threadIdx.x, lane = lane_id(), wid = tid >> 5;
-  const uint32_t lanes_below = (1u << lane) - 1;
   uint32_t *bm = L.bitmaps + (size_t)blockIdx.x * L.bm_words;
   uint32_t *q = L.queues + (size_t)blockIdx.x * L.qcap;
   unsigned long long n_exp = 0, n_edges = 0, n_sets = 0, n_elems = 0, n_uedges = 0, n_usrc = 0;
@@ -118,7 +117,7 @@ ic_bigset_kernel(const __grid_constant__ BigLaunch L) {
     auto take_live = [&](uint32_t live, auto &&at) {
       for (uint32_t bal; (bal = __ballot_sync(FULL, live != 0)) != 0;) {
         if (live) {
-          ev[nev + __popc(bal & lanes_below)] = at((uint32_t)(__ffs(live) - 1));
+          ev[nev + __popc(bal & lanes_below())] = at((uint32_t)(__ffs(live) - 1));
           live &= live - 1;
         }
         nev += __popc(bal);

@@ -152,7 +152,7 @@ ic_fused_kernel(const __grid_constant__ FusedLaunch L) {
           if (!bal) continue;
           uint32_t pos = 0;
           if (lane == (uint32_t)(__ffs(bal) - 1)) pos = atomicAdd(&s_tail, __popc(bal));
-          pos = __shfl_sync(FULL, pos, __ffs(bal) - 1) + __popc(bal & pair_lanes_below());
+          pos = __shfl_sync(FULL, pos, __ffs(bal) - 1) + __popc(bal & lanes_below());
           if (push[t]) {
             if (pos < lcap) {
               if (pos < kSharedLog) s_log[pos] = u[t];

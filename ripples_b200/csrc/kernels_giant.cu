@@ -37,12 +37,6 @@ namespace rip {
 
 namespace {
 
-__device__ __forceinline__ uint32_t lanemask_lt_g() {
-  uint32_t m;
-  asm("mov.u32 %0, %%lanemask_lt;" : "=r"(m));
-  return m;
-}
-
 // Appends x (for lanes with want) to list[*tail ...], one atomic per warp.
 __device__ __forceinline__ void warp_append(bool want, uint32_t x, uint32_t *list,
                                             unsigned int *tail) {
@@ -52,7 +46,7 @@ __device__ __forceinline__ void warp_append(bool want, uint32_t x, uint32_t *lis
   uint32_t base = 0;
   if (lane_id() == leader) base = atomicAdd(tail, (unsigned int)__popc(bal));
   base = __shfl_sync(FULL, base, leader);
-  if (want) list[base + __popc(bal & lanemask_lt_g())] = x;
+  if (want) list[base + __popc(bal & lanes_below())] = x;
 }
 
 template <int CW>
@@ -202,7 +196,7 @@ giant_expand_kernel(const __grid_constant__ GiantLaunch L, uint32_t level) {
   auto append = [&](int k, bool want, uint32_t u) {
     const uint32_t bal = __ballot_sync(FULL, want);
     if (!bal) return;
-    if (want) out.v[k][nout[k] + __popc(bal & pair_lanes_below())] = u;
+    if (want) out.v[k][nout[k] + __popc(bal & lanes_below())] = u;
     nout[k] += __popc(bal);
     if (nout[k] < 32) return;
     nout[k] -= 32;
@@ -389,7 +383,7 @@ __global__ void __launch_bounds__(256) giant_scatter_kernel(GiantLaunch L, uint3
           const uint32_t members = __shfl_sync(FULL, has[g][w], j);
           const uint32_t at = __shfl_sync(FULL, pos[g][w], j);
           if (members >> lane & 1u)
-            L.P.vtx[s_at[w * 32 + j] + at + __popc(members & lanemask_lt_g())] = v[g];
+            L.P.vtx[s_at[w * 32 + j] + at + __popc(members & lanes_below())] = v[g];
         }
       }
     }

@@ -27,12 +27,6 @@ namespace rip {
 
 namespace {
 
-__device__ __forceinline__ uint32_t lanemask_lt() {
-  uint32_t m;
-  asm("mov.u32 %0, %%lanemask_lt;" : "=r"(m));
-  return m;
-}
-
 // In-lists of at least this many 8-edge coin blocks are swept by a whole
 // warp at a time instead of sharing it with other lists.
 constexpr uint32_t kLongBlocks = 32;
@@ -128,7 +122,7 @@ __device__ __forceinline__ SetOutcome ic_plain_set(const DevGraph &G, Key key, c
       overflow = true;
       return;
     }
-    if (isnew) W.q[qlen + __popc(bal & lanemask_lt())] = nu;
+    if (isnew) W.q[qlen + __popc(bal & lanes_below())] = nu;
     qlen += cnt;
   };
   auto block_live = [&](uint32_t b, uint32_t ob, uint32_t oe, uint32_t ovt) -> uint32_t {
@@ -161,7 +155,7 @@ __device__ __forceinline__ SetOutcome ic_plain_set(const DevGraph &G, Key key, c
     if (uniform) set_usrc += __popc(live);
     for (uint32_t bal; (bal = __ballot_sync(FULL, live != 0)) != 0;) {
       if (live) {
-        W.ev[nev + __popc(bal & lanemask_lt())] = at((uint32_t)(__ffs(live) - 1));
+        W.ev[nev + __popc(bal & lanes_below())] = at((uint32_t)(__ffs(live) - 1));
         live &= live - 1;
       }
       nev += __popc(bal);

@@ -39,12 +39,6 @@ namespace rip {
 
 namespace {
 
-__device__ __forceinline__ uint32_t lanemask_lt() {
-  uint32_t m;
-  asm("mov.u32 %0, %%lanemask_lt;" : "=r"(m));
-  return m;
-}
-
 constexpr uint32_t NONE = 0xFFFFFFFFu;
 
 // Sets of at least this many elements are walked by their whole block, 1024
@@ -246,7 +240,7 @@ inverted_kernel(DevPool P, uint64_t S, uint64_t *cursor, uint32_t *inv, uint64_t
         if (valid && leader == lane_id())
           b = atomicAdd(cur + v, (unsigned long long)__popc(peers));
         b = __shfl_sync(FULL, b, leader);
-        if (valid) inv[b + __popc(peers & lanemask_lt())] = (uint32_t)(base + s);
+        if (valid) inv[b + __popc(peers & lanes_below())] = (uint32_t)(base + s);
       },
       [&](uint64_t s, uint32_t v) { inv[atomicAdd(cur + v, 1ull)] = (uint32_t)(base + s); });
 }
@@ -978,7 +972,7 @@ heap_list_kernel(const uint2 *__restrict__ heap, uint32_t n, uint32_t K, uint32_
     if (!bal) continue;
     uint32_t at = 0;
     if (lane_id() == (uint32_t)(__ffs(bal) - 1)) at = atomicAdd(tail, (unsigned int)__popc(bal));
-    at = __shfl_sync(FULL, at, __ffs(bal) - 1) + __popc(bal & lanemask_lt());
+    at = __shfl_sync(FULL, at, __ffs(bal) - 1) + __popc(bal & lanes_below());
     if (want && at < R) {
       list[at] = it.x;
       list[(size_t)R + at] = it.y;

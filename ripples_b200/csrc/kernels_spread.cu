@@ -10,7 +10,7 @@
 // kTileBlocks blocks or more are listed and dealt to all warps in 32-block
 // tiles.  Small levels are packed over the whole CTA (kPackEntries).
 //   IC: out-edge e of a reached vertex fires in replica r iff its coin
-//       (coarse half from sim_ic_block(key, e >> 3, r), fine half from
+//       (coarse half from block e >> 3 of its CoinSet, fine half from
 //       sim_ic_fine on a coarse tie) is below threshold(e) (BFS over live
 //       edges, diffusion_simulation.h:73-127).
 //   LT: the live-edge form of the threshold model (Kempe, Kleinberg, Tardos,
@@ -44,12 +44,6 @@ constexpr uint32_t kTileBlocks = 128;  // lists of at least this many blocks go 
 // larger forms lose by it (2^20 vertices, p ~ U(0, 0.1), 50 hubs: 50.9 -> 53.5).
 constexpr uint32_t kPackEntries = 512;
 constexpr uint32_t kSimLong = 256;  // long lists a level may list
-
-__device__ __forceinline__ uint32_t sim_lanemask_lt() {
-  uint32_t m;
-  asm("mov.u32 %0, %%lanemask_lt;" : "=r"(m));
-  return m;
-}
 
 template <bool SHARED, int THREADS>
 __global__ void __launch_bounds__(THREADS, THREADS == 1024 ? 1 : 4)
@@ -104,7 +98,7 @@ spread_ic_kernel(const __grid_constant__ SpreadLaunch L) {
       if (!bal) return;
       uint32_t pos = 0;
       if (lane == (uint32_t)(__ffs(bal) - 1)) pos = atomicAdd(&s_qlen, (uint32_t)__popc(bal));
-      pos = __shfl_sync(FULL, pos, __ffs(bal) - 1) + __popc(bal & sim_lanemask_lt());
+      pos = __shfl_sync(FULL, pos, __ffs(bal) - 1) + __popc(bal & lanes_below());
       if (isnew && pos < L.qcap) q[pos] = u;
     };
     // Draws 8-edge block b's edges in [ob, oe) (an empty range: none) and follows

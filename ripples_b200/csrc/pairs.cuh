@@ -27,12 +27,6 @@ struct PairWarp {        // a warp's shared memory
 };
 // packed: first pair (10 bits) | first colour in the list (10) | colours - 1 (8)
 
-__device__ __forceinline__ uint32_t pair_lanes_below() {
-  uint32_t m;
-  asm("mov.u32 %0, %%lanemask_lt;" : "=r"(m));
-  return m;
-}
-
 // Coin blocks of a tile of an entry with pc colours, and of a window of it.
 __device__ __forceinline__ uint32_t window_blocks(uint32_t pc) { return kPairWindow / pc; }
 __device__ __forceinline__ uint32_t tile_blocks(uint32_t pc) {
@@ -50,7 +44,7 @@ __device__ __forceinline__ uint32_t fill_window(PairWarp &S, bool want, uint32_t
   const uint32_t total = __shfl_sync(FULL, incl, 31) & 0xFFFFu;
   __syncwarp();
   if (want) {
-    const uint32_t o = __popc(bal & pair_lanes_below());
+    const uint32_t o = __popc(bal & lanes_below());
     uint32_t at = (incl - mine) >> 16;
     S.own[o] = make_uint4(beg, end, beg >> 3, ((incl - mine) & 0xFFFFu) | (at << 10) | ((pc - 1) << 20));
     S.rcp[o] = (1u << 20) / pc + 1;
@@ -154,7 +148,7 @@ __device__ __forceinline__ void sweep_pairs(PairWarp &S, uint32_t npairs, uint32
       const uint32_t bal = __ballot_sync(FULL, live != 0);
       if (!bal) break;
       if (live) {
-        S.ev[nev + __popc(bal & pair_lanes_below())] = make_uint2(e0 + __ffs(live) - 1, pc);
+        S.ev[nev + __popc(bal & lanes_below())] = make_uint2(e0 + __ffs(live) - 1, pc);
         live &= live - 1;
       }
       nev += __popc(bal);

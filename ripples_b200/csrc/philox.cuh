@@ -149,13 +149,6 @@ RIP_HD uint32_t root_of(Key k, uint64_t s, uint32_t n) {
 #endif
 }
 
-// Coarse coins of the 8 edges 8b .. 8b+7 of set s: edge 8b + h is half
-// h & 1 of word h >> 1 (coarse_of).
-RIP_HD u32x4 ic_block(Key k, uint64_t b, uint64_t s) {
-  return philox((uint32_t)b, (uint32_t)(b >> 32), (uint32_t)s,
-                set_hi(s, DOM_IC), k.k0, k.k1);
-}
-
 // What the coin blocks of one set (or spread replica) share.  A block's
 // counter is (b, 0, s_lo, dom << 24 | s_hi) with b < 2^29 (edge ids are below
 // 2^32), so round 0's product of s_lo, and round 1's product of the word that
@@ -176,7 +169,8 @@ RIP_HD CoinSet coin_set(const RK &rk, uint64_t s, uint32_t dom) {
   return CoinSet{set_hi(s, dom) ^ rk.r1(0), lo1 ^ rk.r0(1), hi0 ^ rk.r1(1), lo0 ^ rk.r1(2)};
 }
 
-// ic_block() (sim_ic_block()) of block b for the set whose CoinSet is given.
+// Coarse coins of the 8 edges 8b .. 8b+7 of the set (or spread replica) whose
+// CoinSet is given: edge 8b + h is half h & 1 of word h >> 1 (coarse_of).
 template <class RK>
 RIP_HD u32x4 coin_block(const RK &rk, const CoinSet &S, uint32_t b) {
   uint32_t hi0, lo0, hi1, lo1;
@@ -225,12 +219,6 @@ RIP_HD bool ic_live(Key k, uint64_t s, uint64_t e, uint32_t coarse, uint32_t thr
 #else
   return coarse < th || (coarse == th && ic_fine(k, e, s) < (thr & 0xFFFFu));
 #endif
-}
-
-// Coarse coins of the 8 forward edges 8b .. 8b+7 in spread replica r.
-RIP_HD u32x4 sim_ic_block(Key k, uint64_t b, uint64_t r) {
-  return philox((uint32_t)b, (uint32_t)(b >> 32), (uint32_t)r,
-                set_hi(r, DOM_SIM_IC), k.k0, k.k1);
 }
 
 // Fine (low) 16 bits of the coin of forward edge e in spread replica r.

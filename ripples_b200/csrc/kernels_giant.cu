@@ -15,18 +15,19 @@
 //             its colour in the source's visited mask and, if it is new there,
 //             in its pending mask, and puts the source on the next level's
 //             frontier (once per level: a per-vertex level stamp).
-// What bounds expand: issue (58% of the slots busy, 45% of the warps resident);
-// a pair is some 350 instructions, 75 of them its coins.  An IMM query (k = 20,
-// eps = 0.5) on an R-MAT graph with 2^18 vertices, some 15 of 256 colours a
-// vertex and level, expands in 20.9 ms; a thread per block looping over its
-// colours took 20.3 but a scan of the blocks and an atomic per warp and append
-// besides: the query took 52.7 ms and takes 46.7.
 // A hub's in-edge list is therefore split over the whole grid, and a vertex
 // reached by many sets in the same level is read once for all of them.  When
 // the frontier is empty the members are counted per colour, placed in the
 // pool (host-reserved range), and the masks cleared -- only for vertices the
 // batch touched (a first-touch list).  Coins are the same (set, edge) Philox
 // draws as every other sampler, so the sets are bit-identical to theirs.
+//
+// What bounds expand: issue (58% of the slots busy, 45% of the warps resident);
+// a pair is some 350 instructions, 75 of them its coins.  An IMM query (k = 20,
+// eps = 0.5) on an R-MAT graph with 2^18 vertices, some 15 of 256 colours a
+// vertex and level, expands in 20.9 ms; a thread per block looping over its
+// colours took 20.3, but needed a scan of the blocks and an atomic per warp and
+// append besides (prep 4.5 ms where the items take 1.06).
 #include <algorithm>
 
 #include "device.cuh"
@@ -73,11 +74,6 @@ __global__ void __launch_bounds__(256) giant_seed_kernel(GiantLaunch L) {
 // the list's}: the short entries among them, or a tile of a long one.
 constexpr uint32_t kWindow = 0x80000000u;
 
-// Level prep: entry i of the frontier takes its vertex's pending colours; the
-// warp's entries become work items.  Masks move a whole sector at a time and a
-// block reserves its items with one atomic: with 8-byte accesses (each a partial
-// sector write) and an atomic a warp the launch waited 33 us where it now takes
-// 8 (57 000 entries a level on average).
 // A vertex's mask of CW words in one access (a whole 32-byte sector for CW = 4).
 template <int CW>
 __device__ __forceinline__ void load_mask(const uint64_t *p, uint64_t *m) {
@@ -98,6 +94,11 @@ __device__ __forceinline__ void store_mask(uint64_t *p, const uint64_t *m) {
   else *p = m[0];
 }
 
+// Level prep: entry i of the frontier takes its vertex's pending colours; the
+// warp's entries become work items.  Masks move a whole sector at a time and a
+// block reserves its items with one atomic: with 8-byte accesses (each a partial
+// sector write) and an atomic a warp the launch waited 33 us where it now takes
+// 8 (57 000 entries a level on average).
 template <int CW>
 __global__ void __launch_bounds__(256) giant_prep_kernel(GiantLaunch L, uint32_t nf) {
   __shared__ unsigned long long s_sum[8][4];

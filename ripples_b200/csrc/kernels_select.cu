@@ -284,7 +284,7 @@ __device__ __forceinline__ unsigned long long pick_key(uint32_t c, uint32_t v) {
 // A sharded pick's cover with its decrements listed instead of applied:
 // marks this shard's uncovered sets holding the vertex covered and appends
 // their members to `out` (each entry: that vertex's summed count drops by
-// one), a warp per set as cover_kernel.  At most the shard's element count
+// one), a warp per set.  At most the shard's element count
 // is written.
 __global__ void __launch_bounds__(256) cover_list_kernel(CoverLaunch C, uint32_t *out,
                                                          unsigned long long *cursor) {

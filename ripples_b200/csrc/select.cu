@@ -275,8 +275,9 @@ extern "C" int rip_select(rip_pool *p, uint64_t S, uint32_t k, int tiebreak,
   const int max_blocks = c->num_sms * 4;
   unsigned char *hb = static_cast<unsigned char *>(h_cand.p);
   unsigned char *db = static_cast<unsigned char *>(h_cand.dev);
-  // One pick: mark v's uncovered sets covered and decrement their members, one
-  // warp per set of v's inverted list (`gain` of them are still uncovered).
+  // One pick: mark v's uncovered sets (`gain` of its inverted list) covered and
+  // decrement their members, a warp for some of them at a time, a block for long
+  // ones.
   auto cover = [&](uint32_t v, uint64_t gain) -> int {
     C.vertex = v;
     C.blocks = (int)std::min<uint64_t>(max_blocks * 4, std::max<uint64_t>(1, (gain + 7) / 8));

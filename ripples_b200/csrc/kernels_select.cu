@@ -429,11 +429,16 @@ __global__ void __launch_bounds__(kBlock) cover_gather_kernel(CoverLaunch C, con
 // re-reads only those, then reduces the chunk maxima in the last block.
 constexpr uint32_t SEL_CHUNK = 1024;
 constexpr uint32_t kLoopCtas = 8, kLoopThreads = 512;
-constexpr uint32_t kLoopChunks = 2048;  // chunk maxima a block keeps
-// Elements of a round up to which one cluster makes all its picks: the two
-// rounds just below it of a weighted-cascade query on 2^20 Erdos-Renyi vertices
-// took 3.5 ms this way and 3.7 grid-wide; far above it the first covers alone
-// keep eight SMs busy longer than the grid takes for all picks.
+constexpr uint32_t kLoopChunks = 64;  // chunk maxima a block keeps
+// A round is one cluster's if its chunks (kLoopCtas * kLoopChunks: 2^19 vertices)
+// and elements are few enough; far above either, the chunks that covers touch
+// (every one is read again, 4 KB) or the first covers alone keep eight SMs busy
+// longer than the grid takes for all picks.  One cluster and grid-wide, lowest-id
+// IMMs of 150 seeds on R-MAT graphs of degree 8, weighted cascade (LT): 2^19
+// vertices 12.8 and 14.4 (7.2 and 8.3) ms, 2^20 20.5 and 16.2 (9.6 and 9.0), 2^21
+// 28.7 and 22.6 (18.0 and 12.7), 2^22 48.7 and 27.9 (23.4 and 11.1).  Elements: the
+// two rounds just below 8 M of a weighted-cascade query on Erdos-Renyi vertices 3.5
+// and 3.7 ms.
 constexpr double kLoopElements = 8.0 * (1 << 20);
 
 __device__ __forceinline__ unsigned long long sel_key(uint32_t c, uint32_t v) {

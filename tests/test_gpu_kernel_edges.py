@@ -255,6 +255,29 @@ def test_device_picks_in_one_launch_and_grid_wide(ctx, copies):
     dg.close()
 
 
+@pytest.mark.parametrize("n", [1 << 19, (1 << 19) + 1, 1100003])
+def test_device_picks_by_the_number_of_chunks(ctx, n):
+    """Small rounds of up to 512 chunks of 1024 vertices are one launch, those of more
+    go pick by pick: the last chunks full, of one vertex, ragged."""
+    r = np.random.RandomState(5)
+    sets = [np.unique(np.concatenate([[n - 1 - i % 3], r.randint(0, n, 1 + i % 90)]))
+            for i in range(3000)]
+    off = np.zeros(len(sets) + 1, dtype=np.uint64)
+    np.cumsum([len(x) for x in sets], out=off[1:])
+    vtx = np.concatenate(sets).astype(np.uint32)
+    g = rb.HostGraph(n, np.zeros(n + 1, np.uint64), np.zeros(0, np.uint32), np.zeros(0, np.float32))
+    dg = rb.DeviceGraph(ctx, g, "IC")
+    p = rb.Pool(dg)
+    p.import_sets(off, vtx)
+    for s, k in ((3000, 3), (2999, 60), (100, 40)):
+        e = int(off[s])
+        of, oseeds, ogains, _ = O.select(n, off[: s + 1], vtx[:e], k, rb.TIE_LOWEST_ID)
+        oseeds, ogains = oseeds[ogains > 0], ogains[ogains > 0]
+        f, seeds, gains = p.select(k, s, rb.TIE_LOWEST_ID)
+        assert f == of and seeds.tolist() == oseeds.tolist() and gains.tolist() == ogains.tolist()
+    dg.close()
+
+
 @pytest.mark.parametrize("total", [0.7, 5.0])
 def test_lt_pack_over_list_lengths(ctx, total):
     """Cumulative weights of lists that end on and off the scan's 32-edge and

@@ -40,9 +40,11 @@ constexpr uint32_t kTileBlocks = 128;  // lists of at least this many blocks go 
 // bitmap in shared memory: a warp's share of a small level leaves lanes without a
 // block, and its passes over live edges wait for each other, which is what replicas
 // of a few thousand vertices spend their time on.  R-MAT, p ~ U(0, 0.02), 5 hubs as
-// seeds, 1500 replicas: 2^16 vertices 0.86 -> 0.75 ms, 2^18 3.67 -> 3.47.  The
-// larger forms lose by it (2^20 vertices, p ~ U(0, 0.1), 50 hubs: 50.9 -> 53.5).
-constexpr uint32_t kPackEntries = 512;
+// seeds, 1500 replicas: 2^16 vertices 0.86 -> 0.755 ms, 2^18 3.67 -> 3.48.  Packing
+// levels of up to 512 entries gains more there (0.73), but loses where the seeds are
+// 178 hubs (0.68 -> 0.76 at p ~ U(0, 0.05)).  The larger forms lose by it (2^20
+// vertices, p ~ U(0, 0.1), 50 hubs: 50.9 -> 53.5).
+constexpr uint32_t kPackEntries = 128;
 constexpr uint32_t kSimLong = 256;  // long lists a level may list
 
 template <bool SHARED, int THREADS>
@@ -54,8 +56,8 @@ spread_ic_kernel(const __grid_constant__ SpreadLaunch L) {
   constexpr bool KEEP = THREADS == 1024;
   constexpr bool PACK = SHARED && !KEEP;
   extern __shared__ uint4 s_dyn[];  // SHARED: the reached bitmap
-  constexpr uint32_t ROOM = PACK ? kPackEntries : kSimLong;
-  __shared__ uint32_t s_beg[ROOM], s_end[ROOM];  // a packed level's entries, or long lists
+  static_assert(kPackEntries <= kSimLong, "one room for both");
+  __shared__ uint32_t s_beg[kSimLong], s_end[kSimLong];  // a packed level's entries, or long lists
   __shared__ uint32_t s_off[PACK ? kPackEntries : 1], s_warp[32];
   __shared__ uint32_t s_qlen, s_nlong, s_next;  // the last two zero between levels
   __shared__ unsigned long long s_rep;
@@ -149,10 +151,8 @@ spread_ic_kernel(const __grid_constant__ SpreadLaunch L) {
           } else {
             x = __ldg(&L.G.edges[(b << 3) + h].x);
           }
-          if (!KEEP || !together.value) {
-            const uint32_t word = SHARED ? bm[x >> 5] : __ldcg(&bm[x >> 5]);  // bits are only set
-            want = !((word >> (x & 31)) & 1u);
-          }
+          // (bits are only set: a plain read spares the atomic where it is as near)
+          if (SHARED && (!KEEP || !together.value)) want = !((bm[x >> 5] >> (x & 31)) & 1u);
         }
         if (together.value) {
           reach(want, x);
@@ -640,7 +640,7 @@ spread_lt_small_kernel(const __grid_constant__ SpreadLaunch L) {
 // Shared memory of an SM's CTAs, and what a spread CTA takes besides its dynamic
 // part (static and reserved, rounded up).
 constexpr size_t kSmShared = 227 * 1024;
-constexpr size_t kSpreadStatic = 8192;
+constexpr size_t kSpreadStatic = 5120;
 // Dynamic shared memory of the kernels below at most, by CTAs an SM.
 constexpr size_t kIcShared4 = (kSmShared / 4 - kSpreadStatic) & ~(size_t)15;
 constexpr size_t kIcShared1 = kSmShared - kSpreadStatic;

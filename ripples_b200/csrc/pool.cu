@@ -306,17 +306,22 @@ static int ensure_big_scratch(rip_pool *p, uint32_t slots, uint32_t qcap) {
 
 // Block shape for `count` heavy sets: many sets run best one to a small block
 // (more of them in flight, fewer warps at a barrier), few need larger ones to
-// fill the device.  Sampling 400 000 sets at 2^24 vertices, weighted cascade
+// fill the device -- the largest only where the reverse BFS is supercritical and
+// levels are wide.  Sampling 400 000 sets at 2^24 vertices, weighted cascade
 // (20 000 to 60 000 heavy sets a launch): 41.7 ms with 128 threads, 44.5 with
 // 256, 55 with 512; 600 heavy sets of a 2^14-vertex graph: 1.62 ms with 512
 // threads, 1.79 with 256, 2.17 with 128, 1.93 with 1024.  On seven other graphs
 // (weighted cascade and uniform, 2^14 to 2^22 vertices) and 10 000 or 100 000 sets
-// a call the rule is at most 5% slower than the best fixed shape; on 1000 sets of
-// Erdos-Renyi graphs 512 threads would take 1.4 ms where it takes 1.6.
+// a call the rule is at most 5% slower than the best fixed shape.  A few heavy sets
+// (100 to 1000 a call): weighted cascade, Erdos-Renyi and R-MAT, 2^18 to 2^21
+// vertices, 1.1 to 2.6 ms with 512 threads and 1.1 to 3.1 with 1024; supercritical
+// graphs, 2^14 to 2^17 vertices, 0.43 to 1.5 and 0.40 to 1.25.
 static uint32_t big_shape(const rip_pool *p, uint32_t count) {
   if (p->big_threads) return p->big_threads;
   const uint32_t sms = (uint32_t)p->ctx->num_sms;
-  return count >= 20 * sms ? 128 : count > 5 * sms ? 256 : count > sms ? 512 : 1024;
+  if (count >= 20 * sms) return 128;
+  if (count > 5 * sms) return 256;
+  return count > sms || p->g->branching <= kSupercritical ? 512 : 1024;
 }
 
 // Grows the sets first+ids[i] 64*cw at a time, each batch by the whole grid

@@ -436,8 +436,9 @@ spread_lt_kernel(SpreadLaunch L) {
 // 2^16 as chains have no vertex twice.
 // 2000 replicas: an R-MAT graph's 20 hubs (2^16 vertices, 768 K edges) 26.1 ms by
 // sweeps to the end, 8.2 by levels, 2.5 by halving; 2^16 Erdos-Renyi vertices of
-// degree 10, 50 (5) seeds 20.6 (11.4), 47.5 (20.3), 3.0 (3.3).  The searches' read
-// latency bounds it, two of them in flight a thread.
+// degree 10, 50 (5) seeds 20.6 (11.4), 47.5 (20.3), 3.0 (3.3).  What bounds it: half
+// the issue slots are busy; the draw waits for the searches' reads, two of them in
+// flight a thread, the halving at the CTA's barriers.
 constexpr uint32_t kSweepShare = 64;  // (those 3.0 (3.3) ms: 4.3 (4.8) at 16, 14.6 (11.0) at 2)
 
 template <int THREADS, bool LEVELS>
